@@ -66,6 +66,8 @@ struct PropsLaunch {
     int reg;         // 64^3 FP32: register-resident step kernels (reg64.cu) instead of the shared-memory ones
     int persist;     // one persistent launch per contour step instead of four (register kernels, or the
                      // shared-memory kernels of the compile-time shapes)
+    int pair;        // the pair-packed step kernels (pair.cuh), where the grid has them
+    int step_grid_pair;  // CTAs of their persistent launch (0: none)
     int step_grid;   // CTAs of the register kernels' persistent launch
     int step_grid_pf, step_pf_smem;  // CTAs and dynamic shared memory of the shared-memory kernels' one
 };
@@ -79,6 +81,14 @@ void reg64_pencil(const PropsArgs<float> &a, int nslots, int both, cudaStream_t 
 int reg64_sync_ints(int Ns, int nslots);
 int reg64_step_grid();
 void reg64_step(const PropsArgs<float> &a, int nslots, int s, int grid, cudaStream_t st);
+
+// FP64 step kernels on q + i q^dagger (pair.cuh): spectra [slot][half step, full step][x][kz][y position]
+bool pair_applicable(int m0, int m1, int m2);
+int pair_setup(int m0, int m1, int m2, int *step_grid);
+void pair_mid(const PropsArgs<double> &a, int nslots, int s, cudaStream_t st);
+void pair_combine(const PropsArgs<double> &a, int nslots, int s, int mode, cudaStream_t st);
+void pair_pencil(const PropsArgs<double> &a, int nslots, int both, int wide, cudaStream_t st);
+void pair_step(const PropsArgs<double> &a, int nslots, int s, int wide, int grid, cudaStream_t st);
 
 void pf_smem_bytes(int id, int fp32, int &mid, int &comb);
 // dynamic shared memory of k_pencil_sh for tiles of tc columns

@@ -1,0 +1,298 @@
+// pair.cu -- kernels and launchers of the FP64 contour step on q + i q^dagger
+// (pair.cuh).
+//
+// FP32 keeps the real transforms of props_kernels.cu: in single precision the
+// densities follow the rounding of the transforms, and these kernels moved them
+// by up to 5e-5 (2-norm) and their error against FP64 by up to twice.
+#include "pair.cuh"
+#include "step_order.cuh"
+
+namespace scft {
+namespace {
+
+using T = double;
+
+constexpr int kSmemCta = 227 * 1024;  // dynamic shared memory a CTA may have
+constexpr int kSms = 148;
+
+// slab shapes (m1, m2) and x lengths with kernels
+#define PAIR_SLABS(X) X(16, 16) X(24, 24) X(32, 32) X(40, 40) X(48, 48) X(64, 64) X(64, 96) X(80, 80) X(96, 96)
+#define PAIR_AXES(X) X(16) X(24) X(32) X(40) X(48) X(64) X(80) X(96) X(128)
+// grids with a persistent step kernel
+#define PAIR_GRIDS(X) X(32, 32, 32) X(48, 48, 48) X(64, 64, 64) X(64, 64, 96) X(96, 96, 96)
+
+constexpr int kTile = 32;         // columns per x tile; the wide form takes twice as many
+constexpr int kPencilThreads = 256;
+
+template <int M1, int M2>
+constexpr bool kSlabFits = PairSlab<M1, M2>::SMEM <= kSmemCta;
+
+constexpr int pencil_minb(int m0) { return m0 > 80 ? 2 : 3; }
+
+template <int M1, int M2>
+__global__ void __launch_bounds__(PairSlab<M1, M2>::NT, PairSlab<M1, M2>::MINB) k_pair_mid(PropsArgs<T> a, int s)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    pair_mid_body<M1, M2>(a, s, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
+}
+
+template <int M1, int M2>
+__global__ void __launch_bounds__(PairSlab<M1, M2>::NT, PairSlab<M1, M2>::MINB)
+    k_pair_combine(PropsArgs<T> a, int s, int mode)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    pair_combine_body<M1, M2>(a, s, mode, blockIdx.x, gridDim.y == 1 ? -1 : (int)blockIdx.y, blockIdx.z, smem_raw);
+}
+
+template <int M0, int TC>
+__global__ void __launch_bounds__(kPencilThreads, pencil_minb(M0)) k_pair_pencil(PropsArgs<T> a, int ra, int rb)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    // slots (and tiles) in the opposite order of the slab kernels before and
+    // after: what those touched last is still in L2
+    pair_pencil_body<M0, TC, kPencilThreads>(a, gridDim.x - 1 - blockIdx.x, blockIdx.y, gridDim.z - 1 - blockIdx.z, ra, rb,
+                                                smem_raw);
+}
+
+__device__ __forceinline__ int ld_acquire_gpu(const int *p)
+{
+    int v;
+    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+constexpr uint32_t kStepSpin = 1u << 22;
+
+// The four launches of a step as work items of one launch: both spectra's x
+// tiles, the slabs of mid (two per x), the half-step spectrum's x tiles, the
+// slabs of combine, each phase ordered by slot.  CTAs claim items from a
+// counter in the order of step_order.cuh, and an item waits only for the
+// previous phase of its own slot.  Items are claimed in order by running CTAs,
+// so whatever an item waits for is held by a CTA that is running or done; no
+// residency is assumed.  Every wait is bounded and records error 3 when it
+// gives up, which ends the kernel.
+template <int M0, int M1, int M2, int TC>
+__global__ void __launch_bounds__(PairSlab<M1, M2>::NT, PairSlab<M1, M2>::MINB)
+    k_pair_step(PropsArgs<T> a, int s, int nslots)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ int item_sh[3], ok_sh;
+    using PS = PairSlab<M1, M2>;
+    constexpr int NT = PS::NT, ntiles = (M1 * M2 + TC - 1) / TC;
+    int ra, rb;
+    PS::radices(ra, rb);
+    const int per[4] = {2 * ntiles, 2 * M0, ntiles, M0};
+    int *claim = a.sync + s;      // this step's claim counter
+    int *done = a.sync + a.g.Ns;  // [phase][slot] completion counters, cumulative over the steps
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int ph = -1, gr = 0, un = 0;
+            if (!step_item(atomicAdd(claim, 1), nslots, per, ph, gr, un)) ph = -1;
+            item_sh[0] = ph;
+            item_sh[1] = gr;
+            item_sh[2] = un;
+            ok_sh = 1;
+            if (ph > 0) {
+                const int need = per[ph - 1] * (s + 1);
+                const int *cnt = done + (ph - 1) * nslots + gr;
+                uint32_t i = 0;
+                while (ld_acquire_gpu(cnt) < need && i < kStepSpin) {
+                    __nanosleep(32);
+                    i++;
+                }
+                if (i >= kStepSpin) {
+                    ok_sh = 0;
+                    *a.err = 3;
+                }
+            }
+        }
+        __syncthreads();
+        const int phase = item_sh[0], slot = item_sh[1], unit = item_sh[2];
+        if (phase < 0 || !ok_sh) break;
+        if (phase == 0)
+            pair_pencil_body<M0, TC, NT>(a, unit % ntiles, unit / ntiles, slot, ra, rb, smem_raw);
+        else if (phase == 1)
+            pair_mid_body<M1, M2>(a, s, unit >> 1, unit & 1, slot, smem_raw);
+        else if (phase == 2)
+            pair_pencil_body<M0, TC, NT>(a, unit, 0, slot, ra, rb, smem_raw);
+        else
+            pair_combine_body<M1, M2>(a, s, 0, unit, -1, slot, smem_raw);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(done + phase * nslots + slot, 1);
+        }
+    }
+}
+
+template <int M0, int M1, int M2, int TC>
+constexpr int step_smem()
+{
+    return PairSlab<M1, M2>::SMEM > PairPencil<M0, TC>::SMEM ? PairSlab<M1, M2>::SMEM
+                                                                   : PairPencil<M0, TC>::SMEM;
+}
+
+// Launch of a step kernel: it may start while the kernel before it on the
+// stream finishes (see pdl_wait); cluster: the CTAs along y form one cluster.
+template <class... Args>
+void launch_step(void (*fn)(Args...), dim3 grid, int threads, int smem, bool cluster, cudaStream_t st, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = 1;
+    at[1].val.clusterDim.y = grid.y;
+    at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
+bool slab_ok(int m1, int m2)
+{
+#define X(A, B) \
+    if (m1 == A && m2 == B) return kSlabFits<A, B>;
+    PAIR_SLABS(X)
+#undef X
+    return false;
+}
+
+bool axis_ok(int m0)
+{
+#define X(A) \
+    if (m0 == A) return true;
+    PAIR_AXES(X)
+#undef X
+    return false;
+}
+
+}  // namespace
+
+bool pair_applicable(int m0, int m1, int m2)
+{
+    return slab_ok(m1, m2) && axis_ok(m0);
+}
+
+// raises the kernels' shared-memory limits; *grid = CTAs of the persistent step launch (0: none)
+int pair_setup(int m0, int m1, int m2, int *grid)
+{
+    cudaError_t e = cudaSuccess;
+    auto up = [&](auto *fn, int bytes) {
+        if (e == cudaSuccess) e = raise_dyn_smem(fn, bytes);
+    };
+#define X(A, B)                                                \
+    if (m1 == A && m2 == B) {                                  \
+        if constexpr (kSlabFits<A, B>) {                       \
+            up(k_pair_mid<A, B>, PairSlab<A, B>::SMEM);     \
+            up(k_pair_combine<A, B>, PairSlab<A, B>::SMEM); \
+        }                                                      \
+    }
+    PAIR_SLABS(X)
+#undef X
+#define X(A)                                                               \
+    if (m0 == A) {                                                         \
+        up(k_pair_pencil<A, kTile>, PairPencil<A, kTile>::SMEM);         \
+        up(k_pair_pencil<A, 2 * kTile>, PairPencil<A, 2 * kTile>::SMEM); \
+    }
+    PAIR_AXES(X)
+#undef X
+    *grid = 0;
+#define X(A, B, C)                                                                                             \
+    if (m0 == A && m1 == B && m2 == C) {                                                                       \
+        if constexpr (kSlabFits<B, C>) {                                                                       \
+            up(k_pair_step<A, B, C, kTile>, step_smem<A, B, C, kTile>());                                       \
+            up(k_pair_step<A, B, C, 2 * kTile>, step_smem<A, B, C, 2 * kTile>());                               \
+            int per_sm = 0;                                                                                    \
+            if (e == cudaSuccess &&                                                                            \
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_step<A, B, C, 2 * kTile>,         \
+                                                              PairSlab<B, C>::NT,                           \
+                                                              step_smem<A, B, C, 2 * kTile>()) == cudaSuccess)  \
+                *grid = per_sm * kSms;                                                                         \
+        }                                                                                                      \
+    }
+    PAIR_GRIDS(X)
+#undef X
+    return e == cudaSuccess ? 0 : -1;
+}
+
+void pair_mid(const PropsArgs<T> &a, int nslots, int s, cudaStream_t st)
+{
+    const Geo &g = a.g;
+#define X(A, B)                                                                                              \
+    if (g.m1 == A && g.m2 == B) {                                                                            \
+        using P = PairSlab<A, B>;                                                                         \
+        if constexpr (kSlabFits<A, B>)                                                                       \
+            launch_step(k_pair_mid<A, B>, dim3(g.m0, 2, nslots), P::NT, P::SMEM, false, st, a, s);            \
+        return;                                                                                              \
+    }
+    PAIR_SLABS(X)
+#undef X
+}
+
+void pair_combine(const PropsArgs<T> &a, int nslots, int s, int mode, cudaStream_t st)
+{
+    const Geo &g = a.g;
+    // two CTAs per slab while both find an SM of their own: the chain of a CTA
+    // is then two slab transforms instead of three
+    const int split = 2 * g.m0 * nslots <= kSms && s + 1 < g.Ns ? 2 : 1;
+#define X(A, B)                                                                                                     \
+    if (g.m1 == A && g.m2 == B) {                                                                                   \
+        using P = PairSlab<A, B>;                                                                                \
+        if constexpr (kSlabFits<A, B>)                                                                              \
+            launch_step(k_pair_combine<A, B>, dim3(g.m0, split, nslots), P::NT, P::SMEM, split > 1, st, a, s, mode); \
+        return;                                                                                                     \
+    }
+    PAIR_SLABS(X)
+#undef X
+}
+
+void pair_pencil(const PropsArgs<T> &a, int nslots, int both, int wide, cudaStream_t st)
+{
+    const Geo &g = a.g;
+    const int tc = wide ? 2 * kTile : kTile;
+    int ra = 1, rb = 1;
+#define X(A, B)                        \
+    if (g.m1 == A && g.m2 == B) {      \
+        PairSlab<A, B>::radices(ra, rb); \
+    }
+    PAIR_SLABS(X)
+#undef X
+    const dim3 grid((g.m1 * g.m2 + tc - 1) / tc, both ? 2 : 1, nslots);
+#define X(A)                                                                                                 \
+    if (g.m0 == A) {                                                                                         \
+        if (wide)                                                                                            \
+            launch_step(k_pair_pencil<A, 2 * kTile>, grid, kPencilThreads, PairPencil<A, 2 * kTile>::SMEM, false, st, a, ra, rb);  \
+        else                                                                                                 \
+            launch_step(k_pair_pencil<A, kTile>, grid, kPencilThreads, PairPencil<A, kTile>::SMEM, false, st, a, ra, rb);          \
+        return;                                                                                              \
+    }
+    PAIR_AXES(X)
+#undef X
+}
+
+void pair_step(const PropsArgs<T> &a, int nslots, int s, int wide, int grid, cudaStream_t st)
+{
+    const Geo &g = a.g;
+#define X(A, B, C)                                                                                                   \
+    if (g.m0 == A && g.m1 == B && g.m2 == C) {                                                                       \
+        if constexpr (kSlabFits<B, C>) {                                                                             \
+            constexpr int NT = PairSlab<B, C>::NT;                                                                \
+            if (wide)                                                                                                \
+                k_pair_step<A, B, C, 2 * kTile><<<grid, NT, step_smem<A, B, C, 2 * kTile>(), st>>>(a, s, nslots);     \
+            else                                                                                                     \
+                k_pair_step<A, B, C, kTile><<<grid, NT, step_smem<A, B, C, kTile>(), st>>>(a, s, nslots);             \
+        }                                                                                                            \
+        return;                                                                                                      \
+    }
+    PAIR_GRIDS(X)
+#undef X
+}
+
+}  // namespace scft

@@ -1,0 +1,572 @@
+// pair.cuh -- the contour step on q + i q^dagger (density.h:129-220).
+//
+// Every operation of the Richardson step is either a pointwise product with a
+// real table (E4, E2 of the field that q or q^dagger sees) or a convolution
+// with a real, even kernel (K1, K2).  Both keep the real and the imaginary part
+// of a complex field apart, so q and q^dagger of a replica travel as ONE complex
+// field c = q + i q^dagger: one complex 3-D transform replaces two real ones
+// with no packing, unpacking or Hermitian bookkeeping in between.
+//
+// Each 1-D transform of length N = R1 R2 is done in place, in two register
+// passes with one trip through shared memory between them:
+//   forward  n = j + R2 r:  R1-point DFTs over r, for every j, written back to
+//            j + R2 k1; then times w^(j k1) and R2-point DFTs over j, written to
+//            R2 k1 + k2.  Position R2 k1 + k2 then holds frequency k1 + R1 k2.
+//   inverse  the same passes backwards.
+// A pass reads and writes the same positions, so a transform needs one barrier
+// between its two passes and none inside them.  A slab (fixed x) transforms y
+// (M1 = RA RB), then z (M2 = RZ RC); the small second y pass and first z pass
+// share registers where both fit.  The outer passes meet global memory in
+// registers: the RA-point y pass with lanes along z, so that tables, partial
+// results and the propagator store move in whole rows, and the RC-point z pass
+// with lanes along y positions, so that a spectrum slab is stored [kz][p] in
+// whole rows (p the y position of ky = p/RB + RA (p mod RB)); only the diffusion
+// factors need to know that order.
+//
+// Bank conflicts: rows of a slab sit at an odd stride of complex elements, so
+// both lanes along z and lanes along y positions touch different banks.
+// Twiddle factors are applied in the R2-point passes, where (nearly) a whole
+// warp shares k1 and the table reads are broadcasts.
+#pragma once
+#include "common.cuh"
+#include "dft.cuh"
+#include "kernels.h"
+
+namespace scft {
+
+using cplxd = cplx<double>;
+
+// 16-byte accesses (cplx<double> itself is only 8-byte aligned)
+__device__ __forceinline__ cplxd ldc(const cplxd *p)
+{
+    const double2 v = *reinterpret_cast<const double2 *>(p);
+    return {v.x, v.y};
+}
+// through L2: spectra and partial results written by other CTAs of an earlier phase
+__device__ __forceinline__ cplxd ldc_cg(const cplxd *p)
+{
+    const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
+    return {v.x, v.y};
+}
+__device__ __forceinline__ cplxd ldc_ro(const cplxd *p)
+{
+    const double2 v = __ldg(reinterpret_cast<const double2 *>(p));
+    return {v.x, v.y};
+}
+__device__ __forceinline__ void stc(cplxd *p, cplxd v)
+{
+    *reinterpret_cast<double2 *>(p) = make_double2(v.x, v.y);
+}
+
+// x / 3, correctly rounded but for double rounding below the normal range: one
+// Newton correction of x * (1/3), five operations instead of a divide's
+// subroutine; infinities stay infinite
+__device__ __forceinline__ double third(double x)
+{
+    const double c = 1.0 / 3.0, big = 1.7976931348623157e308;
+    const double q = x * c;
+    const double r = fma(fma(-3.0, q, x), c, q);
+    return fabs(q) <= big ? r : q;
+}
+
+// Programmatic dependent launch: the kernels of a step let the next one start
+// as their last CTAs run (its CTAs set up and read constant tables), and wait
+// here for the whole previous kernel before they touch what it wrote.  Both are
+// no-ops in a kernel launched without the attribute.
+__device__ __forceinline__ void pdl_trigger()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// asks for `bytes` at p to be brought into L2 (16-byte multiples); a hint, no wait
+__device__ __forceinline__ void prefetch_l2(const void *p, int bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+// the two CTAs of a split combine: each has read its input slab (arrive) before
+// either overwrites it (wait)
+__device__ __forceinline__ void pair_arrive()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void pair_wait()
+{
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ const double *pair_etab(const PropsArgs<double> &a, int slot, int fld, int s)
+{
+    const Geo &g = a.g;
+    if (g.jon && s == (fld == 0 ? g.jq : g.jqd)) return a.jtab + (size_t)slot * g.M;
+    const int sel = fld == 0 ? (s < g.n1 ? 0 : 1) : (s < g.n2 ? 1 : 0);
+    return a.etab + ((size_t)slot * 2 + sel) * g.M;
+}
+
+// Transform plan of an M1 x M2 slab: M1 = RA RB, M2 = RZ RC.  MERGE: the
+// RB-point y pass and the RZ-point z pass share registers (RB RZ elements per
+// thread), so a 2-D transform makes two trips through shared memory instead of
+// three.  WANT: threads per SM the registers are budgeted for.
+template <int M1, int M2>
+struct PairPlan;
+#define PAIR_PLAN(m1, m2, ra, rb, rz, rc, merge, nt, want)                                 \
+    template <>                                                                             \
+    struct PairPlan<m1, m2> {                                                                      \
+        static constexpr int RA = ra, RB = rb, RZ = rz, RC = rc, NT = nt;                             \
+        static constexpr bool MERGE = merge;                                                          \
+        static constexpr int WANT = want;  \
+    };
+PAIR_PLAN(16, 16, 8, 2, 2, 8, true, 64, 768)
+PAIR_PLAN(24, 24, 8, 3, 3, 8, true, 96, 768)
+PAIR_PLAN(32, 32, 8, 4, 4, 8, true, 128, 512)
+PAIR_PLAN(40, 40, 10, 4, 4, 10, true, 160, 480)
+PAIR_PLAN(48, 48, 12, 4, 4, 12, true, 192, 576)
+PAIR_PLAN(64, 64, 16, 4, 4, 16, true, 256, 512)
+PAIR_PLAN(64, 96, 8, 8, 12, 8, false, 256, 512)
+PAIR_PLAN(80, 80, 10, 8, 10, 8, false, 416, 416)
+PAIR_PLAN(96, 96, 12, 8, 12, 8, false, 384, 384)
+PAIR_PLAN(128, 128, 16, 8, 16, 8, false, 512, 512)
+#undef PAIR_PLAN
+
+template <int M1, int M2>
+struct PairSlab : PairPlan<M1, M2> {
+    using T = double;
+    using Plan = PairPlan<M1, M2>;
+    using Plan::MERGE;
+    using Plan::NT;
+    using Plan::RA;
+    using Plan::RB;
+    using Plan::RC;
+    using Plan::RZ;
+    static_assert(RA * RB == M1 && RZ * RC == M2, "plan");
+    static constexpr int S = M2 | 1;
+    static constexpr int SMEM = (M1 * S + M1 + M2) * (int)sizeof(cplx<T>);
+    static constexpr int FIT = 227 * 1024 / (SMEM + 1024), REG = Plan::WANT / NT;
+    static constexpr int MINB = FIT < 1 ? 1 : FIT < REG ? FIT : REG < 1 ? 1 : REG;
+
+    cplx<T> *buf, *twy, *twz;
+
+    // radices of the y transform that the spectrum order depends on
+    static __host__ __device__ void radices(int &ra, int &rb)
+    {
+        ra = RA;
+        rb = RB;
+    }
+
+    __device__ __forceinline__ PairSlab(unsigned char *smem)
+    {
+        buf = reinterpret_cast<cplx<T> *>(smem);
+        twy = buf + M1 * S;
+        twz = twy + M1;
+    }
+
+    __device__ __forceinline__ void load_tables(const cplx<T> *tw, int m0)
+    {
+        for (int i = threadIdx.x; i < M1 + M2; i += NT) stc(twy + i, ldc_ro(tw + m0 + i));
+    }
+
+    // loop of a pass over COUNT butterflies
+    template <int COUNT, class F>
+    static __device__ __forceinline__ void each(F f)
+    {
+        if constexpr (COUNT <= NT) {
+            if (COUNT == NT || (int)threadIdx.x < COUNT) f((int)threadIdx.x);
+        } else {
+#pragma unroll 1
+            for (int b = threadIdx.x; b < COUNT; b += NT) f(b);
+        }
+    }
+
+    // spectrum slab src -> buf, up to the last (RA-point y) pass
+    __device__ __forceinline__ void inverse_passes(const cplx<T> *src, bool split = false) const
+    {
+        each<M1 * RZ>([&](int b) {
+            const int y = b % M1, k1 = b / M1;
+            cplx<T> v[RC], *p = buf + y * S + RC * k1;
+#pragma unroll
+            for (int i = 0; i < RC; i++) v[i] = ldc_cg(src + i * (RZ * M1) + b);
+            Reg<T, RC, 1>::run(v);
+            stc(p, v[0]);
+#pragma unroll
+            for (int i = 1; i < RC; i++) stc(p + i, cmulc(v[i], ldc(twz + k1 * i)));
+        });
+        __syncthreads();
+        if (split) pair_arrive();
+        if constexpr (MERGE) {
+            each<RA * RC>([&](int b) {
+                const int j = b % RC, k1 = b / RC;
+                cplx<T> v[RB][RZ], *p = buf + RB * k1 * S + j;
+#pragma unroll
+                for (int i = 0; i < RB; i++) {
+#pragma unroll
+                    for (int r = 0; r < RZ; r++) v[i][r] = ldc(p + i * S + RC * r);
+                    Reg<T, RZ, 1>::run(v[i]);
+                }
+#pragma unroll
+                for (int r = 0; r < RZ; r++) {
+                    cplx<T> u[RB];
+#pragma unroll
+                    for (int i = 0; i < RB; i++) u[i] = v[i][r];
+                    Reg<T, RB, 1>::run(u);
+#pragma unroll
+                    for (int i = 0; i < RB; i++) v[i][r] = u[i];
+                }
+#pragma unroll
+                for (int i = 0; i < RB; i++) {
+                    const cplx<T> w = ldc(twy + k1 * i);
+#pragma unroll
+                    for (int r = 0; r < RZ; r++) stc(p + i * S + RC * r, i > 0 ? cmulc(v[i][r], w) : v[i][r]);
+                }
+            });
+        } else {
+            each<M1 * RC>([&](int b) {
+                const int y = b % M1, j = b / M1;
+                cplx<T> v[RZ], *p = buf + y * S + j;
+#pragma unroll
+                for (int r = 0; r < RZ; r++) v[r] = ldc(p + RC * r);
+                Reg<T, RZ, 1>::run(v);
+#pragma unroll
+                for (int r = 0; r < RZ; r++) stc(p + RC * r, v[r]);
+            });
+            __syncthreads();
+            each<RA * M2>([&](int b) {
+                const int z = b % M2, k1 = b / M2;
+                cplx<T> v[RB], *p = buf + RB * k1 * S + z;
+#pragma unroll
+                for (int i = 0; i < RB; i++) v[i] = ldc(p + i * S);
+                Reg<T, RB, 1>::run(v);
+                stc(p, v[0]);
+#pragma unroll
+                for (int i = 1; i < RB; i++) stc(p + i * S, cmulc(v[i], ldc(twy + k1 * i)));
+            });
+        }
+        __syncthreads();
+    }
+
+    // The RA-point y passes around real space: butterfly (z, j) holds the points
+    // y = j + RB r of column z, lanes along z.  f(v, offset of (j, z) in the
+    // slab) changes them in place (or fills them: INV = false); element r is at
+    // offset + ROW r.  With FWD the first forward y pass follows in registers.
+    static constexpr int ROW = RB * M2;
+    template <bool INV, bool FWD, class F>
+    __device__ __forceinline__ void real_space(F f) const
+    {
+        each<RB * M2>([&](int b) {
+            const int z = b % M2, j = b / M2;
+            cplx<T> v[RA], *p = buf + j * S + z;
+            if (INV) {
+#pragma unroll
+                for (int r = 0; r < RA; r++) v[r] = ldc(p + RB * r * S);
+                Reg<T, RA, 1>::run(v);
+            }
+            f(v, b);
+            if (FWD) {
+                Reg<T, RA, -1>::run(v);
+#pragma unroll
+                for (int r = 0; r < RA; r++) stc(p + RB * r * S, v[r]);
+            }
+        });
+    }
+
+    // buf after the first forward y pass -> spectrum slab dst
+    __device__ __forceinline__ void forward_passes(cplx<T> *dst, bool split, bool last) const
+    {
+        __syncthreads();
+        if constexpr (MERGE) {
+            each<RA * RC>([&](int b) {
+                const int j = b % RC, k1 = b / RC;
+                cplx<T> v[RB][RZ], *p = buf + RB * k1 * S + j;
+#pragma unroll
+                for (int i = 0; i < RB; i++) {
+                    const cplx<T> w = ldc(twy + k1 * i);
+#pragma unroll
+                    for (int r = 0; r < RZ; r++) {
+                        v[i][r] = ldc(p + i * S + RC * r);
+                        if (i > 0) v[i][r] = cmul(v[i][r], w);
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < RZ; r++) {
+                    cplx<T> u[RB];
+#pragma unroll
+                    for (int i = 0; i < RB; i++) u[i] = v[i][r];
+                    Reg<T, RB, -1>::run(u);
+#pragma unroll
+                    for (int i = 0; i < RB; i++) v[i][r] = u[i];
+                }
+#pragma unroll
+                for (int i = 0; i < RB; i++) {
+                    Reg<T, RZ, -1>::run(v[i]);
+#pragma unroll
+                    for (int r = 0; r < RZ; r++) stc(p + i * S + RC * r, v[i][r]);
+                }
+            });
+        } else {
+            each<RA * M2>([&](int b) {
+                const int z = b % M2, k1 = b / M2;
+                cplx<T> v[RB], *p = buf + RB * k1 * S + z;
+                v[0] = ldc(p);
+#pragma unroll
+                for (int i = 1; i < RB; i++) v[i] = cmul(ldc(p + i * S), ldc(twy + k1 * i));
+                Reg<T, RB, -1>::run(v);
+#pragma unroll
+                for (int i = 0; i < RB; i++) stc(p + i * S, v[i]);
+            });
+            __syncthreads();
+            each<M1 * RC>([&](int b) {
+                const int y = b % M1, j = b / M1;
+                cplx<T> v[RZ], *p = buf + y * S + j;
+#pragma unroll
+                for (int r = 0; r < RZ; r++) v[r] = ldc(p + RC * r);
+                Reg<T, RZ, -1>::run(v);
+#pragma unroll
+                for (int r = 0; r < RZ; r++) stc(p + RC * r, v[r]);
+            });
+        }
+        __syncthreads();
+        if (split) pair_wait();
+        if (last) pdl_trigger();
+        each<M1 * RZ>([&](int b) {
+            const int y = b % M1, k1 = b / M1;
+            cplx<T> v[RC], *p = buf + y * S + RC * k1;
+            v[0] = ldc(p);
+#pragma unroll
+            for (int i = 1; i < RC; i++) v[i] = cmul(ldc(p + i), ldc(twz + k1 * i));
+            Reg<T, RC, -1>::run(v);
+#pragma unroll
+            for (int i = 0; i < RC; i++) stc(dst + i * (RZ * M1) + b, v[i]);
+        });
+    }
+};
+
+// mid, slab x of a slot: sp = 0 the half-step spectrum (inverse slab, times E2,
+// forward slab), sp = 1 the full-step spectrum (inverse slab, P = E2 qs1)
+template <int M1, int M2>
+__device__ __forceinline__ void pair_mid_body(const PropsArgs<double> &a, int s, int x, int sp, int slot, unsigned char *smem)
+{
+    using T = double;
+    const Geo &g = a.g;
+    constexpr int AREA = M1 * M2;
+    using PS = PairSlab<M1, M2>;
+    PS B(smem);
+    B.load_tables(a.tw, g.m0);
+    const size_t off = (size_t)x * AREA;
+    cplx<T> *spec = a.spec + ((size_t)slot * 2 + sp) * g.M + off;
+    const T *Eq = pair_etab(a, slot, 0, s) + off, *Ep = pair_etab(a, slot, 1, s) + off;
+    if (threadIdx.x == 0) {
+        prefetch_l2(Eq, AREA * sizeof(T));
+        prefetch_l2(Ep, AREA * sizeof(T));
+    }
+    __syncthreads();
+    pdl_wait();
+    B.inverse_passes(spec);
+    if (sp == 0) {
+        B.template real_space<true, true>([&](cplx<T> *v, int o) {
+#pragma unroll
+            for (int r = 0; r < PS::RA; r++) {
+                const T e0 = __ldg(Eq + o + PS::ROW * r), e1 = __ldg(Ep + o + PS::ROW * r);
+                v[r].x *= e0 * e0;
+                v[r].y *= e1 * e1;
+            }
+        });
+        B.forward_passes(spec, false, true);
+    } else {
+        cplx<T> *P = reinterpret_cast<cplx<T> *>(a.pbuf) + (size_t)slot * g.M + off;
+        B.template real_space<true, false>([&](cplx<T> *v, int o) {
+#pragma unroll
+            for (int r = 0; r < PS::RA; r++) {
+                const T e0 = __ldg(Eq + o + PS::ROW * r), e1 = __ldg(Ep + o + PS::ROW * r);
+                stc(P + o + PS::ROW * r, cplx<T>{v[r].x * (e0 * e0), v[r].y * (e1 * e1)});
+            }
+        });
+    }
+}
+
+// combine, slab x of a slot: finishes step s (mode 0: Richardson combination;
+// mode 1: q(s+1) = 1; mode 2: q(s+1) from the propagator store) and starts step
+// s + 1.  half: -1 one CTA makes both spectra; 0 / 1 this CTA makes only the
+// half-step / full-step one (both repeat the inverse transform, which shortens
+// the chain when the batch leaves SMs idle; they are a cluster of two) and half
+// 0 stores q.
+template <int M1, int M2>
+__device__ __forceinline__ void pair_combine_body(const PropsArgs<double> &a, int s, int mode, int x, int half, int slot,
+                                                  unsigned char *smem)
+{
+    using T = double;
+    const Geo &g = a.g;
+    constexpr int AREA = M1 * M2;
+    using PS = PairSlab<M1, M2>;
+    PS B(smem);
+    B.load_tables(a.tw, g.m0);
+    const size_t M = g.M, off = (size_t)x * AREA;
+    cplx<T> *specA = a.spec + (size_t)slot * 2 * M + off, *specB = specA + M;
+    const int sn = s + 1;
+    T *q0 = a.hist + ((size_t)slot * (g.Ns + 1) + sn) * 2 * M + off, *q1 = q0 + M;
+    const bool next = sn < g.Ns, store = half != 1;
+    const T *Nq = pair_etab(a, slot, 0, next ? sn : 0) + off, *Np = pair_etab(a, slot, 1, next ? sn : 0) + off;
+    const T *Eq = pair_etab(a, slot, 0, s) + off, *Ep = pair_etab(a, slot, 1, s) + off;
+    if (mode == 0 && threadIdx.x == 0) {
+        prefetch_l2(Eq, AREA * sizeof(T));
+        prefetch_l2(Ep, AREA * sizeof(T));
+    }
+    __syncthreads();
+    pdl_wait();
+    if (mode == 0) {
+        const cplx<T> *P = reinterpret_cast<const cplx<T> *>(a.pbuf) + (size_t)slot * M + off;
+        if (threadIdx.x == 0) prefetch_l2(P, AREA * sizeof(cplx<T>));
+        B.inverse_passes(specA, half >= 0);
+        // Richardson, GPU_kernels.h:199-203
+        auto finish = [&](cplx<T> *v, int o) {
+#pragma unroll
+            for (int r = 0; r < PS::RA; r++) {
+                const cplx<T> p = ldc_cg(P + o + PS::ROW * r);
+                v[r].x = third(v[r].x * __ldg(Eq + o + PS::ROW * r) * (T)4 - p.x);
+                v[r].y = third(v[r].y * __ldg(Ep + o + PS::ROW * r) * (T)4 - p.y);
+                if (store) {
+                    q0[o + PS::ROW * r] = v[r].x;
+                    q1[o + PS::ROW * r] = v[r].y;
+                }
+            }
+        };
+        if (!next) {
+            B.template real_space<true, false>(finish);
+            return;
+        }
+        B.template real_space<true, true>([&](cplx<T> *v, int o) {
+            finish(v, o);
+#pragma unroll
+            for (int r = 0; r < PS::RA; r++) {
+                T e0 = __ldg(Nq + o + PS::ROW * r), e1 = __ldg(Np + o + PS::ROW * r);
+                if (half == 1) {
+                    e0 *= e0;
+                    e1 *= e1;
+                }
+                v[r].x *= e0;
+                v[r].y *= e1;
+            }
+        });
+    } else {
+        auto start = [&](cplx<T> *v, int o) {
+#pragma unroll
+            for (int r = 0; r < PS::RA; r++) {
+                v[r] = mode == 1 ? cplx<T>{(T)1, (T)1} : cplx<T>{q0[o + PS::ROW * r], q1[o + PS::ROW * r]};
+                if (mode == 1 && store) {
+                    q0[o + PS::ROW * r] = (T)1;
+                    q1[o + PS::ROW * r] = (T)1;
+                }
+                T e0 = __ldg(Nq + o + PS::ROW * r), e1 = __ldg(Np + o + PS::ROW * r);
+                if (half == 1) {
+                    e0 *= e0;
+                    e1 *= e1;
+                }
+                v[r].x *= e0;
+                v[r].y *= e1;
+            }
+        };
+        B.template real_space<false, true>(start);
+        if (!next) return;
+    }
+    B.forward_passes(half == 1 ? specB : specA, half >= 0 && mode == 0, half >= 0);
+    if (half >= 0) return;
+    // full step input E2' q', from the slice this thread has just stored
+    __syncthreads();
+    B.template real_space<false, true>([&](cplx<T> *v, int o) {
+#pragma unroll
+        for (int r = 0; r < PS::RA; r++) {
+            const T e0 = __ldg(Nq + o + PS::ROW * r), e1 = __ldg(Np + o + PS::ROW * r);
+            v[r] = {q0[o + PS::ROW * r] * (e0 * e0), q1[o + PS::ROW * r] * (e1 * e1)};
+        }
+    });
+    B.forward_passes(specB, false, true);
+}
+
+// x pass of one tile of TC columns of spectrum sp (0: times K2, 1: times K1):
+// forward transform, diffusion factor (Mult_self, GPU_kernels.h:175-181) and
+// inverse transform; the 8-point passes around the factor share registers.
+// Column c is [kz][p], p the y position of ky = p/rb + ra (p mod rb).
+template <int M0, int TC>
+struct PairPencil {
+    static constexpr int SMEM = (M0 * TC + M0) * (int)sizeof(cplx<double>) + (M0 + TC) * (int)sizeof(double);
+};
+
+template <int M0, int TC, int NT>
+__device__ __forceinline__ void pair_pencil_body(const PropsArgs<double> &a, int tile, int sp, int slot, int ra, int rb,
+                                                 unsigned char *smem)
+{
+    using T = double;
+    constexpr int R1 = M0 / 8, R2 = 8;
+    const Geo &g = a.g;
+    const int m1 = g.m1, m2 = g.m2, ncol = m1 * m2, c0 = tile * TC;
+    cplx<T> *buf = reinterpret_cast<cplx<T> *>(smem);
+    cplx<T> *tw = buf + M0 * TC;
+    T *gx = reinterpret_cast<T *>(tw + M0), *colf = gx + M0;
+    cplx<T> *spec = a.spec + ((size_t)slot * 2 + sp) * g.M + c0;
+    const T *kf = a.kfac + (size_t)__ldg(a.slot_rep + slot) * a.kf_stride;  // the replica's box
+    for (int i = threadIdx.x; i < M0; i += NT) {
+        stc(tw + i, ldc_ro(a.tw + i));
+        gx[i] = __ldg(kf + i);
+    }
+    for (int t = threadIdx.x; t < TC; t += NT) {
+        const int c = c0 + t, kz = c / m1, p = c - kz * m1, ky = p / rb + ra * (p % rb);
+        colf[t] = c < ncol ? __ldg(kf + M0 + ky) * __ldg(kf + M0 + m1 + (2 * kz > m2 ? m2 - kz : kz)) : (T)0;
+    }
+    pdl_wait();
+#pragma unroll 1
+    for (int b = threadIdx.x; b < R2 * TC; b += NT) {
+        const int t = b % TC, j = b / TC;
+        if (c0 + t < ncol) {
+            cplx<T> v[R1];
+#pragma unroll
+            for (int r = 0; r < R1; r++) v[r] = ldc_cg(spec + (size_t)(j + R2 * r) * ncol + t);
+            Reg<T, R1, -1>::run(v);
+#pragma unroll
+            for (int r = 0; r < R1; r++) stc(buf + (j + R2 * r) * TC + t, v[r]);
+        }
+    }
+    __syncthreads();
+    const T invM = a.invM, Mreal = a.Mreal;
+#pragma unroll 1
+    for (int b = threadIdx.x; b < R1 * TC; b += NT) {
+        const int t = b % TC, k1 = b / TC;
+        if (c0 + t < ncol) {
+            cplx<T> v[R2], *p = buf + R2 * k1 * TC + t;
+            v[0] = ldc(p);
+#pragma unroll
+            for (int i = 1; i < R2; i++) v[i] = cmul(ldc(p + i * TC), ldc(tw + k1 * i));
+            Reg<T, R2, -1>::run(v);
+            // K2 = g/M, K1 = g^2/M  (Prepare_dev_expKsq2_expKsq, GPU_kernels.h:207-213)
+            const T ct = colf[t];
+#pragma unroll
+            for (int i = 0; i < R2; i++) {
+                const T k2 = gx[k1 + R1 * i] * ct * invM;
+                const T f = sp == 0 ? k2 : k2 * k2 * Mreal;
+                v[i].x *= f;
+                v[i].y *= f;
+            }
+            Reg<T, R2, 1>::run(v);
+            stc(p, v[0]);
+#pragma unroll
+            for (int i = 1; i < R2; i++) stc(p + i * TC, cmulc(v[i], ldc(tw + k1 * i)));
+        }
+    }
+    __syncthreads();
+    pdl_trigger();
+#pragma unroll 1
+    for (int b = threadIdx.x; b < R2 * TC; b += NT) {
+        const int t = b % TC, j = b / TC;
+        if (c0 + t < ncol) {
+            cplx<T> v[R1];
+#pragma unroll
+            for (int r = 0; r < R1; r++) v[r] = ldc(buf + (j + R2 * r) * TC + t);
+            Reg<T, R1, 1>::run(v);
+#pragma unroll
+            for (int r = 0; r < R1; r++) stc(spec + (size_t)(j + R2 * r) * ncol + t, v[r]);
+        }
+    }
+}
+
+}  // namespace scft

@@ -1116,6 +1116,12 @@ constexpr bool kReg64 = sizeof(T) == 4 && F0 == 64 && F1 == 64 && F2 == 64;
 template <typename T, int MT, int F0, int F1, int F2>
 void launch_combine(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gs, int s, int mode, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8) {
+        if (L.pair) {
+            pair_combine(a, gs.z, s, mode, st);
+            return;
+        }
+    }
     if constexpr (kReg64<T, F0, F1, F2>) {
         if (L.reg) {
             reg64_combine(a, gs.z, s, mode, st);
@@ -1134,6 +1140,12 @@ void launch_combine(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gs, int s,
 template <typename T, int MT, int F0, int F1, int F2>
 void launch_mid(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gs, int s, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8) {
+        if (L.pair) {
+            pair_mid(a, gs.z, s, st);
+            return;
+        }
+    }
     if constexpr (kReg64<T, F0, F1, F2>) {
         if (L.reg) {
             reg64_mid(a, gs.z, s, st);
@@ -1152,6 +1164,12 @@ void launch_mid(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gs, int s, cud
 template <typename T, int MT, int F0, int F1, int F2>
 void launch_pencil(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gp, int both, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8) {
+        if (L.pair) {
+            pair_pencil(a, gp.z, both, L.ptile_wide, st);
+            return;
+        }
+    }
     if constexpr (kReg64<T, F0, F1, F2>) {
         if (L.reg) {
             reg64_pencil(a, gp.z, both, st);
@@ -1193,6 +1211,15 @@ int launch_props_mt(const PropsArgs<T> &a, const PropsLaunch &L, int nslots, cud
     dim3 gs(g.m0, 2, nslots), gp(g.ncol_tiles, 2, nslots);
     k_prepare<T><<<dim3(L.ew_blocks, nslots), 256, 0, st>>>(a);
     int n = 6;
+    if constexpr (sizeof(T) == 8) {
+        if (L.pair && L.persist) {
+            // one persistent launch per contour step; its counters start at zero
+            cudaMemsetAsync(a.sync, 0, sizeof(int) * reg64_sync_ints(g.Ns, nslots), st);
+            pair_combine(a, nslots, -1, 1, st);
+            for (int s = 0; s < g.Ns; s++) pair_step(a, nslots, s, L.ptile_wide, L.step_grid_pair, st);
+            n += g.Ns;
+        }
+    }
     if constexpr (kReg64<T, F0, F1, F2>) {
         if (L.reg && L.persist) {
             // one persistent launch per contour step (reg64.cu); its counters start at zero
@@ -1203,7 +1230,7 @@ int launch_props_mt(const PropsArgs<T> &a, const PropsLaunch &L, int nslots, cud
         }
     }
     if constexpr (F1 != 0) {
-        if (n == 6 && !L.reg && L.persist && L.pf && L.tma_pencil && a.sync) {
+        if (n == 6 && !L.reg && !L.pair && L.persist && L.pf && L.tma_pencil && a.sync) {
             // one persistent launch per contour step on the shared-memory kernels
             constexpr int TC = kTile<T>::value;
             cudaMemsetAsync(a.sync, 0, sizeof(int) * reg64_sync_ints(g.Ns, nslots), st);

@@ -846,7 +846,15 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
             L.step_grid = reg64_step_grid();
             L.persist = 1;
         }
-        ctx->persist_ok = (L.reg || L.step_grid_pf > 0) && ctx->sync;
+        L.pair = T == 8 && pair_applicable(g.m0, g.m1, g.m2);
+        if (L.pair && pair_setup(g.m0, g.m1, g.m2, &L.step_grid_pair) != 0) {
+            ctx->lasterr = "cudaFuncSetAttribute(max dynamic shared memory) failed";
+            rc = SCFT_CUDA_ERROR;
+            goto done;
+        }
+        if (const char *ev = getenv("SCFT_PENCIL_TILE_WIDE"))
+            if (L.pair) L.ptile_wide = ev[0] == '1';
+        ctx->persist_ok = (L.pair ? L.step_grid_pair > 0 : (L.reg || L.step_grid_pf > 0)) && ctx->sync;
         if (const char *ev = getenv("SCFT_PERSIST")) L.persist = ev[0] == '1' ? 1 : 0;
         if (const char *ev = getenv("SCFT_NO_PERSIST"))
             if (ev[0] == '1') ctx->persist_ok = false;
@@ -2280,7 +2288,7 @@ scft_status scft_autotune_ex(scft_ctx *ctx, int *groups_out, int *wide_out, int 
     // axes: slot groups (1, 2, 4) x x-pencil tile width (default, wide;
     // tensor-map pencils of the shared-memory kernels only) x launches per
     // contour step (four, or one persistent launch); c = gi + 3 wide + 6 persist
-    const int nw = (!ctx->L.reg && ctx->L.tmap_wide) ? 2 : 1;
+    const int nw = (ctx->L.pair || (!ctx->L.reg && ctx->L.tmap_wide)) ? 2 : 1;
     const int np = ctx->persist_ok ? 2 : 1;
     for (int c = 0; c < kTuneCandidates; c++) {
         const int ng = 1 << (c % 3), wide = (c / 3) & 1, persist = c / 6;

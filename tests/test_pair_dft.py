@@ -1,0 +1,70 @@
+"""The register DFTs of the pair-packed step kernels (scft_string_b200/csrc/dft.cuh),
+built for the host and checked against numpy's FFT for every length they have,
+both signs, in double precision.  No GPU."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from test_reg64_host import _cuda_include
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+LENGTHS = [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16]
+
+SRC = r"""
+#define __device__
+#define __host__
+#define __forceinline__ inline
+#include <cuda_runtime.h>
+#undef __device__
+#undef __host__
+#undef __forceinline__
+#define __device__
+#define __host__
+#define __forceinline__ inline
+#include "dft.cuh"
+using namespace scft;
+template <int R> static void go(int sign, cplx<double> *v)
+{
+    if (sign < 0) Reg<double, R, -1>::run(v); else Reg<double, R, 1>::run(v);
+}
+extern "C" void h_dft(int n, int sign, double *v)
+{
+    cplx<double> *c = reinterpret_cast<cplx<double> *>(v);
+    switch (n) {
+%s
+    }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    inc = _cuda_include()
+    if inc is None or shutil.which("g++") is None:
+        pytest.skip("needs g++ and the CUDA headers")
+    d = tmp_path_factory.mktemp("dft")
+    src = d / "dft_host.cpp"
+    src.write_text(SRC % "\n".join(f"        case {n}: go<{n}>(sign, c); break;" for n in LENGTHS))
+    out = str(d / "libdft_host.so")
+    csrc = os.path.join(HERE, "..", "scft_string_b200", "csrc")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + inc, "-I" + csrc, "-o", out, str(src)],
+                   check=True)
+    L = C.CDLL(out)
+    L.h_dft.argtypes = [C.c_int, C.c_int, np.ctypeslib.ndpointer(np.float64, flags="C_CONTIGUOUS")]
+    return L
+
+
+@pytest.mark.parametrize("n", LENGTHS)
+@pytest.mark.parametrize("sign", [-1, 1])
+def test_register_dft(lib, n, sign):
+    rng = np.random.default_rng(n)
+    x = rng.normal(size=n) + 1j * rng.normal(size=n)
+    ref = np.fft.fft(x) if sign < 0 else np.fft.ifft(x) * n
+    v = np.ascontiguousarray(x.view(np.float64))
+    lib.h_dft(n, sign, v)
+    # a few roundings of n terms of size 1
+    assert np.abs(v.view(np.complex128) - ref).max() <= 8 * n * np.finfo(float).eps
