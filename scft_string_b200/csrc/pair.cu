@@ -4,6 +4,8 @@
 // FP32 keeps the real transforms of props_kernels.cu: in single precision the
 // densities follow the rounding of the transforms, and these kernels moved them
 // by up to 5e-5 (2-norm) and their error against FP64 by up to twice.
+#include <algorithm>
+
 #include "pair.cuh"
 #include "step_order.cuh"
 
@@ -33,7 +35,7 @@ template <int M1, int M2>
 __global__ void __launch_bounds__(PairSlab<M1, M2>::NT, PairSlab<M1, M2>::MINB) k_pair_mid(PropsArgs<T> a, int s)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    pair_mid_body<M1, M2>(a, s, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
+    pair_mid_body(PairSlab<M1, M2>(smem_raw), a, s, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 template <int M1, int M2>
@@ -41,7 +43,8 @@ __global__ void __launch_bounds__(PairSlab<M1, M2>::NT, PairSlab<M1, M2>::MINB)
     k_pair_combine(PropsArgs<T> a, int s, int mode)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    pair_combine_body<M1, M2>(a, s, mode, blockIdx.x, gridDim.y == 1 ? -1 : (int)blockIdx.y, blockIdx.z, smem_raw);
+    pair_combine_body(PairSlab<M1, M2>(smem_raw), a, s, mode, blockIdx.x, gridDim.y == 1 ? -1 : (int)blockIdx.y,
+                      blockIdx.z);
 }
 
 template <int M0, int TC>
@@ -52,6 +55,29 @@ __global__ void __launch_bounds__(kPencilThreads, pencil_minb(M0)) k_pair_pencil
     // after: what those touched last is still in L2
     pair_pencil_body<M0, TC, kPencilThreads>(a, gridDim.x - 1 - blockIdx.x, blockIdx.y, gridDim.z - 1 - blockIdx.z, ra, rb,
                                                 smem_raw);
+}
+
+// shapes without kernels of their own
+template <int RA>
+__global__ void __launch_bounds__(512, 1) k_pair_mid_any(PropsArgs<T> a, int s, PairAny q)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    pair_mid_body(PairSlabAny<RA>(smem_raw, q), a, s, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+template <int RA>
+__global__ void __launch_bounds__(512, 1) k_pair_combine_any(PropsArgs<T> a, int s, int mode, PairAny q)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    pair_combine_body(PairSlabAny<RA>(smem_raw, q), a, s, mode, blockIdx.x, gridDim.y == 1 ? -1 : (int)blockIdx.y,
+                      blockIdx.z);
+}
+
+template <int R2>
+__global__ void __launch_bounds__(kPencilThreads, 2) k_pair_pencil_any(PropsArgs<T> a, int ra, int rb)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    pair_pencil_any_body<R2, kTile>(a, gridDim.x - 1 - blockIdx.x, blockIdx.y, gridDim.z - 1 - blockIdx.z, ra, rb, smem_raw);
 }
 
 __device__ __forceinline__ int ld_acquire_gpu(const int *p)
@@ -113,11 +139,11 @@ __global__ void __launch_bounds__(PairSlab<M1, M2>::NT, PairSlab<M1, M2>::MINB)
         if (phase == 0)
             pair_pencil_body<M0, TC, NT>(a, unit % ntiles, unit / ntiles, slot, ra, rb, smem_raw);
         else if (phase == 1)
-            pair_mid_body<M1, M2>(a, s, unit >> 1, unit & 1, slot, smem_raw);
+            pair_mid_body(PS(smem_raw), a, s, unit >> 1, unit & 1, slot);
         else if (phase == 2)
             pair_pencil_body<M0, TC, NT>(a, unit, 0, slot, ra, rb, smem_raw);
         else
-            pair_combine_body<M1, M2>(a, s, 0, unit, -1, slot, smem_raw);
+            pair_combine_body(PS(smem_raw), a, s, 0, unit, -1, slot);
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
@@ -173,11 +199,60 @@ bool axis_ok(int m0)
     return false;
 }
 
+// n = r1 r2 with both radices available and the larger one as small as it gets
+// (at equal size the first the larger: real space and global memory are met with
+// more elements per thread); false if there are none
+bool two_radices(int n, int &r1, int &r2)
+{
+    static const int rad[] = {
+#define X(Q) Q,
+        PAIR_RADICES(X)
+#undef X
+    };
+    int best = 1 << 30;
+    for (int a : rad)
+        for (int b : rad)
+            if (a >= b && a * b == n && a < best) {
+                best = a;
+                r1 = a;
+                r2 = b;
+            }
+    return best < (1 << 30);
+}
+
+int any_smem(const PairAny &q) { return (q.m1 * q.S + q.m1 + q.m2) * (int)sizeof(cplxd); }
+int any_pencil_smem(int m0) { return (m0 * kTile + m0) * (int)sizeof(cplxd) + (m0 + kTile) * (int)sizeof(double); }
+
+bool any_plan(int m1, int m2, PairAny &q)
+{
+    if (m1 < 2 || m2 < 2) return false;
+    if (!two_radices(m1, q.ra, q.rb) || !two_radices(m2, q.rc, q.rz)) return false;
+    q.m1 = m1;
+    q.m2 = m2;
+    q.S = m2 | 1;
+    q.mag1 = (unsigned)((1ull << 32) / m1) + 1;
+    q.mag2 = (unsigned)((1ull << 32) / m2) + 1;
+    return any_smem(q) <= kSmemCta;
+}
+
+// threads of a slab kernel of such a shape: one butterfly each in its widest
+// pass, up to 256, or 512 where shared memory leaves one CTA per SM
+int any_threads(const PairAny &q)
+{
+    const int n = std::max(std::max(q.m1 * q.rz, q.m1 * q.rc), std::max(q.ra * q.m2, q.rb * q.m2));
+    const int most = 2 * (any_smem(q) + 1024) <= 228 * 1024 ? 256 : 512;
+    return std::min(most, (n + 31) / 32 * 32);
+}
+
+bool any_axis(int m0, int &r1, int &r2) { return two_radices(m0, r2, r1) && any_pencil_smem(m0) <= kSmemCta; }
+
 }  // namespace
 
 bool pair_applicable(int m0, int m1, int m2)
 {
-    return slab_ok(m1, m2) && axis_ok(m0);
+    PairAny q;
+    int r1, r2;
+    return (slab_ok(m1, m2) || any_plan(m1, m2, q)) && (axis_ok(m0) || any_axis(m0, r1, r2));
 }
 
 // raises the kernels' shared-memory limits; *grid = CTAs of the persistent step launch (0: none)
@@ -203,6 +278,23 @@ int pair_setup(int m0, int m1, int m2, int *grid)
     }
     PAIR_AXES(X)
 #undef X
+    PairAny q;
+    int r1, r2;
+    if (!slab_ok(m1, m2) && any_plan(m1, m2, q)) switch (q.ra) {
+#define X(A)                                           \
+    case A:                                            \
+        up(k_pair_mid_any<A>, any_smem(q));            \
+        up(k_pair_combine_any<A>, any_smem(q));        \
+        break;
+            PAIR_RADICES(X)
+#undef X
+        }
+    if (!axis_ok(m0) && any_axis(m0, r1, r2)) switch (r2) {
+#define X(A) \
+    case A: up(k_pair_pencil_any<A>, any_pencil_smem(m0)); break;
+            PAIR_RADICES(X)
+#undef X
+        }
     *grid = 0;
 #define X(A, B, C)                                                                                             \
     if (m0 == A && m1 == B && m2 == C) {                                                                       \
@@ -234,6 +326,13 @@ void pair_mid(const PropsArgs<T> &a, int nslots, int s, cudaStream_t st)
     }
     PAIR_SLABS(X)
 #undef X
+    PairAny q;
+    if (any_plan(g.m1, g.m2, q)) switch (q.ra) {
+#define X(A)                                                                                                           \
+    case A: launch_step(k_pair_mid_any<A>, dim3(g.m0, 2, nslots), any_threads(q), any_smem(q), false, st, a, s, q); break;
+            PAIR_RADICES(X)
+#undef X
+        }
 }
 
 void pair_combine(const PropsArgs<T> &a, int nslots, int s, int mode, cudaStream_t st)
@@ -251,6 +350,16 @@ void pair_combine(const PropsArgs<T> &a, int nslots, int s, int mode, cudaStream
     }
     PAIR_SLABS(X)
 #undef X
+    PairAny q;
+    if (any_plan(g.m1, g.m2, q)) switch (q.ra) {
+#define X(A)                                                                                                         \
+    case A:                                                                                                          \
+        launch_step(k_pair_combine_any<A>, dim3(g.m0, split, nslots), any_threads(q), any_smem(q), split > 1, st, a, \
+                    s, mode, q);                                                                                     \
+        break;
+            PAIR_RADICES(X)
+#undef X
+        }
 }
 
 void pair_pencil(const PropsArgs<T> &a, int nslots, int both, int wide, cudaStream_t st)
@@ -264,6 +373,22 @@ void pair_pencil(const PropsArgs<T> &a, int nslots, int both, int wide, cudaStre
     }
     PAIR_SLABS(X)
 #undef X
+    PairAny q;
+    if (!slab_ok(g.m1, g.m2) && any_plan(g.m1, g.m2, q)) {
+        ra = q.ra;
+        rb = q.rb;
+    }
+    int r1, r2;
+    if (!axis_ok(g.m0) && any_axis(g.m0, r1, r2)) {
+        const dim3 grid((g.m1 * g.m2 + kTile - 1) / kTile, both ? 2 : 1, nslots);
+        switch (r2) {
+#define X(A) \
+    case A: launch_step(k_pair_pencil_any<A>, grid, kPencilThreads, any_pencil_smem(g.m0), false, st, a, ra, rb); break;
+            PAIR_RADICES(X)
+#undef X
+        }
+        return;
+    }
     const dim3 grid((g.m1 * g.m2 + tc - 1) / tc, both ? 2 : 1, nslots);
 #define X(A)                                                                                                 \
     if (g.m0 == A) {                                                                                         \

@@ -82,9 +82,11 @@ __device__ __forceinline__ void pdl_wait()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// asks for `bytes` at p to be brought into L2 (16-byte multiples); a hint, no wait
+// asks for `bytes` at p to be brought into L2; a hint, no wait.  The copy engine
+// wants 16-byte multiples; slabs of an odd number of doubles go without.
 __device__ __forceinline__ void prefetch_l2(const void *p, int bytes)
 {
+    if (((unsigned)(size_t)p | (unsigned)bytes) & 15u) return;
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
@@ -164,7 +166,7 @@ struct PairSlab : PairPlan<M1, M2> {
         twz = twy + M1;
     }
 
-    __device__ __forceinline__ void load_tables(const cplx<T> *tw, int m0)
+    __device__ __forceinline__ void load_tables(const cplx<T> *tw, int m0) const
     {
         for (int i = threadIdx.x; i < M1 + M2; i += NT) stc(twy + i, ldc_ro(tw + m0 + i));
     }
@@ -250,8 +252,9 @@ struct PairSlab : PairPlan<M1, M2> {
     // The RA-point y passes around real space: butterfly (z, j) holds the points
     // y = j + RB r of column z, lanes along z.  f(v, offset of (j, z) in the
     // slab) changes them in place (or fills them: INV = false); element r is at
-    // offset + ROW r.  With FWD the first forward y pass follows in registers.
-    static constexpr int ROW = RB * M2;
+    // offset + row() r.  With FWD the first forward y pass follows in registers.
+    static __device__ __forceinline__ int row() { return RB * M2; }
+    static __device__ __forceinline__ int area() { return M1 * M2; }
     template <bool INV, bool FWD, class F>
     __device__ __forceinline__ void real_space(F f) const
     {
@@ -343,23 +346,147 @@ struct PairSlab : PairPlan<M1, M2> {
     }
 };
 
+// ---------------------------------------------------------------- other slab shapes
+// The same slab transforms with sizes and radices known at run time: every axis
+// of a length R1 R2 with both radices among 1-10, 12, 14, 15, 16.  The passes are
+// out-of-line functions of the radix, shared by all kernels; only the real-space
+// radix RA is a template parameter of the slab.  The small y and z passes stay
+// apart (no merged pass).
+#define PAIR_RADICES(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(12) X(14) X(15) X(16)
+
+struct PairAny {
+    int m1, m2, ra, rb, rz, rc, S;
+    unsigned mag1, mag2;  // floor(2^32 / m) + 1: b / m = umulhi(b, mag), exact for b m < 2^32
+};
+
+// Butterfly b = i + n k reads src[i si + k sk + r sr] and writes
+// dst[i di + k dk + r dr], r < R; TW: times w^(k r), before a forward DFT, after
+// an inverse one.
+template <int R, int SIGN, bool TW, bool FROM_GLOBAL, bool TO_GLOBAL>
+__device__ __noinline__ void pair_any_pass(const cplxd *src, cplxd *dst, const cplxd *tw, int count, int n, unsigned mag,
+                                           int si, int sk, int sr, int di, int dk, int dr)
+{
+    if (!FROM_GLOBAL) __builtin_assume(__isShared(src));
+    if (!TO_GLOBAL) __builtin_assume(__isShared(dst));
+    if (TW) __builtin_assume(__isShared(tw));
+#pragma unroll 1
+    for (int b = threadIdx.x; b < count; b += blockDim.x) {
+        const int k = (int)__umulhi((unsigned)b, mag), i = b - k * n;
+        const cplxd *p = src + i * si + k * sk;
+        cplxd v[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            v[r] = FROM_GLOBAL ? ldc_cg(p + r * sr) : ldc(p + r * sr);
+            if (TW && SIGN < 0 && r > 0) v[r] = cmul(v[r], ldc(tw + k * r));
+        }
+        Reg<double, R, SIGN>::run(v);
+        cplxd *o = dst + i * di + k * dk;
+#pragma unroll
+        for (int r = 0; r < R; r++) stc(o + r * dr, TW && SIGN > 0 && r > 0 ? cmulc(v[r], ldc(tw + k * r)) : v[r]);
+    }
+}
+
+template <int SIGN, bool TW, bool FROM_GLOBAL, bool TO_GLOBAL = false>
+__device__ __forceinline__ void pair_any(int R, const cplxd *src, cplxd *dst, const cplxd *tw, int count, int n,
+                                         unsigned mag, int si, int sk, int sr, int di, int dk, int dr)
+{
+    switch (R) {
+#define X(Q) \
+    case Q: pair_any_pass<Q, SIGN, TW, FROM_GLOBAL, TO_GLOBAL>(src, dst, tw, count, n, mag, si, sk, sr, di, dk, dr); break;
+        PAIR_RADICES(X)
+#undef X
+    }
+}
+
+template <int RA_>
+struct PairSlabAny {
+    using T = double;
+    static constexpr int RA = RA_;
+    PairAny q;
+    cplx<T> *buf, *twy, *twz;
+
+    __device__ __forceinline__ PairSlabAny(unsigned char *smem, const PairAny &plan) : q(plan)
+    {
+        buf = reinterpret_cast<cplx<T> *>(smem);
+        twy = buf + q.m1 * q.S;
+        twz = twy + q.m1;
+    }
+    __device__ __forceinline__ int row() const { return q.rb * q.m2; }
+    __device__ __forceinline__ int area() const { return q.m1 * q.m2; }
+
+    __device__ __forceinline__ void load_tables(const cplx<T> *tw, int m0) const
+    {
+        for (int i = threadIdx.x; i < q.m1 + q.m2; i += blockDim.x) stc(twy + i, ldc_ro(tw + m0 + i));
+    }
+
+    __device__ __forceinline__ void inverse_passes(const cplx<T> *src, bool split = false) const
+    {
+        pair_any<1, true, true>(q.rc, src, buf, twz, q.m1 * q.rz, q.m1, q.mag1, 1, q.m1, q.rz * q.m1, q.S, q.rc, 1);
+        __syncthreads();
+        if (split) pair_arrive();
+        if (q.rz > 1) {
+            pair_any<1, false, false>(q.rz, buf, buf, twz, q.m1 * q.rc, q.m1, q.mag1, q.S, 1, q.rc, q.S, 1, q.rc);
+            __syncthreads();
+        }
+        if (q.rb > 1) {
+            pair_any<1, true, false>(q.rb, buf, buf, twy, q.ra * q.m2, q.m2, q.mag2, 1, q.rb * q.S, q.S, 1, q.rb * q.S, q.S);
+            __syncthreads();
+        }
+    }
+
+    template <bool INV, bool FWD, class F>
+    __device__ __forceinline__ void real_space(F f) const
+    {
+#pragma unroll 1
+        for (int b = threadIdx.x; b < q.rb * q.m2; b += blockDim.x) {
+            const int j = (int)__umulhi((unsigned)b, q.mag2), z = b - j * q.m2, step = q.rb * q.S;
+            cplx<T> v[RA], *p = buf + j * q.S + z;
+            if (INV) {
+#pragma unroll
+                for (int r = 0; r < RA; r++) v[r] = ldc(p + step * r);
+                Reg<T, RA, 1>::run(v);
+            }
+            f(v, b);
+            if (FWD) {
+                Reg<T, RA, -1>::run(v);
+#pragma unroll
+                for (int r = 0; r < RA; r++) stc(p + step * r, v[r]);
+            }
+        }
+    }
+
+    __device__ __forceinline__ void forward_passes(cplx<T> *dst, bool split, bool last) const
+    {
+        __syncthreads();
+        if (q.rb > 1) {
+            pair_any<-1, true, false>(q.rb, buf, buf, twy, q.ra * q.m2, q.m2, q.mag2, 1, q.rb * q.S, q.S, 1, q.rb * q.S, q.S);
+            __syncthreads();
+        }
+        if (q.rz > 1) {
+            pair_any<-1, false, false>(q.rz, buf, buf, twz, q.m1 * q.rc, q.m1, q.mag1, q.S, 1, q.rc, q.S, 1, q.rc);
+            __syncthreads();
+        }
+        if (split) pair_wait();
+        if (last) pdl_trigger();
+        pair_any<-1, true, false, true>(q.rc, buf, dst, twz, q.m1 * q.rz, q.m1, q.mag1, q.S, q.rc, 1, 1, q.m1, q.rz * q.m1);
+    }
+};
+
 // mid, slab x of a slot: sp = 0 the half-step spectrum (inverse slab, times E2,
 // forward slab), sp = 1 the full-step spectrum (inverse slab, P = E2 qs1)
-template <int M1, int M2>
-__device__ __forceinline__ void pair_mid_body(const PropsArgs<double> &a, int s, int x, int sp, int slot, unsigned char *smem)
+template <class PS>
+__device__ __forceinline__ void pair_mid_body(const PS &B, const PropsArgs<double> &a, int s, int x, int sp, int slot)
 {
     using T = double;
     const Geo &g = a.g;
-    constexpr int AREA = M1 * M2;
-    using PS = PairSlab<M1, M2>;
-    PS B(smem);
+    const int area = B.area(), row = B.row();
     B.load_tables(a.tw, g.m0);
-    const size_t off = (size_t)x * AREA;
+    const size_t off = (size_t)x * area;
     cplx<T> *spec = a.spec + ((size_t)slot * 2 + sp) * g.M + off;
     const T *Eq = pair_etab(a, slot, 0, s) + off, *Ep = pair_etab(a, slot, 1, s) + off;
     if (threadIdx.x == 0) {
-        prefetch_l2(Eq, AREA * sizeof(T));
-        prefetch_l2(Ep, AREA * sizeof(T));
+        prefetch_l2(Eq, area * sizeof(T));
+        prefetch_l2(Ep, area * sizeof(T));
     }
     __syncthreads();
     pdl_wait();
@@ -368,7 +495,7 @@ __device__ __forceinline__ void pair_mid_body(const PropsArgs<double> &a, int s,
         B.template real_space<true, true>([&](cplx<T> *v, int o) {
 #pragma unroll
             for (int r = 0; r < PS::RA; r++) {
-                const T e0 = __ldg(Eq + o + PS::ROW * r), e1 = __ldg(Ep + o + PS::ROW * r);
+                const T e0 = __ldg(Eq + o + row * r), e1 = __ldg(Ep + o + row * r);
                 v[r].x *= e0 * e0;
                 v[r].y *= e1 * e1;
             }
@@ -379,8 +506,8 @@ __device__ __forceinline__ void pair_mid_body(const PropsArgs<double> &a, int s,
         B.template real_space<true, false>([&](cplx<T> *v, int o) {
 #pragma unroll
             for (int r = 0; r < PS::RA; r++) {
-                const T e0 = __ldg(Eq + o + PS::ROW * r), e1 = __ldg(Ep + o + PS::ROW * r);
-                stc(P + o + PS::ROW * r, cplx<T>{v[r].x * (e0 * e0), v[r].y * (e1 * e1)});
+                const T e0 = __ldg(Eq + o + row * r), e1 = __ldg(Ep + o + row * r);
+                stc(P + o + row * r, cplx<T>{v[r].x * (e0 * e0), v[r].y * (e1 * e1)});
             }
         });
     }
@@ -392,17 +519,15 @@ __device__ __forceinline__ void pair_mid_body(const PropsArgs<double> &a, int s,
 // half-step / full-step one (both repeat the inverse transform, which shortens
 // the chain when the batch leaves SMs idle; they are a cluster of two) and half
 // 0 stores q.
-template <int M1, int M2>
-__device__ __forceinline__ void pair_combine_body(const PropsArgs<double> &a, int s, int mode, int x, int half, int slot,
-                                                  unsigned char *smem)
+template <class PS>
+__device__ __forceinline__ void pair_combine_body(const PS &B, const PropsArgs<double> &a, int s, int mode, int x, int half,
+                                                  int slot)
 {
     using T = double;
     const Geo &g = a.g;
-    constexpr int AREA = M1 * M2;
-    using PS = PairSlab<M1, M2>;
-    PS B(smem);
+    const int area = B.area(), row = B.row();
     B.load_tables(a.tw, g.m0);
-    const size_t M = g.M, off = (size_t)x * AREA;
+    const size_t M = g.M, off = (size_t)x * area;
     cplx<T> *specA = a.spec + (size_t)slot * 2 * M + off, *specB = specA + M;
     const int sn = s + 1;
     T *q0 = a.hist + ((size_t)slot * (g.Ns + 1) + sn) * 2 * M + off, *q1 = q0 + M;
@@ -410,25 +535,25 @@ __device__ __forceinline__ void pair_combine_body(const PropsArgs<double> &a, in
     const T *Nq = pair_etab(a, slot, 0, next ? sn : 0) + off, *Np = pair_etab(a, slot, 1, next ? sn : 0) + off;
     const T *Eq = pair_etab(a, slot, 0, s) + off, *Ep = pair_etab(a, slot, 1, s) + off;
     if (mode == 0 && threadIdx.x == 0) {
-        prefetch_l2(Eq, AREA * sizeof(T));
-        prefetch_l2(Ep, AREA * sizeof(T));
+        prefetch_l2(Eq, area * sizeof(T));
+        prefetch_l2(Ep, area * sizeof(T));
     }
     __syncthreads();
     pdl_wait();
     if (mode == 0) {
         const cplx<T> *P = reinterpret_cast<const cplx<T> *>(a.pbuf) + (size_t)slot * M + off;
-        if (threadIdx.x == 0) prefetch_l2(P, AREA * sizeof(cplx<T>));
+        if (threadIdx.x == 0) prefetch_l2(P, area * sizeof(cplx<T>));
         B.inverse_passes(specA, half >= 0);
         // Richardson, GPU_kernels.h:199-203
         auto finish = [&](cplx<T> *v, int o) {
 #pragma unroll
             for (int r = 0; r < PS::RA; r++) {
-                const cplx<T> p = ldc_cg(P + o + PS::ROW * r);
-                v[r].x = third(v[r].x * __ldg(Eq + o + PS::ROW * r) * (T)4 - p.x);
-                v[r].y = third(v[r].y * __ldg(Ep + o + PS::ROW * r) * (T)4 - p.y);
+                const cplx<T> p = ldc_cg(P + o + row * r);
+                v[r].x = third(v[r].x * __ldg(Eq + o + row * r) * (T)4 - p.x);
+                v[r].y = third(v[r].y * __ldg(Ep + o + row * r) * (T)4 - p.y);
                 if (store) {
-                    q0[o + PS::ROW * r] = v[r].x;
-                    q1[o + PS::ROW * r] = v[r].y;
+                    q0[o + row * r] = v[r].x;
+                    q1[o + row * r] = v[r].y;
                 }
             }
         };
@@ -440,7 +565,7 @@ __device__ __forceinline__ void pair_combine_body(const PropsArgs<double> &a, in
             finish(v, o);
 #pragma unroll
             for (int r = 0; r < PS::RA; r++) {
-                T e0 = __ldg(Nq + o + PS::ROW * r), e1 = __ldg(Np + o + PS::ROW * r);
+                T e0 = __ldg(Nq + o + row * r), e1 = __ldg(Np + o + row * r);
                 if (half == 1) {
                     e0 *= e0;
                     e1 *= e1;
@@ -453,12 +578,12 @@ __device__ __forceinline__ void pair_combine_body(const PropsArgs<double> &a, in
         auto start = [&](cplx<T> *v, int o) {
 #pragma unroll
             for (int r = 0; r < PS::RA; r++) {
-                v[r] = mode == 1 ? cplx<T>{(T)1, (T)1} : cplx<T>{q0[o + PS::ROW * r], q1[o + PS::ROW * r]};
+                v[r] = mode == 1 ? cplx<T>{(T)1, (T)1} : cplx<T>{q0[o + row * r], q1[o + row * r]};
                 if (mode == 1 && store) {
-                    q0[o + PS::ROW * r] = (T)1;
-                    q1[o + PS::ROW * r] = (T)1;
+                    q0[o + row * r] = (T)1;
+                    q1[o + row * r] = (T)1;
                 }
-                T e0 = __ldg(Nq + o + PS::ROW * r), e1 = __ldg(Np + o + PS::ROW * r);
+                T e0 = __ldg(Nq + o + row * r), e1 = __ldg(Np + o + row * r);
                 if (half == 1) {
                     e0 *= e0;
                     e1 *= e1;
@@ -477,8 +602,8 @@ __device__ __forceinline__ void pair_combine_body(const PropsArgs<double> &a, in
     B.template real_space<false, true>([&](cplx<T> *v, int o) {
 #pragma unroll
         for (int r = 0; r < PS::RA; r++) {
-            const T e0 = __ldg(Nq + o + PS::ROW * r), e1 = __ldg(Np + o + PS::ROW * r);
-            v[r] = {q0[o + PS::ROW * r] * (e0 * e0), q1[o + PS::ROW * r] * (e1 * e1)};
+            const T e0 = __ldg(Nq + o + row * r), e1 = __ldg(Np + o + row * r);
+            v[r] = {q0[o + row * r] * (e0 * e0), q1[o + row * r] * (e1 * e1)};
         }
     });
     B.forward_passes(specB, false, true);
@@ -566,6 +691,73 @@ __device__ __forceinline__ void pair_pencil_body(const PropsArgs<double> &a, int
 #pragma unroll
             for (int r = 0; r < R1; r++) stc(spec + (size_t)(j + R2 * r) * ncol + t, v[r]);
         }
+    }
+}
+
+// The same x pass with m0 = r1 R2 and the first radix known at run time.
+template <int R2, int TC>
+__device__ __forceinline__ void pair_pencil_any_body(const PropsArgs<double> &a, int tile, int sp, int slot, int ra, int rb,
+                                                     unsigned char *smem)
+{
+    using T = double;
+    const Geo &g = a.g;
+    const int m0 = g.m0, m1 = g.m1, m2 = g.m2, ncol = m1 * m2, c0 = tile * TC, r1 = m0 / R2;
+    const int nc = ncol - c0 < TC ? ncol - c0 : TC;
+    cplx<T> *buf = reinterpret_cast<cplx<T> *>(smem);
+    cplx<T> *tw = buf + m0 * TC;
+    T *gx = reinterpret_cast<T *>(tw + m0), *colf = gx + m0;
+    cplx<T> *spec = a.spec + ((size_t)slot * 2 + sp) * g.M + c0;
+    const T *kf = a.kfac + (size_t)__ldg(a.slot_rep + slot) * a.kf_stride;
+    for (int i = threadIdx.x; i < m0; i += blockDim.x) {
+        stc(tw + i, ldc_ro(a.tw + i));
+        gx[i] = __ldg(kf + i);
+    }
+    for (int t = threadIdx.x; t < nc; t += blockDim.x) {
+        const int c = c0 + t, kz = c / m1, p = c - kz * m1, ky = p / rb + ra * (p % rb);
+        colf[t] = __ldg(kf + m0 + ky) * __ldg(kf + m0 + m1 + (2 * kz > m2 ? m2 - kz : kz));
+    }
+    pdl_wait();
+    const unsigned mag = 0xffffffffu / (unsigned)nc + 1u;  // nc = 1: butterfly b is (0, b)
+    auto outer = [&](int b, int &t, int &j) {
+        j = nc > 1 ? (int)__umulhi((unsigned)b, mag) : b;
+        t = b - j * nc;
+    };
+    if (nc > 1) {
+        pair_any<-1, false, true>(r1, spec, buf, tw, nc * R2, nc, mag, 1, ncol, R2 * ncol, 1, TC, R2 * TC);
+    } else {
+        // one column left: butterfly index b = R2-point position
+        pair_any<-1, false, true>(r1, spec, buf, tw, R2, 1 << 30, 0, ncol, 0, R2 * ncol, TC, 0, R2 * TC);
+    }
+    __syncthreads();
+    const T invM = a.invM, Mreal = a.Mreal;
+#pragma unroll 1
+    for (int b = threadIdx.x; b < r1 * nc; b += blockDim.x) {
+        int t, k1;
+        outer(b, t, k1);
+        cplx<T> v[R2], *p = buf + R2 * k1 * TC + t;
+        v[0] = ldc(p);
+#pragma unroll
+        for (int i = 1; i < R2; i++) v[i] = cmul(ldc(p + i * TC), ldc(tw + k1 * i));
+        Reg<T, R2, -1>::run(v);
+        const T ct = colf[t];
+#pragma unroll
+        for (int i = 0; i < R2; i++) {
+            const T k2 = gx[k1 + r1 * i] * ct * invM;
+            const T f = sp == 0 ? k2 : k2 * k2 * Mreal;
+            v[i].x *= f;
+            v[i].y *= f;
+        }
+        Reg<T, R2, 1>::run(v);
+        stc(p, v[0]);
+#pragma unroll
+        for (int i = 1; i < R2; i++) stc(p + i * TC, cmulc(v[i], ldc(tw + k1 * i)));
+    }
+    __syncthreads();
+    pdl_trigger();
+    if (nc > 1) {
+        pair_any<1, false, false, true>(r1, buf, spec, tw, nc * R2, nc, mag, 1, TC, R2 * TC, 1, ncol, R2 * ncol);
+    } else {
+        pair_any<1, false, false, true>(r1, buf, spec, tw, R2, 1 << 30, 0, TC, 0, R2 * TC, ncol, 0, R2 * ncol);
     }
 }
 

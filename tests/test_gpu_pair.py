@@ -1,6 +1,6 @@
 """The FP64 contour step on q + i q^dagger (csrc/pair.cuh) against the FP64
-oracle, on every slab shape it has (merged and unmerged passes) and with an x
-axis of its own, as one replica (the combine of two CTAs per slab where the
+oracle, on every slab shape it has (merged and unmerged passes, run-time sizes)
+and with an x axis of its own, and on shapes it leaves to the general kernels, as one replica (the combine of two CTAs per slab where the
 batch is small) and in a batch of several (one CTA per slab)."""
 import numpy as np
 import pytest
@@ -11,7 +11,10 @@ import scft_string_b200 as S
 pytestmark = pytest.mark.gpu
 
 GRIDS = [(16, 16, 16), (24, 24, 24), (40, 40, 40), (80, 80, 80), (16, 64, 64), (96, 24, 24), (80, 64, 96),
-         (128, 16, 16), (24, 96, 96), (48, 48, 48)]
+         (128, 16, 16), (24, 96, 96), (48, 48, 48),
+         # run-time sizes: every radix, prime axes, the smallest ones, one column left over
+         (35, 54, 45), (2, 2, 2), (3, 5, 7), (9, 100, 98), (6, 15, 16), (112, 14, 12), (10, 3, 3),
+         (30, 108, 112), (64, 25, 27), (1, 12, 10), (12, 1, 10), (12, 10, 1), (4, 125, 6)]
 
 
 @pytest.mark.parametrize("m", GRIDS)
