@@ -18,7 +18,7 @@ constexpr int kSmemCta = 227 * 1024;  // dynamic shared memory a CTA may have
 constexpr int kSms = 148;
 
 // slab shapes (m1, m2) and x lengths with kernels
-#define PAIR_SLABS(X) X(16, 16) X(24, 24) X(32, 32) X(40, 40) X(48, 48) X(64, 64) X(64, 96) X(80, 80) X(96, 96)
+#define PAIR_SLABS(X) X(16, 16) X(24, 24) X(32, 32) X(40, 40) X(48, 48) X(64, 64) X(64, 96) X(80, 80) X(96, 96) X(128, 128)
 #define PAIR_AXES(X) X(16) X(24) X(32) X(40) X(48) X(64) X(80) X(96) X(128)
 // grids with a persistent step kernel
 #define PAIR_GRIDS(X) X(32, 32, 32) X(48, 48, 48) X(64, 64, 64) X(64, 64, 96) X(96, 96, 96)
@@ -26,25 +26,22 @@ constexpr int kSms = 148;
 constexpr int kTile = 32;         // columns per x tile; the wide form takes twice as many
 constexpr int kPencilThreads = 256;
 
-template <int M1, int M2>
-constexpr bool kSlabFits = PairSlab<M1, M2>::SMEM <= kSmemCta;
-
 constexpr int pencil_minb(int m0) { return m0 > 80 ? 2 : 3; }
 
-template <int M1, int M2>
-__global__ void __launch_bounds__(PairSlab<M1, M2>::NT, PairSlab<M1, M2>::MINB) k_pair_mid(PropsArgs<T> a, int s)
+template <int M1, int M2, int CL>
+__global__ void __launch_bounds__(PairSlab<M1, M2, CL>::NT, PairSlab<M1, M2, CL>::MINB) k_pair_mid(PropsArgs<T> a, int s)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    pair_mid_body(PairSlab<M1, M2>(smem_raw), a, s, blockIdx.x, blockIdx.y, blockIdx.z);
+    pair_mid_body(PairSlab<M1, M2, CL>(smem_raw), a, s, blockIdx.x / CL, blockIdx.y, blockIdx.z);
 }
 
-template <int M1, int M2>
-__global__ void __launch_bounds__(PairSlab<M1, M2>::NT, PairSlab<M1, M2>::MINB)
+template <int M1, int M2, int CL>
+__global__ void __launch_bounds__(PairSlab<M1, M2, CL>::NT, PairSlab<M1, M2, CL>::MINB)
     k_pair_combine(PropsArgs<T> a, int s, int mode)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    pair_combine_body(PairSlab<M1, M2>(smem_raw), a, s, mode, blockIdx.x, gridDim.y == 1 ? -1 : (int)blockIdx.y,
-                      blockIdx.z);
+    pair_combine_body(PairSlab<M1, M2, CL>(smem_raw), a, s, mode, blockIdx.x / CL,
+                      gridDim.y == 1 ? -1 : (int)blockIdx.y, blockIdx.z);
 }
 
 template <int M0, int TC>
@@ -98,12 +95,12 @@ constexpr uint32_t kStepSpin = 1u << 22;
 // residency is assumed.  Every wait is bounded and records error 3 when it
 // gives up, which ends the kernel.
 template <int M0, int M1, int M2, int TC>
-__global__ void __launch_bounds__(PairSlab<M1, M2>::NT, PairSlab<M1, M2>::MINB)
+__global__ void __launch_bounds__(PairSlab<M1, M2, 1>::NT, PairSlab<M1, M2, 1>::MINB)
     k_pair_step(PropsArgs<T> a, int s, int nslots)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ int item_sh[3], ok_sh;
-    using PS = PairSlab<M1, M2>;
+    using PS = PairSlab<M1, M2, 1>;
     constexpr int NT = PS::NT, ntiles = (M1 * M2 + TC - 1) / TC;
     int ra, rb;
     PS::radices(ra, rb);
@@ -155,14 +152,14 @@ __global__ void __launch_bounds__(PairSlab<M1, M2>::NT, PairSlab<M1, M2>::MINB)
 template <int M0, int M1, int M2, int TC>
 constexpr int step_smem()
 {
-    return PairSlab<M1, M2>::SMEM > PairPencil<M0, TC>::SMEM ? PairSlab<M1, M2>::SMEM
+    return PairSlab<M1, M2, 1>::SMEM > PairPencil<M0, TC>::SMEM ? PairSlab<M1, M2, 1>::SMEM
                                                                    : PairPencil<M0, TC>::SMEM;
 }
 
 // Launch of a step kernel: it may start while the kernel before it on the
-// stream finishes (see pdl_wait); cluster: the CTAs along y form one cluster.
+// stream finishes (see pdl_wait), in clusters of (cx, cy) CTAs.
 template <class... Args>
-void launch_step(void (*fn)(Args...), dim3 grid, int threads, int smem, bool cluster, cudaStream_t st, Args... args)
+void launch_step(void (*fn)(Args...), dim3 grid, int threads, int smem, int cx, int cy, cudaStream_t st, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -173,18 +170,24 @@ void launch_step(void (*fn)(Args...), dim3 grid, int threads, int smem, bool clu
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = 1;
-    at[1].val.clusterDim.y = grid.y;
+    at[1].val.clusterDim.x = cx;
+    at[1].val.clusterDim.y = cy;
     at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = cluster ? 2 : 1;
+    cfg.numAttrs = cx * cy > 1 ? 2 : 1;
     cudaLaunchKernelEx(&cfg, fn, args...);
 }
+
+// CTAs per slab: one where the slab fits a CTA's shared memory.  Two were slower
+// on every shape that fits (one replica step: 64^3 34.2 us with one, 37.1 with
+// two; 48^3 22.9 and 27.3; 96^3 84.9 and 91.6).
+template <int M1, int M2>
+constexpr int kCl = PairSlab<M1, M2, 1>::SMEM <= kSmemCta ? 1 : 2;
 
 bool slab_ok(int m1, int m2)
 {
 #define X(A, B) \
-    if (m1 == A && m2 == B) return kSlabFits<A, B>;
+    if (m1 == A && m2 == B) return true;
     PAIR_SLABS(X)
 #undef X
     return false;
@@ -262,12 +265,11 @@ int pair_setup(int m0, int m1, int m2, int *grid)
     auto up = [&](auto *fn, int bytes) {
         if (e == cudaSuccess) e = raise_dyn_smem(fn, bytes);
     };
-#define X(A, B)                                                \
-    if (m1 == A && m2 == B) {                                  \
-        if constexpr (kSlabFits<A, B>) {                       \
-            up(k_pair_mid<A, B>, PairSlab<A, B>::SMEM);     \
-            up(k_pair_combine<A, B>, PairSlab<A, B>::SMEM); \
-        }                                                      \
+#define X(A, B)                                                     \
+    if (m1 == A && m2 == B) {                                       \
+        constexpr int CL = kCl<A, B>;                               \
+        up(k_pair_mid<A, B, CL>, PairSlab<A, B, CL>::SMEM);         \
+        up(k_pair_combine<A, B, CL>, PairSlab<A, B, CL>::SMEM);     \
     }
     PAIR_SLABS(X)
 #undef X
@@ -298,13 +300,13 @@ int pair_setup(int m0, int m1, int m2, int *grid)
     *grid = 0;
 #define X(A, B, C)                                                                                             \
     if (m0 == A && m1 == B && m2 == C) {                                                                       \
-        if constexpr (kSlabFits<B, C>) {                                                                       \
+        if constexpr (kCl<B, C> == 1) {                                                                       \
             up(k_pair_step<A, B, C, kTile>, step_smem<A, B, C, kTile>());                                       \
             up(k_pair_step<A, B, C, 2 * kTile>, step_smem<A, B, C, 2 * kTile>());                               \
             int per_sm = 0;                                                                                    \
             if (e == cudaSuccess &&                                                                            \
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_step<A, B, C, 2 * kTile>,         \
-                                                              PairSlab<B, C>::NT,                           \
+                                                              PairSlab<B, C, 1>::NT,                           \
                                                               step_smem<A, B, C, 2 * kTile>()) == cudaSuccess)  \
                 *grid = per_sm * kSms;                                                                         \
         }                                                                                                      \
@@ -317,19 +319,19 @@ int pair_setup(int m0, int m1, int m2, int *grid)
 void pair_mid(const PropsArgs<T> &a, int nslots, int s, cudaStream_t st)
 {
     const Geo &g = a.g;
-#define X(A, B)                                                                                              \
-    if (g.m1 == A && g.m2 == B) {                                                                            \
-        using P = PairSlab<A, B>;                                                                         \
-        if constexpr (kSlabFits<A, B>)                                                                       \
-            launch_step(k_pair_mid<A, B>, dim3(g.m0, 2, nslots), P::NT, P::SMEM, false, st, a, s);            \
-        return;                                                                                              \
+#define X(A, B)                                                                                                      \
+    if (g.m1 == A && g.m2 == B) {                                                                                    \
+        constexpr int CL = kCl<A, B>;                                                                                \
+        using P = PairSlab<A, B, CL>;                                                                                \
+        launch_step(k_pair_mid<A, B, CL>, dim3(CL * g.m0, 2, nslots), P::NT, P::SMEM, CL, 1, st, a, s);               \
+        return;                                                                                                      \
     }
     PAIR_SLABS(X)
 #undef X
     PairAny q;
     if (any_plan(g.m1, g.m2, q)) switch (q.ra) {
 #define X(A)                                                                                                           \
-    case A: launch_step(k_pair_mid_any<A>, dim3(g.m0, 2, nslots), any_threads(q), any_smem(q), false, st, a, s, q); break;
+    case A: launch_step(k_pair_mid_any<A>, dim3(g.m0, 2, nslots), any_threads(q), any_smem(q), 1, 1, st, a, s, q); break;
             PAIR_RADICES(X)
 #undef X
         }
@@ -341,12 +343,13 @@ void pair_combine(const PropsArgs<T> &a, int nslots, int s, int mode, cudaStream
     // two CTAs per slab while both find an SM of their own: the chain of a CTA
     // is then two slab transforms instead of three
     const int split = 2 * g.m0 * nslots <= kSms && s + 1 < g.Ns ? 2 : 1;
-#define X(A, B)                                                                                                     \
-    if (g.m1 == A && g.m2 == B) {                                                                                   \
-        using P = PairSlab<A, B>;                                                                                \
-        if constexpr (kSlabFits<A, B>)                                                                              \
-            launch_step(k_pair_combine<A, B>, dim3(g.m0, split, nslots), P::NT, P::SMEM, split > 1, st, a, s, mode); \
-        return;                                                                                                     \
+#define X(A, B)                                                                                                      \
+    if (g.m1 == A && g.m2 == B) {                                                                                    \
+        constexpr int CL = kCl<A, B>;                                                                                \
+        const int half = CL > 1 ? 1 : split;                                                                         \
+        using P = PairSlab<A, B, CL>;                                                                                \
+        launch_step(k_pair_combine<A, B, CL>, dim3(CL * g.m0, half, nslots), P::NT, P::SMEM, CL, half, st, a, s, mode); \
+        return;                                                                                                      \
     }
     PAIR_SLABS(X)
 #undef X
@@ -354,7 +357,7 @@ void pair_combine(const PropsArgs<T> &a, int nslots, int s, int mode, cudaStream
     if (any_plan(g.m1, g.m2, q)) switch (q.ra) {
 #define X(A)                                                                                                         \
     case A:                                                                                                          \
-        launch_step(k_pair_combine_any<A>, dim3(g.m0, split, nslots), any_threads(q), any_smem(q), split > 1, st, a, \
+        launch_step(k_pair_combine_any<A>, dim3(g.m0, split, nslots), any_threads(q), any_smem(q), 1, split, st, a, \
                     s, mode, q);                                                                                     \
         break;
             PAIR_RADICES(X)
@@ -369,7 +372,7 @@ void pair_pencil(const PropsArgs<T> &a, int nslots, int both, int wide, cudaStre
     int ra = 1, rb = 1;
 #define X(A, B)                        \
     if (g.m1 == A && g.m2 == B) {      \
-        PairSlab<A, B>::radices(ra, rb); \
+        PairSlab<A, B, 1>::radices(ra, rb); \
     }
     PAIR_SLABS(X)
 #undef X
@@ -383,7 +386,7 @@ void pair_pencil(const PropsArgs<T> &a, int nslots, int both, int wide, cudaStre
         const dim3 grid((g.m1 * g.m2 + kTile - 1) / kTile, both ? 2 : 1, nslots);
         switch (r2) {
 #define X(A) \
-    case A: launch_step(k_pair_pencil_any<A>, grid, kPencilThreads, any_pencil_smem(g.m0), false, st, a, ra, rb); break;
+    case A: launch_step(k_pair_pencil_any<A>, grid, kPencilThreads, any_pencil_smem(g.m0), 1, 1, st, a, ra, rb); break;
             PAIR_RADICES(X)
 #undef X
         }
@@ -393,9 +396,9 @@ void pair_pencil(const PropsArgs<T> &a, int nslots, int both, int wide, cudaStre
 #define X(A)                                                                                                 \
     if (g.m0 == A) {                                                                                         \
         if (wide)                                                                                            \
-            launch_step(k_pair_pencil<A, 2 * kTile>, grid, kPencilThreads, PairPencil<A, 2 * kTile>::SMEM, false, st, a, ra, rb);  \
+            launch_step(k_pair_pencil<A, 2 * kTile>, grid, kPencilThreads, PairPencil<A, 2 * kTile>::SMEM, 1, 1, st, a, ra, rb);  \
         else                                                                                                 \
-            launch_step(k_pair_pencil<A, kTile>, grid, kPencilThreads, PairPencil<A, kTile>::SMEM, false, st, a, ra, rb);          \
+            launch_step(k_pair_pencil<A, kTile>, grid, kPencilThreads, PairPencil<A, kTile>::SMEM, 1, 1, st, a, ra, rb);          \
         return;                                                                                              \
     }
     PAIR_AXES(X)
@@ -407,8 +410,8 @@ void pair_step(const PropsArgs<T> &a, int nslots, int s, int wide, int grid, cud
     const Geo &g = a.g;
 #define X(A, B, C)                                                                                                   \
     if (g.m0 == A && g.m1 == B && g.m2 == C) {                                                                       \
-        if constexpr (kSlabFits<B, C>) {                                                                             \
-            constexpr int NT = PairSlab<B, C>::NT;                                                                \
+        if constexpr (kCl<B, C> == 1) {                                                                             \
+            constexpr int NT = PairSlab<B, C, 1>::NT;                                                                \
             if (wide)                                                                                                \
                 k_pair_step<A, B, C, 2 * kTile><<<grid, NT, step_smem<A, B, C, 2 * kTile>(), st>>>(a, s, nslots);     \
             else                                                                                                     \

@@ -101,6 +101,20 @@ __device__ __forceinline__ void pair_wait()
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ int cluster_rank()
+{
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return (int)r;
+}
+// the same shared-memory object of CTA `rank` of the cluster, as a generic address
+__device__ __forceinline__ cplxd *cluster_map(cplxd *p, int rank)
+{
+    unsigned long long o;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(o) : "l"((unsigned long long)p), "r"(rank));
+    return reinterpret_cast<cplxd *>(o);
+}
+
 __device__ __forceinline__ const double *pair_etab(const PropsArgs<double> &a, int slot, int fld, int s)
 {
     const Geo &g = a.g;
@@ -131,26 +145,33 @@ PAIR_PLAN(64, 64, 16, 4, 4, 16, true, 256, 512)
 PAIR_PLAN(64, 96, 8, 8, 12, 8, false, 256, 512)
 PAIR_PLAN(80, 80, 10, 8, 10, 8, false, 416, 416)
 PAIR_PLAN(96, 96, 12, 8, 12, 8, false, 384, 384)
-PAIR_PLAN(128, 128, 16, 8, 16, 8, false, 512, 512)
+PAIR_PLAN(128, 128, 16, 8, 16, 8, false, 1024, 512)  // two CTAs per slab only
 #undef PAIR_PLAN
 
-template <int M1, int M2>
+// threads of one of CL CTAs
+__host__ __device__ constexpr int pair_nt(int nt, int cl) { return cl == 1 ? nt : (nt / cl + 31) / 32 * 32; }
+
+// CL CTAs of a cluster may share a slab: each holds M1/CL of its rows (y
+// positions).  Every pass but the RA-point y pass stays within those rows; that
+// one takes M2/CL columns per CTA and reads and writes the other CTAs' rows
+// through distributed shared memory, in place, between two cluster barriers.
+template <int M1, int M2, int CL>
 struct PairSlab : PairPlan<M1, M2> {
     using T = double;
     using Plan = PairPlan<M1, M2>;
     using Plan::MERGE;
-    using Plan::NT;
     using Plan::RA;
     using Plan::RB;
     using Plan::RC;
     using Plan::RZ;
-    static_assert(RA * RB == M1 && RZ * RC == M2, "plan");
-    static constexpr int S = M2 | 1;
-    static constexpr int SMEM = (M1 * S + M1 + M2) * (int)sizeof(cplx<T>);
+    static_assert(RA * RB == M1 && RZ * RC == M2 && RA % CL == 0 && M2 % CL == 0, "plan");
+    static constexpr int NT = pair_nt(Plan::NT, CL), L = M1 / CL, RAL = RA / CL, S = M2 | 1;
+    static constexpr int SMEM = (L * S + M1 + M2) * (int)sizeof(cplx<T>);
     static constexpr int FIT = 227 * 1024 / (SMEM + 1024), REG = Plan::WANT / NT;
     static constexpr int MINB = FIT < 1 ? 1 : FIT < REG ? FIT : REG < 1 ? 1 : REG;
 
-    cplx<T> *buf, *twy, *twz;
+    cplx<T> *buf, *twy, *twz, *part[CL];
+    int rank;
 
     // radices of the y transform that the spectrum order depends on
     static __host__ __device__ void radices(int &ra, int &rb)
@@ -162,13 +183,36 @@ struct PairSlab : PairPlan<M1, M2> {
     __device__ __forceinline__ PairSlab(unsigned char *smem)
     {
         buf = reinterpret_cast<cplx<T> *>(smem);
-        twy = buf + M1 * S;
+        twy = buf + L * S;
         twz = twy + M1;
+        rank = 0;
+        part[0] = buf;
+        if constexpr (CL > 1) {
+            rank = cluster_rank();
+#pragma unroll
+            for (int i = 0; i < CL; i++) part[i] = cluster_map(buf, i);
+        }
     }
 
     __device__ __forceinline__ void load_tables(const cplx<T> *tw, int m0) const
     {
         for (int i = threadIdx.x; i < M1 + M2; i += NT) stc(twy + i, ldc_ro(tw + m0 + i));
+    }
+
+    // all of the slab's CTAs
+    static __device__ __forceinline__ void sync()
+    {
+        if constexpr (CL > 1) {
+            pair_arrive();
+            pair_wait();
+        } else {
+            __syncthreads();
+        }
+    }
+    // after the last access to another CTA's rows
+    static __device__ __forceinline__ void finish()
+    {
+        if constexpr (CL > 1) sync();
     }
 
     // loop of a pass over COUNT butterflies
@@ -186,11 +230,12 @@ struct PairSlab : PairPlan<M1, M2> {
     // spectrum slab src -> buf, up to the last (RA-point y) pass
     __device__ __forceinline__ void inverse_passes(const cplx<T> *src, bool split = false) const
     {
-        each<M1 * RZ>([&](int b) {
-            const int y = b % M1, k1 = b / M1;
+        const cplx<T> *own = src + rank * L;
+        each<L * RZ>([&](int b) {
+            const int y = b % L, k1 = b / L;
             cplx<T> v[RC], *p = buf + y * S + RC * k1;
 #pragma unroll
-            for (int i = 0; i < RC; i++) v[i] = ldc_cg(src + i * (RZ * M1) + b);
+            for (int i = 0; i < RC; i++) v[i] = ldc_cg(own + (i * RZ + k1) * M1 + y);
             Reg<T, RC, 1>::run(v);
             stc(p, v[0]);
 #pragma unroll
@@ -199,7 +244,7 @@ struct PairSlab : PairPlan<M1, M2> {
         __syncthreads();
         if (split) pair_arrive();
         if constexpr (MERGE) {
-            each<RA * RC>([&](int b) {
+            each<RAL * RC>([&](int b) {
                 const int j = b % RC, k1 = b / RC;
                 cplx<T> v[RB][RZ], *p = buf + RB * k1 * S + j;
 #pragma unroll
@@ -219,14 +264,14 @@ struct PairSlab : PairPlan<M1, M2> {
                 }
 #pragma unroll
                 for (int i = 0; i < RB; i++) {
-                    const cplx<T> w = ldc(twy + k1 * i);
+                    const cplx<T> w = ldc(twy + (rank * RAL + k1) * i);
 #pragma unroll
                     for (int r = 0; r < RZ; r++) stc(p + i * S + RC * r, i > 0 ? cmulc(v[i][r], w) : v[i][r]);
                 }
             });
         } else {
-            each<M1 * RC>([&](int b) {
-                const int y = b % M1, j = b / M1;
+            each<L * RC>([&](int b) {
+                const int y = b % L, j = b / L;
                 cplx<T> v[RZ], *p = buf + y * S + j;
 #pragma unroll
                 for (int r = 0; r < RZ; r++) v[r] = ldc(p + RC * r);
@@ -235,7 +280,7 @@ struct PairSlab : PairPlan<M1, M2> {
                 for (int r = 0; r < RZ; r++) stc(p + RC * r, v[r]);
             });
             __syncthreads();
-            each<RA * M2>([&](int b) {
+            each<RAL * M2>([&](int b) {
                 const int z = b % M2, k1 = b / M2;
                 cplx<T> v[RB], *p = buf + RB * k1 * S + z;
 #pragma unroll
@@ -243,10 +288,10 @@ struct PairSlab : PairPlan<M1, M2> {
                 Reg<T, RB, 1>::run(v);
                 stc(p, v[0]);
 #pragma unroll
-                for (int i = 1; i < RB; i++) stc(p + i * S, cmulc(v[i], ldc(twy + k1 * i)));
+                for (int i = 1; i < RB; i++) stc(p + i * S, cmulc(v[i], ldc(twy + (rank * RAL + k1) * i)));
             });
         }
-        __syncthreads();
+        sync();
     }
 
     // The RA-point y passes around real space: butterfly (z, j) holds the points
@@ -258,19 +303,19 @@ struct PairSlab : PairPlan<M1, M2> {
     template <bool INV, bool FWD, class F>
     __device__ __forceinline__ void real_space(F f) const
     {
-        each<RB * M2>([&](int b) {
-            const int z = b % M2, j = b / M2;
-            cplx<T> v[RA], *p = buf + j * S + z;
+        each<RB * M2 / CL>([&](int b) {
+            const int z = rank * (M2 / CL) + b % (M2 / CL), j = b / (M2 / CL), at = j * S + z;
+            cplx<T> v[RA];
             if (INV) {
 #pragma unroll
-                for (int r = 0; r < RA; r++) v[r] = ldc(p + RB * r * S);
+                for (int r = 0; r < RA; r++) v[r] = ldc(part[r / RAL] + at + RB * (r % RAL) * S);
                 Reg<T, RA, 1>::run(v);
             }
-            f(v, b);
+            f(v, j * M2 + z);
             if (FWD) {
                 Reg<T, RA, -1>::run(v);
 #pragma unroll
-                for (int r = 0; r < RA; r++) stc(p + RB * r * S, v[r]);
+                for (int r = 0; r < RA; r++) stc(part[r / RAL] + at + RB * (r % RAL) * S, v[r]);
             }
         });
     }
@@ -278,14 +323,14 @@ struct PairSlab : PairPlan<M1, M2> {
     // buf after the first forward y pass -> spectrum slab dst
     __device__ __forceinline__ void forward_passes(cplx<T> *dst, bool split, bool last) const
     {
-        __syncthreads();
+        sync();
         if constexpr (MERGE) {
-            each<RA * RC>([&](int b) {
+            each<RAL * RC>([&](int b) {
                 const int j = b % RC, k1 = b / RC;
                 cplx<T> v[RB][RZ], *p = buf + RB * k1 * S + j;
 #pragma unroll
                 for (int i = 0; i < RB; i++) {
-                    const cplx<T> w = ldc(twy + k1 * i);
+                    const cplx<T> w = ldc(twy + (rank * RAL + k1) * i);
 #pragma unroll
                     for (int r = 0; r < RZ; r++) {
                         v[i][r] = ldc(p + i * S + RC * r);
@@ -309,19 +354,19 @@ struct PairSlab : PairPlan<M1, M2> {
                 }
             });
         } else {
-            each<RA * M2>([&](int b) {
+            each<RAL * M2>([&](int b) {
                 const int z = b % M2, k1 = b / M2;
                 cplx<T> v[RB], *p = buf + RB * k1 * S + z;
                 v[0] = ldc(p);
 #pragma unroll
-                for (int i = 1; i < RB; i++) v[i] = cmul(ldc(p + i * S), ldc(twy + k1 * i));
+                for (int i = 1; i < RB; i++) v[i] = cmul(ldc(p + i * S), ldc(twy + (rank * RAL + k1) * i));
                 Reg<T, RB, -1>::run(v);
 #pragma unroll
                 for (int i = 0; i < RB; i++) stc(p + i * S, v[i]);
             });
             __syncthreads();
-            each<M1 * RC>([&](int b) {
-                const int y = b % M1, j = b / M1;
+            each<L * RC>([&](int b) {
+                const int y = b % L, j = b / L;
                 cplx<T> v[RZ], *p = buf + y * S + j;
 #pragma unroll
                 for (int r = 0; r < RZ; r++) v[r] = ldc(p + RC * r);
@@ -333,15 +378,16 @@ struct PairSlab : PairPlan<M1, M2> {
         __syncthreads();
         if (split) pair_wait();
         if (last) pdl_trigger();
-        each<M1 * RZ>([&](int b) {
-            const int y = b % M1, k1 = b / M1;
+        cplx<T> *own = dst + rank * L;
+        each<L * RZ>([&](int b) {
+            const int y = b % L, k1 = b / L;
             cplx<T> v[RC], *p = buf + y * S + RC * k1;
             v[0] = ldc(p);
 #pragma unroll
             for (int i = 1; i < RC; i++) v[i] = cmul(ldc(p + i), ldc(twz + k1 * i));
             Reg<T, RC, -1>::run(v);
 #pragma unroll
-            for (int i = 0; i < RC; i++) stc(dst + i * (RZ * M1) + b, v[i]);
+            for (int i = 0; i < RC; i++) stc(own + (i * RZ + k1) * M1 + y, v[i]);
         });
     }
 };
@@ -411,6 +457,8 @@ struct PairSlabAny {
         twy = buf + q.m1 * q.S;
         twz = twy + q.m1;
     }
+    static __device__ __forceinline__ void sync() { __syncthreads(); }
+    static __device__ __forceinline__ void finish() {}
     __device__ __forceinline__ int row() const { return q.rb * q.m2; }
     __device__ __forceinline__ int area() const { return q.m1 * q.m2; }
 
@@ -510,6 +558,7 @@ __device__ __forceinline__ void pair_mid_body(const PS &B, const PropsArgs<doubl
                 stc(P + o + row * r, cplx<T>{v[r].x * (e0 * e0), v[r].y * (e1 * e1)});
             }
         });
+        B.finish();
     }
 }
 
@@ -559,6 +608,7 @@ __device__ __forceinline__ void pair_combine_body(const PS &B, const PropsArgs<d
         };
         if (!next) {
             B.template real_space<true, false>(finish);
+            B.finish();
             return;
         }
         B.template real_space<true, true>([&](cplx<T> *v, int o) {
@@ -592,13 +642,13 @@ __device__ __forceinline__ void pair_combine_body(const PS &B, const PropsArgs<d
                 v[r].y *= e1;
             }
         };
+        B.sync();  // every CTA of the slab runs before its rows are written
         B.template real_space<false, true>(start);
-        if (!next) return;
     }
     B.forward_passes(half == 1 ? specB : specA, half >= 0 && mode == 0, half >= 0);
     if (half >= 0) return;
     // full step input E2' q', from the slice this thread has just stored
-    __syncthreads();
+    B.sync();
     B.template real_space<false, true>([&](cplx<T> *v, int o) {
 #pragma unroll
         for (int r = 0; r < PS::RA; r++) {

@@ -11,7 +11,7 @@ import scft_string_b200 as S
 pytestmark = pytest.mark.gpu
 
 GRIDS = [(16, 16, 16), (24, 24, 24), (40, 40, 40), (80, 80, 80), (16, 64, 64), (96, 24, 24), (80, 64, 96),
-         (128, 16, 16), (24, 96, 96), (48, 48, 48),
+         (128, 16, 16), (24, 96, 96), (48, 48, 48), (8, 128, 128),
          # run-time sizes: every radix, prime axes, the smallest ones, one column left over
          (35, 54, 45), (2, 2, 2), (3, 5, 7), (9, 100, 98), (6, 15, 16), (112, 14, 12), (10, 3, 3),
          (30, 108, 112), (64, 25, 27), (1, 12, 10), (12, 1, 10), (12, 10, 1), (4, 125, 6)]
