@@ -1396,19 +1396,22 @@ int run_op(int op, const PropsArgs<T> *a, const PropsLaunch &L, int n, cudaStrea
 template <typename T>
 int dispatch(int op, const PropsArgs<T> *a, const PropsLaunch &L, int n, cudaStream_t st)
 {
-    switch (L.fixed) {
-        case 32: return run_op<T, 256, 32, 32, 32>(op, a, L, n, st);
-        case 48: return run_op<T, 256, 48, 48, 48>(op, a, L, n, st);
-        case 64: return run_op<T, 256, 64, 64, 64>(op, a, L, n, st);
-        case 96: return run_op<T, 256, 96, 96, 96>(op, a, L, n, st);
-        case 128: return run_op<T, 512, 128, 128, 128>(op, a, L, n, st);
-        case 6496: return run_op<T, 256, 64, 64, 96>(op, a, L, n, st);
-        default: break;
+    if constexpr (sizeof(T) == 4) {
+        switch (L.fixed) {
+            case 32: return run_op<T, 256, 32, 32, 32>(op, a, L, n, st);
+            case 48: return run_op<T, 256, 48, 48, 48>(op, a, L, n, st);
+            case 64: return run_op<T, 256, 64, 64, 64>(op, a, L, n, st);
+            case 96: return run_op<T, 256, 96, 96, 96>(op, a, L, n, st);
+            case 128: return run_op<T, 512, 128, 128, 128>(op, a, L, n, st);
+            case 6496: return run_op<T, 256, 64, 64, 96>(op, a, L, n, st);
+            default: break;
+        }
     }
     return L.big ? run_op<T, 1024, 0, 0, 0>(op, a, L, n, st) : run_op<T, 256, 0, 0, 0>(op, a, L, n, st);
 }
 
-// compile-time shape id for a grid (0: runtime-shaped kernels)
+// compile-time shape id of an FP32 grid (0: runtime-shaped kernels); the FP64
+// grids of these shapes run the kernels of pair.cu
 int fixed_shape_id(int m0, int m1, int m2)
 {
     if (m0 == m1 && m1 == m2 && (m0 == 32 || m0 == 48 || m0 == 64 || m0 == 96 || m0 == 128)) return m0;

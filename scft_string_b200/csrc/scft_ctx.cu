@@ -680,7 +680,7 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
     L.pencil_threads = std::min(1024, std::max(128, round32(threads_for(g.px, g.tc))));
     L.big = (L.slab_threads > 256 || L.pencil_threads > 256) ? 1 : 0;
     const int rt_slab_threads = L.slab_threads, rt_pencil_threads = L.pencil_threads;
-    L.fixed = fixed_shape_id(g.m0, g.m1, g.m2);
+    L.fixed = T == 4 ? fixed_shape_id(g.m0, g.m1, g.m2) : 0;
     if (L.fixed) L.slab_threads = L.pencil_threads = fixed_shape_threads(L.fixed);
     // 64^3 FP32: the register-resident step kernels (reg64.cu) with SCFT_REG64=1;
     // the shared-memory kernels otherwise (measured faster on a B200)
@@ -757,7 +757,8 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
         CKC(cudaMalloc(&ctx->hist, ctx->nostore ? T * 2 * M : T * 2 * M * (size_t)(g.Ns + 1) * S));
         CKC(cudaMalloc(&ctx->spec, T * 2 * 4 * (size_t)g.Mk * S));
         CKC(cudaMalloc(&ctx->pbuf, T * 2 * M * S));
-        if (L.reg || L.fixed) {  // counters of the persistent step launch
+        L.pair = T == 8 && pair_applicable(g.m0, g.m1, g.m2);
+        if (L.reg || L.fixed || L.pair) {  // counters of the persistent step launch
             ctx->sync_stride = reg64_sync_ints(g.Ns, (int)S);
             CKC(cudaMalloc(&ctx->sync, sizeof(int) * 2 * (size_t)ctx->sync_stride));
         }
@@ -846,7 +847,6 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
             L.step_grid = reg64_step_grid();
             L.persist = 1;
         }
-        L.pair = T == 8 && pair_applicable(g.m0, g.m1, g.m2);
         if (L.pair && pair_setup(g.m0, g.m1, g.m2, &L.step_grid_pair) != 0) {
             ctx->lasterr = "cudaFuncSetAttribute(max dynamic shared memory) failed";
             rc = SCFT_CUDA_ERROR;
