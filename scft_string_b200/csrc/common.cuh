@@ -41,12 +41,31 @@ __device__ __forceinline__ cplx<T> csub(cplx<T> a, cplx<T> b)
 constexpr int kMaxStages = 12;
 constexpr int kPairLanes = 8;  // slab pack/unpack: mk2 <= 32*kPairLanes
 
+// Quotients by a run-time divisor n: b / n = umulhi(b, mag), mag = floor(2^32/n)
+// + 1 (0 for n = 1), exact while b n < 2^32.  A 32-bit division is about 20
+// instructions; the run-time shaped transforms take several per butterfly.
+__host__ __device__ __forceinline__ unsigned div_mag(int n) { return n > 1 ? 0xffffffffu / (unsigned)n + 1u : 0u; }
+__device__ __forceinline__ int div_by(int b, unsigned mag) { return mag ? (int)__umulhi((unsigned)b, mag) : b; }
+
 // Mixed-radix factorisation of one FFT length (radices 2, 3, 4, 5, 7, 8).
 struct Plan1D {
     int n;
     int nst;
     int radix[kMaxStages];
+    unsigned mag_nr[kMaxStages], mag_ns[kMaxStages];  // div_mag of n / radix and of the accumulated size, per stage
+    int tw_step[kMaxStages];                          // twiddle table stride of the stage
 };
+
+inline void plan_mags(Plan1D &p)
+{
+    int ns = 1;
+    for (int s = 0; s < p.nst; s++) {
+        p.mag_nr[s] = div_mag(p.n / p.radix[s]);
+        p.mag_ns[s] = div_mag(ns);
+        ns *= p.radix[s];
+        p.tw_step[s] = p.n / ns;
+    }
+}
 
 // Everything a propagator kernel needs to know about the grid.
 struct Geo {

@@ -147,18 +147,22 @@ struct Slots {
     static constexpr int value = kStageBudget / R;
 };
 
-// One Stockham stage over `nlines` lines of length n.  Element i of line l is
+// One Stockham stage (sign SIGN) over `nlines` lines of length n; buf and tw are
+// in shared memory.  Element i of line l is
 // buf[l*ls + i*es].  line_fast selects the butterfly->thread order: consecutive
 // threads walk lines (good when ls == 1) or butterflies (good when es == 1).
-template <typename T, int R>
+template <typename T, int R, int SIGN>
 __device__ __noinline__ void fft_stage(cplx<T> *__restrict__ buf, int n, int nlines, int es,
                                      int ls, bool line_fast, int Ns,
-                                     const cplx<T> *__restrict__ tw, int sign, int *err)
+                                     const cplx<T> *__restrict__ tw, int *err, unsigned mag_lines,
+                                     unsigned mag_nr, unsigned mag_ns, int tstep)
 {
+    __builtin_assume(__isShared(buf));
+    __builtin_assume(__isShared(tw));
     constexpr int SL = Slots<R>::value;
-    const int nR = n / R;
+    constexpr int sign = SIGN;
+    const int nR = R == 8 ? n >> 3 : R == 4 ? n >> 2 : R == 2 ? n >> 1 : n / R;
     const int nb = nlines * nR;
-    const int tstep = n / (Ns * R);
     const int nthr = blockDim.x;
     cplx<T> v[SL][R];
 #pragma unroll
@@ -167,13 +171,13 @@ __device__ __noinline__ void fft_stage(cplx<T> *__restrict__ buf, int n, int nli
         if (b < nb) {
             int line, j;
             if (line_fast) {
-                line = b % nlines;
-                j = b / nlines;
+                j = div_by(b, mag_lines);
+                line = b - j * nlines;
             } else {
-                j = b % nR;
-                line = b / nR;
+                line = div_by(b, mag_nr);
+                j = b - line * nR;
             }
-            const int k = j % Ns;
+            const int k = j - div_by(j, mag_ns) * Ns;
             const cplx<T> *src = buf + line * ls + j * es;
 #pragma unroll
             for (int r = 0; r < R; r++) {
@@ -195,13 +199,13 @@ __device__ __noinline__ void fft_stage(cplx<T> *__restrict__ buf, int n, int nli
         if (b < nb) {
             int line, j;
             if (line_fast) {
-                line = b % nlines;
-                j = b / nlines;
+                j = div_by(b, mag_lines);
+                line = b - j * nlines;
             } else {
-                j = b % nR;
-                line = b / nR;
+                line = div_by(b, mag_nr);
+                j = b - line * nR;
             }
-            const int k = j % Ns;
+            const int k = j - div_by(j, mag_ns) * Ns;
             cplx<T> *dst = buf + line * ls + ((j - k) * R + k) * es;
 #pragma unroll
             for (int r = 0; r < R; r++) dst[r * Ns * es] = v[sl][r];
@@ -215,15 +219,26 @@ __device__ void cta_fft(cplx<T> *buf, const Plan1D &p, int nlines, int es, int l
                         const cplx<T> *tw, int sign, int *err)
 {
     int Ns = 1;
+    const unsigned ml = div_mag(nlines);
     for (int st = 0; st < p.nst; st++) {
         const int R = p.radix[st];
+        const unsigned mr = p.mag_nr[st], ms = p.mag_ns[st];
+        const int step = p.tw_step[st];
         switch (R) {
-            case 8: fft_stage<T, 8>(buf, p.n, nlines, es, ls, line_fast, Ns, tw, sign, err); break;
-            case 4: fft_stage<T, 4>(buf, p.n, nlines, es, ls, line_fast, Ns, tw, sign, err); break;
-            case 2: fft_stage<T, 2>(buf, p.n, nlines, es, ls, line_fast, Ns, tw, sign, err); break;
-            case 3: fft_stage<T, 3>(buf, p.n, nlines, es, ls, line_fast, Ns, tw, sign, err); break;
-            case 5: fft_stage<T, 5>(buf, p.n, nlines, es, ls, line_fast, Ns, tw, sign, err); break;
-            case 7: fft_stage<T, 7>(buf, p.n, nlines, es, ls, line_fast, Ns, tw, sign, err); break;
+#define SCFT_STAGE(Q)                                                                                              \
+    case Q:                                                                                                        \
+        if (sign < 0)                                                                                              \
+            fft_stage<T, Q, -1>(buf, p.n, nlines, es, ls, line_fast, Ns, tw, err, ml, mr, ms, step);               \
+        else                                                                                                       \
+            fft_stage<T, Q, 1>(buf, p.n, nlines, es, ls, line_fast, Ns, tw, err, ml, mr, ms, step);                \
+        break;
+            SCFT_STAGE(8)
+            SCFT_STAGE(4)
+            SCFT_STAGE(2)
+            SCFT_STAGE(3)
+            SCFT_STAGE(5)
+            SCFT_STAGE(7)
+#undef SCFT_STAGE
             default: *err = 2; return;
         }
         Ns *= R;

@@ -60,6 +60,7 @@ bool factor7(int n, Plan1D &p)
             p.radix[p.nst++] = R;
             rem /= R;
         }
+    plan_mags(p);
     return rem == 1;
 }
 

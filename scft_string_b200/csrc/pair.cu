@@ -156,28 +156,6 @@ constexpr int step_smem()
                                                                    : PairPencil<M0, TC>::SMEM;
 }
 
-// Launch of a step kernel: it may start while the kernel before it on the
-// stream finishes (see pdl_wait), in clusters of (cx, cy) CTAs.
-template <class... Args>
-void launch_step(void (*fn)(Args...), dim3 grid, int threads, int smem, int cx, int cy, cudaStream_t st, Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = cx;
-    at[1].val.clusterDim.y = cy;
-    at[1].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = cx * cy > 1 ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, fn, args...);
-}
-
 // CTAs per slab: one where the slab fits a CTA's shared memory.  Two were slower
 // on every shape that fits (one replica step: 64^3 34.2 us with one, 37.1 with
 // two; 48^3 22.9 and 27.3; 96^3 84.9 and 91.6).

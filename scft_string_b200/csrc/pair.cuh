@@ -31,6 +31,7 @@
 #include "common.cuh"
 #include "dft.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace scft {
 
@@ -67,27 +68,6 @@ __device__ __forceinline__ double third(double x)
     const double q = x * c;
     const double r = fma(fma(-3.0, q, x), c, q);
     return fabs(q) <= big ? r : q;
-}
-
-// Programmatic dependent launch: the kernels of a step let the next one start
-// as their last CTAs run (its CTAs set up and read constant tables), and wait
-// here for the whole previous kernel before they touch what it wrote.  Both are
-// no-ops in a kernel launched without the attribute.
-__device__ __forceinline__ void pdl_trigger()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void pdl_wait()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-// asks for `bytes` at p to be brought into L2; a hint, no wait.  The copy engine
-// wants 16-byte multiples; slabs of an odd number of doubles go without.
-__device__ __forceinline__ void prefetch_l2(const void *p, int bytes)
-{
-    if (((unsigned)(size_t)p | (unsigned)bytes) & 15u) return;
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
 // the two CTAs of a split combine: each has read its input slab (arrive) before

@@ -1,0 +1,52 @@
+// pdl.cuh -- overlap of the launches of a contour step: programmatic dependent
+// launch, L2 prefetch, and the launch call that both take.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace scft {
+
+// Programmatic dependent launch: the kernels of a step let the next one start
+// as their last CTAs run (its CTAs set up and read constant tables), and wait
+// here for the whole previous kernel before they touch what it wrote.  Both are
+// no-ops in a kernel launched without the attribute.
+__device__ __forceinline__ void pdl_trigger()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// asks for `bytes` at p to be brought into L2; a hint, no wait.  The copy engine
+// wants 16-byte multiples; slabs of an odd number of doubles go without.
+__device__ __forceinline__ void prefetch_l2(const void *p, int bytes)
+{
+    if (((unsigned)(size_t)p | (unsigned)bytes) & 15u) return;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+// Launch of a step kernel: it may start while the kernel before it on the
+// stream finishes (see pdl_wait), in clusters of (cx, cy) CTAs.
+template <class... Params, class... Args>
+inline void launch_step(void (*fn)(Params...), dim3 grid, int threads, int smem, int cx, int cy, cudaStream_t st,
+                        const Args &...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cx;
+    at[1].val.clusterDim.y = cy;
+    at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cx * cy > 1 ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, fn, Params(args)...);
+}
+
+}  // namespace scft

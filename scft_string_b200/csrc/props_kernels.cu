@@ -18,6 +18,7 @@
 #include "common.cuh"
 #include "fft.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 #include "tma.cuh"
 #include "step_order.cuh"
 
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     const int m0 = FX ? FM0 : g.m0, M = m0 * m1 * m2, Mk = m0 * m1 * mk2;
     const int slab_c = m1 * mk2 + m2 + 32;
     const int nthr = FX ? MT : (int)blockDim.x;
+    const unsigned mag = FX ? 0 : div_mag(m2);
     cplx<T> *buf = reinterpret_cast<cplx<T> *>(smem_raw);
     cplx<T> *twy = buf + slab_c;
     cplx<T> *twz = twy + m1;
@@ -141,6 +143,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     T *qn = a.hist + hist_off<T>(g, slot, sn, fld) + slab_r;
     const int npair = (m1 + 1) / 2, npz = npair * m2;
 
+    pdl_wait();
     if (mode == 0) {
         for (int i = threadIdx.x; i < m1 * mk2; i += nthr) buf[i] = specA[slab_k + i];
         __syncthreads();
@@ -148,7 +151,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
         const T *E4 = etab_ptr(a, slot, etab_sel(g, fld, s)) + slab_r;
         const T *P = a.pbuf + ((size_t)slot * 2 + fld) * M + slab_r;
         for (int e = threadIdx.x; e < npz; e += nthr) {
-            const int p = e / m2, z = e - p * m2;
+            const int p = FX ? e / m2 : div_by(e, mag), z = e - p * m2;
             cplx<T> &c = buf[prow<FM2>(p, mk2) + z];
             const int r0 = 2 * p * m2 + z;
             // Richardson, GPU_kernels.h:199-203
@@ -164,7 +167,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
         }
     } else if (mode == 1) {
         for (int e = threadIdx.x; e < npz; e += nthr) {
-            const int p = e / m2, z = e - p * m2;
+            const int p = FX ? e / m2 : div_by(e, mag), z = e - p * m2;
             const int r0 = 2 * p * m2 + z;
             const bool hb = 2 * p + 1 < m1;
             buf[prow<FM2>(p, mk2) + z] = {(T)1, hb ? (T)1 : (T)0};
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
         }
     } else {
         for (int e = threadIdx.x; e < npz; e += nthr) {
-            const int p = e / m2, z = e - p * m2;
+            const int p = FX ? e / m2 : div_by(e, mag), z = e - p * m2;
             const int r0 = 2 * p * m2 + z;
             const bool hb = 2 * p + 1 < m1;
             buf[prow<FM2>(p, mk2) + z] = {qn[r0], hb ? qn[r0 + m2] : (T)0};
@@ -184,7 +187,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     const T *E4n = etab_ptr(a, slot, etab_sel(g, fld, sn)) + slab_r;
     // half step input E4' q'
     for (int e = threadIdx.x; e < npz; e += nthr) {
-        const int p = e / m2, z = e - p * m2;
+        const int p = FX ? e / m2 : div_by(e, mag), z = e - p * m2;
         cplx<T> &c = buf[prow<FM2>(p, mk2) + z];
         const int r0 = 2 * p * m2 + z;
         c.x *= E4n[r0];
@@ -196,7 +199,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     __syncthreads();
     // full step input E2' q' (q' re-read from the propagator store written above)
     for (int e = threadIdx.x; e < npz; e += nthr) {
-        const int p = e / m2, z = e - p * m2;
+        const int p = FX ? e / m2 : div_by(e, mag), z = e - p * m2;
         const int r0 = 2 * p * m2 + z;
         const T e0 = E4n[r0];
         T v0 = qn[r0] * (e0 * e0), v1 = (T)0;
@@ -208,6 +211,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     }
     __syncthreads();
     slab_fwd<T, MT, FM1, FM2>(buf, g, twy, twz, a.err);
+    pdl_trigger();
     for (int i = threadIdx.x; i < m1 * mk2; i += nthr) specB[slab_k + i] = buf[i];
 }
 
@@ -222,6 +226,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     const int m0 = FX ? FM0 : g.m0, M = m0 * m1 * m2, Mk = m0 * m1 * mk2;
     const int slab_c = m1 * mk2 + m2 + 32;
     const int nthr = FX ? MT : (int)blockDim.x;
+    const unsigned mag = FX ? 0 : div_mag(m2);
     cplx<T> *buf = reinterpret_cast<cplx<T> *>(smem_raw);
     cplx<T> *twy = buf + slab_c;
     cplx<T> *twz = twy + m1;
@@ -237,11 +242,12 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     const int npz = ((m1 + 1) / 2) * m2;
 
     // full step: P = E2 * qs1
+    pdl_wait();
     for (int i = threadIdx.x; i < m1 * mk2; i += nthr) buf[i] = specB[slab_k + i];
     __syncthreads();
     slab_inv<T, MT, FM1, FM2>(buf, g, twy, twz, a.err);
     for (int e = threadIdx.x; e < npz; e += nthr) {
-        const int p = e / m2, z = e - p * m2;
+        const int p = FX ? e / m2 : div_by(e, mag), z = e - p * m2;
         const cplx<T> c = buf[prow<FM2>(p, mk2) + z];
         const int r0 = 2 * p * m2 + z;
         const T e0 = E4[r0];
@@ -257,7 +263,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     __syncthreads();
     slab_inv<T, MT, FM1, FM2>(buf, g, twy, twz, a.err);
     for (int e = threadIdx.x; e < npz; e += nthr) {
-        const int p = e / m2, z = e - p * m2;
+        const int p = FX ? e / m2 : div_by(e, mag), z = e - p * m2;
         cplx<T> &c = buf[prow<FM2>(p, mk2) + z];
         const int r0 = 2 * p * m2 + z;
         const T e0 = E4[r0];
@@ -271,6 +277,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     }
     __syncthreads();
     slab_fwd<T, MT, FM1, FM2>(buf, g, twy, twz, a.err);
+    pdl_trigger();
     for (int i = threadIdx.x; i < m1 * mk2; i += nthr) specA[slab_k + i] = buf[i];
 }
 
@@ -289,29 +296,32 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     const int m1 = FX ? FM1 : g.m1, mk2 = (FX ? FM2 : g.m2) / 2 + 1;
     const int Mk = m0 * m1 * mk2;
     const int nthr = FX ? MT : (int)blockDim.x;
+    const unsigned mag = FX ? 0 : div_mag(tc), mag_k = FX ? 0 : div_mag(mk2);
     cplx<T> *buf = reinterpret_cast<cplx<T> *>(smem_raw);
     cplx<T> *twx = buf + tc * m0;
     T *colf = reinterpret_cast<T *>(twx + m0);
     T *gx = colf + tc;
     for (int i = threadIdx.x; i < m0; i += nthr) twx[i] = a.tw[i];
-    const int tile = blockIdx.x, fld = blockIdx.y, slot = blockIdx.z;
+    // opposite order of the slab kernels before and after: what they touched last is still in L2
+    const int tile = gridDim.x - 1 - blockIdx.x, fld = gridDim.y - 1 - blockIdx.y, slot = gridDim.z - 1 - blockIdx.z;
     const int ncol = m1 * mk2;
     const int c0 = tile * tc;
     const T *kf = a.kfac + (size_t)a.slot_rep[slot] * a.kf_stride;  // the replica's box
     for (int t = threadIdx.x; t < tc; t += nthr) {
         const int c = c0 + t;
-        const int y = c / mk2, kz = c - y * mk2;
+        const int y = FX ? c / mk2 : div_by(c, mag_k), kz = c - y * mk2;
         colf[t] = c < ncol ? kf[m0 + y] * kf[m0 + m1 + kz] : (T)0;
     }
     for (int i = threadIdx.x; i < m0; i += nthr) gx[i] = kf[i];
     const T invM = a.invM;
     cplx<T> *spec = a.spec + ((size_t)slot * 2 + fld) * 2 * Mk;
     const int npass = both ? 2 : 1;
+    pdl_wait();
     for (int pass = 0; pass < npass; pass++) {
         cplx<T> *sp = spec + (size_t)pass * Mk;
         __syncthreads();
         for (int e = threadIdx.x; e < tc * m0; e += nthr) {
-            const int x = e / tc, t = e - x * tc;
+            const int x = FX ? e / tc : div_by(e, mag), t = e - x * tc;
             const int c = c0 + t;
             buf[e] = c < ncol ? sp[(size_t)x * ncol + c] : cplx<T>{(T)0, (T)0};
         }
@@ -321,7 +331,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
         else
             cta_fft(buf, g.px, tc, tc, 1, true, twx, -1, a.err);
         for (int e = threadIdx.x; e < tc * m0; e += nthr) {
-            const int x = e / tc, t = e - x * tc;
+            const int x = FX ? e / tc : div_by(e, mag), t = e - x * tc;
             const T k2 = gx[x] * colf[t];
             // pass 0: K2 = g/M ; pass 1: K1 = g^2/M  (Prepare_dev_expKsq2_expKsq, GPU_kernels.h:207-213)
             const T f = pass == 0 ? k2 * invM : (k2 * invM) * (k2 * invM) * a.Mreal;
@@ -333,8 +343,9 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
             fft_fixed<T, FM0, TCF, TCF, 1, true, MT>(buf, twx, +1);
         else
             cta_fft(buf, g.px, tc, tc, 1, true, twx, +1, a.err);
+        if (pass == npass - 1) pdl_trigger();
         for (int e = threadIdx.x; e < tc * m0; e += nthr) {
-            const int x = e / tc, t = e - x * tc;
+            const int x = FX ? e / tc : div_by(e, mag), t = e - x * tc;
             const int c = c0 + t;
             if (c < ncol) sp[(size_t)x * ncol + c] = buf[e];
         }
@@ -383,10 +394,11 @@ __device__ __forceinline__ void mid_pf_body(const PropsArgs<T> &a, int s, int x,
     if (threadIdx.x == 0) {
         for (int i = 0; i < 3; i++) mbar_init(&bars[i], 1);
         mbar_fence_init();
+        mbar_expect_tx(&bars[1], L::REAL_BYTES);
+        bulk_g2s(E4s, E4g, L::REAL_BYTES, &bars[1]);  // constant over the chain
+        pdl_wait();
         mbar_expect_tx(&bars[0], L::SPEC_BYTES);
         bulk_g2s(bufB, specB + slab_k, L::SPEC_BYTES, &bars[0]);
-        mbar_expect_tx(&bars[1], L::REAL_BYTES);
-        bulk_g2s(E4s, E4g, L::REAL_BYTES, &bars[1]);
         mbar_expect_tx(&bars[2], L::SPEC_BYTES);
         bulk_g2s(bufA, specA + slab_k, L::SPEC_BYTES, &bars[2]);
     }
@@ -426,6 +438,7 @@ __device__ __forceinline__ void mid_pf_body(const PropsArgs<T> &a, int s, int x,
     }
     __syncthreads();
     slab_forward_fixed<T, m1, m2, MT>(bufA, twy, twz);
+    pdl_trigger();
     for (int i = threadIdx.x; i < m1 * mk2; i += MT) specA[slab_k + i] = bufA[i];
 }
 
@@ -459,6 +472,11 @@ __device__ __forceinline__ void combine_pf_body(const PropsArgs<T> &a, int s, in
     if (threadIdx.x == 0) {
         for (int i = 0; i < 3; i++) mbar_init(&bars[i], 1);
         mbar_fence_init();
+        if (mode == 0 || next) {
+            mbar_expect_tx(&bars[2], L::REAL_BYTES);
+            bulk_g2s(E, etab_ptr(a, slot, sel_s) + slab_r, L::REAL_BYTES, &bars[2]);  // constant over the chain
+        }
+        pdl_wait();
         if (mode == 0) {
             mbar_expect_tx(&bars[0], L::SPEC_BYTES);
             bulk_g2s(buf, specA + slab_k, L::SPEC_BYTES, &bars[0]);
@@ -467,10 +485,6 @@ __device__ __forceinline__ void combine_pf_body(const PropsArgs<T> &a, int s, in
         } else if (mode == 2) {
             mbar_expect_tx(&bars[1], L::REAL_BYTES);
             bulk_g2s(Q, qn, L::REAL_BYTES, &bars[1]);
-        }
-        if (mode == 0 || next) {
-            mbar_expect_tx(&bars[2], L::REAL_BYTES);
-            bulk_g2s(E, etab_ptr(a, slot, sel_s) + slab_r, L::REAL_BYTES, &bars[2]);
         }
     }
     for (int i = threadIdx.x; i < m1; i += MT) twy[i] = a.tw[FM0 + i];
@@ -533,6 +547,7 @@ __device__ __forceinline__ void combine_pf_body(const PropsArgs<T> &a, int s, in
     }
     __syncthreads();
     slab_forward_fixed<T, m1, m2, MT>(buf, twy, twz);
+    pdl_trigger();
     for (int i = threadIdx.x; i < m1 * mk2; i += MT) specB[slab_k + i] = buf[i];
 }
 
@@ -562,6 +577,7 @@ __device__ __forceinline__ void pencil_tma_body(const CUtensorMap &tmap, const P
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
         mbar_fence_init();
+        pdl_wait();
         mbar_expect_tx(&bars[0], BOX_BYTES);
         tma_load_2d(bufA, &tmap, x, y0, &bars[0]);
         if (both) {
@@ -596,6 +612,7 @@ __device__ __forceinline__ void pencil_tma_body(const CUtensorMap &tmap, const P
         });
         fence_proxy_async_smem();
         __syncthreads();
+        if (pass == npass - 1) pdl_trigger();
         if (threadIdx.x == 0) tma_store_2d(&tmap, x, y0 + pass * m0, buf);
     }
     if (threadIdx.x == 0) tma_store_wait_read();
@@ -606,7 +623,9 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1)
     k_pencil_tma(const __grid_constant__ CUtensorMap tmap, PropsArgs<T> a, int both)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    pencil_tma_body<T, MT, FM0, FM1, FM2, TC>(tmap, a, both, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
+    // opposite order of the slab kernels before and after: what they touched last is still in L2
+    pencil_tma_body<T, MT, FM0, FM1, FM2, TC>(tmap, a, both, gridDim.x - 1 - blockIdx.x, gridDim.y - 1 - blockIdx.y,
+                                              gridDim.z - 1 - blockIdx.z, smem_raw);
 }
 
 // ---------------------------------------------------------------- shuffle pencil (m0 = 64)
@@ -1130,11 +1149,11 @@ void launch_combine(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gs, int s,
     }
     if constexpr (F1 != 0) {
         if (L.pf) {
-            k_combine_pf<T, MT, F0, F1, F2><<<gs, MT, L.combine_pf_smem, st>>>(a, s, mode);
+            launch_step(k_combine_pf<T, MT, F0, F1, F2>, gs, MT, L.combine_pf_smem, 1, 1, st, a, s, mode);
             return;
         }
     }
-    k_combine<T, MT, F0, F1, F2><<<gs, L.slab_threads, L.slab_smem, st>>>(a, s, mode);
+    launch_step(k_combine<T, MT, F0, F1, F2>, gs, L.slab_threads, L.slab_smem, 1, 1, st, a, s, mode);
 }
 
 template <typename T, int MT, int F0, int F1, int F2>
@@ -1154,11 +1173,11 @@ void launch_mid(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gs, int s, cud
     }
     if constexpr (F1 != 0) {
         if (L.pf) {
-            k_mid_pf<T, MT, F0, F1, F2><<<gs, MT, L.mid_pf_smem, st>>>(a, s);
+            launch_step(k_mid_pf<T, MT, F0, F1, F2>, gs, MT, L.mid_pf_smem, 1, 1, st, a, s);
             return;
         }
     }
-    k_mid<T, MT, F0, F1, F2><<<gs, L.slab_threads, L.slab_smem, st>>>(a, s);
+    launch_step(k_mid<T, MT, F0, F1, F2>, gs, L.slab_threads, L.slab_smem, 1, 1, st, a, s);
 }
 
 template <typename T, int MT, int F0, int F1, int F2>
@@ -1193,15 +1212,15 @@ void launch_pencil(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gp, int bot
                 }
             }
             if (L.ptile_wide)
-                k_pencil_tma<T, MT, F0, F1, F2, 2 * TC><<<dim3((ncol + 2 * TC - 1) / (2 * TC), gp.y, gp.z), MT,
-                                                          L.pencil_tma_smem_wide, st>>>(*L.tmap_wide, a, both);
+                launch_step(k_pencil_tma<T, MT, F0, F1, F2, 2 * TC>, dim3((ncol + 2 * TC - 1) / (2 * TC), gp.y, gp.z), MT,
+                            L.pencil_tma_smem_wide, 1, 1, st, *L.tmap_wide, a, both);
             else
-                k_pencil_tma<T, MT, F0, F1, F2, TC><<<dim3((ncol + TC - 1) / TC, gp.y, gp.z), MT, L.pencil_tma_smem,
-                                                      st>>>(*L.tmap, a, both);
+                launch_step(k_pencil_tma<T, MT, F0, F1, F2, TC>, dim3((ncol + TC - 1) / TC, gp.y, gp.z), MT,
+                            L.pencil_tma_smem, 1, 1, st, *L.tmap, a, both);
             return;
         }
     }
-    k_pencil<T, MT, F0, F1, F2><<<gp, L.pencil_threads, L.pencil_smem, st>>>(a, both);
+    launch_step(k_pencil<T, MT, F0, F1, F2>, gp, L.pencil_threads, L.pencil_smem, 1, 1, st, a, both);
 }
 
 template <typename T, int MT, int F0, int F1, int F2>

@@ -43,7 +43,7 @@ bool factor(int n, Plan1D &p)
             p.radix[p.nst++] = R;
             rem /= R;
         }
-    // a radix-2 stage after radix 8/4 stages is better merged: 8*2 -> 4*4
+    plan_mags(p);
     return rem == 1;
 }
 

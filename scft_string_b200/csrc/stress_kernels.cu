@@ -56,6 +56,7 @@ __device__ __forceinline__ double bsum(double v, double *sh)
 template <typename T>
 __global__ void k_stress_slab_fwd(StressArgs<T> a, StressPairs P)
 {
+    const unsigned mag = div_mag(a.g.m2);
     extern __shared__ unsigned char smem_raw[];
     const Geo &g = a.g;
     cplx<T> *buf = reinterpret_cast<cplx<T> *>(smem_raw);
@@ -72,7 +73,7 @@ __global__ void k_stress_slab_fwd(StressArgs<T> a, StressPairs P)
     for (int pass = 0; pass < 2; pass++) {
         __syncthreads();
         for (int e = threadIdx.x; e < npz; e += blockDim.x) {
-            const int pp = e / m2, z = e - pp * m2;
+            const int pp = div_by(e, mag), z = e - pp * m2;
             const int r0 = 2 * pp * m2 + z;
             T e0 = E4[r0], v1 = (T)0;
             if (pass) e0 *= e0;
@@ -115,6 +116,7 @@ __global__ void k_stress_pencil1(StressArgs<T> a)
     __shared__ double sh[32];
     const Geo &g = a.g;
     const int tc = g.tc, m0 = g.m0, ncol = g.m1 * g.mk2;
+    const unsigned mag = div_mag(tc);
     cplx<T> *bx = reinterpret_cast<cplx<T> *>(smem_raw);
     cplx<T> *by = bx + tc * m0;
     cplx<T> *twx = by + tc * m0;
@@ -126,7 +128,7 @@ __global__ void k_stress_pencil1(StressArgs<T> a)
         const cplx<T> *sx = a.S2 + ((size_t)p * 2 + 0) * g.Mk, *sy = a.S2 + ((size_t)p * 2 + 1) * g.Mk;
         __syncthreads();
         for (int e = threadIdx.x; e < tc * m0; e += blockDim.x) {
-            const int xx = e / tc, t = e - xx * tc, c = c0 + t;
+            const int xx = div_by(e, mag), t = e - xx * tc, c = c0 + t;
             bx[e] = c < ncol ? sx[(size_t)xx * ncol + c] : cplx<T>{(T)0, (T)0};
             by[e] = c < ncol ? sy[(size_t)xx * ncol + c] : cplx<T>{(T)0, (T)0};
         }
@@ -135,7 +137,7 @@ __global__ void k_stress_pencil1(StressArgs<T> a)
         cta_fft(by, g.px, tc, tc, 1, true, twx, -1, a.err);
         double acc[3] = {0, 0, 0};
         for (int e = threadIdx.x; e < tc * m0; e += blockDim.x) {
-            const int xx = e / tc, t = e - xx * tc, c = c0 + t;
+            const int xx = div_by(e, mag), t = e - xx * tc, c = c0 + t;
             if (c >= ncol) continue;
             double wi[3], K2, hw;
             dk_weights(a, xx, c, wi, K2, hw);
@@ -153,13 +155,13 @@ __global__ void k_stress_pencil1(StressArgs<T> a)
         cplx<T> *s4 = a.S4 + ((size_t)p * 2 + xy) * g.Mk, *s4p = a.S4p + ((size_t)p * 2 + xy) * g.Mk;
         __syncthreads();
         for (int e = threadIdx.x; e < tc * m0; e += blockDim.x) {
-            const int xx = e / tc, t = e - xx * tc, c = c0 + t;
+            const int xx = div_by(e, mag), t = e - xx * tc, c = c0 + t;
             bx[e] = c < ncol ? s4[(size_t)xx * ncol + c] : cplx<T>{(T)0, (T)0};
         }
         __syncthreads();
         cta_fft(bx, g.px, tc, tc, 1, true, twx, -1, a.err);
         for (int e = threadIdx.x; e < tc * m0; e += blockDim.x) {
-            const int xx = e / tc, t = e - xx * tc, c = c0 + t;
+            const int xx = div_by(e, mag), t = e - xx * tc, c = c0 + t;
             if (c < ncol) s4[(size_t)xx * ncol + c] = bx[e];
             const int yk = c / g.mk2, kz = c - yk * g.mk2;
             const T f = c < ncol ? a.kfac[xx] * a.kfac[m0 + yk] * a.kfac[m0 + g.m1 + kz] * a.invM : (T)0;
@@ -169,7 +171,7 @@ __global__ void k_stress_pencil1(StressArgs<T> a)
         __syncthreads();
         cta_fft(bx, g.px, tc, tc, 1, true, twx, +1, a.err);
         for (int e = threadIdx.x; e < tc * m0; e += blockDim.x) {
-            const int xx = e / tc, t = e - xx * tc, c = c0 + t;
+            const int xx = div_by(e, mag), t = e - xx * tc, c = c0 + t;
             if (c < ncol) s4p[(size_t)xx * ncol + c] = bx[e];
         }
     }
@@ -179,6 +181,7 @@ __global__ void k_stress_pencil1(StressArgs<T> a)
 template <typename T>
 __global__ void k_stress_slab_mid(StressArgs<T> a, StressPairs P)
 {
+    const unsigned mag = div_mag(a.g.m2);
     extern __shared__ unsigned char smem_raw[];
     const Geo &g = a.g;
     cplx<T> *buf = reinterpret_cast<cplx<T> *>(smem_raw);
@@ -196,7 +199,7 @@ __global__ void k_stress_slab_mid(StressArgs<T> a, StressPairs P)
     slab_inverse(buf, g, twy, twz, a.err);
     const int npz = g.npair * m2;
     for (int e = threadIdx.x; e < npz; e += blockDim.x) {
-        const int pp = e / m2, z = e - pp * m2;
+        const int pp = div_by(e, mag), z = e - pp * m2;
         cplx<T> &c = buf[2 * pp * mk2 + z];
         const int r0 = 2 * pp * m2 + z;
         const T e0 = E4[r0];
@@ -221,6 +224,7 @@ __global__ void k_stress_pencil2(StressArgs<T> a)
     __shared__ double sh[32];
     const Geo &g = a.g;
     const int tc = g.tc, m0 = g.m0, ncol = g.m1 * g.mk2;
+    const unsigned mag = div_mag(tc);
     cplx<T> *bx = reinterpret_cast<cplx<T> *>(smem_raw);
     cplx<T> *by = bx + tc * m0;
     cplx<T> *twx = by + tc * m0;
@@ -231,7 +235,7 @@ __global__ void k_stress_pencil2(StressArgs<T> a)
     const cplx<T> *ux = a.S4 + ((size_t)p * 2 + 0) * g.Mk, *uy = a.S4 + ((size_t)p * 2 + 1) * g.Mk;
     __syncthreads();
     for (int e = threadIdx.x; e < tc * m0; e += blockDim.x) {
-        const int xx = e / tc, t = e - xx * tc, c = c0 + t;
+        const int xx = div_by(e, mag), t = e - xx * tc, c = c0 + t;
         bx[e] = c < ncol ? wx[(size_t)xx * ncol + c] : cplx<T>{(T)0, (T)0};
         by[e] = c < ncol ? wy[(size_t)xx * ncol + c] : cplx<T>{(T)0, (T)0};
     }
@@ -240,7 +244,7 @@ __global__ void k_stress_pencil2(StressArgs<T> a)
     cta_fft(by, g.px, tc, tc, 1, true, twx, -1, a.err);
     double acc[3] = {0, 0, 0};
     for (int e = threadIdx.x; e < tc * m0; e += blockDim.x) {
-        const int xx = e / tc, t = e - xx * tc, c = c0 + t;
+        const int xx = div_by(e, mag), t = e - xx * tc, c = c0 + t;
         if (c >= ncol) continue;
         double wi[3], K2, hw;
         dk_weights(a, xx, c, wi, K2, hw);
@@ -291,15 +295,16 @@ __device__ void jn_pencil_tile(const StressArgs<T> &a, cplx<T> *bx, const cplx<T
 {
     const Geo &g = a.g;
     const int tc = g.tc, m0 = g.m0, ncol = g.m1 * g.mk2;
+    const unsigned mag = div_mag(tc);
     __syncthreads();
     for (int e = threadIdx.x; e < tc * m0; e += blockDim.x) {
-        const int xx = e / tc, t = e - xx * tc, c = c0 + t;
+        const int xx = div_by(e, mag), t = e - xx * tc, c = c0 + t;
         bx[e] = c < ncol ? src[(size_t)xx * ncol + c] : cplx<T>{(T)0, (T)0};
     }
     __syncthreads();
     cta_fft(bx, g.px, tc, tc, 1, true, twx, -1, a.err);
     for (int e = threadIdx.x; e < tc * m0; e += blockDim.x) {
-        const int xx = e / tc, t = e - xx * tc, c = c0 + t;
+        const int xx = div_by(e, mag), t = e - xx * tc, c = c0 + t;
         const int yk = c / g.mk2, kz = c - yk * g.mk2;
         T f = (T)0;
         if (c < ncol) {
@@ -312,7 +317,7 @@ __device__ void jn_pencil_tile(const StressArgs<T> &a, cplx<T> *bx, const cplx<T
     __syncthreads();
     cta_fft(bx, g.px, tc, tc, 1, true, twx, +1, a.err);
     for (int e = threadIdx.x; e < tc * m0; e += blockDim.x) {
-        const int xx = e / tc, t = e - xx * tc, c = c0 + t;
+        const int xx = div_by(e, mag), t = e - xx * tc, c = c0 + t;
         if (c < ncol) dst[(size_t)xx * ncol + c] = bx[e];
     }
 }
@@ -336,6 +341,7 @@ template <typename T>
 __device__ void jn_slab_to_real(const StressArgs<T> &a, cplx<T> *buf, const cplx<T> *twy, const cplx<T> *twz,
                                 const cplx<T> *src, T *dst)
 {
+    const unsigned mag = div_mag(a.g.m2);
     const Geo &g = a.g;
     const int m1 = g.m1, m2 = g.m2, mk2 = g.mk2;
     __syncthreads();
@@ -343,7 +349,7 @@ __device__ void jn_slab_to_real(const StressArgs<T> &a, cplx<T> *buf, const cplx
     __syncthreads();
     slab_inverse(buf, g, twy, twz, a.err);
     for (int e = threadIdx.x; e < g.npair * m2; e += blockDim.x) {
-        const int pp = e / m2, z = e - pp * m2;
+        const int pp = div_by(e, mag), z = e - pp * m2;
         const cplx<T> c = buf[2 * pp * mk2 + z];
         const int r0 = 2 * pp * m2 + z;
         dst[r0] = c.x;
@@ -354,6 +360,7 @@ __device__ void jn_slab_to_real(const StressArgs<T> &a, cplx<T> *buf, const cplx
 template <typename T>
 __global__ void k_jn_slab(StressArgs<T> a, int pass)
 {
+    const unsigned mag = div_mag(a.g.m2);
     extern __shared__ unsigned char smem_raw[];
     const Geo &g = a.g;
     cplx<T> *buf = reinterpret_cast<cplx<T> *>(smem_raw);
@@ -375,7 +382,7 @@ __global__ void k_jn_slab(StressArgs<T> a, int pass)
     const T *E4 = etab_of(a, 2) + slab_r;
     __syncthreads();
     for (int e = threadIdx.x; e < g.npair * m2; e += blockDim.x) {
-        const int pp = e / m2, z = e - pp * m2;
+        const int pp = div_by(e, mag), z = e - pp * m2;
         const int r0 = 2 * pp * m2 + z;
         const T e0 = E4[r0];
         T v1 = (T)0;
