@@ -83,18 +83,19 @@ __global__ void k_dens_final(const double *__restrict__ acc, size_t M, const dou
     }
 }
 
-// phis and the W+ residual sum into the replica's scalar record
+// phis and the W+ residual sum into the replica's scalar record; a warp per sum
 __global__ void k_dens_phis(const double *__restrict__ part, int nblk, size_t M, double *__restrict__ rs)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double v[6];
-    for (int k = 0; k < 6; k++) {
-        double t = 0;
-        for (int i = 0; i < nblk; i++) t += part[k * nblk + i];
-        v[k] = t;
-    }
-    for (int k = 0; k < 5; k++) rs[kRsPhis + k] = v[k] / (double)M;
-    rs[kRsDev2] = v[5];
+    const int k = threadIdx.x >> 5;
+    double t = 0;
+    for (int i = threadIdx.x & 31; i < nblk; i += 32) t += part[k * nblk + i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) != 0) return;
+    if (k < 5)
+        rs[kRsPhis + k] = t / (double)M;
+    else
+        rs[kRsDev2] = t;
 }
 
 }  // namespace
@@ -110,7 +111,7 @@ int launch_density_final(const double *acc, size_t M, double *rs_row, double ds,
                          double *part, int nblk, cudaStream_t st)
 {
     k_dens_final<<<nblk, 256, 0, st>>>(acc, M, rs_row, ds, chi, conc, part);
-    k_dens_phis<<<1, 32, 0, st>>>(part, nblk, M, rs_row);
+    k_dens_phis<<<1, 192, 0, st>>>(part, nblk, M, rs_row);
     return 2;
 }
 

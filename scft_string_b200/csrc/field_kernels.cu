@@ -231,13 +231,16 @@ __global__ void k_freee(FieldArgs a, double f)
     put_partial(a.partials, 2 * j + 1, s1, sh);
 }
 
+// a warp per row, in a fixed order
 __global__ void k_reduce_final(const double *partials, int nrows, int nblk, double *out)
 {
-    const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (row >= nrows) return;
     double t = 0;
-    for (int i = 0; i < nblk; i++) t += partials[(size_t)row * nblk + i];
-    out[row] = t;
+    for (int i = threadIdx.x & 31; i < nblk; i += 32) t += partials[(size_t)row * nblk + i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0) out[row] = t;
 }
 
 SmallVec to_vec(const double *v, int n)
@@ -300,7 +303,7 @@ void launch_freee(const FieldArgs &a, int n, double f, int nblk, cudaStream_t st
 
 void launch_reduce_final(const double *partials, int nrows, int nblk, double *out, cudaStream_t st)
 {
-    k_reduce_final<<<(nrows + 127) / 128, 128, 0, st>>>(partials, nrows, nblk, out);
+    k_reduce_final<<<(nrows + 3) / 4, 128, 0, st>>>(partials, nrows, nblk, out);
 }
 
 }  // namespace scft

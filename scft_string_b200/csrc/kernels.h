@@ -46,11 +46,17 @@ struct PropsArgs {
     int *sync;              // claim and completion counters of the persistent step kernel (reg64.cu)
 };
 
+// most blocks per slot of the density pass, and threads that share a point's
+// contour on grids of fewer than kDensPoints points
+constexpr int kDensBlocks = 8 * 148, kDensParts = 4, kDensPoints = 150000;
+
 struct PropsLaunch {
     int slab_threads, slab_smem;
     int pencil_threads, pencil_smem;
     int ew_blocks;   // elementwise grid (per slot)
     int red_blocks;  // reduction grid (per slot)
+    int q_blocks;    // grid of the partition function sums (per slot)
+    int dens_blocks, dens_parts;  // grid of the density pass (per slot), threads per point
     int big;         // FFT kernels need more than 256 threads per CTA
     int fixed;       // compile-time shape id (0: runtime-shaped kernels)
     int pf;          // prefetching (bulk-copy) slab kernels for the fixed shape

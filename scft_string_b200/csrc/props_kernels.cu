@@ -972,19 +972,29 @@ __global__ void k_qsum(PropsArgs<T> a)
     }
 }
 
-// Q2, QC, lnQ and the ensemble weights (density.h:376-399); one block per slot
+// sum of n partials by one warp, in a fixed order (lanes strided, then a tree);
+// valid in every lane.  One thread adding 148 of them took 8 us.
+__device__ __forceinline__ double warp_row_sum(const double *p, int n)
+{
+    double t = 0;
+    for (int i = threadIdx.x & 31; i < n; i += 32) t += p[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
+// Q2, QC, lnQ and the ensemble weights (density.h:376-399); one block of two warps per slot
 template <typename T>
 __global__ void k_qfinal(PropsArgs<T> a, int nblk)
 {
-    const int slot = blockIdx.x;
+    __shared__ double sums[2];
+    const int slot = blockIdx.x, w = threadIdx.x >> 5;
+    const double t = warp_row_sum(a.partials + (size_t)slot * a.npart_stride + w * nblk, nblk);
+    if ((threadIdx.x & 31) == 0) sums[w] = t;
+    __syncthreads();
     if (threadIdx.x != 0) return;
-    const double *pp = a.partials + (size_t)slot * a.npart_stride;
-    double Q2 = 0, QC = 0;
-    for (int i = 0; i < nblk; i++) Q2 += pp[i];
-    for (int i = 0; i < nblk; i++) QC += pp[nblk + i];
     const double M = (double)a.g.M;
-    Q2 /= M;
-    QC /= M;
+    const double Q2 = sums[0] / M, QC = sums[1] / M;
     const int rep = a.slot_rep[slot];
     double *rs = a.rs + (size_t)rep * kRsStride;
     const double phic = a.phic, alpha = a.alpha;
@@ -1013,7 +1023,7 @@ __device__ __forceinline__ void kahan_add(double &sum, double &c, double term)
     sum = t;
 }
 
-// sum += w_s u(s) v(t - s) for s in [s0, s1) with Simpson interior weights
+// sum += w_s u(s) v(t - s) over part `part` of `parts` of s in [s0, s1) with Simpson interior weights
 // 4, 2, 4, ... from s0 (the reference's loops, density.h:404-422), Kahan
 // compensated, in the reference's order.  u, v are fields fu, fv of the
 // propagator store at point r.  The loads of four consecutive terms are
@@ -1021,10 +1031,12 @@ __device__ __forceinline__ void kahan_add(double &sum, double &c, double term)
 // instead of two.
 template <typename T>
 __device__ __forceinline__ void simpson_run(const T *h, size_t M, int r, int s0, int s1, int fu, int fv, int t,
-                                            double &sum, double &c)
+                                            double &sum, double &c, int part, int parts)
 {
-    int s = s0;
-    for (; s + 3 < s1; s += 4) {
+    const int len = s1 > s0 ? s1 - s0 : 0;
+    const int end = s0 + len * (part + 1) / parts;
+    int s = s0 + len * part / parts;
+    for (; s + 3 < end; s += 4) {
         double u[4], v[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -1034,7 +1046,7 @@ __device__ __forceinline__ void simpson_run(const T *h, size_t M, int r, int s0,
 #pragma unroll
         for (int k = 0; k < 4; k++) kahan_add(sum, c, (((s + k - s0) & 1) ? 2 : 4) * u[k] * v[k]);
     }
-    for (; s < s1; s++)
+    for (; s < end; s++)
         kahan_add(sum, c, (((s - s0) & 1) ? 2 : 4) * (double)h[((size_t)s * 2 + fu) * M + r] *
                               (double)h[((size_t)(t - s) * 2 + fv) * M + r]);
 }
@@ -1045,10 +1057,17 @@ __device__ __forceinline__ void simpson_run(const T *h, size_t M, int r, int s0,
 // correction, as in the reference.  Products are formed and summed in FP64
 // with Kahan compensation.  Also emits per-block partial sums of
 // rC, rA, rB, rhA, rhB and (chi*(phiA+phiB-1))^2.
-template <typename T>
-__global__ void k_density(PropsArgs<T> a)
+// The pass reads every slice once and is bound by memory: it needs the loads of
+// about 1000 threads per SM in flight.  One block per SM reached 1.4 TB/s at 64^3
+// (one replica); here a thread takes one point (64^3: 1024 blocks), and on grids
+// with fewer points than that PARTS threads share a point's contour.  PARTS
+// follows from the grid alone, so a replica's densities do not depend on its batch.
+template <typename T, int PARTS>
+__global__ void __launch_bounds__(256) k_density(PropsArgs<T> a)
 {
-    __shared__ double sh[32];
+    constexpr int PTS = 256 / PARTS;
+    __shared__ double sh[32], part_sum[PARTS > 1 ? 3 * 256 : 1];
+    const int part = threadIdx.x / PTS, lane = threadIdx.x % PTS;
     const Geo &g = a.g;
     const int slot = blockIdx.y;
     const int rep = a.slot_rep[slot];
@@ -1060,16 +1079,36 @@ __global__ void k_density(PropsArgs<T> a)
     const T *h = a.hist + hist_off<T>(g, slot, 0, 0);
     double *conc = a.conc + (size_t)rep * 4 * M;
     double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < (int)M; r += gridDim.x * blockDim.x) {
+    // whole blocks of points: every thread of a block takes the same number of turns
+    for (int r0 = blockIdx.x * PTS; r0 < (int)M; r0 += gridDim.x * PTS) {
+        const bool in = r0 + lane < (int)M;
+        const int r = in ? r0 + lane : (int)M - 1;
 #define Q1(s) ((double)h[((size_t)(s) * 2 + 0) * M + r])
 #define Q2(s) ((double)h[((size_t)(s) * 2 + 1) * M + r])
-        double rhB = 2.0 * Q2(Nh), chB = 0;
-        const double q12 = Q1(n1) * Q2(n2);
-        double rCA = Q2(Ns) + q12, cA = 0;
-        double rCB = Q1(Ns) + q12, cB = 0;
-        simpson_run(h, M, r, 1, Nh, 1, 1, Nh, rhB, chB);     // Q2(s) Q2(Nh - s)
-        simpson_run(h, M, r, 1, n1, 0, 1, Ns, rCA, cA);      // Q1(s) Q2(Ns - s)
-        simpson_run(h, M, r, n1 + 1, Ns, 0, 1, Ns, rCB, cB); // Q1(s) Q2(Ns - s)
+        double rhB = 0, chB = 0, rCA = 0, cA = 0, rCB = 0, cB = 0;
+        if (part == 0) {
+            const double q12 = Q1(n1) * Q2(n2);
+            rhB = 2.0 * Q2(Nh);
+            rCA = Q2(Ns) + q12;
+            rCB = Q1(Ns) + q12;
+        }
+        simpson_run(h, M, r, 1, Nh, 1, 1, Nh, rhB, chB, part, PARTS);     // Q2(s) Q2(Nh - s)
+        simpson_run(h, M, r, 1, n1, 0, 1, Ns, rCA, cA, part, PARTS);      // Q1(s) Q2(Ns - s)
+        simpson_run(h, M, r, n1 + 1, Ns, 0, 1, Ns, rCB, cB, part, PARTS); // Q1(s) Q2(Ns - s)
+        if constexpr (PARTS > 1) {
+            part_sum[threadIdx.x] = rhB;
+            part_sum[256 + threadIdx.x] = rCA;
+            part_sum[512 + threadIdx.x] = rCB;
+            __syncthreads();
+            if (part == 0)
+                for (int i = 1; i < PARTS; i++) {
+                    rhB += part_sum[i * PTS + lane];
+                    rCA += part_sum[256 + i * PTS + lane];
+                    rCB += part_sum[512 + i * PTS + lane];
+                }
+            __syncthreads();
+        }
+        if (part != 0 || !in) continue;
         if (g.jon) {
             // continuous A fraction: theta of the junction step's trapezoid
             // weight moves from the B block to the A block (3/2 here: the sums
@@ -1104,24 +1143,20 @@ __global__ void k_density(PropsArgs<T> a)
     }
 }
 
-// phis (density.h:433-454) and the W+ residual sum of solve_field0 (scft.cu:527-535)
+// phis (density.h:433-454) and the W+ residual sum of solve_field0
+// (scft.cu:527-535); one block of six warps per slot, a warp per sum.  One thread
+// adding the six rows took 28 us.
 template <typename T>
 __global__ void k_dfinal(PropsArgs<T> a, int nblk)
 {
-    const int slot = blockIdx.x;
-    if (threadIdx.x != 0) return;
-    const double *pp = a.partials + (size_t)slot * a.npart_stride;
-    const int rep = a.slot_rep[slot];
-    double *rs = a.rs + (size_t)rep * kRsStride;
-    double v[6];
-    for (int k = 0; k < 6; k++) {
-        double t = 0;
-        for (int i = 0; i < nblk; i++) t += pp[k * nblk + i];
-        v[k] = t;
-    }
-    const double M = (double)a.g.M;
-    for (int k = 0; k < 5; k++) rs[kRsPhis + k] = v[k] / M;
-    rs[kRsDev2] = v[5];
+    const int slot = blockIdx.x, k = threadIdx.x >> 5;
+    const double t = warp_row_sum(a.partials + (size_t)slot * a.npart_stride + k * nblk, nblk);
+    if ((threadIdx.x & 31) != 0) return;
+    double *rs = a.rs + (size_t)a.slot_rep[slot] * kRsStride;
+    if (k < 5)
+        rs[kRsPhis + k] = t / (double)a.g.M;
+    else
+        rs[kRsDev2] = t;
 }
 
 // ---------------------------------------------------------------- launchers
@@ -1275,10 +1310,13 @@ int launch_props_mt(const PropsArgs<T> &a, const PropsLaunch &L, int nslots, cud
         }
         n += 4 * g.Ns;
     }
-    k_qsum<T><<<dim3(L.red_blocks, nslots), 256, 0, st>>>(a);
-    k_qfinal<T><<<nslots, 32, 0, st>>>(a, L.red_blocks);
-    k_density<T><<<dim3(L.red_blocks, nslots), 256, 0, st>>>(a);
-    k_dfinal<T><<<nslots, 32, 0, st>>>(a, L.red_blocks);
+    k_qsum<T><<<dim3(L.q_blocks, nslots), 256, 0, st>>>(a);
+    k_qfinal<T><<<nslots, 64, 0, st>>>(a, L.q_blocks);
+    if (L.dens_parts > 1)
+        k_density<T, kDensParts><<<dim3(L.dens_blocks, nslots), 256, 0, st>>>(a);
+    else
+        k_density<T, 1><<<dim3(L.dens_blocks, nslots), 256, 0, st>>>(a);
+    k_dfinal<T><<<nslots, 192, 0, st>>>(a, L.dens_blocks);
     return n;
 }
 
@@ -1482,8 +1520,8 @@ int launch_prepare(const PropsArgs<T> &a, const PropsLaunch &L, cudaStream_t st)
 template <typename T>
 int launch_qsums(const PropsArgs<T> &a, const PropsLaunch &L, cudaStream_t st)
 {
-    k_qsum<T><<<dim3(L.red_blocks, 1), 256, 0, st>>>(a);
-    k_qfinal<T><<<1, 32, 0, st>>>(a, L.red_blocks);
+    k_qsum<T><<<dim3(L.q_blocks, 1), 256, 0, st>>>(a);
+    k_qfinal<T><<<1, 64, 0, st>>>(a, L.q_blocks);
     return 2;
 }
 

@@ -702,6 +702,9 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
     L.pencil_smem = (int)((g.tc * g.m0 + g.m0) * 2 * T + (g.tc + g.m0) * T);
     L.ew_blocks = std::max(1, std::min(1024, (g.M + 255) / 256));
     L.red_blocks = kRedBlocks;
+    L.q_blocks = std::max(1, std::min(4 * kRedBlocks, (g.M + 255) / 256));
+    L.dens_parts = g.M < kDensPoints ? kDensParts : 1;
+    L.dens_blocks = std::max(1, std::min(kDensBlocks, (int)(((long long)g.M * L.dens_parts + 255) / 256)));
     if (L.slab_smem > (int)prop.sharedMemPerBlockOptin || L.pencil_smem > (int)prop.sharedMemPerBlockOptin) {
         delete ctx;
         return SCFT_BAD_INPUT;
@@ -731,7 +734,7 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
             upload_tables<float>(ctx, twb, kfb);
         else
             upload_tables<double>(ctx, twb, kfb);
-        ctx->npart_stride = 6 * kRedBlocks;
+        ctx->npart_stride = 6 * kDensBlocks;
         ctx->nred_rows = 2 * kMaxStrn + 8;
         CKC(cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking));
         CKC(cudaStreamCreateWithFlags(&ctx->st2, cudaStreamNonBlocking));
@@ -1876,9 +1879,9 @@ scft_status props_ckpt_impl(scft_ctx *ctx, int ii, int K, double *lnQ_out, doubl
     auto flush = [&]() {
         if (P.n == 0) return;
         ctx->stats.kernel_launches += T == 4 ? launch_density_acc<float>((const float *)R.ck, M, P, acc,
-                                                                         ctx->L.red_blocks, ctx->st)
+                                                                         ctx->L.dens_blocks, ctx->st)
                                              : launch_density_acc<double>((const double *)R.ck, M, P, acc,
-                                                                          ctx->L.red_blocks, ctx->st);
+                                                                          ctx->L.dens_blocks, ctx->st);
         P.n = 0;
     };
     auto add = [&](long long x, long long y, double a, double b, double h) {
