@@ -163,6 +163,11 @@ int launch_junction_dtheta(const StressArgs<T> &a, const StressPairs &P, int sla
                            int pencil_threads, int pencil_smem, double *part, int nblk, double *out,
                            cudaStream_t st);
 
+// the same sums on pairs packed as one complex field (pair_stress.cu), FP64 grids of pair_applicable
+constexpr int kStressSumBlocks = 64;
+int pair_stress_setup(int m0, int m1, int m2);
+int pair_stress_chunk(const StressArgs<double> &a, const StressPairs &P, double *out, cudaStream_t st);
+
 // ------------------------------------------------------------------ checkpointed densities
 constexpr int kDensPairs = 32;
 

@@ -7,6 +7,7 @@
 #include <algorithm>
 
 #include "pair.cuh"
+#include "pair_shapes.h"
 #include "step_order.cuh"
 
 namespace scft {
@@ -14,17 +15,12 @@ namespace {
 
 using T = double;
 
-constexpr int kSmemCta = 227 * 1024;  // dynamic shared memory a CTA may have
 constexpr int kSms = 148;
+constexpr int kTile = kPairTile;  // the wide form takes twice as many columns
+constexpr int kPencilThreads = 256;
 
-// slab shapes (m1, m2) and x lengths with kernels
-#define PAIR_SLABS(X) X(16, 16) X(24, 24) X(32, 32) X(40, 40) X(48, 48) X(64, 64) X(64, 96) X(80, 80) X(96, 96) X(128, 128)
-#define PAIR_AXES(X) X(16) X(24) X(32) X(40) X(48) X(64) X(80) X(96) X(128)
 // grids with a persistent step kernel
 #define PAIR_GRIDS(X) X(32, 32, 32) X(48, 48, 48) X(64, 64, 64) X(64, 64, 96) X(96, 96, 96)
-
-constexpr int kTile = 32;         // columns per x tile; the wide form takes twice as many
-constexpr int kPencilThreads = 256;
 
 constexpr int pencil_minb(int m0) { return m0 > 80 ? 2 : 3; }
 
@@ -156,84 +152,13 @@ constexpr int step_smem()
                                                                    : PairPencil<M0, TC>::SMEM;
 }
 
-// CTAs per slab: one where the slab fits a CTA's shared memory.  Two were slower
-// on every shape that fits (one replica step: 64^3 34.2 us with one, 37.1 with
-// two; 48^3 22.9 and 27.3; 96^3 84.9 and 91.6).
-template <int M1, int M2>
-constexpr int kCl = PairSlab<M1, M2, 1>::SMEM <= kSmemCta ? 1 : 2;
-
-bool slab_ok(int m1, int m2)
-{
-#define X(A, B) \
-    if (m1 == A && m2 == B) return true;
-    PAIR_SLABS(X)
-#undef X
-    return false;
-}
-
-bool axis_ok(int m0)
-{
-#define X(A) \
-    if (m0 == A) return true;
-    PAIR_AXES(X)
-#undef X
-    return false;
-}
-
-// n = r1 r2 with both radices available and the larger one as small as it gets
-// (at equal size the first the larger: real space and global memory are met with
-// more elements per thread); false if there are none
-bool two_radices(int n, int &r1, int &r2)
-{
-    static const int rad[] = {
-#define X(Q) Q,
-        PAIR_RADICES(X)
-#undef X
-    };
-    int best = 1 << 30;
-    for (int a : rad)
-        for (int b : rad)
-            if (a >= b && a * b == n && a < best) {
-                best = a;
-                r1 = a;
-                r2 = b;
-            }
-    return best < (1 << 30);
-}
-
-int any_smem(const PairAny &q) { return (q.m1 * q.S + q.m1 + q.m2) * (int)sizeof(cplxd); }
-int any_pencil_smem(int m0) { return (m0 * kTile + m0) * (int)sizeof(cplxd) + (m0 + kTile) * (int)sizeof(double); }
-
-bool any_plan(int m1, int m2, PairAny &q)
-{
-    if (m1 < 2 || m2 < 2) return false;
-    if (!two_radices(m1, q.ra, q.rb) || !two_radices(m2, q.rc, q.rz)) return false;
-    q.m1 = m1;
-    q.m2 = m2;
-    q.S = m2 | 1;
-    q.mag1 = (unsigned)((1ull << 32) / m1) + 1;
-    q.mag2 = (unsigned)((1ull << 32) / m2) + 1;
-    return any_smem(q) <= kSmemCta;
-}
-
-// threads of a slab kernel of such a shape: one butterfly each in its widest
-// pass, up to 256, or 512 where shared memory leaves one CTA per SM
-int any_threads(const PairAny &q)
-{
-    const int n = std::max(std::max(q.m1 * q.rz, q.m1 * q.rc), std::max(q.ra * q.m2, q.rb * q.m2));
-    const int most = 2 * (any_smem(q) + 1024) <= 228 * 1024 ? 256 : 512;
-    return std::min(most, (n + 31) / 32 * 32);
-}
-
-bool any_axis(int m0, int &r1, int &r2) { return two_radices(m0, r2, r1) && any_pencil_smem(m0) <= kSmemCta; }
-
 }  // namespace
 
 bool pair_applicable(int m0, int m1, int m2)
 {
     PairAny q;
     int r1, r2;
-    return (slab_ok(m1, m2) || any_plan(m1, m2, q)) && (axis_ok(m0) || any_axis(m0, r1, r2));
+    return (pair_slab_fixed(m1, m2) || pair_any_plan(m1, m2, q)) && (pair_axis_fixed(m0) || pair_x_radices(m0, r1, r2));
 }
 
 // raises the kernels' shared-memory limits; *grid = CTAs of the persistent step launch (0: none)
@@ -260,18 +185,18 @@ int pair_setup(int m0, int m1, int m2, int *grid)
 #undef X
     PairAny q;
     int r1, r2;
-    if (!slab_ok(m1, m2) && any_plan(m1, m2, q)) switch (q.ra) {
+    if (!pair_slab_fixed(m1, m2) && pair_any_plan(m1, m2, q)) switch (q.ra) {
 #define X(A)                                           \
     case A:                                            \
-        up(k_pair_mid_any<A>, any_smem(q));            \
-        up(k_pair_combine_any<A>, any_smem(q));        \
+        up(k_pair_mid_any<A>, pair_any_smem(q));            \
+        up(k_pair_combine_any<A>, pair_any_smem(q));        \
         break;
             PAIR_RADICES(X)
 #undef X
         }
-    if (!axis_ok(m0) && any_axis(m0, r1, r2)) switch (r2) {
+    if (!pair_axis_fixed(m0) && pair_x_radices(m0, r1, r2)) switch (r2) {
 #define X(A) \
-    case A: up(k_pair_pencil_any<A>, any_pencil_smem(m0)); break;
+    case A: up(k_pair_pencil_any<A>, pair_any_pencil_smem(m0)); break;
             PAIR_RADICES(X)
 #undef X
         }
@@ -307,9 +232,9 @@ void pair_mid(const PropsArgs<T> &a, int nslots, int s, cudaStream_t st)
     PAIR_SLABS(X)
 #undef X
     PairAny q;
-    if (any_plan(g.m1, g.m2, q)) switch (q.ra) {
+    if (pair_any_plan(g.m1, g.m2, q)) switch (q.ra) {
 #define X(A)                                                                                                           \
-    case A: launch_step(k_pair_mid_any<A>, dim3(g.m0, 2, nslots), any_threads(q), any_smem(q), 1, 1, st, a, s, q); break;
+    case A: launch_step(k_pair_mid_any<A>, dim3(g.m0, 2, nslots), pair_any_threads(q), pair_any_smem(q), 1, 1, st, a, s, q); break;
             PAIR_RADICES(X)
 #undef X
         }
@@ -332,10 +257,10 @@ void pair_combine(const PropsArgs<T> &a, int nslots, int s, int mode, cudaStream
     PAIR_SLABS(X)
 #undef X
     PairAny q;
-    if (any_plan(g.m1, g.m2, q)) switch (q.ra) {
+    if (pair_any_plan(g.m1, g.m2, q)) switch (q.ra) {
 #define X(A)                                                                                                         \
     case A:                                                                                                          \
-        launch_step(k_pair_combine_any<A>, dim3(g.m0, split, nslots), any_threads(q), any_smem(q), 1, split, st, a, \
+        launch_step(k_pair_combine_any<A>, dim3(g.m0, split, nslots), pair_any_threads(q), pair_any_smem(q), 1, split, st, a, \
                     s, mode, q);                                                                                     \
         break;
             PAIR_RADICES(X)
@@ -348,23 +273,13 @@ void pair_pencil(const PropsArgs<T> &a, int nslots, int both, int wide, cudaStre
     const Geo &g = a.g;
     const int tc = wide ? 2 * kTile : kTile;
     int ra = 1, rb = 1;
-#define X(A, B)                        \
-    if (g.m1 == A && g.m2 == B) {      \
-        PairSlab<A, B, 1>::radices(ra, rb); \
-    }
-    PAIR_SLABS(X)
-#undef X
-    PairAny q;
-    if (!slab_ok(g.m1, g.m2) && any_plan(g.m1, g.m2, q)) {
-        ra = q.ra;
-        rb = q.rb;
-    }
+    pair_y_radices(g.m1, g.m2, ra, rb);
     int r1, r2;
-    if (!axis_ok(g.m0) && any_axis(g.m0, r1, r2)) {
+    if (!pair_axis_fixed(g.m0) && pair_x_radices(g.m0, r1, r2)) {
         const dim3 grid((g.m1 * g.m2 + kTile - 1) / kTile, both ? 2 : 1, nslots);
         switch (r2) {
 #define X(A) \
-    case A: launch_step(k_pair_pencil_any<A>, grid, kPencilThreads, any_pencil_smem(g.m0), 1, 1, st, a, ra, rb); break;
+    case A: launch_step(k_pair_pencil_any<A>, grid, kPencilThreads, pair_any_pencil_smem(g.m0), 1, 1, st, a, ra, rb); break;
             PAIR_RADICES(X)
 #undef X
         }

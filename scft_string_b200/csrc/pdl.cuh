@@ -26,11 +26,11 @@ __device__ __forceinline__ void prefetch_l2(const void *p, int bytes)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
-// Launch of a step kernel: it may start while the kernel before it on the
-// stream finishes (see pdl_wait), in clusters of (cx, cy) CTAs.
+// Launch in clusters of (cx, cy) CTAs.  pdl: it may start while the kernel before
+// it on the stream finishes; only for kernels that call pdl_wait.
 template <class... Params, class... Args>
-inline void launch_step(void (*fn)(Params...), dim3 grid, int threads, int smem, int cx, int cy, cudaStream_t st,
-                        const Args &...args)
+inline void launch_ex(bool pdl, void (*fn)(Params...), dim3 grid, int threads, int smem, int cx, int cy, cudaStream_t st,
+                      const Args &...args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -39,7 +39,7 @@ inline void launch_step(void (*fn)(Params...), dim3 grid, int threads, int smem,
     cfg.stream = st;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
     at[1].id = cudaLaunchAttributeClusterDimension;
     at[1].val.clusterDim.x = cx;
     at[1].val.clusterDim.y = cy;
@@ -47,6 +47,13 @@ inline void launch_step(void (*fn)(Params...), dim3 grid, int threads, int smem,
     cfg.attrs = at;
     cfg.numAttrs = cx * cy > 1 ? 2 : 1;
     cudaLaunchKernelEx(&cfg, fn, Params(args)...);
+}
+
+template <class... Params, class... Args>
+inline void launch_step(void (*fn)(Params...), dim3 grid, int threads, int smem, int cx, int cy, cudaStream_t st,
+                        const Args &...args)
+{
+    launch_ex(true, fn, grid, threads, smem, cx, cy, st, args...);
 }
 
 }  // namespace scft

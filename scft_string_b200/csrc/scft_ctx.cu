@@ -1491,8 +1491,12 @@ scft_status stress_alloc(scft_ctx *ctx)
     CK(cudaMalloc(&ctx->st_S4, sz));
     CK(cudaMalloc(&ctx->st_S2, sz));
     CK(cudaMalloc(&ctx->st_S4p, sz));
-    CK(cudaMalloc(&ctx->st_part, sizeof(double) * 9 * (size_t)g.ncol_tiles * kStressPairs));
-    CK(cudaMalloc(&ctx->st_out, sizeof(double) * 3 * kStressPairs));
+    CK(cudaMalloc(&ctx->st_part, sizeof(double) * 9 * (size_t)std::max(g.ncol_tiles, kStressSumBlocks) * kStressPairs));
+    CK(cudaMalloc(&ctx->st_out, sizeof(double) * 3 * (size_t)(g.Ns + g.Nh)));  // every pair of a call
+    if (ctx->L.pair && pair_stress_setup(g.m0, g.m1, g.m2) != 0) {
+        ctx->lasterr = "stress kernels: shared memory attribute";
+        return SCFT_CUDA_ERROR;
+    }
     if ((T == 4 ? set_stress_smem<float>(ctx->rt_slab_smem, ctx->rt_pencil_smem)
                 : set_stress_smem<double>(ctx->rt_slab_smem, ctx->rt_pencil_smem)) != 0) {
         ctx->lasterr = "stress kernels: shared memory attribute";
@@ -1507,7 +1511,7 @@ scft_status stress_pairs(scft_ctx *ctx, int rep, int slot, const void *hist, con
 {
     const Geo &g = ctx->g;
     const double *Lr = &ctx->Dr[3 * (size_t)rep];  // the replica's box
-    std::vector<double> out(3 * kStressPairs);
+    std::vector<double> out(3 * pairs.size());
     for (size_t c0 = 0; c0 < pairs.size(); c0 += kStressPairs) {
         StressPairs P;
         std::memset(&P, 0, sizeof(P));
@@ -1529,7 +1533,7 @@ scft_status stress_pairs(scft_ctx *ctx, int rep, int slot, const void *hist, con
                                 {Lr[0], Lr[1], Lr[2]}, (float)(1.0 / g.M), ctx->err};
             a.jtab = (const float *)ctx->jtab;
             nl = launch_stress_chunk<float>(a, P, ctx->rt_slab_threads, ctx->rt_slab_smem,
-                                            ctx->rt_pencil_threads, ctx->rt_pencil_smem, ctx->st_out, ctx->st);
+                                            ctx->rt_pencil_threads, ctx->rt_pencil_smem, ctx->st_out + 3 * c0, ctx->st);
         } else {
             StressArgs<double> a{g, slot, (const double *)hist, (const double *)ctx->etab,
                                  (const cplx<double> *)ctx->tw, (const double *)ctx->kfac + (size_t)rep * ctx->kf_n,
@@ -1537,17 +1541,20 @@ scft_status stress_pairs(scft_ctx *ctx, int rep, int slot, const void *hist, con
                                  (cplx<double> *)ctx->st_S4p, ctx->st_part,
                                  {Lr[0], Lr[1], Lr[2]}, 1.0 / g.M, ctx->err};
             a.jtab = (const double *)ctx->jtab;
-            nl = launch_stress_chunk<double>(a, P, ctx->rt_slab_threads, ctx->rt_slab_smem,
-                                             ctx->rt_pencil_threads, ctx->rt_pencil_smem, ctx->st_out, ctx->st);
+            nl = ctx->L.pair ? pair_stress_chunk(a, P, ctx->st_out + 3 * c0, ctx->st)
+                             : launch_stress_chunk<double>(a, P, ctx->rt_slab_threads, ctx->rt_slab_smem,
+                                                           ctx->rt_pencil_threads, ctx->rt_pencil_smem,
+                                                           ctx->st_out + 3 * c0, ctx->st);
         }
         ctx->stats.kernel_launches += nl;
-        CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(out.data(), ctx->st_out, sizeof(double) * 3 * P.n, cudaMemcpyDeviceToHost, ctx->st));
-        scft_status s = check_device_err(ctx);
-        if (s != SCFT_OK) return s;
-        for (int p = 0; p < P.n; p++)
-            for (int i = 0; i < 3; i++) (pairs[c0 + p].homo ? dQ2 : dQC)[i] += out[3 * p + i];
     }
+    CK(cudaGetLastError());
+    // one wait for all chunks
+    CK(cudaMemcpyAsync(out.data(), ctx->st_out, sizeof(double) * out.size(), cudaMemcpyDeviceToHost, ctx->st));
+    scft_status s = check_device_err(ctx);
+    if (s != SCFT_OK) return s;
+    for (size_t p = 0; p < pairs.size(); p++)
+        for (int i = 0; i < 3; i++) (pairs[p].homo ? dQ2 : dQC)[i] += out[3 * p + i];
     return SCFT_OK;
 }
 
@@ -1962,9 +1969,8 @@ extern "C" {
 // QC depends on f:  dQC/dtheta = (1/M) <q^dagger(N-1-n1), dS_J/dtheta q(n1)>
 // (the adjoint of the junction step, stress_kernels.cu).  dF/df = -d lnQ/df
 // at a converged saddle point.
-scft_status scft_dF_df(scft_ctx *ctx, int ii, double *dlnQ_df, double *dF_df)
+static scft_status dF_df_impl(scft_ctx *ctx, int ii, bool fresh, double *dlnQ_df, double *dF_df)
 {
-    if (!ctx || ii < 0 || ii >= ctx->strn) return SCFT_BAD_INPUT;
     if (ctx->nostore) {
         ctx->lasterr = "scft_dF_df needs the full propagator store (context created with nostore)";
         return SCFT_UNSUPPORTED;
@@ -1978,8 +1984,10 @@ scft_status scft_dF_df(scft_ctx *ctx, int ii, double *dlnQ_df, double *dF_df)
     if (s != SCFT_OK) return s;
     const size_t T = ctx->prec == SCFT_FP32 ? 4 : 8;
     if (!ctx->jd_rbuf) CK(cudaMalloc(&ctx->jd_rbuf, T * 6 * (size_t)g.M));
-    s = props_list(ctx, {ii});
-    if (s != SCFT_OK) return s;
+    if (fresh) {
+        s = props_list(ctx, {ii});
+        if (s != SCFT_OK) return s;
+    }
     const int slot = ctx->slot_of[ii];
     const double QC = rsv(ctx, ii, kRsQC), zC = rsv(ctx, ii, kRsZC);
     StressPairs P;
@@ -2032,6 +2040,12 @@ scft_status scft_dF_df(scft_ctx *ctx, int ii, double *dlnQ_df, double *dF_df)
     return SCFT_OK;
 }
 
+scft_status scft_dF_df(scft_ctx *ctx, int ii, double *dlnQ_df, double *dF_df)
+{
+    if (!ctx || ii < 0 || ii >= ctx->strn) return SCFT_BAD_INPUT;
+    return dF_df_impl(ctx, ii, true, dlnQ_df, dF_df);
+}
+
 // All parameter derivatives of replica ii at its current fields in one call:
 // dF/dL (scft_stress), dF/dchiN (scft_dF_dchi) and, for a continuous A
 // fraction, dF/df (scft_dF_df); dF/df is NaN otherwise (f enters the
@@ -2043,7 +2057,7 @@ scft_status scft_gradients(scft_ctx *ctx, int ii, double *dF_dL, double *dF_dchi
     if (s == SCFT_OK && dF_dchi) s = scft_dF_dchi(ctx, ii, dF_dchi);
     if (s == SCFT_OK && dF_df) {
         if (ctx->g.jon)
-            s = scft_dF_df(ctx, ii, nullptr, dF_df);
+            s = dF_df_impl(ctx, ii, false, nullptr, dF_df);  // on the propagators that scft_stress left
         else
             *dF_df = std::nan("");
     }
