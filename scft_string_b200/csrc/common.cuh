@@ -45,7 +45,14 @@ constexpr int kPairLanes = 8;  // slab pack/unpack: mk2 <= 32*kPairLanes
 // + 1 (0 for n = 1), exact while b n < 2^32.  A 32-bit division is about 20
 // instructions; the run-time shaped transforms take several per butterfly.
 __host__ __device__ __forceinline__ unsigned div_mag(int n) { return n > 1 ? 0xffffffffu / (unsigned)n + 1u : 0u; }
-__device__ __forceinline__ int div_by(int b, unsigned mag) { return mag ? (int)__umulhi((unsigned)b, mag) : b; }
+__host__ __device__ __forceinline__ int div_by(int b, unsigned mag)
+{
+#ifdef __CUDA_ARCH__
+    return mag ? (int)__umulhi((unsigned)b, mag) : b;
+#else
+    return mag ? (int)(((unsigned long long)(unsigned)b * mag) >> 32) : b;
+#endif
+}
 
 // Mixed-radix factorisation of one FFT length (radices 2, 3, 4, 5, 7, 8).
 struct Plan1D {

@@ -248,5 +248,9 @@ template <typename T, int SIGN>
 struct Reg<T, 14, SIGN> : RegCoprime<T, 2, 7, SIGN> {};
 template <typename T, int SIGN>
 struct Reg<T, 15, SIGN> : RegCoprime<T, 3, 5, SIGN> {};
+template <typename T, int SIGN>
+struct Reg<T, 20, SIGN> : RegCoprime<T, 4, 5, SIGN> {};
+template <typename T, int SIGN>
+struct Reg<T, 24, SIGN> : RegCoprime<T, 8, 3, SIGN> {};
 
 }  // namespace scft

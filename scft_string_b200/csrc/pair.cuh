@@ -122,9 +122,9 @@ PAIR_PLAN(32, 32, 8, 4, 4, 8, true, 128, 512)
 PAIR_PLAN(40, 40, 10, 4, 4, 10, true, 160, 480)
 PAIR_PLAN(48, 48, 12, 4, 4, 12, true, 192, 576)
 PAIR_PLAN(64, 64, 16, 4, 4, 16, true, 256, 512)
-PAIR_PLAN(64, 96, 8, 8, 12, 8, false, 256, 512)
-PAIR_PLAN(80, 80, 10, 8, 10, 8, false, 416, 416)
-PAIR_PLAN(96, 96, 12, 8, 12, 8, false, 384, 384)
+PAIR_PLAN(64, 96, 16, 4, 4, 24, true, 384, 384)
+PAIR_PLAN(80, 80, 20, 4, 4, 20, true, 320, 320)
+PAIR_PLAN(96, 96, 24, 4, 4, 24, true, 384, 384)
 PAIR_PLAN(128, 128, 16, 8, 16, 8, false, 1024, 512)  // two CTAs per slab only
 #undef PAIR_PLAN
 

@@ -12,19 +12,10 @@ import pytest
 from test_reg64_host import _cuda_include
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-LENGTHS = [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16]
+LENGTHS = [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16, 20, 24]
 
 SRC = r"""
-#define __device__
-#define __host__
-#define __forceinline__ inline
 #include <cuda_runtime.h>
-#undef __device__
-#undef __host__
-#undef __forceinline__
-#define __device__
-#define __host__
-#define __forceinline__ inline
 #include "dft.cuh"
 using namespace scft;
 template <int R> static void go(int sign, cplx<double> *v)
@@ -68,3 +59,19 @@ def test_register_dft(lib, n, sign):
     lib.h_dft(n, sign, v)
     # a few roundings of n terms of size 1
     assert np.abs(v.view(np.complex128) - ref).max() <= 8 * n * np.finfo(float).eps
+
+
+def test_quotients_by_reciprocal(tmp_path):
+    """div_by with div_mag(n) is b // n for every divisor and range that the
+    run-time sizes use (axes up to 510, butterfly and element counts below 2^16)."""
+    inc = _cuda_include()
+    if inc is None or shutil.which("g++") is None:
+        pytest.skip("needs g++ and the CUDA headers")
+    src, out = tmp_path / "div.cpp", str(tmp_path / "libdiv.so")
+    src.write_text('#include "common.cuh"\nextern "C" int bad(int nmax, int bmax) { for (int n = 1; n <= nmax; n++) {'
+                   " unsigned m = scft::div_mag(n); for (int b = 0; b < bmax; b++)"
+                   " if (scft::div_by(b, m) != b / n) return n; } return 0; }\n")
+    csrc = os.path.join(HERE, "..", "scft_string_b200", "csrc")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I" + inc, "-I" + csrc, "-o", out, str(src)],
+                   check=True)
+    assert C.CDLL(out).bad(2048, 65536) == 0
