@@ -72,7 +72,7 @@ struct scft_ctx {
     double f;  // rounded A fraction
     cudaStream_t st = nullptr, st2 = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, fork = nullptr, join = nullptr;
-    int ngroups = 2;
+    int ngroups = 0;  // slot groups of a round; 0: default_groups
     cudaEvent_t tev[4] = {nullptr, nullptr, nullptr, nullptr};
     PropsLaunch L;
     std::string lasterr;
@@ -246,6 +246,27 @@ int effective_groups(int ngroups, int nb)
     return (ng > 1 && nb >= 2 * ng) ? ng : 1;
 }
 
+// The count where none is configured: two, and on the pair-packed kernels twice
+// as many as long as the replicas of the two groups that run at a time hold more
+// than L2 keeps (spectra, tables and partial result: 64 bytes a point) and a
+// group still has slabs for most SMs.  64^3, us per replica step with 2 / 4
+// groups: 16 replicas 15.1 / 14.2, 14 replicas 15.2 / 14.2, 10 replicas 14.7 /
+// 15.5, 8 replicas 14.2 / 15.2; 48^3, 16 replicas 5.9 / 6.2.
+int default_groups(const scft_ctx *ctx, int nb)
+{
+    constexpr double kLive = 135e6;
+    constexpr int kSlabs = 192;
+    int ng = 2;
+    if (ctx->L.pair)
+        while (2.0 * ((nb + ng - 1) / ng) * 64.0 * ctx->M > kLive && nb / (2 * ng) * ctx->g.m0 >= kSlabs) ng *= 2;
+    return nb >= 2 * ng ? ng : 1;
+}
+
+int groups_for(const scft_ctx *ctx, int nb)
+{
+    return ctx->ngroups > 0 ? effective_groups(ctx->ngroups, nb) : default_groups(ctx, nb);
+}
+
 // density::props for a list of replicas; scalars land in ctx->rs_h.  Without a
 // full store (nostore) each replica runs from checkpoints.
 scft_status props_list(scft_ctx *ctx, const std::vector<int> &reps)
@@ -280,7 +301,7 @@ scft_status props_list(scft_ctx *ctx, const std::vector<int> &reps)
         // last wave of one group's launch overlaps the other group's work;
         // with more than two groups each stream runs its groups one after
         // another (fewer spectra live at once)
-        const int ng = effective_groups(ctx->ngroups, nb);
+        const int ng = groups_for(ctx, nb);
         auto launch = [&]() {
             int n = 0;
             if (ng > 1) {
@@ -2334,7 +2355,8 @@ scft_status scft_autotune_ex(scft_ctx *ctx, int *groups_out, int *wide_out, int 
         }
     }
     drop_graphs();
-    ctx->ngroups = best_g;
+    // where it is what the default takes, the default stays: it also knows partial batches
+    ctx->ngroups = best_g == default_groups(ctx, ctx->strn) ? 0 : best_g;
     ctx->L.ptile_wide = best_w;
     ctx->L.persist = best_p;
     ctx->stats = keep;
