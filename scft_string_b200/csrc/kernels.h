@@ -96,6 +96,12 @@ void pair_combine(const PropsArgs<double> &a, int nslots, int s, int mode, cudaS
 void pair_pencil(const PropsArgs<double> &a, int nslots, int both, int wide, cudaStream_t st);
 void pair_step(const PropsArgs<double> &a, int nslots, int s, int wide, int grid, cudaStream_t st);
 
+// FP32 slab kernels of the compile-time shapes (real_slab.cuh)
+bool real_slab_has(int m1, int m2);
+int real_slab_setup(int m1, int m2);
+void real_mid(const PropsArgs<float> &a, int nslots, int s, cudaStream_t st);
+void real_combine(const PropsArgs<float> &a, int nslots, int s, int mode, cudaStream_t st);
+
 void pf_smem_bytes(int id, int fp32, int &mid, int &comb);
 // dynamic shared memory of k_pencil_sh for tiles of tc columns
 int pencil_sh_smem_bytes(int fp32, int tc, int m0);

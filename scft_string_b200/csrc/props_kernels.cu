@@ -757,20 +757,6 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1)
     pencil_sh_body<T, MT, FM0, FM1, FM2, TC>(tmap, a, both, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
 }
 
-template <typename T, int MT, int FM0, int FM1, int FM2>
-__global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 4 : 2) : 1) k_mid_pf(PropsArgs<T> a, int s)
-{
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    mid_pf_body<T, MT, FM0, FM1, FM2>(a, s, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
-}
-
-template <typename T, int MT, int FM0, int FM1, int FM2>
-__global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 4 : 2) : 1) k_combine_pf(PropsArgs<T> a, int s, int mode)
-{
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    combine_pf_body<T, MT, FM0, FM1, FM2>(a, s, mode, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
-}
-
 // ---------------------------------------------------------------- one launch per contour step
 // The persistent form of the four launches above for the compile-time
 // shapes: CTAs claim work items from a counter in a fixed order -- every
@@ -1184,7 +1170,7 @@ void launch_combine(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gs, int s,
     }
     if constexpr (F1 != 0) {
         if (L.pf) {
-            launch_step(k_combine_pf<T, MT, F0, F1, F2>, gs, MT, L.combine_pf_smem, 1, 1, st, a, s, mode);
+            if constexpr (sizeof(T) == 4) real_combine(a, gs.z, s, mode, st);
             return;
         }
     }
@@ -1208,7 +1194,7 @@ void launch_mid(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gs, int s, cud
     }
     if constexpr (F1 != 0) {
         if (L.pf) {
-            launch_step(k_mid_pf<T, MT, F0, F1, F2>, gs, MT, L.mid_pf_smem, 1, 1, st, a, s);
+            if constexpr (sizeof(T) == 4) real_mid(a, gs.z, s, st);
             return;
         }
     }
@@ -1376,8 +1362,7 @@ int set_smem_mt(const PropsLaunch &L)
             }
         }
         if (e4 == cudaSuccess && L.pf) {
-            e4 = raise_dyn_smem(k_combine_pf<T, MT, F0, F1, F2>, L.combine_pf_smem);
-            e5 = raise_dyn_smem(k_mid_pf<T, MT, F0, F1, F2>, L.mid_pf_smem);
+            if (real_slab_setup(F1, F2) != 0) e5 = cudaErrorInvalidValue;
         }
     }
     int e6 = 0;

@@ -1,0 +1,427 @@
+// real_slab.cuh -- the FP32 slab kernels of the compile-time shapes.
+//
+// The same transforms as slab_forward_fixed / slab_inverse_fixed (fft.cuh): two
+// real rows per complex z line, the kz = 0 and kz = M2/2 columns as one complex y
+// column, every butterfly with the same inputs, twiddle factors and order of
+// operations, so the results are the same bits.  What differs is how a thread
+// covers a line: an M = 8 R point line takes a radix-8 pass and one pass over the
+// R remaining points, whose stages (12 = 4 3, 16 = 8 2, ...) share registers; the
+// unpacking of row pairs is done by the thread that transforms both rows' y
+// columns, in place; spectra are read from and written to global memory by the
+// outer passes themselves, and real space is met in registers.  A slab transform
+// makes three trips through shared memory; it made five to seven, with a barrier
+// before and after each stage.
+//
+// Products that feed an addition directly are rounded on their own (__fmul_rn):
+// they went through shared memory before, and a fused multiply-add would round
+// differently.
+#pragma once
+#include "common.cuh"
+#include "fft.cuh"
+#include "kernels.h"
+#include "pdl.cuh"
+
+namespace scft {
+
+using cplxf = cplx<float>;
+
+__device__ __forceinline__ cplxf ldf(const cplxf *p)
+{
+    const float2 v = *reinterpret_cast<const float2 *>(p);
+    return {v.x, v.y};
+}
+__device__ __forceinline__ cplxf ldf_cg(const cplxf *p)
+{
+    const float2 v = __ldcg(reinterpret_cast<const float2 *>(p));
+    return {v.x, v.y};
+}
+__device__ __forceinline__ void stf(cplxf *p, cplxf v) { *reinterpret_cast<float2 *>(p) = make_float2(v.x, v.y); }
+
+// a w and a conj(w), with the roundings that cmul and cmulc compile to in the
+// shared-memory stages (which product is rounded, which is fused)
+template <int SIGN>
+__device__ __forceinline__ cplxf twiddle(cplxf a, cplxf w)
+{
+    if (SIGN < 0) return {__fmaf_rn(a.x, w.x, -__fmul_rn(a.y, w.y)), __fmaf_rn(a.y, w.x, __fmul_rn(a.x, w.y))};
+    return {__fmaf_rn(a.x, w.x, __fmul_rn(a.y, w.y)), __fmaf_rn(a.y, w.x, -__fmul_rn(a.x, w.y))};
+}
+
+// second stage radix of the R points left after radix 8 (1: one stage)
+__host__ __device__ constexpr int tail_b(int r) { return r == 6 || r == 12 ? 3 : r == 16 ? 2 : 1; }
+
+// The stages after the radix-8 one of a length-N line (N = 8 RA RB): inputs j = 0
+// .. RA RB - 1 of output class k1, result slot t holds index k1 + 8 t.
+template <int RA, int RB, int SIGN>
+__device__ __forceinline__ void tail_run(cplxf *v, int k1, const cplxf *tw)
+{
+    constexpr int R = RA * RB;
+    cplxf o[R];
+#pragma unroll
+    for (int j = 0; j < RB; j++) {
+        cplxf u[RA];
+#pragma unroll
+        for (int a = 0; a < RA; a++) {
+            u[a] = v[j + RB * a];
+            if (a > 0) u[a] = twiddle<SIGN>(u[a], ldf(tw + RB * a * k1));
+        }
+        Dft<float, RA>::run(u, SIGN, nullptr, 0);
+#pragma unroll
+        for (int a = 0; a < RA; a++) {
+            if (RB > 1 && j > 0) u[a] = twiddle<SIGN>(u[a], ldf(tw + j * (k1 + 8 * a)));
+            o[RB * a + j] = u[a];
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < RA; a++) {
+        if constexpr (RB > 1) Dft<float, RB>::run(o + RB * a, SIGN, nullptr, 0);
+#pragma unroll
+        for (int b = 0; b < RB; b++) v[a + RA * b] = o[RB * a + b];
+    }
+}
+
+template <int M1, int M2>
+struct RealSlab {
+    static constexpr int RY = M1 / 8, RZ = M2 / 8, H = M2 / 2, MK2 = H + 1, NP = M1 / 2, S = M2 + 1, NT = 4 * M1;
+    static constexpr int BY = tail_b(RY), BZ = tail_b(RZ);
+    static constexpr bool FUSED = RZ == 8;  // the last inverse and the first forward z pass hold the same points
+    static constexpr int SMEM = (NP * S + M1 + M1 + M2) * (int)sizeof(cplxf);
+    static constexpr int FIT = 227 * 1024 / (SMEM + 1024), REG = 1024 / NT;
+    static constexpr int MINB = FIT < 1 ? 1 : FIT < REG ? FIT : REG < 1 ? 1 : REG;
+    static_assert(RY % 2 == 0 && M1 % 8 == 0 && M2 % 8 == 0, "shape");
+
+    cplxf *buf, *col, *twy, *twz;
+
+    __device__ __forceinline__ RealSlab(unsigned char *smem)
+    {
+        buf = reinterpret_cast<cplxf *>(smem);
+        col = buf + NP * S;
+        twy = col + M1;
+        twz = twy + M1;
+    }
+
+    __device__ __forceinline__ void load_tables(const cplxf *tw, int m0) const
+    {
+        for (int i = threadIdx.x; i < M1 + M2; i += NT) stf(twy + i, ldf(tw + m0 + i));
+    }
+
+    template <int COUNT, class F>
+    static __device__ __forceinline__ void each(F f)
+    {
+        if constexpr (COUNT <= NT) {
+            if (COUNT == NT || (int)threadIdx.x < COUNT) f((int)threadIdx.x);
+        } else {
+#pragma unroll 1
+            for (int b = threadIdx.x; b < COUNT; b += NT) f(b);
+        }
+    }
+
+    // Row pair of index t where 8 lanes cover z: the two row pairs of a half-warp
+    // are 8 apart, 8 S = 8 (mod 16) elements, in the other half of the banks.
+    static __device__ __forceinline__ int prow(int t)
+    {
+        if constexpr (NP % 16 == 0)
+            return (t & ~15) + ((t & 15) >> 1) + ((t & 1) << 3);
+        else
+            return t;
+    }
+    // slot of the partner column of kz in a packed row
+    static __device__ __forceinline__ int mirror(int kz) { return kz ? M2 - kz : H; }
+
+    // spectrum slab src [ky][kz] -> packed rows, up to the last z pass
+    __device__ __forceinline__ void inverse_passes(const cplxf *src) const
+    {
+        each<H * RY>([&](int b) {
+            const int kz = b % H, kk = b / H;
+            cplxf v[8];
+#pragma unroll
+            for (int r = 0; r < 8; r++) v[r] = ldf_cg(src + (kk + RY * r) * MK2 + kz);
+            if (kz == 0) {
+#pragma unroll
+                for (int r = 0; r < 8; r++) {
+                    const cplxf ch = ldf_cg(src + (kk + RY * r) * MK2 + H);
+                    v[r] = {v[r].x - ch.y, v[r].y + ch.x};
+                }
+            }
+            Dft<float, 8>::run(v, 1, nullptr, 0);
+            cplxf *p = buf + 4 * kk * S;
+#pragma unroll
+            for (int n = 0; n < 8; n += 2) {
+                stf(p + (n / 2) * S + kz, v[n]);
+                stf(p + (n / 2) * S + mirror(kz), v[n + 1]);
+            }
+        });
+        __syncthreads();
+        each<H * 4>([&](int b) {
+            const int kz = b % H, n = b / H;
+            cplxf e[RY], o[RY], *p = buf + n * S + kz, *q = buf + n * S + mirror(kz);
+#pragma unroll
+            for (int k = 0; k < RY; k++) {
+                e[k] = ldf(p + 4 * k * S);
+                o[k] = ldf(q + 4 * k * S);
+            }
+            tail_run<RY / BY, BY, 1>(e, 2 * n, twy);
+            tail_run<RY / BY, BY, 1>(o, 2 * n + 1, twy);
+            // rows 2p and 2p + 1 as one complex row
+#pragma unroll
+            for (int t = 0; t < RY; t++) {
+                const cplxf A = e[t], B = o[t];
+                if (kz) {
+                    stf(p + 4 * t * S, {A.x - B.y, A.y + B.x});
+                    stf(q + 4 * t * S, {A.x + B.y, B.x - A.y});
+                } else {
+                    stf(p + 4 * t * S, {A.x, B.x});
+                    stf(q + 4 * t * S, {A.y, B.y});
+                }
+            }
+        });
+        __syncthreads();
+        constexpr int PER = (NP * RZ + NT - 1) / NT;
+        cplxf v[PER][8];
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int b = threadIdx.x + i * NT;
+            if ((NP * RZ) % NT == 0 || b < NP * RZ) {
+                const int p = b % NP, kk = b / NP;
+#pragma unroll
+                for (int r = 0; r < 8; r++) v[i][r] = ldf(buf + p * S + kk + RZ * r);
+                Dft<float, 8>::run(v[i], 1, nullptr, 0);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            const int b = threadIdx.x + i * NT;
+            if ((NP * RZ) % NT == 0 || b < NP * RZ) {
+                const int p = b % NP, kk = b / NP;
+#pragma unroll
+                for (int r = 0; r < 8; r++) stf(buf + p * S + r + 8 * kk, v[i][r]);
+            }
+        }
+        __syncthreads();
+    }
+
+    // Real space: a thread holds the points z = n + 8 t, t < RZ, of rows 2p (.x) and
+    // 2p + 1 (.y).  f(v, offset of (2p, n) in the slab) changes (INV) or fills them;
+    // FWD hands them to forward_passes.
+    template <bool INV, bool FWD, class F>
+    __device__ __forceinline__ void real_space(F f) const
+    {
+        const int n = threadIdx.x & 7, p = prow(threadIdx.x >> 3);
+        cplxf v[RZ], *q = buf + p * S + n;
+        if (INV) {
+#pragma unroll
+            for (int t = 0; t < RZ; t++) v[t] = ldf(q + 8 * t);
+            tail_run<RZ / BZ, BZ, 1>(v, n, twz);
+        }
+        f(v, 2 * p * M2 + n);
+        if (FWD) {
+            if constexpr (FUSED) Dft<float, 8>::run(v, -1, nullptr, 0);
+#pragma unroll
+            for (int t = 0; t < RZ; t++) stf(q + 8 * t, v[t]);
+        }
+    }
+
+    // packed rows -> spectrum slab dst [ky][kz]
+    __device__ __forceinline__ void forward_passes(cplxf *dst, bool last) const
+    {
+        __syncthreads();
+        if constexpr (!FUSED) {
+            each<NP * RZ>([&](int b) {
+                const int j = b % RZ, p = b / RZ;
+                cplxf v[8], *q = buf + p * S + j;
+#pragma unroll
+                for (int r = 0; r < 8; r++) v[r] = ldf(q + RZ * r);
+                Dft<float, 8>::run(v, -1, nullptr, 0);
+#pragma unroll
+                for (int r = 0; r < 8; r++) stf(q + RZ * r, v[r]);
+            });
+            __syncthreads();
+        }
+        {
+            const int p = threadIdx.x % NP, k1 = threadIdx.x / NP;  // NT = 8 NP
+            cplxf v[RZ];
+#pragma unroll
+            for (int i = 0; i < RZ; i++) v[i] = ldf(buf + p * S + RZ * k1 + i);
+            tail_run<RZ / BZ, BZ, -1>(v, k1, twz);
+            __syncthreads();
+#pragma unroll
+            for (int t = 0; t < RZ; t++) stf(buf + p * S + k1 + 8 * t, v[t]);
+        }
+        __syncthreads();
+        each<H * (RY / 2)>([&](int b) {
+            const int kz = b % H, a = b / H;
+            cplxf e[8], o[8], *p = buf + a * S + kz, *q = buf + a * S + mirror(kz);
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                const cplxf ck = ldf(p + (RY / 2) * r * S), cm = ldf(q + (RY / 2) * r * S);
+                if (kz) {
+                    e[r] = {(ck.x + cm.x) * 0.5f, (ck.y - cm.y) * 0.5f};
+                    o[r] = {(ck.y + cm.y) * 0.5f, (cm.x - ck.x) * 0.5f};
+                } else {
+                    e[r] = {ck.x, cm.x};
+                    o[r] = {ck.y, cm.y};
+                }
+            }
+            Dft<float, 8>::run(e, -1, nullptr, 0);
+            Dft<float, 8>::run(o, -1, nullptr, 0);
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                stf(p + (RY / 2) * r * S, e[r]);
+                stf(q + (RY / 2) * r * S, o[r]);
+            }
+        });
+        __syncthreads();
+        if (last) pdl_trigger();
+        each<H * 8>([&](int b) {
+            const int kz = b % H, k1 = b / H;
+            cplxf v[RY], *p = buf + (RY / 2) * k1 * S + kz, *q = buf + (RY / 2) * k1 * S + mirror(kz);
+#pragma unroll
+            for (int j = 0; j < RY; j += 2) {
+                v[j] = ldf(p + (j / 2) * S);
+                v[j + 1] = ldf(q + (j / 2) * S);
+            }
+            tail_run<RY / BY, BY, -1>(v, k1, twy);
+            if (kz) {
+#pragma unroll
+                for (int t = 0; t < RY; t++) stf(dst + (k1 + 8 * t) * MK2 + kz, v[t]);
+            } else {
+#pragma unroll
+                for (int t = 0; t < RY; t++) stf(col + k1 + 8 * t, v[t]);
+            }
+        });
+        __syncthreads();
+        // the spectra of the kz = 0 and kz = H columns
+        each<M1>([&](int k) {
+            const cplxf c = ldf(col + k), cm = ldf(col + (k ? M1 - k : 0));
+            stf(dst + k * MK2, {(c.x + cm.x) * 0.5f, (c.y - cm.y) * 0.5f});
+            stf(dst + k * MK2 + H, {(c.y + cm.y) * 0.5f, (cm.x - c.x) * 0.5f});
+        });
+    }
+};
+
+__device__ __forceinline__ const float *real_etab(const PropsArgs<float> &a, int slot, int fld, int s)
+{
+    const Geo &g = a.g;
+    if (g.jon && s == (fld == 0 ? g.jq : g.jqd)) return a.jtab + (size_t)slot * g.M;
+    const int sel = fld == 0 ? (s < g.n1 ? 0 : 1) : (s < g.n2 ? 1 : 0);
+    return a.etab + ((size_t)slot * 2 + sel) * g.M;
+}
+
+// mid: sp = 0 the half-step spectrum (inverse slab, times E2, forward slab), sp = 1
+// the full-step one (inverse slab, P = E2 qs1)
+template <int M1, int M2>
+__global__ void __launch_bounds__(RealSlab<M1, M2>::NT, RealSlab<M1, M2>::MINB) k_real_mid(PropsArgs<float> a, int s)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    using R = RealSlab<M1, M2>;
+    const R B(smem_raw);
+    const Geo &g = a.g;
+    const int x = blockIdx.x, fld = blockIdx.y & 1, sp = blockIdx.y >> 1, slot = blockIdx.z;
+    const size_t off = (size_t)x * M1 * M2;
+    cplxf *spec = a.spec + (((size_t)slot * 2 + fld) * 2 + sp) * g.Mk + (size_t)x * M1 * R::MK2;
+    const float *E = real_etab(a, slot, fld, s) + off;
+    if (threadIdx.x == 0) prefetch_l2(E, M1 * M2 * sizeof(float));
+    B.load_tables(a.tw, g.m0);
+    __syncthreads();
+    pdl_wait();
+    B.inverse_passes(spec);
+    if (sp == 0) {
+        B.template real_space<true, true>([&](cplxf *v, int o) {
+#pragma unroll
+            for (int t = 0; t < R::RZ; t++) {
+                const float e0 = __ldg(E + o + 8 * t), e1 = __ldg(E + o + M2 + 8 * t);
+                v[t].x = __fmul_rn(v[t].x, __fmul_rn(e0, e0));
+                v[t].y = __fmul_rn(v[t].y, __fmul_rn(e1, e1));
+            }
+        });
+        B.forward_passes(spec, true);
+    } else {
+        float *P = a.pbuf + ((size_t)slot * 2 + fld) * g.M + off;
+        B.template real_space<true, false>([&](cplxf *v, int o) {
+#pragma unroll
+            for (int t = 0; t < R::RZ; t++) {
+                const float e0 = __ldg(E + o + 8 * t), e1 = __ldg(E + o + M2 + 8 * t);
+                P[o + 8 * t] = __fmul_rn(v[t].x, __fmul_rn(e0, e0));
+                P[o + M2 + 8 * t] = __fmul_rn(v[t].y, __fmul_rn(e1, e1));
+            }
+        });
+    }
+}
+
+// combine: modes as k_combine_pf
+template <int M1, int M2>
+__global__ void __launch_bounds__(RealSlab<M1, M2>::NT, RealSlab<M1, M2>::MINB)
+    k_real_combine(PropsArgs<float> a, int s, int mode)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    using R = RealSlab<M1, M2>;
+    const R B(smem_raw);
+    const Geo &g = a.g;
+    const int x = blockIdx.x, fld = blockIdx.y, slot = blockIdx.z, sn = s + 1;
+    const size_t off = (size_t)x * M1 * M2;
+    cplxf *specA = a.spec + ((size_t)slot * 2 + fld) * 2 * g.Mk + (size_t)x * M1 * R::MK2, *specB = specA + g.Mk;
+    float *qn = a.hist + (((size_t)slot * (g.Ns + 1) + sn) * 2 + fld) * (size_t)g.M + off;
+    const bool next = sn < g.Ns;
+    const float *E = real_etab(a, slot, fld, s) + off, *En = real_etab(a, slot, fld, next ? sn : 0) + off;
+    const float *P = a.pbuf + ((size_t)slot * 2 + fld) * g.M + off;
+    if (threadIdx.x == 0) prefetch_l2(mode == 0 ? E : En, M1 * M2 * sizeof(float));
+    B.load_tables(a.tw, g.m0);
+    __syncthreads();
+    pdl_wait();
+    // Richardson, GPU_kernels.h:199-203
+    auto finish = [&](cplxf *v, int o) {
+#pragma unroll
+        for (int t = 0; t < R::RZ; t++) {
+            const float q0 = (v[t].x * __ldg(E + o + 8 * t) * 4.0f - __ldcg(P + o + 8 * t)) / 3.0f;
+            const float q1 = (v[t].y * __ldg(E + o + M2 + 8 * t) * 4.0f - __ldcg(P + o + M2 + 8 * t)) / 3.0f;
+            qn[o + 8 * t] = q0;
+            qn[o + M2 + 8 * t] = q1;
+            v[t] = {q0, q1};
+        }
+    };
+    auto scale = [&](cplxf *v, int o) {  // half step input E4' q'
+#pragma unroll
+        for (int t = 0; t < R::RZ; t++)
+            v[t] = {__fmul_rn(v[t].x, __ldg(En + o + 8 * t)), __fmul_rn(v[t].y, __ldg(En + o + M2 + 8 * t))};
+    };
+    if (mode == 0) {
+        if (threadIdx.x == 0) prefetch_l2(P, M1 * M2 * sizeof(float));
+        B.inverse_passes(specA);
+        if (!next) {
+            B.template real_space<true, false>(finish);
+            return;
+        }
+        B.template real_space<true, true>([&](cplxf *v, int o) {
+            finish(v, o);
+            scale(v, o);
+        });
+    } else {
+        B.template real_space<false, true>([&](cplxf *v, int o) {
+#pragma unroll
+            for (int t = 0; t < R::RZ; t++) {
+                if (mode == 1) {
+                    v[t] = {1.0f, 1.0f};
+                    qn[o + 8 * t] = 1.0f;
+                    qn[o + M2 + 8 * t] = 1.0f;
+                } else {
+                    v[t] = {qn[o + 8 * t], qn[o + M2 + 8 * t]};
+                }
+            }
+            if (next) scale(v, o);
+        });
+        if (!next) return;
+    }
+    B.forward_passes(specA, false);
+    // full step input E2' q', from the slice this thread has just stored
+    __syncthreads();
+    B.template real_space<false, true>([&](cplxf *v, int o) {
+#pragma unroll
+        for (int t = 0; t < R::RZ; t++) {
+            const float e0 = __ldg(En + o + 8 * t), e1 = __ldg(En + o + M2 + 8 * t);
+            v[t] = {__fmul_rn(qn[o + 8 * t], __fmul_rn(e0, e0)), __fmul_rn(qn[o + M2 + 8 * t], __fmul_rn(e1, e1))};
+        }
+    });
+    B.forward_passes(specB, true);
+}
+
+}  // namespace scft
