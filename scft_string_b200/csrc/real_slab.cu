@@ -19,7 +19,7 @@ int real_slab_setup(int m1, int m2)
     cudaError_t e = cudaSuccess;
 #define X(A, B)                                                                               \
     if (m1 == A && m2 == B) {                                                                 \
-        e = raise_dyn_smem(k_real_mid<A, B>, RealSlab<A, B>::SMEM);                           \
+        e = raise_dyn_smem(k_real_mid<A, B>, RealSlab<A, B>::SMEM_MID);                          \
         if (e == cudaSuccess) e = raise_dyn_smem(k_real_combine<A, B>, RealSlab<A, B>::SMEM); \
     }
     REAL_SLABS(X)
@@ -32,7 +32,7 @@ void real_mid(const PropsArgs<float> &a, int nslots, int s, cudaStream_t st)
     const Geo &g = a.g;
 #define X(A, B)                                                                                                   \
     if (g.m1 == A && g.m2 == B)                                                                                   \
-        launch_step(k_real_mid<A, B>, dim3(g.m0, 4, nslots), RealSlab<A, B>::NT, RealSlab<A, B>::SMEM, 1, 1, st, a, s);
+        launch_step(k_real_mid<A, B>, dim3(g.m0, 4, nslots), RealSlab<A, B>::NT, RealSlab<A, B>::SMEM_MID, 1, 1, st, a, s);
     REAL_SLABS(X)
 #undef X
 }

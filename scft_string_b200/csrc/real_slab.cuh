@@ -12,6 +12,13 @@
 // makes three trips through shared memory; it made five to seven, with a barrier
 // before and after each stage.
 //
+// The real-space operands (the E table, P, q) come and go through padded copies
+// in shared memory, moved by bulk copies a row pair at a time: a thread holds the
+// points n + 8 t of two rows, so a warp would touch global memory in runs of 32
+// bytes, four wavefronts an access (they were 40 % of the LSU's work at 64^3; 16
+// replicas of 64^3 9.15 -> 8.75 us per replica step).  Slabs of 96 and 128 rows go
+// without: the copies would halve the CTAs per SM (96^3 44 us without, 57 with).
+//
 // Products that feed an addition directly are rounded on their own (__fmul_rn):
 // they went through shared memory before, and a fused multiply-add would round
 // differently.
@@ -20,6 +27,7 @@
 #include "fft.cuh"
 #include "kernels.h"
 #include "pdl.cuh"
+#include "tma.cuh"
 
 namespace scft {
 
@@ -84,16 +92,48 @@ struct RealSlab {
     static constexpr int RY = M1 / 8, RZ = M2 / 8, H = M2 / 2, MK2 = H + 1, NP = M1 / 2, S = M2 + 1, NT = 4 * M1;
     static constexpr int BY = tail_b(RY), BZ = tail_b(RZ);
     static constexpr bool FUSED = RZ == 8;  // the last inverse and the first forward z pass hold the same points
-    static constexpr int SMEM = (NP * S + M1 + M1 + M2) * (int)sizeof(cplxf);
+    // staged copy of a real slab: row pair p at stage_at(p), padded so that the four
+    // row pairs of a warp fall into different banks
+    static constexpr int STAGE = NP * (2 * M2 + 8) + 16 * (NP / 8);  // floats
+    static constexpr int BASE = 128 + (NP * S + M1 + M1 + M2) * (int)sizeof(cplxf);
+    static constexpr bool STAGED = M1 <= 64;
+    static constexpr int SMEM_MID = BASE + (STAGED ? STAGE * 4 : 0), SMEM = BASE + (STAGED ? 2 * STAGE * 4 : 0);
     static constexpr int FIT = 227 * 1024 / (SMEM + 1024), REG = 1024 / NT;
     static constexpr int MINB = FIT < 1 ? 1 : FIT < REG ? FIT : REG < 1 ? 1 : REG;
     static_assert(RY % 2 == 0 && M1 % 8 == 0 && M2 % 8 == 0, "shape");
 
+    uint64_t *bars;
     cplxf *buf, *col, *twy, *twz;
+    float *Es, *Qs;  // staged E table; staged P, then q'
+
+    static __device__ __forceinline__ int stage_at(int p) { return p * (2 * M2 + 8) + 16 * (p >> 3); }
+
+    // Bulk copies of a real slab, a row pair each, by warp 0.
+    __device__ __forceinline__ void stage_in(float *dst, const float *src, uint64_t *bar) const
+    {
+        if (threadIdx.x >= 32) return;
+        if (threadIdx.x == 0) mbar_expect_tx(bar, M1 * M2 * sizeof(float));
+        __syncwarp();
+        for (int p = threadIdx.x; p < NP; p += 32) bulk_g2s(dst + stage_at(p), src + p * 2 * M2, 2 * M2 * sizeof(float), bar);
+    }
+    // after a fence by the writers and a barrier; stage_out_done before the CTA exits
+    __device__ __forceinline__ void stage_out(float *dst, const float *src) const
+    {
+        if (threadIdx.x >= 32) return;
+        for (int p = threadIdx.x; p < NP; p += 32) bulk_s2g(dst + p * 2 * M2, src + stage_at(p), 2 * M2 * sizeof(float));
+        bulk_commit();
+    }
+    __device__ __forceinline__ void stage_out_done() const
+    {
+        if (threadIdx.x < 32) tma_store_wait_read();
+    }
 
     __device__ __forceinline__ RealSlab(unsigned char *smem)
     {
-        buf = reinterpret_cast<cplxf *>(smem);
+        bars = reinterpret_cast<uint64_t *>(smem);
+        buf = reinterpret_cast<cplxf *>(smem + 128);
+        Es = reinterpret_cast<float *>(smem + BASE);
+        Qs = Es + STAGE;
         col = buf + NP * S;
         twy = col + M1;
         twz = twy + M1;
@@ -201,8 +241,8 @@ struct RealSlab {
     }
 
     // Real space: a thread holds the points z = n + 8 t, t < RZ, of rows 2p (.x) and
-    // 2p + 1 (.y).  f(v, offset of (2p, n) in the slab) changes (INV) or fills them;
-    // FWD hands them to forward_passes.
+    // 2p + 1 (.y).  f(v, offset of (2p, n) in the slab, in a staged copy) changes (INV)
+    // or fills them; FWD hands them to forward_passes.
     template <bool INV, bool FWD, class F>
     __device__ __forceinline__ void real_space(F f) const
     {
@@ -213,7 +253,7 @@ struct RealSlab {
             for (int t = 0; t < RZ; t++) v[t] = ldf(q + 8 * t);
             tail_run<RZ / BZ, BZ, 1>(v, n, twz);
         }
-        f(v, 2 * p * M2 + n);
+        f(v, 2 * p * M2 + n, stage_at(p) + n);
         if (FWD) {
             if constexpr (FUSED) Dft<float, 8>::run(v, -1, nullptr, 0);
 #pragma unroll
@@ -320,35 +360,54 @@ __global__ void __launch_bounds__(RealSlab<M1, M2>::NT, RealSlab<M1, M2>::MINB) 
     const size_t off = (size_t)x * M1 * M2;
     cplxf *spec = a.spec + (((size_t)slot * 2 + fld) * 2 + sp) * g.Mk + (size_t)x * M1 * R::MK2;
     const float *E = real_etab(a, slot, fld, s) + off;
-    if (threadIdx.x == 0) prefetch_l2(E, M1 * M2 * sizeof(float));
+    float *P = a.pbuf + ((size_t)slot * 2 + fld) * g.M + off;
+    // table value and P at offset i of the slab, is of a staged copy
+    auto e_at = [&](int i, int is) { return R::STAGED ? B.Es[is] : __ldg(E + i); };
+    if constexpr (R::STAGED) {
+        if (threadIdx.x == 0) {
+            mbar_init(&B.bars[0], 1);
+            mbar_fence_init();
+        }
+        B.stage_in(B.Es, E, &B.bars[0]);  // constant over the chain
+    } else {
+        if (threadIdx.x == 0) prefetch_l2(E, M1 * M2 * sizeof(float));
+    }
     B.load_tables(a.tw, g.m0);
     __syncthreads();
     pdl_wait();
     B.inverse_passes(spec);
+    if constexpr (R::STAGED) mbar_wait(&B.bars[0], 0, a.err);
     if (sp == 0) {
-        B.template real_space<true, true>([&](cplxf *v, int o) {
+        B.template real_space<true, true>([&](cplxf *v, int o, int os) {
 #pragma unroll
             for (int t = 0; t < R::RZ; t++) {
-                const float e0 = __ldg(E + o + 8 * t), e1 = __ldg(E + o + M2 + 8 * t);
+                const float e0 = e_at(o + 8 * t, os + 8 * t), e1 = e_at(o + M2 + 8 * t, os + M2 + 8 * t);
                 v[t].x = __fmul_rn(v[t].x, __fmul_rn(e0, e0));
                 v[t].y = __fmul_rn(v[t].y, __fmul_rn(e1, e1));
             }
         });
         B.forward_passes(spec, true);
     } else {
-        float *P = a.pbuf + ((size_t)slot * 2 + fld) * g.M + off;
-        B.template real_space<true, false>([&](cplxf *v, int o) {
+        B.template real_space<true, false>([&](cplxf *v, int o, int os) {
 #pragma unroll
             for (int t = 0; t < R::RZ; t++) {
-                const float e0 = __ldg(E + o + 8 * t), e1 = __ldg(E + o + M2 + 8 * t);
-                P[o + 8 * t] = __fmul_rn(v[t].x, __fmul_rn(e0, e0));
-                P[o + M2 + 8 * t] = __fmul_rn(v[t].y, __fmul_rn(e1, e1));
+                const float e0 = e_at(o + 8 * t, os + 8 * t), e1 = e_at(o + M2 + 8 * t, os + M2 + 8 * t);
+                const float p0 = __fmul_rn(v[t].x, __fmul_rn(e0, e0)), p1 = __fmul_rn(v[t].y, __fmul_rn(e1, e1));
+                (R::STAGED ? B.Es + os : P + o)[8 * t] = p0;
+                (R::STAGED ? B.Es + os : P + o)[M2 + 8 * t] = p1;
             }
         });
+        if constexpr (R::STAGED) {
+            fence_proxy_async_smem();
+            __syncthreads();
+            B.stage_out(P, B.Es);
+            B.stage_out_done();
+        }
     }
 }
 
-// combine: modes as k_combine_pf
+// combine: finishes step s (mode 0: Richardson combination; mode 1: q(s+1) = 1;
+// mode 2: q(s+1) from the propagator store) and starts step s + 1
 template <int M1, int M2>
 __global__ void __launch_bounds__(RealSlab<M1, M2>::NT, RealSlab<M1, M2>::MINB)
     k_real_combine(PropsArgs<float> a, int s, int mode)
@@ -362,66 +421,98 @@ __global__ void __launch_bounds__(RealSlab<M1, M2>::NT, RealSlab<M1, M2>::MINB)
     cplxf *specA = a.spec + ((size_t)slot * 2 + fld) * 2 * g.Mk + (size_t)x * M1 * R::MK2, *specB = specA + g.Mk;
     float *qn = a.hist + (((size_t)slot * (g.Ns + 1) + sn) * 2 + fld) * (size_t)g.M + off;
     const bool next = sn < g.Ns;
-    const float *E = real_etab(a, slot, fld, s) + off, *En = real_etab(a, slot, fld, next ? sn : 0) + off;
+    const float *En = real_etab(a, slot, fld, next ? sn : 0) + off;
+    const float *E = mode == 0 ? real_etab(a, slot, fld, s) + off : En;
     const float *P = a.pbuf + ((size_t)slot * 2 + fld) * g.M + off;
-    if (threadIdx.x == 0) prefetch_l2(mode == 0 ? E : En, M1 * M2 * sizeof(float));
+    const bool same = E == En;  // the next step's table, unless the chain changes blocks here
+    // table of step s, of step s + 1, P, and q' at offset i of the slab, is of a staged copy
+    auto e_at = [&](int i, int is) { return R::STAGED ? B.Es[is] : __ldg(E + i); };
+    auto en_at = [&](int i, int is) { return R::STAGED && same ? B.Es[is] : __ldg(En + i); };
+    auto p_at = [&](int i, int is) { return R::STAGED ? B.Qs[is] : __ldcg(P + i); };
+    auto q_at = [&](int i, int is) -> float & { return R::STAGED ? B.Qs[is] : qn[i]; };
+    if constexpr (R::STAGED) {
+        if (threadIdx.x == 0) {
+            mbar_init(&B.bars[0], 1);
+            mbar_init(&B.bars[1], 1);
+            mbar_fence_init();
+        }
+        B.stage_in(B.Es, E, &B.bars[0]);  // constant over the chain
+    } else {
+        if (threadIdx.x == 0) prefetch_l2(E, M1 * M2 * sizeof(float));
+    }
     B.load_tables(a.tw, g.m0);
     __syncthreads();
     pdl_wait();
+    if constexpr (R::STAGED) {
+        if (mode != 1) B.stage_in(B.Qs, mode == 0 ? P : qn, &B.bars[1]);
+    } else {
+        if (mode == 0 && threadIdx.x == 0) prefetch_l2(P, M1 * M2 * sizeof(float));
+    }
+    auto scale = [&](cplxf *v, int o, int os) {  // half step input E4' q'
+#pragma unroll
+        for (int t = 0; t < R::RZ; t++)
+            v[t] = {__fmul_rn(v[t].x, en_at(o + 8 * t, os + 8 * t)), __fmul_rn(v[t].y, en_at(o + M2 + 8 * t, os + M2 + 8 * t))};
+    };
     // Richardson, GPU_kernels.h:199-203
-    auto finish = [&](cplxf *v, int o) {
+    auto finish = [&](cplxf *v, int o, int os) {
 #pragma unroll
         for (int t = 0; t < R::RZ; t++) {
-            const float q0 = (v[t].x * __ldg(E + o + 8 * t) * 4.0f - __ldcg(P + o + 8 * t)) / 3.0f;
-            const float q1 = (v[t].y * __ldg(E + o + M2 + 8 * t) * 4.0f - __ldcg(P + o + M2 + 8 * t)) / 3.0f;
-            qn[o + 8 * t] = q0;
-            qn[o + M2 + 8 * t] = q1;
+            const int i = o + 8 * t, is = os + 8 * t;
+            const float q0 = (v[t].x * e_at(i, is) * 4.0f - p_at(i, is)) / 3.0f;
+            const float q1 = (v[t].y * e_at(i + M2, is + M2) * 4.0f - p_at(i + M2, is + M2)) / 3.0f;
+            q_at(i, is) = q0;
+            q_at(i + M2, is + M2) = q1;
             v[t] = {q0, q1};
         }
     };
-    auto scale = [&](cplxf *v, int o) {  // half step input E4' q'
-#pragma unroll
-        for (int t = 0; t < R::RZ; t++)
-            v[t] = {__fmul_rn(v[t].x, __ldg(En + o + 8 * t)), __fmul_rn(v[t].y, __ldg(En + o + M2 + 8 * t))};
-    };
     if (mode == 0) {
-        if (threadIdx.x == 0) prefetch_l2(P, M1 * M2 * sizeof(float));
         B.inverse_passes(specA);
-        if (!next) {
-            B.template real_space<true, false>(finish);
-            return;
+        if constexpr (R::STAGED) {
+            mbar_wait(&B.bars[0], 0, a.err);
+            mbar_wait(&B.bars[1], 0, a.err);
         }
-        B.template real_space<true, true>([&](cplxf *v, int o) {
-            finish(v, o);
-            scale(v, o);
-        });
+        if (next)
+            B.template real_space<true, true>([&](cplxf *v, int o, int os) {
+                finish(v, o, os);
+                scale(v, o, os);
+            });
+        else
+            B.template real_space<true, false>(finish);
     } else {
-        B.template real_space<false, true>([&](cplxf *v, int o) {
+        if constexpr (R::STAGED) {
+            mbar_wait(&B.bars[0], 0, a.err);
+            if (mode == 2) mbar_wait(&B.bars[1], 0, a.err);
+        }
+        B.template real_space<false, true>([&](cplxf *v, int o, int os) {
 #pragma unroll
             for (int t = 0; t < R::RZ; t++) {
-                if (mode == 1) {
-                    v[t] = {1.0f, 1.0f};
-                    qn[o + 8 * t] = 1.0f;
-                    qn[o + M2 + 8 * t] = 1.0f;
-                } else {
-                    v[t] = {qn[o + 8 * t], qn[o + M2 + 8 * t]};
-                }
+                const int i = o + 8 * t, is = os + 8 * t;
+                if (mode == 1) q_at(i, is) = q_at(i + M2, is + M2) = 1.0f;
+                v[t] = mode == 1 ? cplxf{1.0f, 1.0f} : cplxf{q_at(i, is), q_at(i + M2, is + M2)};
             }
-            if (next) scale(v, o);
+            scale(v, o, os);
         });
-        if (!next) return;
     }
-    B.forward_passes(specA, false);
-    // full step input E2' q', from the slice this thread has just stored
-    __syncthreads();
-    B.template real_space<false, true>([&](cplxf *v, int o) {
+    if constexpr (R::STAGED) {
+        fence_proxy_async_smem();
+        __syncthreads();
+        if (mode != 2) B.stage_out(qn, B.Qs);
+    }
+    if (next) {
+        B.forward_passes(specA, false);
+        // full step input E2' q'
+        __syncthreads();
+        B.template real_space<false, true>([&](cplxf *v, int o, int os) {
 #pragma unroll
-        for (int t = 0; t < R::RZ; t++) {
-            const float e0 = __ldg(En + o + 8 * t), e1 = __ldg(En + o + M2 + 8 * t);
-            v[t] = {__fmul_rn(qn[o + 8 * t], __fmul_rn(e0, e0)), __fmul_rn(qn[o + M2 + 8 * t], __fmul_rn(e1, e1))};
-        }
-    });
-    B.forward_passes(specB, true);
+            for (int t = 0; t < R::RZ; t++) {
+                const int i = o + 8 * t, is = os + 8 * t;
+                const float e0 = en_at(i, is), e1 = en_at(i + M2, is + M2);
+                v[t] = {__fmul_rn(q_at(i, is), __fmul_rn(e0, e0)), __fmul_rn(q_at(i + M2, is + M2), __fmul_rn(e1, e1))};
+            }
+        });
+        B.forward_passes(specB, true);
+    }
+    if constexpr (R::STAGED) B.stage_out_done();
 }
 
 }  // namespace scft

@@ -94,6 +94,14 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int x, int 
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 
+// bulk copy shared -> global, 16-byte aligned multiples of 16; completes with tma_store_wait_read
+__device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes)
+{
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_addr(src)), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+
 __device__ __forceinline__ void tma_store_wait_read()
 {
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
