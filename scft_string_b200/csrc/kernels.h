@@ -101,6 +101,8 @@ bool real_slab_has(int m1, int m2);
 int real_slab_setup(int m1, int m2);
 void real_mid(const PropsArgs<float> &a, int nslots, int s, cudaStream_t st);
 void real_combine(const PropsArgs<float> &a, int nslots, int s, int mode, cudaStream_t st);
+int real_pencil_setup(int m0);
+void real_pencil(const PropsArgs<float> &a, int nslots, int both, int wide, cudaStream_t st);
 
 void pf_smem_bytes(int id, int fp32, int &mid, int &comb);
 // dynamic shared memory of k_pencil_sh for tiles of tc columns

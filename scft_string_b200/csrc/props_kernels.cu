@@ -618,16 +618,6 @@ __device__ __forceinline__ void pencil_tma_body(const CUtensorMap &tmap, const P
     if (threadIdx.x == 0) tma_store_wait_read();
 }
 
-template <typename T, int MT, int FM0, int FM1, int FM2, int TC>
-__global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1)
-    k_pencil_tma(const __grid_constant__ CUtensorMap tmap, PropsArgs<T> a, int both)
-{
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    // opposite order of the slab kernels before and after: what they touched last is still in L2
-    pencil_tma_body<T, MT, FM0, FM1, FM2, TC>(tmap, a, both, gridDim.x - 1 - blockIdx.x, gridDim.y - 1 - blockIdx.y,
-                                              gridDim.z - 1 - blockIdx.z, smem_raw);
-}
-
 // ---------------------------------------------------------------- shuffle pencil (m0 = 64)
 // Opt-in (SCFT_PENCIL_SHUFFLE=1): on the 16-replica 64^3 string it measured
 // as fast as the Stockham pencil at the same tile width and 2 % slower than
@@ -1216,28 +1206,21 @@ void launch_pencil(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gp, int bot
             return;
         }
     }
-    if constexpr (F1 != 0) {
-        if (L.tma_pencil) {
-            // tile width: kTile columns, or twice that (two butterflies per
-            // thread between barriers) when the autotuner picked it
+    if constexpr (F1 != 0 && sizeof(T) == 4) {
+        if (L.pf && !L.pencil_sh) {
+            real_pencil(a, gp.z, both, L.ptile_wide, st);
+            return;
+        }
+    }
+    if constexpr (F0 == 64 && sizeof(T) == 4) {
+        if (L.pencil_sh) {
             constexpr int TC = kTile<T>::value, ncol = F1 * (F2 / 2 + 1);
-            if constexpr (F0 == 64) {
-                if (L.pencil_sh) {
-                    if (L.ptile_wide)
-                        k_pencil_sh<T, MT, F0, F1, F2, 2 * TC><<<dim3((ncol + 2 * TC - 1) / (2 * TC), gp.y, gp.z), MT,
-                                                                 L.pencil_tma_smem_wide, st>>>(*L.tmap_wide, a, both);
-                    else
-                        k_pencil_sh<T, MT, F0, F1, F2, TC><<<dim3((ncol + TC - 1) / TC, gp.y, gp.z), MT,
-                                                             L.pencil_tma_smem, st>>>(*L.tmap, a, both);
-                    return;
-                }
-            }
             if (L.ptile_wide)
-                launch_step(k_pencil_tma<T, MT, F0, F1, F2, 2 * TC>, dim3((ncol + 2 * TC - 1) / (2 * TC), gp.y, gp.z), MT,
-                            L.pencil_tma_smem_wide, 1, 1, st, *L.tmap_wide, a, both);
+                k_pencil_sh<T, MT, F0, F1, F2, 2 * TC><<<dim3((ncol + 2 * TC - 1) / (2 * TC), gp.y, gp.z), MT,
+                                                         L.pencil_tma_smem_wide, st>>>(*L.tmap_wide, a, both);
             else
-                launch_step(k_pencil_tma<T, MT, F0, F1, F2, TC>, dim3((ncol + TC - 1) / TC, gp.y, gp.z), MT,
-                            L.pencil_tma_smem, 1, 1, st, *L.tmap, a, both);
+                k_pencil_sh<T, MT, F0, F1, F2, TC><<<dim3((ncol + TC - 1) / TC, gp.y, gp.z), MT, L.pencil_tma_smem,
+                                                     st>>>(*L.tmap, a, both);
             return;
         }
     }
@@ -1349,9 +1332,6 @@ int set_smem_mt(const PropsLaunch &L)
     cudaError_t e4 = cudaSuccess, e5 = cudaSuccess;
     if constexpr (F1 != 0) {
         if (L.tma_pencil) {
-            e4 = raise_dyn_smem(k_pencil_tma<T, MT, F0, F1, F2, kTile<T>::value>, L.pencil_tma_smem);
-            if (e4 == cudaSuccess && L.tmap_wide)
-                e4 = raise_dyn_smem(k_pencil_tma<T, MT, F0, F1, F2, 2 * kTile<T>::value>, L.pencil_tma_smem_wide);
             if constexpr (F0 == 64) {
                 if (e4 == cudaSuccess && L.pencil_sh) {
                     e4 = raise_dyn_smem(k_pencil_sh<T, MT, F0, F1, F2, kTile<T>::value>, L.pencil_tma_smem);
@@ -1362,7 +1342,7 @@ int set_smem_mt(const PropsLaunch &L)
             }
         }
         if (e4 == cudaSuccess && L.pf) {
-            if (real_slab_setup(F1, F2) != 0) e5 = cudaErrorInvalidValue;
+            if (real_slab_setup(F1, F2) != 0 || real_pencil_setup(F0) != 0) e5 = cudaErrorInvalidValue;
         }
     }
     int e6 = 0;

@@ -48,4 +48,46 @@ void real_combine(const PropsArgs<float> &a, int nslots, int s, int mode, cudaSt
 #undef X
 }
 
+#define REAL_AXES(X) X(32) X(48) X(64) X(96) X(128)
+constexpr int kRealTile = 32;
+
+int real_pencil_setup(int m0)
+{
+    cudaError_t e = cudaSuccess;
+#define X(A)                                                                                            \
+    if (m0 == A) {                                                                                      \
+        e = raise_dyn_smem(k_real_pencil<A, kRealTile>, RealPencil<A, kRealTile>::SMEM);                \
+        if (e == cudaSuccess)                                                                           \
+            e = raise_dyn_smem(k_real_pencil<A, 2 * kRealTile>, RealPencil<A, 2 * kRealTile>::SMEM);    \
+    }
+    REAL_AXES(X)
+#undef X
+    return e == cudaSuccess ? 0 : -1;
+}
+
+void real_pencil(const PropsArgs<float> &a, int nslots, int both, int wide, cudaStream_t st)
+{
+    const Geo &g = a.g;
+    // Wide tiles where they still fill the SMs four times: 512-byte rows (16 replicas
+    // of 64^3 8.8 us per replica step against 9.2, of 48^3 79.7 us a step against
+    // 82.0).  Small batches want more blocks (one replica 24.2 us wide, 22.1
+    // narrow), and the longer axes spill at twice the butterflies per thread (eight
+    // replicas of 128^3 109 us wide, 93 narrow).
+    const int ncol = g.m1 * g.mk2, wtiles = (ncol + 2 * kRealTile - 1) / (2 * kRealTile);
+    wide = wide || (g.m0 <= 64 && wtiles * (both ? 4 : 2) * nslots >= 4 * 148);
+    const int tc = wide ? 2 * kRealTile : kRealTile;
+    const dim3 grid((ncol + tc - 1) / tc, both ? 4 : 2, nslots);
+#define X(A)                                                                                                        \
+    if (g.m0 == A) {                                                                                                \
+        if (wide)                                                                                                   \
+            launch_step(k_real_pencil<A, 2 * kRealTile>, grid, kRealPencilThreads, RealPencil<A, 2 * kRealTile>::SMEM, \
+                        1, 1, st, a);                                                                               \
+        else                                                                                                        \
+            launch_step(k_real_pencil<A, kRealTile>, grid, kRealPencilThreads, RealPencil<A, kRealTile>::SMEM, 1, 1, \
+                        st, a);                                                                                     \
+    }
+    REAL_AXES(X)
+#undef X
+}
+
 }  // namespace scft

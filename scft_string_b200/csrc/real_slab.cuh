@@ -515,4 +515,119 @@ __global__ void __launch_bounds__(RealSlab<M1, M2>::NT, RealSlab<M1, M2>::MINB)
     if constexpr (R::STAGED) B.stage_out_done();
 }
 
+// ---------------------------------------------------------------- x pass
+// The inverse of tail_run for the x pass: slots t = a + RA b (frequency k1 + 8 t)
+// back to points m = 0 .. RA RB - 1, in the stage order of fft_pair_fused (the
+// radices reversed), then the factor of the radix-8 stage that follows.
+template <int RA, int RB>
+__device__ __forceinline__ void tail_back(cplxf *v, int k1, const cplxf *tw)
+{
+    constexpr int R = RA * RB;
+    cplxf o[R];
+#pragma unroll
+    for (int a = 0; a < RA; a++) {
+        cplxf u[RB];
+#pragma unroll
+        for (int b = 0; b < RB; b++) u[b] = v[a + RA * b];
+        if constexpr (RB > 1) Dft<float, RB>::run(u, 1, nullptr, 0);
+#pragma unroll
+        for (int b = 0; b < RB; b++) o[RA * b + a] = (RB > 1 && a > 0) ? twiddle<1>(u[b], ldf(tw + 8 * a * b)) : u[b];
+    }
+#pragma unroll
+    for (int b = 0; b < RB; b++) {
+        Dft<float, RA>::run(o + RA * b, 1, nullptr, 0);
+#pragma unroll
+        for (int r = 0; r < RA; r++) {
+            const int m = b + RB * r;
+            v[m] = m > 0 ? twiddle<1>(o[RA * b + r], ldf(tw + k1 * m)) : o[RA * b + r];
+        }
+    }
+}
+
+template <int M0, int TC>
+struct RealPencil {
+    static constexpr int SMEM = (M0 * TC + M0) * (int)sizeof(cplxf) + (M0 + TC) * (int)sizeof(float);
+};
+constexpr int kRealPencilThreads = 256;
+
+// One tile of TC columns of one spectrum: forward x transform, diffusion factor
+// (Mult_self, GPU_kernels.h:175-181), inverse transform, with one trip through
+// shared memory on each side of the factor.  sp 0: times K2, 1: times K1.
+template <int M0, int TC>
+__global__ void __launch_bounds__(kRealPencilThreads, 4) k_real_pencil(PropsArgs<float> a)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    constexpr int R2 = M0 / 8, RB = tail_b(R2), RA = R2 / RB, NT = kRealPencilThreads;
+    const Geo &g = a.g;
+    // opposite order of the slab kernels before and after: what they touched last is still in L2
+    const int tile = gridDim.x - 1 - blockIdx.x, slot = gridDim.z - 1 - blockIdx.z;
+    const int fld = blockIdx.y & 1, sp = blockIdx.y >> 1;
+    const int ncol = g.m1 * g.mk2, c0 = tile * TC;
+    cplxf *buf = reinterpret_cast<cplxf *>(smem_raw), *tw = buf + M0 * TC;
+    float *gx = reinterpret_cast<float *>(tw + M0), *colf = gx + M0;
+    cplxf *spec = a.spec + (((size_t)slot * 2 + fld) * 2 + sp) * g.Mk + c0;
+    const float *kf = a.kfac + (size_t)__ldg(a.slot_rep + slot) * a.kf_stride;  // the replica's box
+    for (int i = threadIdx.x; i < M0; i += NT) {
+        stf(tw + i, ldf(a.tw + i));
+        gx[i] = __ldg(kf + i);
+    }
+    for (int t = threadIdx.x; t < TC; t += NT) {
+        const int c = c0 + t, y = c / g.mk2, kz = c - y * g.mk2;
+        colf[t] = c < ncol ? __ldg(kf + M0 + y) * __ldg(kf + M0 + g.m1 + kz) : 0.0f;
+    }
+    pdl_wait();
+#pragma unroll 1
+    for (int b = threadIdx.x; b < R2 * TC; b += NT) {
+        const int t = b % TC, j = b / TC;
+        if (c0 + t < ncol) {
+            cplxf v[8];
+#pragma unroll
+            for (int r = 0; r < 8; r++) v[r] = ldf_cg(spec + (size_t)(j + R2 * r) * ncol + t);
+            Dft<float, 8>::run(v, -1, nullptr, 0);
+#pragma unroll
+            for (int r = 0; r < 8; r++) stf(buf + (j + R2 * r) * TC + t, v[r]);
+        }
+    }
+    __syncthreads();
+    const float invM = a.invM, Mreal = a.Mreal;
+#pragma unroll 1
+    for (int b = threadIdx.x; b < 8 * TC; b += NT) {
+        const int t = b % TC, k1 = b / TC;
+        if (c0 + t < ncol) {
+            cplxf v[R2], *p = buf + R2 * k1 * TC + t;
+#pragma unroll
+            for (int i = 0; i < R2; i++) v[i] = ldf(p + i * TC);
+            tail_run<RA, RB, -1>(v, k1, tw);
+            // K2 = g/M, K1 = g^2/M  (Prepare_dev_expKsq2_expKsq, GPU_kernels.h:207-213);
+            // the product may fuse with the additions that follow, as it does in
+            // fft_pair_fused
+            const float ct = colf[t];
+#pragma unroll
+            for (int i = 0; i < R2; i++) {
+                const float k2 = gx[k1 + 8 * i] * ct;
+                const float f = sp == 0 ? k2 * invM : (k2 * invM) * (k2 * invM) * Mreal;
+                v[i].x *= f;
+                v[i].y *= f;
+            }
+            tail_back<RA, RB>(v, k1, tw);
+#pragma unroll
+            for (int i = 0; i < R2; i++) stf(p + i * TC, v[i]);
+        }
+    }
+    __syncthreads();
+    pdl_trigger();
+#pragma unroll 1
+    for (int b = threadIdx.x; b < R2 * TC; b += NT) {
+        const int t = b % TC, m = b / TC;
+        if (c0 + t < ncol) {
+            cplxf v[8];
+#pragma unroll
+            for (int r = 0; r < 8; r++) v[r] = ldf(buf + (m + R2 * r) * TC + t);
+            Dft<float, 8>::run(v, 1, nullptr, 0);
+#pragma unroll
+            for (int r = 0; r < 8; r++) stf(spec + (size_t)(m + R2 * r) * ncol + t, v[r]);
+        }
+    }
+}
+
 }  // namespace scft
