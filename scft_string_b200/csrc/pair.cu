@@ -50,29 +50,6 @@ __global__ void __launch_bounds__(kPencilThreads, pencil_minb(M0)) k_pair_pencil
                                                 smem_raw);
 }
 
-// shapes without kernels of their own
-template <int RA>
-__global__ void __launch_bounds__(512, 1) k_pair_mid_any(PropsArgs<T> a, int s, PairAny q)
-{
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    pair_mid_body(PairSlabAny<RA>(smem_raw, q), a, s, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
-template <int RA>
-__global__ void __launch_bounds__(512, 1) k_pair_combine_any(PropsArgs<T> a, int s, int mode, PairAny q)
-{
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    pair_combine_body(PairSlabAny<RA>(smem_raw, q), a, s, mode, blockIdx.x, gridDim.y == 1 ? -1 : (int)blockIdx.y,
-                      blockIdx.z);
-}
-
-template <int R2>
-__global__ void __launch_bounds__(kPencilThreads, 2) k_pair_pencil_any(PropsArgs<T> a, int ra, int rb)
-{
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    pair_pencil_any_body<R2, kTile>(a, gridDim.x - 1 - blockIdx.x, blockIdx.y, gridDim.z - 1 - blockIdx.z, ra, rb, smem_raw);
-}
-
 __device__ __forceinline__ int ld_acquire_gpu(const int *p)
 {
     int v;
@@ -183,23 +160,7 @@ int pair_setup(int m0, int m1, int m2, int *grid)
     }
     PAIR_AXES(X)
 #undef X
-    PairAny q;
-    int r1, r2;
-    if (!pair_slab_fixed(m1, m2) && pair_any_plan(m1, m2, q)) switch (q.ra) {
-#define X(A)                                           \
-    case A:                                            \
-        up(k_pair_mid_any<A>, pair_any_smem(q));            \
-        up(k_pair_combine_any<A>, pair_any_smem(q));        \
-        break;
-            PAIR_RADICES(X)
-#undef X
-        }
-    if (!pair_axis_fixed(m0) && pair_x_radices(m0, r1, r2)) switch (r2) {
-#define X(A) \
-    case A: up(k_pair_pencil_any<A>, pair_any_pencil_smem(m0)); break;
-            PAIR_RADICES(X)
-#undef X
-        }
+    if (e == cudaSuccess && pair_any_setup(m0, m1, m2) != 0) return -1;
     *grid = 0;
 #define X(A, B, C)                                                                                             \
     if (m0 == A && m1 == B && m2 == C) {                                                                       \
@@ -231,13 +192,7 @@ void pair_mid(const PropsArgs<T> &a, int nslots, int s, cudaStream_t st)
     }
     PAIR_SLABS(X)
 #undef X
-    PairAny q;
-    if (pair_any_plan(g.m1, g.m2, q)) switch (q.ra) {
-#define X(A)                                                                                                           \
-    case A: launch_step(k_pair_mid_any<A>, dim3(g.m0, 2, nslots), pair_any_threads(q), pair_any_smem(q), 1, 1, st, a, s, q); break;
-            PAIR_RADICES(X)
-#undef X
-        }
+    pair_any_mid(a, nslots, s, st);
 }
 
 void pair_combine(const PropsArgs<T> &a, int nslots, int s, int mode, cudaStream_t st)
@@ -256,16 +211,7 @@ void pair_combine(const PropsArgs<T> &a, int nslots, int s, int mode, cudaStream
     }
     PAIR_SLABS(X)
 #undef X
-    PairAny q;
-    if (pair_any_plan(g.m1, g.m2, q)) switch (q.ra) {
-#define X(A)                                                                                                         \
-    case A:                                                                                                          \
-        launch_step(k_pair_combine_any<A>, dim3(g.m0, split, nslots), pair_any_threads(q), pair_any_smem(q), 1, split, st, a, \
-                    s, mode, q);                                                                                     \
-        break;
-            PAIR_RADICES(X)
-#undef X
-        }
+    pair_any_combine(a, nslots, s, mode, split, st);
 }
 
 void pair_pencil(const PropsArgs<T> &a, int nslots, int both, int wide, cudaStream_t st)
@@ -274,15 +220,8 @@ void pair_pencil(const PropsArgs<T> &a, int nslots, int both, int wide, cudaStre
     const int tc = wide ? 2 * kTile : kTile;
     int ra = 1, rb = 1;
     pair_y_radices(g.m1, g.m2, ra, rb);
-    int r1, r2;
-    if (!pair_axis_fixed(g.m0) && pair_x_radices(g.m0, r1, r2)) {
-        const dim3 grid((g.m1 * g.m2 + kTile - 1) / kTile, both ? 2 : 1, nslots);
-        switch (r2) {
-#define X(A) \
-    case A: launch_step(k_pair_pencil_any<A>, grid, kPencilThreads, pair_any_pencil_smem(g.m0), 1, 1, st, a, ra, rb); break;
-            PAIR_RADICES(X)
-#undef X
-        }
+    if (!pair_axis_fixed(g.m0)) {
+        pair_any_pencil(a, nslots, both, ra, rb, st);
         return;
     }
     const dim3 grid((g.m1 * g.m2 + tc - 1) / tc, both ? 2 : 1, nslots);

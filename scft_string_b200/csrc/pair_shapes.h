@@ -103,4 +103,10 @@ inline void pair_y_radices(int m1, int m2, int &ra, int &rb)
 #undef X
 }
 
+// launches of pair_any.cu
+int pair_any_setup(int m0, int m1, int m2);
+void pair_any_mid(const PropsArgs<double> &a, int nslots, int s, cudaStream_t st);
+void pair_any_combine(const PropsArgs<double> &a, int nslots, int s, int mode, int split, cudaStream_t st);
+void pair_any_pencil(const PropsArgs<double> &a, int nslots, int both, int ra, int rb, cudaStream_t st);
+
 }  // namespace scft

@@ -674,9 +674,12 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
     }
 
     int dev = p->device;
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return SCFT_UNSUPPORTED;
-    if (prop.major != 10) return SCFT_UNSUPPORTED;
+    // two attributes: the whole property record takes 2.5 ms to fetch
+    int major = 0, smem_optin = 0;
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return SCFT_UNSUPPORTED;
+    if (major != 10) return SCFT_UNSUPPORTED;
     if (cudaSetDevice(dev) != cudaSuccess) return SCFT_UNSUPPORTED;
 
     scft_ctx *ctx = new scft_ctx();
@@ -711,7 +714,7 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
     L.pf = 0;
     if (L.fixed) {
         pf_smem_bytes(L.fixed, T == 4, L.mid_pf_smem, L.combine_pf_smem);
-        L.pf = (std::max(L.mid_pf_smem, L.combine_pf_smem) <= (int)prop.sharedMemPerBlockOptin) ? 1 : 0;
+        L.pf = (std::max(L.mid_pf_smem, L.combine_pf_smem) <= smem_optin) ? 1 : 0;
         if (const char *ev = getenv("SCFT_NO_PREFETCH")) L.pf = ev[0] == '1' ? 0 : L.pf;
     }
     if (threads_for(g.pz, g.npair) > 1024 || threads_for(g.py, g.mk2) > 1024 ||
@@ -726,7 +729,7 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
     L.q_blocks = std::max(1, std::min(4 * kRedBlocks, (g.M + 255) / 256));
     L.dens_parts = g.M < kDensPoints ? kDensParts : 1;
     L.dens_blocks = std::max(1, std::min(kDensBlocks, (int)(((long long)g.M * L.dens_parts + 255) / 256)));
-    if (L.slab_smem > (int)prop.sharedMemPerBlockOptin || L.pencil_smem > (int)prop.sharedMemPerBlockOptin) {
+    if (L.slab_smem > smem_optin || L.pencil_smem > smem_optin) {
         delete ctx;
         return SCFT_BAD_INPUT;
     }
@@ -839,7 +842,7 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
                     L.tmap = &ctx->tmap;
                     L.pencil_tma_smem = smem_for(tc);
                     // the wide tile (2 tc columns; box width 4 tc reals <= 256, or 4 boxes of the swizzled map)
-                    if (4 * tc <= 256 && smem_for(2 * tc) <= (int)prop.sharedMemPerBlockOptin &&
+                    if (4 * tc <= 256 && smem_for(2 * tc) <= smem_optin &&
                         encode(&ctx->tmap_wide, 2 * tc) == CUDA_SUCCESS) {
                         L.tmap_wide = &ctx->tmap_wide;
                         L.pencil_tma_smem_wide = smem_for(2 * tc);
@@ -855,7 +858,7 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
         if (L.fixed && L.pf && L.tma_pencil) {
             int sm = std::max(L.mid_pf_smem, std::max(L.combine_pf_smem, L.pencil_tma_smem));
             if (L.tmap_wide) sm = std::max(sm, L.pencil_tma_smem_wide);
-            if (sm <= (int)prop.sharedMemPerBlockOptin) L.step_pf_smem = sm;
+            if (sm <= smem_optin) L.step_pf_smem = sm;
         }
         if ((T == 4 ? set_props_smem<float>(L) : set_props_smem<double>(L)) != 0) {
             ctx->lasterr = "cudaFuncSetAttribute(max dynamic shared memory) failed";
