@@ -26,6 +26,7 @@ using namespace scft;
 
 // schedules scft_autotune_ex times: slot groups (1, 2, 4) x tile width x launch form
 constexpr int kTuneCandidates = 12;
+constexpr size_t kStageBytes = 128 * 1024;  // host copies of up to this size go through pinned staging
 
 namespace {
 
@@ -112,7 +113,14 @@ struct scft_ctx {
     // host state
     std::vector<int> doiis;
     std::vector<int> slot_of;   // replica -> slot of its last props (-1 unknown)
-    std::vector<double> rs_h;   // [rep][kRsStride]
+    // pinned and mapped: the error word that the kernels write (err: its device
+    // address), staging for small host copies (kStageBytes in, as much out) and the
+    // host copy of rs, [rep][kRsStride]
+    void *host_mem = nullptr;
+    unsigned char *stage_in = nullptr, *stage_out = nullptr;
+    volatile int *err_h = nullptr;
+    double *rs_h = nullptr;
+    std::vector<int> rep_cur;   // what rep_dev holds
     std::vector<double> red_h;
     scft_stats stats{};
     bool timing_pending = false;
@@ -212,11 +220,10 @@ FieldArgs field_args(scft_ctx *ctx, const int *rep_list)
 // context stays usable.
 scft_status check_device_err(scft_ctx *ctx)
 {
-    int e = 0;
-    CK(cudaMemcpyAsync(&e, ctx->err, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
+    const int e = *ctx->err_h;
     if (e == 0) return SCFT_OK;
-    CK(cudaMemsetAsync(ctx->err, 0, sizeof(int), ctx->st));
+    *ctx->err_h = 0;  // nothing of this context is in flight
     if (e == 3) {
         ctx->lasterr = "a bounded device wait for a bulk copy gave up";
         return SCFT_TIMEOUT;
@@ -225,9 +232,35 @@ scft_status check_device_err(scft_ctx *ctx)
     return SCFT_CUDA_ERROR;
 }
 
+// Host arrays of up to kStageBytes go through pinned staging: a pageable copy of 64
+// KB takes 48 us, a copy into staging and from there 14.  One copy each way per
+// call, which waits for its stream before it returns.
+scft_status copy_in(scft_ctx *ctx, void *dst, const void *src, size_t bytes)
+{
+    if (bytes <= kStageBytes) {
+        std::memcpy(ctx->stage_in, src, bytes);
+        src = ctx->stage_in;
+    }
+    CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->st));
+    return SCFT_OK;
+}
+
+scft_status copy_out_start(scft_ctx *ctx, void *dst, const void *src, size_t bytes)
+{
+    CK(cudaMemcpyAsync(bytes <= kStageBytes ? ctx->stage_out : dst, src, bytes, cudaMemcpyDeviceToHost, ctx->st));
+    return SCFT_OK;
+}
+// after the stream has been waited for
+void copy_out_finish(scft_ctx *ctx, void *dst, size_t bytes)
+{
+    if (bytes <= kStageBytes) std::memcpy(dst, ctx->stage_out, bytes);
+}
+
 // uploads a replica list to the device (pageable copy: staged before return)
 scft_status upload_list(scft_ctx *ctx, const std::vector<int> &reps)
 {
+    if (reps == ctx->rep_cur) return SCFT_OK;
+    ctx->rep_cur = reps;
     CK(cudaMemcpyAsync(ctx->rep_dev, reps.data(), sizeof(int) * reps.size(), cudaMemcpyHostToDevice,
                        ctx->st));
     return SCFT_OK;
@@ -280,7 +313,7 @@ scft_status props_list(scft_ctx *ctx, const std::vector<int> &reps)
             ctx->slot_of[r] = -1;
         }
         CK(cudaEventRecord(ctx->ev1, ctx->st));
-        CK(cudaMemcpyAsync(ctx->rs_h.data(), ctx->rs, sizeof(double) * ctx->rs_h.size(), cudaMemcpyDeviceToHost,
+        CK(cudaMemcpyAsync(ctx->rs_h, ctx->rs, sizeof(double) * kRsStride * ctx->nrep_alloc, cudaMemcpyDeviceToHost,
                            ctx->st));
         scft_status s = check_device_err(ctx);
         if (s != SCFT_OK) return s;
@@ -349,8 +382,8 @@ scft_status props_list(scft_ctx *ctx, const std::vector<int> &reps)
     }
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev1, ctx->st));
-    CK(cudaMemcpyAsync(ctx->rs_h.data(), ctx->rs, sizeof(double) * ctx->rs_h.size(),
-                       cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(ctx->rs_h, ctx->rs, sizeof(double) * kRsStride * ctx->nrep_alloc, cudaMemcpyDeviceToHost,
+                       ctx->st));
     s = check_device_err(ctx);
     if (s != SCFT_OK) return s;
     float ms = 0;
@@ -616,11 +649,12 @@ void scft_destroy(scft_ctx *ctx)
 {
     if (!ctx) return;
     void *ptrs[] = {ctx->W, ctx->conc, ctx->DEV, ctx->dWda, ctx->rs, ctx->partials, ctx->redout,
-                    ctx->rep_dev, ctx->err, ctx->etab, ctx->hist, ctx->spec, ctx->pbuf, ctx->tw,
+                    ctx->rep_dev, ctx->etab, ctx->hist, ctx->spec, ctx->pbuf, ctx->tw,
                     ctx->kfac, ctx->knots, ctx->st_S4, ctx->st_S2, ctx->st_S4p, ctx->st_part,
                     ctx->st_out, ctx->and_X, ctx->and_D, ctx->ck_mem, ctx->jtab, ctx->jd_rbuf, ctx->sync};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    if (ctx->host_mem) cudaFreeHost(ctx->host_mem);
     for (auto &e : ctx->tev)
         if (e) cudaEventDestroy(e);
     for (auto &g : ctx->graphs)
@@ -777,7 +811,14 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
                        sizeof(double) * std::max<size_t>(ctx->npart_stride * S, (size_t)ctx->nred_rows * kRedBlocks)));
         CKC(cudaMalloc(&ctx->redout, sizeof(double) * ctx->nred_rows));
         CKC(cudaMalloc(&ctx->rep_dev, sizeof(int) * (R + 1)));
-        CKC(cudaMalloc(&ctx->err, sizeof(int)));
+        CKC(cudaHostAlloc(&ctx->host_mem, 64 + 2 * kStageBytes + sizeof(double) * kRsStride * R, cudaHostAllocMapped));
+        ctx->err_h = static_cast<volatile int *>(ctx->host_mem);
+        *ctx->err_h = 0;
+        ctx->stage_in = static_cast<unsigned char *>(ctx->host_mem) + 64;
+        ctx->stage_out = ctx->stage_in + kStageBytes;
+        ctx->rs_h = reinterpret_cast<double *>(ctx->stage_out + kStageBytes);
+        std::memset(ctx->rs_h, 0, sizeof(double) * kRsStride * R);
+        CKC(cudaHostGetDevicePointer((void **)&ctx->err, ctx->host_mem, 0));
         CKC(cudaMalloc(&ctx->etab, T * 2 * M * S));
         if (g.jon) CKC(cudaMalloc(&ctx->jtab, T * M * S));
         // the full propagator store (2 slices per step and slot); a stub without it
@@ -806,7 +847,6 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
         CKC(cudaMemset(ctx->DEV, 0, sizeof(double) * 2 * M * R));
         CKC(cudaMemset(ctx->dWda, 0, sizeof(double) * M * R));
         CKC(cudaMemset(ctx->rs, 0, sizeof(double) * kRsStride * R));
-        CKC(cudaMemset(ctx->err, 0, sizeof(int)));
         // 2-D tensor map of all spectra: rows of 2*m1*mk2 reals, nslots*2*2*m0 rows
         L.tma_pencil = 0;
         if (L.fixed && !getenv("SCFT_NO_TMA_PENCIL")) {
@@ -890,7 +930,6 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
         ctx->graphs.assign((size_t)(R + 1) * (S + 1) + 1, nullptr);
         if (const char *ev = getenv("SCFT_NO_GRAPHS")) ctx->use_graphs = ev[0] != '1';
         ctx->slot_of.assign(R, -1);
-        ctx->rs_h.assign(kRsStride * R, 0.0);
         ctx->red_h.assign(ctx->nred_rows, 0.0);
         auto &S_ = ctx->sf;
         S_.x.assign(ctx->strn, 0.0);
@@ -919,8 +958,8 @@ done:
 scft_status scft_set_fields(scft_ctx *ctx, int ii, const double *w2M)
 {
     if (!ctx || !w2M || ii < 0 || ii >= ctx->strn) return SCFT_BAD_INPUT;
-    CK(cudaMemcpyAsync(ctx->W + (size_t)ii * 2 * ctx->M, w2M, sizeof(double) * 2 * ctx->M,
-                       cudaMemcpyHostToDevice, ctx->st));
+    scft_status s = copy_in(ctx, ctx->W + (size_t)ii * 2 * ctx->M, w2M, sizeof(double) * 2 * ctx->M);
+    if (s != SCFT_OK) return s;
     CK(cudaStreamSynchronize(ctx->st));
     return SCFT_OK;
 }
@@ -929,9 +968,11 @@ scft_status scft_get_fields(const scft_ctx *cctx, int ii, double *w2M)
 {
     scft_ctx *ctx = const_cast<scft_ctx *>(cctx);
     if (!ctx || !w2M || ii < 0 || ii >= ctx->strn) return SCFT_BAD_INPUT;
-    CK(cudaMemcpyAsync(w2M, ctx->W + (size_t)ii * 2 * ctx->M, sizeof(double) * 2 * ctx->M,
-                       cudaMemcpyDeviceToHost, ctx->st));
+    const size_t bytes = sizeof(double) * 2 * ctx->M;
+    scft_status s = copy_out_start(ctx, w2M, ctx->W + (size_t)ii * 2 * ctx->M, bytes);
+    if (s != SCFT_OK) return s;
     CK(cudaStreamSynchronize(ctx->st));
+    copy_out_finish(ctx, w2M, bytes);
     return SCFT_OK;
 }
 
@@ -966,7 +1007,7 @@ scft_status scft_get_conc(const scft_ctx *cctx, int ii, double *out4M, double *l
         CK(cudaMemcpyAsync(out4M, ctx->conc + (size_t)ii * 4 * ctx->M, sizeof(double) * 4 * ctx->M,
                            cudaMemcpyDeviceToHost, ctx->st));
     }
-    CK(cudaMemcpyAsync(ctx->rs_h.data() + (size_t)ii * kRsStride, ctx->rs + (size_t)ii * kRsStride,
+    CK(cudaMemcpyAsync(ctx->rs_h + (size_t)ii * kRsStride, ctx->rs + (size_t)ii * kRsStride,
                        sizeof(double) * kRsStride, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     if (lnQ) *lnQ = rsv(ctx, ii, kRsLnQ);
@@ -1000,13 +1041,14 @@ scft_status scft_props_host(scft_ctx *ctx, double *w, double *lnQ, int ii, int N
     }
     const int sc = ctx->strn;  // scratch replica
     const size_t M = ctx->M;
-    CK(cudaMemcpyAsync(ctx->W + (size_t)sc * 2 * M, w, sizeof(double) * 2 * M, cudaMemcpyHostToDevice,
-                       ctx->st));
-    scft_status s = props_list(ctx, {sc});
+    scft_status s = copy_in(ctx, ctx->W + (size_t)sc * 2 * M, w, sizeof(double) * 2 * M);
     if (s != SCFT_OK) return s;
-    CK(cudaMemcpyAsync(w + 2 * M, ctx->conc + (size_t)sc * 4 * M, sizeof(double) * 4 * M,
-                       cudaMemcpyDeviceToHost, ctx->st));
+    s = props_list(ctx, {sc});
+    if (s != SCFT_OK) return s;
+    s = copy_out_start(ctx, w + 2 * M, ctx->conc + (size_t)sc * 4 * M, sizeof(double) * 4 * M);
+    if (s != SCFT_OK) return s;
     CK(cudaStreamSynchronize(ctx->st));
+    copy_out_finish(ctx, w + 2 * M, sizeof(double) * 4 * M);
     if (lnQ) *lnQ = rsv(ctx, sc, kRsLnQ);
     if (phis)
         for (int k = 0; k < 5; k++) phis[k] = rsv(ctx, sc, kRsPhis + k);
@@ -1024,14 +1066,18 @@ scft_status scft_do_step(scft_ctx *ctx, int ii, const double *in, double *out, i
     const size_t M = ctx->M;
     const size_t T = ctx->prec == SCFT_FP32 ? 4 : 8;
     const size_t slice = 2 * M;
-    std::vector<unsigned char> tmp(slice * T);
-    if (T == 4)
-        for (size_t i = 0; i < slice; i++) ((float *)tmp.data())[i] = (float)in[i];
-    else
-        std::memcpy(tmp.data(), in, slice * 8);
-    CK(cudaMemcpyAsync(ctx->rep_dev, &ii, sizeof(int), cudaMemcpyHostToDevice, ctx->st));
+    // FP64 slices are copied as they are, FP32 ones through a host conversion
+    std::vector<float> tmp;
+    const void *src = in;
+    if (T == 4) {
+        tmp.assign(in, in + slice);
+        src = tmp.data();
+    }
+    scft_status st = upload_list(ctx, {ii});
+    if (st != SCFT_OK) return st;
     unsigned char *h0 = (unsigned char *)ctx->hist + (size_t)s * slice * T;
-    CK(cudaMemcpyAsync(h0, tmp.data(), slice * T, cudaMemcpyHostToDevice, ctx->st));
+    st = copy_in(ctx, h0, src, slice * T);
+    if (st != SCFT_OK) return st;
     int nl;
     if (T == 4)
         nl = launch_single_step<float>(props_args<float>(ctx, ctx->rep_dev), ctx->L, s, ctx->st);
@@ -1039,15 +1085,16 @@ scft_status scft_do_step(scft_ctx *ctx, int ii, const double *in, double *out, i
         nl = launch_single_step<double>(props_args<double>(ctx, ctx->rep_dev), ctx->L, s, ctx->st);
     ctx->stats.kernel_launches += nl;
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(tmp.data(), h0 + slice * T, slice * T, cudaMemcpyDeviceToHost, ctx->st));
-    scft_status st = check_device_err(ctx);
-    if (st != SCFT_OK) return st;
     for (auto &so : ctx->slot_of)
         if (so == 0) so = -1;
+    void *dst = T == 4 ? (void *)tmp.data() : (void *)out;
+    st = copy_out_start(ctx, dst, h0 + slice * T, slice * T);
+    if (st != SCFT_OK) return st;
+    st = check_device_err(ctx);
+    if (st != SCFT_OK) return st;
+    copy_out_finish(ctx, dst, slice * T);
     if (T == 4)
-        for (size_t i = 0; i < slice; i++) out[i] = ((float *)tmp.data())[i];
-    else
-        std::memcpy(out, tmp.data(), slice * 8);
+        for (size_t i = 0; i < slice; i++) out[i] = tmp[i];
     return SCFT_OK;
 }
 
@@ -1066,14 +1113,11 @@ scft_status scft_get_propagator(const scft_ctx *cctx, int ii, int which, int s, 
     }
     const size_t M = ctx->M, T = ctx->prec == SCFT_FP32 ? 4 : 8;
     const size_t off = (((size_t)slot * (ctx->g.Ns + 1) + s) * 2 + (which ? 1 : 0)) * M;
-    std::vector<unsigned char> tmp(M * T);
-    CK(cudaMemcpyAsync(tmp.data(), (unsigned char *)ctx->hist + off * T, M * T, cudaMemcpyDeviceToHost,
-                       ctx->st));
+    std::vector<float> tmp(T == 4 ? M : 0);
+    CK(cudaMemcpyAsync(T == 4 ? (void *)tmp.data() : (void *)outM, (unsigned char *)ctx->hist + off * T, M * T,
+                       cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
-    if (T == 4)
-        for (size_t i = 0; i < M; i++) outM[i] = ((float *)tmp.data())[i];
-    else
-        std::memcpy(outM, tmp.data(), M * 8);
+    for (size_t i = 0; i < tmp.size(); i++) outM[i] = tmp[i];
     return SCFT_OK;
 }
 
