@@ -518,6 +518,7 @@ __device__ __forceinline__ void pair_mid_body(const PS &B, const PropsArgs<doubl
     }
     __syncthreads();
     pdl_wait();
+    if (pdl_early(g.m0)) pdl_trigger();
     B.inverse_passes(spec);
     if (sp == 0) {
         B.template real_space<true, true>([&](cplx<T> *v, int o) {
@@ -569,6 +570,7 @@ __device__ __forceinline__ void pair_combine_body(const PS &B, const PropsArgs<d
     }
     __syncthreads();
     pdl_wait();
+    if (pdl_early(g.m0)) pdl_trigger();
     if (mode == 0) {
         const cplx<T> *P = reinterpret_cast<const cplx<T> *>(a.pbuf) + (size_t)slot * M + off;
         if (threadIdx.x == 0) prefetch_l2(P, area * sizeof(cplx<T>));
@@ -670,6 +672,7 @@ __device__ __forceinline__ void pair_pencil_body(const PropsArgs<double> &a, int
         colf[t] = c < ncol ? __ldg(kf + M0 + ky) * __ldg(kf + M0 + m1 + (2 * kz > m2 ? m2 - kz : kz)) : (T)0;
     }
     pdl_wait();
+    if (pdl_early(g.m0)) pdl_trigger();
 #pragma unroll 1
     for (int b = threadIdx.x; b < R2 * TC; b += NT) {
         const int t = b % TC, j = b / TC;
@@ -747,6 +750,7 @@ __device__ __forceinline__ void pair_pencil_any_body(const PropsArgs<double> &a,
         colf[t] = __ldg(kf + m0 + ky) * __ldg(kf + m0 + m1 + (2 * kz > m2 ? m2 - kz : kz));
     }
     pdl_wait();
+    if (pdl_early(g.m0)) pdl_trigger();
     const unsigned mag = 0xffffffffu / (unsigned)nc + 1u;  // nc = 1: butterfly b is (0, b)
     auto outer = [&](int b, int &t, int &j) {
         j = nc > 1 ? (int)__umulhi((unsigned)b, mag) : b;

@@ -375,6 +375,7 @@ __global__ void __launch_bounds__(RealSlab<M1, M2>::NT, RealSlab<M1, M2>::MINB) 
     B.load_tables(a.tw, g.m0);
     __syncthreads();
     pdl_wait();
+    if (pdl_early(g.m0)) pdl_trigger();
     B.inverse_passes(spec);
     if constexpr (R::STAGED) mbar_wait(&B.bars[0], 0, a.err);
     if (sp == 0) {
@@ -443,6 +444,7 @@ __global__ void __launch_bounds__(RealSlab<M1, M2>::NT, RealSlab<M1, M2>::MINB)
     B.load_tables(a.tw, g.m0);
     __syncthreads();
     pdl_wait();
+    if (pdl_early(g.m0)) pdl_trigger();
     if constexpr (R::STAGED) {
         if (mode != 1) B.stage_in(B.Qs, mode == 0 ? P : qn, &B.bars[1]);
     } else {
@@ -576,6 +578,7 @@ __global__ void __launch_bounds__(kRealPencilThreads, 4) k_real_pencil(PropsArgs
         colf[t] = c < ncol ? __ldg(kf + M0 + y) * __ldg(kf + M0 + g.m1 + kz) : 0.0f;
     }
     pdl_wait();
+    if (pdl_early(g.m0)) pdl_trigger();
 #pragma unroll 1
     for (int b = threadIdx.x; b < R2 * TC; b += NT) {
         const int t = b % TC, j = b / TC;
