@@ -67,7 +67,7 @@ void pair_any_mid(const PropsArgs<T> &a, int nslots, int s, cudaStream_t st)
     PairAny q;
     if (pair_any_plan(g.m1, g.m2, q)) switch (q.ra) {
 #define X(A)                                                                                                           \
-    case A: launch_step(k_pair_mid_any<A>, dim3(g.m0, 2, nslots), pair_any_threads(q), pair_any_smem(q), 1, 1, st, a, s, q); break;
+    case A: launch_step(k_pair_mid_any<A>, dim3(g.m0, 2, nslots), pair_any_threads(q, 2 * g.m0 * nslots), pair_any_smem(q), 1, 1, st, a, s, q); break;
             PAIR_RADICES(X)
 #undef X
         }
@@ -80,7 +80,7 @@ void pair_any_combine(const PropsArgs<T> &a, int nslots, int s, int mode, int sp
     if (pair_any_plan(g.m1, g.m2, q)) switch (q.ra) {
 #define X(A)                                                                                                         \
     case A:                                                                                                          \
-        launch_step(k_pair_combine_any<A>, dim3(g.m0, split, nslots), pair_any_threads(q), pair_any_smem(q), 1, split, st, a, \
+        launch_step(k_pair_combine_any<A>, dim3(g.m0, split, nslots), pair_any_threads(q, split * g.m0 * nslots), pair_any_smem(q), 1, split, st, a, \
                     s, mode, q);                                                                                     \
         break;
             PAIR_RADICES(X)

@@ -75,12 +75,13 @@ inline bool pair_any_plan(int m1, int m2, PairAny &q)
     return pair_any_smem(q) <= kSmemCta;
 }
 
-// threads of a slab kernel of such a shape: one butterfly each in its widest
-// pass, up to 256, or 512 where shared memory leaves one CTA per SM
-inline int pair_any_threads(const PairAny &q)
+// threads of a slab kernel of such a shape in a launch of `ctas` CTAs: one
+// butterfly each in its widest pass, up to 256, or 512 where an SM holds one CTA
+// anyway, by its shared memory or because there are no more
+inline int pair_any_threads(const PairAny &q, int ctas)
 {
     const int n = std::max(std::max(q.m1 * q.rz, q.m1 * q.rc), std::max(q.ra * q.m2, q.rb * q.m2));
-    const int most = 2 * (pair_any_smem(q) + 1024) <= 228 * 1024 ? 256 : 512;
+    const int most = 2 * (pair_any_smem(q) + 1024) <= 228 * 1024 && ctas > 148 ? 256 : 512;
     return std::min(most, (n + 31) / 32 * 32);
 }
 

@@ -296,9 +296,9 @@ int pair_stress_chunk(const StressArgs<T> &a, const StressPairs &P, double *out,
 #define X(A)                                                                                                           \
     case A:                                                                                                            \
         if (mid)                                                                                                       \
-            k_pair_stress_mid_any<A><<<dim3(g.m0, 1, P.n), pair_any_threads(q), pair_any_smem(q), st>>>(a, P, q);       \
+            k_pair_stress_mid_any<A><<<dim3(g.m0, 1, P.n), pair_any_threads(q, 2 * g.m0 * P.n), pair_any_smem(q), st>>>(a, P, q);       \
         else                                                                                                           \
-            k_pair_stress_fwd_any<A><<<dim3(g.m0, 2, P.n), pair_any_threads(q), pair_any_smem(q), st>>>(a, P, q);       \
+            k_pair_stress_fwd_any<A><<<dim3(g.m0, 2, P.n), pair_any_threads(q, 2 * g.m0 * P.n), pair_any_smem(q), st>>>(a, P, q);       \
         break;
                 PAIR_RADICES(X)
 #undef X
