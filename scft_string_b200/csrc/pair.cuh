@@ -70,17 +70,6 @@ __device__ __forceinline__ double third(double x)
     return fabs(q) <= big ? r : q;
 }
 
-// the two CTAs of a split combine: each has read its input slab (arrive) before
-// either overwrites it (wait)
-__device__ __forceinline__ void pair_arrive()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void pair_wait()
-{
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 __device__ __forceinline__ int cluster_rank()
 {
     unsigned r;

@@ -33,6 +33,17 @@ __device__ __forceinline__ void prefetch_l2(const void *p, int bytes)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+// the two CTAs of a split combine: each has read its input slab (arrive) before
+// either overwrites it (wait)
+__device__ __forceinline__ void pair_arrive()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void pair_wait()
+{
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // Launch in clusters of (cx, cy) CTAs.  pdl: it may start while the kernel before
 // it on the stream finishes; only for kernels that call pdl_wait.
 template <class... Params, class... Args>

@@ -117,8 +117,10 @@ __device__ __forceinline__ void slab_inv(cplx<T> *buf, const Geo &g, const cplx<
 // mode 0: finishes step s (q(s+1) = Richardson combination);
 // mode 1: q(s+1) = 1 (Array_set_value, density.h:368-369; called with s = -1);
 // mode 2: q(s+1) is taken from the propagator store (single-step entry).
-// Then starts step s+1 when s+1 < Ns.
-template <typename T, int MT, int FM0, int FM1, int FM2>
+// Then starts step s+1 when s+1 < Ns.  SPLIT: a slab is shared by a cluster of
+// two CTAs along y (small batches): both finish the step, each makes one of
+// the two spectra, the first stores q.
+template <typename T, int MT, int FM0, int FM1, int FM2, bool SPLIT = false>
 __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) k_combine(PropsArgs<T> a, int s, int mode)
 {
     extern __shared__ unsigned char smem_raw[];
@@ -134,7 +136,9 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     cplx<T> *twz = twy + m1;
     for (int i = threadIdx.x; i < m1; i += nthr) twy[i] = a.tw[m0 + i];
     for (int i = threadIdx.x; i < m2; i += nthr) twz[i] = a.tw[m0 + m1 + i];
-    const int x = blockIdx.x, fld = blockIdx.y, slot = blockIdx.z;
+    const int x = blockIdx.x, fld = SPLIT ? blockIdx.y >> 1 : blockIdx.y, slot = blockIdx.z;
+    const int half = SPLIT ? blockIdx.y & 1 : -1;
+    const bool store = half != 1;
     const size_t slab_r = (size_t)x * m1 * m2;  // real offset of this slab
     const size_t slab_k = (size_t)x * m1 * mk2;
     cplx<T> *specA = a.spec + ((size_t)slot * 2 + fld) * 2 * Mk;
@@ -147,6 +151,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     if (mode == 0) {
         for (int i = threadIdx.x; i < m1 * mk2; i += nthr) buf[i] = specA[slab_k + i];
         __syncthreads();
+        if (SPLIT) pair_arrive();
         slab_inv<T, MT, FM1, FM2>(buf, g, twy, twz, a.err);
         const T *E4 = etab_ptr(a, slot, etab_sel(g, fld, s)) + slab_r;
         const T *P = a.pbuf + ((size_t)slot * 2 + fld) * M + slab_r;
@@ -156,11 +161,11 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
             const int r0 = 2 * p * m2 + z;
             // Richardson, GPU_kernels.h:199-203
             c.x = (c.x * E4[r0] * (T)4 - P[r0]) / (T)3;
-            qn[r0] = c.x;
+            if (store) qn[r0] = c.x;
             if (2 * p + 1 < m1) {
                 const int r1 = r0 + m2;
                 c.y = (c.y * E4[r1] * (T)4 - P[r1]) / (T)3;
-                qn[r1] = c.y;
+                if (store) qn[r1] = c.y;
             } else {
                 c.y = (T)0;
             }
@@ -171,8 +176,10 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
             const int r0 = 2 * p * m2 + z;
             const bool hb = 2 * p + 1 < m1;
             buf[prow<FM2>(p, mk2) + z] = {(T)1, hb ? (T)1 : (T)0};
-            qn[r0] = (T)1;
-            if (hb) qn[r0 + m2] = (T)1;
+            if (store) {
+                qn[r0] = (T)1;
+                if (hb) qn[r0 + m2] = (T)1;
+            }
         }
     } else {
         for (int e = threadIdx.x; e < npz; e += nthr) {
@@ -185,17 +192,27 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     if (sn >= g.Ns) return;
     __syncthreads();
     const T *E4n = etab_ptr(a, slot, etab_sel(g, fld, sn)) + slab_r;
-    // half step input E4' q'
+    // half step input E4' q' (half 1: the full step input E2' q')
     for (int e = threadIdx.x; e < npz; e += nthr) {
         const int p = FX ? e / m2 : div_by(e, mag), z = e - p * m2;
         cplx<T> &c = buf[prow<FM2>(p, mk2) + z];
         const int r0 = 2 * p * m2 + z;
-        c.x *= E4n[r0];
-        if (2 * p + 1 < m1) c.y *= E4n[r0 + m2];
+        const T e0 = E4n[r0];
+        c.x *= half == 1 ? e0 * e0 : e0;
+        if (2 * p + 1 < m1) {
+            const T e1 = E4n[r0 + m2];
+            c.y *= half == 1 ? e1 * e1 : e1;
+        }
     }
     __syncthreads();
     slab_fwd<T, MT, FM1, FM2>(buf, g, twy, twz, a.err);
-    for (int i = threadIdx.x; i < m1 * mk2; i += nthr) specA[slab_k + i] = buf[i];
+    if (SPLIT) {
+        if (mode == 0) pair_wait();
+        pdl_trigger();
+    }
+    cplx<T> *first = half == 1 ? specB : specA;
+    for (int i = threadIdx.x; i < m1 * mk2; i += nthr) first[slab_k + i] = buf[i];
+    if (SPLIT) return;
     __syncthreads();
     // full step input E2' q' (q' re-read from the propagator store written above)
     for (int e = threadIdx.x; e < npz; e += nthr) {
@@ -216,7 +233,9 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
 }
 
 // ---------------------------------------------------------------- mid
-template <typename T, int MT, int FM0, int FM1, int FM2>
+// SPLIT: the half step and the full step of a slab are two CTAs, the longer half
+// steps first.
+template <typename T, int MT, int FM0, int FM1, int FM2, bool SPLIT = false>
 __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) k_mid(PropsArgs<T> a, int s)
 {
     extern __shared__ unsigned char smem_raw[];
@@ -232,7 +251,8 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     cplx<T> *twz = twy + m1;
     for (int i = threadIdx.x; i < m1; i += nthr) twy[i] = a.tw[m0 + i];
     for (int i = threadIdx.x; i < m2; i += nthr) twz[i] = a.tw[m0 + m1 + i];
-    const int x = blockIdx.x, fld = blockIdx.y, slot = blockIdx.z;
+    const bool half = SPLIT && blockIdx.y < 2;
+    const int x = blockIdx.x, fld = SPLIT ? blockIdx.y & 1 : blockIdx.y, slot = blockIdx.z;
     const size_t slab_r = (size_t)x * m1 * m2;
     const size_t slab_k = (size_t)x * m1 * mk2;
     const T *E4 = etab_ptr(a, slot, etab_sel(g, fld, s)) + slab_r;
@@ -241,27 +261,30 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
     T *P = a.pbuf + ((size_t)slot * 2 + fld) * M + slab_r;
     const int npz = ((m1 + 1) / 2) * m2;
 
-    // full step: P = E2 * qs1
     pdl_wait();
-    for (int i = threadIdx.x; i < m1 * mk2; i += nthr) buf[i] = specB[slab_k + i];
-    __syncthreads();
-    slab_inv<T, MT, FM1, FM2>(buf, g, twy, twz, a.err);
-    for (int e = threadIdx.x; e < npz; e += nthr) {
-        const int p = FX ? e / m2 : div_by(e, mag), z = e - p * m2;
-        const cplx<T> c = buf[prow<FM2>(p, mk2) + z];
-        const int r0 = 2 * p * m2 + z;
-        const T e0 = E4[r0];
-        P[r0] = c.x * (e0 * e0);
-        if (2 * p + 1 < m1) {
-            const T e1 = E4[r0 + m2];
-            P[r0 + m2] = c.y * (e1 * e1);
+    if (!half) {  // full step: P = E2 * qs1
+        for (int i = threadIdx.x; i < m1 * mk2; i += nthr) buf[i] = specB[slab_k + i];
+        __syncthreads();
+        slab_inv<T, MT, FM1, FM2>(buf, g, twy, twz, a.err);
+        if (SPLIT) pdl_trigger();
+        for (int e = threadIdx.x; e < npz; e += nthr) {
+            const int p = FX ? e / m2 : div_by(e, mag), z = e - p * m2;
+            const cplx<T> c = buf[prow<FM2>(p, mk2) + z];
+            const int r0 = 2 * p * m2 + z;
+            const T e0 = E4[r0];
+            P[r0] = c.x * (e0 * e0);
+            if (2 * p + 1 < m1) {
+                const T e1 = E4[r0 + m2];
+                P[r0 + m2] = c.y * (e1 * e1);
+            }
         }
+        if (SPLIT) return;
+        __syncthreads();
     }
-    __syncthreads();
-    // second half step input: E2 * (first half step)
     for (int i = threadIdx.x; i < m1 * mk2; i += nthr) buf[i] = specA[slab_k + i];
     __syncthreads();
     slab_inv<T, MT, FM1, FM2>(buf, g, twy, twz, a.err);
+    // second half step input: E2 * (first half step)
     for (int e = threadIdx.x; e < npz; e += nthr) {
         const int p = FX ? e / m2 : div_by(e, mag), z = e - p * m2;
         cplx<T> &c = buf[prow<FM2>(p, mk2) + z];
@@ -285,7 +308,7 @@ __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) 
 // x-transform of a tile of tc consecutive (ky, kz) columns, times the
 // diffusion factor (Mult_self, GPU_kernels.h:175-181), inverse x-transform.
 // both != 0: spectrum A with K2 and spectrum B with K1; else A with K2 only.
-template <typename T, int MT, int FM0, int FM1, int FM2>
+template <typename T, int MT, int FM0, int FM1, int FM2, bool SPLIT = false>
 __global__ void __launch_bounds__(MT, MT == 256 ? (sizeof(T) == 4 ? 3 : 2) : 1) k_pencil(PropsArgs<T> a, int both)
 {
     extern __shared__ unsigned char smem_raw[];
@@ -1164,6 +1187,16 @@ void launch_combine(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gs, int s,
             return;
         }
     }
+    if constexpr (F0 == 0) {
+        // two CTAs per slab while each finds an SM of its own (with the split mid, one
+        // FP32 replica step: 35x54x45 102 -> 81 us, 60^3 130 -> 115, 16x12x20 55 -> 48;
+        // a kernel of its own, since the choice at run time costs the large batches
+        // registers: 30x28x36 x8 13.4 -> 14.2)
+        if (4 * gs.x * gs.z <= 148 && s + 1 < a.g.Ns) {
+            launch_step(k_combine<T, MT, 0, 0, 0, true>, dim3(gs.x, 4, gs.z), L.slab_threads, L.slab_smem, 1, 2, st, a, s, mode);
+            return;
+        }
+    }
     launch_step(k_combine<T, MT, F0, F1, F2>, gs, L.slab_threads, L.slab_smem, 1, 1, st, a, s, mode);
 }
 
@@ -1185,6 +1218,18 @@ void launch_mid(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gs, int s, cud
     if constexpr (F1 != 0) {
         if (L.pf) {
             if constexpr (sizeof(T) == 4) real_mid(a, gs.z, s, st);
+            return;
+        }
+    }
+    if constexpr (F0 == 0) {
+        // half and full step in CTAs of their own where that takes fewer rounds of the
+        // chip; a tie goes to one CTA, which reads E once
+        // (FP32, 45^3 x5 28.4 -> 27.1 us, 128x128x64 x2 217 -> 200, 100^3 x4
+        // 177 -> 168)
+        const int per = std::max(1, std::min((MT == 256 && sizeof(T) == 4 ? 768 : MT == 256 ? 512 : 1024) / L.slab_threads, 228 * 1024 / (L.slab_smem + 1024)));
+        const int n = 2 * gs.x * gs.z, fit = 148 * per;
+        if ((2 * n + fit - 1) / fit < 2 * ((n + fit - 1) / fit)) {
+            launch_step(k_mid<T, MT, 0, 0, 0, true>, dim3(gs.x, 4, gs.z), L.slab_threads, L.slab_smem, 1, 1, st, a, s);
             return;
         }
     }
@@ -1328,6 +1373,10 @@ int set_smem_mt(const PropsLaunch &L)
 {
     cudaError_t e1 = raise_dyn_smem(k_combine<T, MT, F0, F1, F2>, L.slab_smem);
     cudaError_t e2 = raise_dyn_smem(k_mid<T, MT, F0, F1, F2>, L.slab_smem);
+    if constexpr (F0 == 0) {
+        if (e1 == cudaSuccess) e1 = raise_dyn_smem(k_combine<T, MT, 0, 0, 0, true>, L.slab_smem);
+        if (e2 == cudaSuccess) e2 = raise_dyn_smem(k_mid<T, MT, 0, 0, 0, true>, L.slab_smem);
+    }
     cudaError_t e3 = raise_dyn_smem(k_pencil<T, MT, F0, F1, F2>, L.pencil_smem);
     cudaError_t e4 = cudaSuccess, e5 = cudaSuccess;
     if constexpr (F1 != 0) {

@@ -56,3 +56,23 @@ def test_step_at_the_block_change(built_lib, m):
         ref = od.do_step(q, s, 4, 8)
         # the tolerance of the other FP32 step tests
         assert np.abs(ctx.do_step(0, q, s) - ref).max() <= 2e-6 * np.abs(ref).max(), s
+
+
+@pytest.mark.parametrize("m,many", [((16, 12, 20), 24), ((35, 14, 45), 11), ((30, 28, 27), 13), ((9, 50, 21), 44)])
+def test_run_time_sizes_same_bits_alone_and_in_a_batch(built_lib, m, many):
+    """At sizes without compile-time kernels a small batch shares each slab between
+    two CTAs; a replica gets the same bits there as in a batch that does not."""
+    M, N = int(np.prod(m)), 11
+    rng = np.random.default_rng(8)
+    wm, wp = rng.normal(0, 3.0, M), rng.normal(0, 1.0, M)
+
+    def run(n):
+        ctx = S.Context(m, (4.0, 4.1, 4.2), N, chi=14, f=0.43, phidb=0.85, ens=2, strn=n, dostring=0, precision="fp32")
+        for ii in range(n):
+            ctx.set_fields(ii, wm, wp)
+        ctx.solve_field0_all(2, 0.0)
+        conc, lnQ, _ = ctx.get_conc(n - 1)
+        return conc, lnQ, ctx.propagator(n - 1, 0, N), ctx.propagator(n - 1, 1, N)
+
+    for a, b in zip(run(1), run(many)):
+        np.testing.assert_array_equal(a, b)
