@@ -158,9 +158,10 @@ __global__ void __launch_bounds__(256, 2) k_pair_stress_pencil(StressArgs<T> a, 
             v[i].y *= f;
         }
         Reg<T, R2, 1>::run(v);
-        stc(q, v[0]);
 #pragma unroll
-        for (int i = 1; i < R2; i++) stc(q + i * TC, cmulc(v[i], ldc(tw + k1 * i)));
+        for (int i = 1; i < R2; i++) v[i] = cmulc(v[i], ldc(tw + k1 * i));
+#pragma unroll
+        for (int i = 0; i < R2; i++) stc(q + i * TC, v[i]);
     }
     if (!back) return;
     __syncthreads();
