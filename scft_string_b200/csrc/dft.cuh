@@ -253,4 +253,16 @@ struct Reg<T, 20, SIGN> : RegCoprime<T, 4, 5, SIGN> {};
 template <typename T, int SIGN>
 struct Reg<T, 24, SIGN> : RegCoprime<T, 8, 3, SIGN> {};
 
+// x / 3, correctly rounded but for double rounding below the normal range: the
+// residual of x * (1/3) by a fused multiply-add, added back once (P. Markstein, IBM J.
+// Res. Dev. 34, 1990); five operations instead of a divide's subroutine; infinities
+// stay infinite
+__device__ __forceinline__ double third(double x)
+{
+    const double c = 1.0 / 3.0, big = 1.7976931348623157e308;
+    const double q = x * c;
+    const double r = fma(fma(-3.0, q, x), c, q);
+    return fabs(q) <= big ? r : q;
+}
+
 }  // namespace scft

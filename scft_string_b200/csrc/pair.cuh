@@ -60,17 +60,6 @@ __device__ __forceinline__ void stc(cplxd *p, cplxd v)
     *reinterpret_cast<double2 *>(p) = make_double2(v.x, v.y);
 }
 
-// x / 3, correctly rounded but for double rounding below the normal range: one
-// Newton correction of x * (1/3), five operations instead of a divide's
-// subroutine; infinities stay infinite
-__device__ __forceinline__ double third(double x)
-{
-    const double c = 1.0 / 3.0, big = 1.7976931348623157e308;
-    const double q = x * c;
-    const double r = fma(fma(-3.0, q, x), c, q);
-    return fabs(q) <= big ? r : q;
-}
-
 __device__ __forceinline__ int cluster_rank()
 {
     unsigned r;

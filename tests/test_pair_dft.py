@@ -15,12 +15,19 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LENGTHS = [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16, 20, 24]
 
 SRC = r"""
+#include <cmath>
 #include <cuda_runtime.h>
+using std::fma;
+using std::fabs;
 #include "dft.cuh"
 using namespace scft;
 template <int R> static void go(int sign, cplx<double> *v)
 {
     if (sign < 0) Reg<double, R, -1>::run(v); else Reg<double, R, 1>::run(v);
+}
+extern "C" void h_third(int n, double *v)
+{
+    for (int i = 0; i < n; i++) v[i] = third(v[i]);
 }
 extern "C" void h_dft(int n, int sign, double *v)
 {
@@ -45,6 +52,7 @@ def lib(tmp_path_factory):
     subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + inc, "-I" + csrc, "-o", out, str(src)],
                    check=True)
     L = C.CDLL(out)
+    L.h_third.argtypes = [C.c_int, np.ctypeslib.ndpointer(np.float64, flags="C_CONTIGUOUS")]
     L.h_dft.argtypes = [C.c_int, C.c_int, np.ctypeslib.ndpointer(np.float64, flags="C_CONTIGUOUS")]
     return L
 
@@ -59,6 +67,18 @@ def test_register_dft(lib, n, sign):
     lib.h_dft(n, sign, v)
     # a few roundings of n terms of size 1
     assert np.abs(v.view(np.complex128) - ref).max() <= 8 * n * np.finfo(float).eps
+
+
+def test_third(lib):
+    """third(x) is x / 3 correctly rounded wherever the quotient and the residual are
+    normal, and x / 3 for infinities and NaN."""
+    rng = np.random.default_rng(3)
+    x = rng.normal(size=200000) * 2.0 ** rng.integers(-900, 900, 200000)
+    top = np.finfo(float).max
+    x = np.concatenate([x, np.arange(-3000.0, 3000.0), [top, -top, np.inf, -np.inf, np.nan]])
+    v = x.copy()
+    lib.h_third(v.size, v)
+    np.testing.assert_array_equal(v, x / 3.0)
 
 
 def test_quotients_by_reciprocal(tmp_path):
