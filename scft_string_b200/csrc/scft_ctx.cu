@@ -260,9 +260,10 @@ void copy_out_finish(scft_ctx *ctx, void *dst, size_t bytes)
 scft_status upload_list(scft_ctx *ctx, const std::vector<int> &reps)
 {
     if (reps == ctx->rep_cur) return SCFT_OK;
-    ctx->rep_cur = reps;
+    ctx->rep_cur.clear();  // until the copy is on its way
     CK(cudaMemcpyAsync(ctx->rep_dev, reps.data(), sizeof(int) * reps.size(), cudaMemcpyHostToDevice,
                        ctx->st));
+    ctx->rep_cur = reps;
     return SCFT_OK;
 }
 
@@ -282,9 +283,10 @@ int effective_groups(int ngroups, int nb)
 // The count where none is configured: two, and on the pair-packed kernels twice
 // as many as long as the replicas of the two groups that run at a time hold more
 // than L2 keeps (spectra, tables and partial result: 64 bytes a point) and a
-// group still has slabs for most SMs.  64^3, us per replica step with 2 / 4
-// groups: 16 replicas 15.1 / 14.2, 14 replicas 15.2 / 14.2, 10 replicas 14.7 /
-// 15.5, 8 replicas 14.2 / 15.2; 48^3, 16 replicas 5.9 / 6.2.
+// group still has slabs for most SMs.  us per replica step with 2 / 4 groups: 64^3,
+// 16 replicas 14.8 / 13.9, 14 replicas 14.7 / 13.8; fewer slabs per group lose (10
+// replicas 14.7 / 15.5, 8 replicas 14.2 / 15.2 when the rule was made, 48^3 x16 5.65
+// / 6.09); 80^3 x16 33.6 / 34.1, 96^3 x8 58.3 / 58.3.
 int default_groups(const scft_ctx *ctx, int nb)
 {
     constexpr double kLive = 135e6;
