@@ -9,6 +9,16 @@ namespace scft {
 // as their last CTAs run (its CTAs set up and read constant tables), and wait
 // here for the whole previous kernel before they touch what it wrote.  Both are
 // no-ops in a kernel launched without the attribute.
+//
+// What a kernel may read before its wait: only what was complete when the kernel
+// before it passed its own, for that kernel's trigger comes after its wait.  A chain
+// is k_prepare, the first combine (modes 1 and 2), then pencil, mid, pencil, combine
+// (mode 0) per step.  So every kernel may read the twiddle and diffusion factors and
+// the replica list, which copies ahead of k_prepare wrote; the E tables, which
+// k_prepare writes, may be read early by all but the first combine: k_prepare has no
+// trigger, and its blocks may be gone before its stores are visible.  Where a chain
+// starts again from a checkpoint, the kernel before the first combine is a copy, and
+// the same rule is kept.  L2 prefetches are hints and may come at any time.
 __device__ __forceinline__ void pdl_trigger()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(RealSlab<M1, M2>::NT, RealSlab<M1, M2>::MINB) 
             mbar_init(&B.bars[0], 1);
             mbar_fence_init();
         }
-        B.stage_in(B.Es, E, &B.bars[0]);  // constant over the chain
+        B.stage_in(B.Es, E, &B.bars[0]);  // settled: never the first kernel of a chain (pdl.cuh)
     } else {
         if (threadIdx.x == 0) prefetch_l2(E, M1 * M2 * sizeof(float));
     }
@@ -437,7 +437,8 @@ __global__ void __launch_bounds__(RealSlab<M1, M2>::NT, RealSlab<M1, M2>::MINB)
             mbar_init(&B.bars[1], 1);
             mbar_fence_init();
         }
-        B.stage_in(B.Es, E, &B.bars[0]);  // constant over the chain
+        // settled unless this is the first kernel of a chain (pdl.cuh)
+        if (mode == 0) B.stage_in(B.Es, E, &B.bars[0]);
     } else {
         if (threadIdx.x == 0) prefetch_l2(E, M1 * M2 * sizeof(float));
     }
@@ -446,6 +447,7 @@ __global__ void __launch_bounds__(RealSlab<M1, M2>::NT, RealSlab<M1, M2>::MINB)
     pdl_wait();
     if (pdl_early(g.m0)) pdl_trigger();
     if constexpr (R::STAGED) {
+        if (mode != 0) B.stage_in(B.Es, E, &B.bars[0]);
         if (mode != 1) B.stage_in(B.Qs, mode == 0 ? P : qn, &B.bars[1]);
     } else {
         if (mode == 0 && threadIdx.x == 0) prefetch_l2(P, M1 * M2 * sizeof(float));

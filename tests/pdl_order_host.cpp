@@ -1,0 +1,165 @@
+// Host build of the step kernels that overlap with the kernel before them
+// (scft_string_b200/csrc/real_slab.cuh, pair.cuh) for tests/test_pdl_order.py: one
+// thread of one CTA runs a kernel body with the copies and loads of csrc/tma.cuh and
+// csrc/pdl.cuh replaced by ones that note which array is read, and whether the wait
+// for the previous kernel came first.  The numbers computed are meaningless.
+#include <cmath>
+#include <cstddef>
+#include <cstdint>
+#include <vector>
+
+#include <cuda_runtime.h>
+
+namespace {
+struct Range {
+    const unsigned char *p;
+    size_t n;
+    int id;
+};
+std::vector<Range> ranges;
+bool waited;
+int early[16];  // reads before the wait, per array
+
+template <class T>
+void note(const T *p)
+{
+    if (waited) return;
+    const unsigned char *q = reinterpret_cast<const unsigned char *>(p);
+    for (const Range &r : ranges)
+        if (q >= r.p && q < r.p + r.n) early[r.id]++;
+}
+}  // namespace
+
+// the device names that the headers use
+static const uint3 threadIdx = {0, 0, 0};
+static uint3 blockIdx;
+static dim3 gridDim, blockDim;
+static inline void __syncthreads() {}
+static inline void __syncwarp() {}
+static inline float __fmul_rn(float a, float b) { return a * b; }
+static inline float __fmaf_rn(float a, float b, float c) { return fmaf(a, b, c); }
+static inline unsigned __umulhi(unsigned a, unsigned b) { return (unsigned)(((unsigned long long)a * b) >> 32); }
+static inline unsigned __reduce_max_sync(unsigned, unsigned v) { return v; }
+static inline unsigned atomicMax(unsigned *p, unsigned v) { return *p > v ? *p : (*p = v); }
+static inline int __double2hiint(double v)
+{
+    uint64_t b;
+    __builtin_memcpy(&b, &v, 8);
+    return (int)(b >> 32);
+}
+static inline double __hiloint2double(int hi, int lo)
+{
+    const uint64_t b = (uint64_t)(uint32_t)hi << 32 | (uint32_t)lo;
+    double v;
+    __builtin_memcpy(&v, &b, 8);
+    return v;
+}
+#define __builtin_assume(x)
+#define __noinline__
+#define __launch_bounds__(...)
+template <class T>
+static inline T __ldg(const T *p)
+{
+    note(p);
+    return *p;
+}
+template <class T>
+static inline T __ldcg(const T *p)
+{
+    note(p);
+    return *p;
+}
+using std::fabs;
+using std::fma;
+using std::max;
+using std::min;
+
+#include "real_slab.cuh"  // copied next to the stand-ins of pdl.cuh and tma.cuh
+#include "pair.cuh"
+
+namespace scft {
+alignas(128) unsigned char smem_raw[1 << 18];  // the kernels' dynamic shared memory
+}
+
+using namespace scft;
+
+enum { W = 0, HIST, ETAB, JTAB, SPEC, PBUF, SCALE, CONST };
+
+template <class T>
+struct Case {
+    PropsArgs<T> a{};
+    std::vector<T> etab, jtab, hist, pbuf, kfac;
+    std::vector<cplx<T>> spec, tw;
+    std::vector<int> rep, sync;
+    int err = 0;
+
+    template <class V>
+    void own(V &v, size_t n, int id)
+    {
+        v.assign(n, typename V::value_type());
+        ranges.push_back({reinterpret_cast<const unsigned char *>(v.data()), n * sizeof(v[0]), id});
+    }
+    Case(int m, int Ns, int mk2)
+    {
+        ranges.clear();
+        for (int &e : early) e = 0;
+        waited = false;
+        Geo &g = a.g;
+        g = Geo();
+        g.m0 = g.m1 = g.m2 = m;
+        g.mk2 = mk2;
+        g.M = m * m * m;
+        g.Mk = m * m * mk2;
+        g.Ns = Ns;
+        g.n1 = Ns / 2;
+        g.n2 = Ns - Ns / 2;
+        own(etab, 2 * (size_t)g.M, ETAB);
+        own(jtab, g.M, JTAB);
+        own(hist, 2 * (size_t)g.M * (Ns + 1), HIST);
+        own(spec, 4 * (size_t)g.Mk, SPEC);
+        own(pbuf, 2 * (size_t)g.M, PBUF);
+        own(tw, 3 * m, CONST);
+        own(kfac, 3 * m, CONST);
+        own(rep, 1, CONST);
+        a.etab = etab.data();
+        a.jtab = jtab.data();
+        a.hist = hist.data();
+        a.spec = spec.data();
+        a.pbuf = pbuf.data();
+        a.tw = tw.data();
+        a.kfac = kfac.data();
+        a.slot_rep = rep.data();
+        a.err = &err;
+        a.invM = a.Mreal = (T)1;
+        blockIdx = {0, 0, 0};
+        gridDim = dim3(1, 2, 1);
+    }
+};
+
+// which: 0 combine, 1 mid, 2 x pass.  counts[0..15]: reads of each array before the wait
+extern "C" int h_early(int fp32, int which, int s, int mode, int *counts)
+{
+    const int m = 32, Ns = 8;
+    if (fp32) {
+        Case<float> c(m, Ns, m / 2 + 1);
+        blockDim = dim3(RealSlab<32, 32>::NT);
+        if (which == 0)
+            k_real_combine<32, 32>(c.a, s, mode);
+        else if (which == 1)
+            k_real_mid<32, 32>(c.a, s);
+        else
+            k_real_pencil<32, 32>(c.a);
+    } else {
+        Case<double> c(m, Ns, m);
+        using P = PairSlab<32, 32, 1>;
+        blockDim = dim3(P::NT);
+        if (which == 0)
+            pair_combine_body(P(smem_raw), c.a, s, mode, 0, -1, 0);
+        else if (which == 1)
+            pair_mid_body(P(smem_raw), c.a, s, 0, 1, 0);
+        else
+            pair_pencil_body<32, 32, 256>(c.a, 0, 0, 0, P::RA, P::RB, smem_raw);
+    }
+    for (int i = 0; i < 16; i++) counts[i] = early[i];
+    return waited ? 0 : -1;
+}
