@@ -44,6 +44,7 @@ struct PropsArgs {
     int slot0;              // first slot of this launch within the spectra tensor map
     T *jtab;                // [slot][M]  junction-step E4 (continuous A fraction only)
     int *sync;              // claim and completion counters of the persistent step kernel (reg64.cu)
+    int *pexp;              // [slot][Ns+1][2] binary exponents of the sizes of q(s), q^dagger(s) (pair.cuh)
 };
 
 // most blocks per slot of the density pass, and threads that share a point's
@@ -93,7 +94,8 @@ bool pair_applicable(int m0, int m1, int m2);
 int pair_setup(int m0, int m1, int m2, int *step_grid);
 void pair_mid(const PropsArgs<double> &a, int nslots, int s, cudaStream_t st);
 void pair_combine(const PropsArgs<double> &a, int nslots, int s, int mode, cudaStream_t st);
-void pair_pencil(const PropsArgs<double> &a, int nslots, int both, int wide, cudaStream_t st);
+// both = 1: both spectra of step s; 0: the half-step one, and the exponents of step s + 1
+void pair_pencil(const PropsArgs<double> &a, int nslots, int s, int both, int wide, cudaStream_t st);
 void pair_step(const PropsArgs<double> &a, int nslots, int s, int wide, int grid, cudaStream_t st);
 
 // FP32 slab kernels of the compile-time shapes (real_slab.cuh)
@@ -140,6 +142,7 @@ struct StressPairs {
     int xs[kStressPairs], xf[kStressPairs];  // slice s and field (0 q, 1 q^dagger) of x
     int ys[kStressPairs], yf[kStressPairs];  // of the adjoint y
     int sel[kStressPairs];                   // E table of the step (0 A, 1 B)
+    int xe[kStressPairs], ye[kStressPairs];  // 2 (contour step) + field of x and y: their sizes in pexp
 };
 
 template <typename T>
@@ -157,6 +160,7 @@ struct StressArgs {
     const T *jtab;           // [slot][M] junction-step E4 (table 2), continuous A fraction only
     T *rbuf;                 // [6][M] real work arrays of the junction derivative
     const double *wminus;    // W- of the replica (junction derivative)
+    const int *pexp;         // [slot][Ns+1][2] binary exponents of the sizes (pair.cuh)
 };
 
 template <typename T>

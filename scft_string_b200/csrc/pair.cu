@@ -41,13 +41,19 @@ __global__ void __launch_bounds__(PairSlab<M1, M2, CL>::NT, PairSlab<M1, M2, CL>
 }
 
 template <int M0, int TC>
-__global__ void __launch_bounds__(kPencilThreads, pencil_minb(M0)) k_pair_pencil(PropsArgs<T> a, int ra, int rb)
+__global__ void __launch_bounds__(kPencilThreads, pencil_minb(M0)) k_pair_pencil(PropsArgs<T> a, int s, int nsum, int ra, int rb)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     // slots (and tiles) in the opposite order of the slab kernels before and
     // after: what those touched last is still in L2
-    pair_pencil_body<M0, TC, kPencilThreads>(a, gridDim.x - 1 - blockIdx.x, blockIdx.y, gridDim.z - 1 - blockIdx.z, ra, rb,
-                                                smem_raw);
+    const int tile = gridDim.x - 1 - blockIdx.x, slot = gridDim.z - 1 - blockIdx.z;
+    if (tile * TC >= a.g.m1 * a.g.m2) {  // a tile past the last: the exponents of step s + 1
+        pdl_wait();
+        pdl_trigger();
+        pair_next_exponents(a, slot, s, nsum);
+        return;
+    }
+    pair_pencil_body<M0, TC, kPencilThreads>(a, tile, blockIdx.y, slot, ra, rb, smem_raw);
 }
 
 __device__ __forceinline__ int ld_acquire_gpu(const int *p)
@@ -60,8 +66,8 @@ __device__ __forceinline__ int ld_acquire_gpu(const int *p)
 constexpr uint32_t kStepSpin = 1u << 22;
 
 // The four launches of a step as work items of one launch: both spectra's x
-// tiles, the slabs of mid (two per x), the half-step spectrum's x tiles, the
-// slabs of combine, each phase ordered by slot.  CTAs claim items from a
+// tiles, the slabs of mid (two per x), the half-step spectrum's x tiles and the
+// exponents of the next step, the slabs of combine, each phase ordered by slot.  CTAs claim items from a
 // counter in the order of step_order.cuh, and an item waits only for the
 // previous phase of its own slot.  Items are claimed in order by running CTAs,
 // so whatever an item waits for is held by a CTA that is running or done; no
@@ -77,7 +83,7 @@ __global__ void __launch_bounds__(PairSlab<M1, M2, 1>::NT, PairSlab<M1, M2, 1>::
     constexpr int NT = PS::NT, ntiles = (M1 * M2 + TC - 1) / TC;
     int ra, rb;
     PS::radices(ra, rb);
-    const int per[4] = {2 * ntiles, 2 * M0, ntiles, M0};
+    const int per[4] = {2 * ntiles, 2 * M0, ntiles + 1, M0};
     int *claim = a.sync + s;      // this step's claim counter
     int *done = a.sync + a.g.Ns;  // [phase][slot] completion counters, cumulative over the steps
     for (;;) {
@@ -110,6 +116,8 @@ __global__ void __launch_bounds__(PairSlab<M1, M2, 1>::NT, PairSlab<M1, M2, 1>::
             pair_pencil_body<M0, TC, NT>(a, unit % ntiles, unit / ntiles, slot, ra, rb, smem_raw);
         else if (phase == 1)
             pair_mid_body(PS(smem_raw), a, s, unit >> 1, unit & 1, slot);
+        else if (phase == 2 && unit == ntiles)
+            pair_next_exponents(a, slot, s, M0);
         else if (phase == 2)
             pair_pencil_body<M0, TC, NT>(a, unit, 0, slot, ra, rb, smem_raw);
         else
@@ -214,23 +222,24 @@ void pair_combine(const PropsArgs<T> &a, int nslots, int s, int mode, cudaStream
     pair_any_combine(a, nslots, s, mode, split, st);
 }
 
-void pair_pencil(const PropsArgs<T> &a, int nslots, int both, int wide, cudaStream_t st)
+void pair_pencil(const PropsArgs<T> &a, int nslots, int s, int both, int wide, cudaStream_t st)
 {
     const Geo &g = a.g;
     const int tc = wide ? 2 * kTile : kTile;
     int ra = 1, rb = 1;
     pair_y_radices(g.m1, g.m2, ra, rb);
+    const int nsum = pair_slab_ctas(g.m1, g.m2) * g.m0;  // partial sums of mid
     if (!pair_axis_fixed(g.m0)) {
-        pair_any_pencil(a, nslots, both, ra, rb, st);
+        pair_any_pencil(a, nslots, s, both, nsum, ra, rb, st);
         return;
     }
-    const dim3 grid((g.m1 * g.m2 + tc - 1) / tc, both ? 2 : 1, nslots);
+    const dim3 grid((g.m1 * g.m2 + tc - 1) / tc + !both, both ? 2 : 1, nslots);
 #define X(A)                                                                                                 \
     if (g.m0 == A) {                                                                                         \
         if (wide)                                                                                            \
-            launch_step(k_pair_pencil<A, 2 * kTile>, grid, kPencilThreads, PairPencil<A, 2 * kTile>::SMEM, 1, 1, st, a, ra, rb);  \
+            launch_step(k_pair_pencil<A, 2 * kTile>, grid, kPencilThreads, PairPencil<A, 2 * kTile>::SMEM, 1, 1, st, a, s, nsum, ra, rb);  \
         else                                                                                                 \
-            launch_step(k_pair_pencil<A, kTile>, grid, kPencilThreads, PairPencil<A, kTile>::SMEM, 1, 1, st, a, ra, rb);          \
+            launch_step(k_pair_pencil<A, kTile>, grid, kPencilThreads, PairPencil<A, kTile>::SMEM, 1, 1, st, a, s, nsum, ra, rb);          \
         return;                                                                                              \
     }
     PAIR_AXES(X)

@@ -7,6 +7,12 @@
 // field c = q + i q^dagger: one complex 3-D transform replaces two real ones
 // with no packing, unpacking or Hermitian bookkeeping in between.
 //
+// The transforms round both parts relative to the larger one, and where W- has a mean
+// q and q^dagger drift apart by exp(2 <W-> s).  So the field is c = q + i 2^k q^dagger,
+// k per replica and step, from the root mean squares of the full-step result P (which
+// mid has in registers and which is of the size of the next q): a power of two costs
+// no rounding, and either propagator keeps the precision of a transform of its own.
+//
 // Each 1-D transform of length N = R1 R2 is done in place, in two register
 // passes with one trip through shared memory between them:
 //   forward  n = j + R2 r:  R1-point DFTs over r, for every j, written back to
@@ -124,6 +130,7 @@ struct PairSlab : PairPlan<M1, M2> {
     using Plan::RC;
     using Plan::RZ;
     static_assert(RA * RB == M1 && RZ * RC == M2 && RA % CL == 0 && M2 % CL == 0, "plan");
+    static constexpr int CTAS = CL;
     static constexpr int NT = pair_nt(Plan::NT, CL), L = M1 / CL, RAL = RA / CL, S = M2 | 1;
     static constexpr int SMEM = (L * S + M1 + M2) * (int)sizeof(cplx<T>);
     static constexpr int FIT = 227 * 1024 / (SMEM + 1024), REG = Plan::WANT / NT;
@@ -416,7 +423,7 @@ __device__ __forceinline__ void pair_any(int R, const cplxd *src, cplxd *dst, co
 template <int RA_>
 struct PairSlabAny {
     using T = double;
-    static constexpr int RA = RA_;
+    static constexpr int RA = RA_, CTAS = 1, rank = 0;
     PairAny q;
     cplx<T> *buf, *twy, *twz;
 
@@ -489,8 +496,123 @@ struct PairSlabAny {
     }
 };
 
+// ---------------------------------------------------------------- sizes of q and q^dagger
+// a.pexp[slot][s][field]: binary exponent of the root mean square of q(s) and
+// q^dagger(s); 0 for q(0) = 1.
+
+// k of a step whose exponents are e0, e1; bounded as the powers are, which stay normal
+__device__ __forceinline__ int pair_shift(int e0, int e1) { return min(max(e0 - e1, -1000), 1000); }
+__device__ __forceinline__ double pair_pow2(int k) { return __hiloint2double((1023 + min(max(k, -1000), 1000)) << 20, 0); }
+
+// sums over the CTA's threads of x and y -> out[0], out[1]
+__device__ __forceinline__ void pair_cta_sums(double x, double y, double *out)
+{
+    __shared__ double sh[2][32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        x += __shfl_xor_sync(0xffffffffu, x, o);
+        y += __shfl_xor_sync(0xffffffffu, y, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][threadIdx.x >> 5] = x;
+        sh[1][threadIdx.x >> 5] = y;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double t = 0;
+        for (int i = 0; i < (int)(blockDim.x >> 5); i++) t += sh[threadIdx.x][i];
+        out[threadIdx.x] = t;
+    }
+}
+
+// Floors of the binary exponents of the root mean squares that n pairs of partial sums
+// of squares give; bits 0 and 1 of the result: that sum was a normal number.  One warp,
+// every lane has the result.
+__device__ __forceinline__ int pair_rms_exponents(const double *sums, int n, double invM, int2 &e)
+{
+    double t0 = 0, t1 = 0;
+    for (int i = threadIdx.x & 31; i < n; i += 32) {
+        const double2 v = __ldcg(reinterpret_cast<const double2 *>(sums) + i);
+        t0 += v.x;
+        t1 += v.y;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        t0 += __shfl_xor_sync(0xffffffffu, t0, o);
+        t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+    }
+    // times 1.7: a uniform field of ones is not at the edge of a binade, where the last
+    // bit of a sum would decide
+    const int b0 = __double2hiint(t0 * invM * 1.7) >> 20, b1 = __double2hiint(t1 * invM * 1.7) >> 20;
+    e = {(b0 - 1023) >> 1, (b1 - 1023) >> 1};
+    return (b0 > 0 && b0 < 2047) | (b1 > 0 && b1 < 2047) << 1;
+}
+
+// Exponents of step s + 1 of a slot from mid's n partial sums of step s, whose terms
+// were scaled by 2^-(exponent of q(s)) (and by 2^k in the second part); those of step s
+// where a sum is no use.  Any CTA.
+__device__ __forceinline__ void pair_next_exponents(const PropsArgs<double> &a, int slot, int s, int n)
+{
+    if (threadIdx.x >= 32) return;
+    int2 *e = reinterpret_cast<int2 *>(a.pexp) + (size_t)slot * (a.g.Ns + 1) + s, d;
+    const int2 now = __ldcg(e);
+    const bool ok = pair_rms_exponents(a.partials + (size_t)slot * a.npart_stride, n, a.invM, d) == 3;
+    if (threadIdx.x != 0) return;
+    e[1] = ok ? make_int2(now.x + d.x, now.x + d.y - pair_shift(now.x, now.y)) : now;
+}
+
+// Exponents of a slice that no step led to, from the sums that n blocks took at three
+// scales (pair_block_sums): in every thread of the CTA.
+__device__ __forceinline__ int2 pair_slice_exponents(const double *sums, int n, double invM)
+{
+    __shared__ int2 sh;
+    if (threadIdx.x < 32) {
+        int2 e = {0, 0}, d;
+        int got = 0;
+        for (int j = 0; j < 3 && got < 3; j++) {
+            const int have = pair_rms_exponents(sums + 2 * j * n, n, invM, d) & ~got, c = j == 0 ? 0 : j == 1 ? 600 : -600;
+            if (have & 1) e.x = d.x - c;
+            if (have & 2) e.y = d.y - c;
+            got |= have;
+        }
+        if (threadIdx.x == 0) sh = e;
+    }
+    __syncthreads();
+    return sh;
+}
+
+// Sums of squares of q and q^dagger at q, per block, at the scales 2^0, 2^600, 2^-600:
+// no size of a normal number is lost.  For a grid of blocks along x.
+__device__ __forceinline__ void pair_block_sums(const double *q, int M, double *sums)
+{
+    __shared__ double sh[6][32];
+    const double c[3] = {1.0, pair_pow2(600), pair_pow2(-600)};
+    double t[6] = {0, 0, 0, 0, 0, 0};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
+        const double x = q[i], y = q[i + M];
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            t[2 * j] = fma(x * c[j], x * c[j], t[2 * j]);
+            t[2 * j + 1] = fma(y * c[j], y * c[j], t[2 * j + 1]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+        if ((threadIdx.x & 31) == 0) sh[k][threadIdx.x >> 5] = t[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        double v = 0;
+        for (int i = 0; i < (int)(blockDim.x >> 5); i++) v += sh[threadIdx.x][i];
+        sums[2 * ((threadIdx.x >> 1) * gridDim.x + blockIdx.x) + (threadIdx.x & 1)] = v;
+    }
+}
+
 // mid, slab x of a slot: sp = 0 the half-step spectrum (inverse slab, times E2,
-// forward slab), sp = 1 the full-step spectrum (inverse slab, P = E2 qs1)
+// forward slab), sp = 1 the full-step spectrum (inverse slab, P = E2 qs1, and the sums
+// of its squares)
 template <class PS>
 __device__ __forceinline__ void pair_mid_body(const PS &B, const PropsArgs<double> &a, int s, int x, int sp, int slot)
 {
@@ -521,6 +643,7 @@ __device__ __forceinline__ void pair_mid_body(const PS &B, const PropsArgs<doubl
         B.forward_passes(spec, false, true);
     } else {
         cplx<T> *P = reinterpret_cast<cplx<T> *>(a.pbuf) + (size_t)slot * g.M + off;
+        T sx = 0, sy = 0;
         B.template real_space<true, false>([&](cplx<T> *v, int o) {
 #pragma unroll
             for (int r = 0; r < PS::RA; r++) {
@@ -528,19 +651,26 @@ __device__ __forceinline__ void pair_mid_body(const PS &B, const PropsArgs<doubl
                 v[r].x *= e0 * e0;
                 v[r].y *= e1 * e1;
             }
+            const T c = pair_pow2(-__ldcg(a.pexp + ((size_t)slot * (a.g.Ns + 1) + s) * 2));
 #pragma unroll
-            for (int r = 0; r < PS::RA; r++) stc(P + o + row * r, v[r]);
+            for (int r = 0; r < PS::RA; r++) {
+                stc(P + o + row * r, v[r]);
+                const T x0 = v[r].x * c, y0 = v[r].y * c;
+                sx = fma(x0, x0, sx);
+                sy = fma(y0, y0, sy);
+            }
         });
+        pair_cta_sums(sx, sy, a.partials + (size_t)slot * a.npart_stride + 2 * (x * PS::CTAS + B.rank));
         B.finish();
     }
 }
 
 // combine, slab x of a slot: finishes step s (mode 0: Richardson combination;
-// mode 1: q(s+1) = 1; mode 2: q(s+1) from the propagator store) and starts step
-// s + 1.  half: -1 one CTA makes both spectra; 0 / 1 this CTA makes only the
+// mode 1: q(s+1) = 1; mode 2: q(s+1) from the propagator store; mode 2 + n: the same,
+// its sizes from the sums of n blocks) and starts step s + 1.  half: -1 one CTA makes both spectra; 0 / 1 this CTA makes only the
 // half-step / full-step one (both repeat the inverse transform, which shortens
 // the chain when the batch leaves SMs idle; they are a cluster of two) and half
-// 0 stores q.
+// 0 stores q.  up: 2^k of step s + 1, down: 2^-k of step s.
 template <class PS>
 __device__ __forceinline__ void pair_combine_body(const PS &B, const PropsArgs<double> &a, int s, int mode, int x, int half,
                                                   int slot)
@@ -563,17 +693,24 @@ __device__ __forceinline__ void pair_combine_body(const PS &B, const PropsArgs<d
     __syncthreads();
     pdl_wait();
     if (pdl_early(g.m0)) pdl_trigger();
+    int *ex = a.pexp + ((size_t)slot * (g.Ns + 1) + sn) * 2;
+    int2 now = {0, 0}, nxt = {0, 0};  // exponents of steps s and s + 1; 0 for q(0) = 1
+    T up = 1, down = 1;
+    if (mode != 1) nxt = __ldcg(reinterpret_cast<const int2 *>(ex));
     if (mode == 0) {
+        now = __ldcg(reinterpret_cast<const int2 *>(ex) - 1);
         const cplx<T> *P = reinterpret_cast<const cplx<T> *>(a.pbuf) + (size_t)slot * M + off;
         if (threadIdx.x == 0) prefetch_l2(P, area * sizeof(cplx<T>));
         B.inverse_passes(specA, half >= 0);
+        up = pair_pow2(nxt.x - nxt.y);  // here: the loads have had the passes to arrive
+        down = pair_pow2(now.y - now.x);
         // Richardson, GPU_kernels.h:199-203
         auto finish = [&](cplx<T> *v, int o) {
 #pragma unroll
             for (int r = 0; r < PS::RA; r++) {
                 const cplx<T> p = ldc_cg(P + o + row * r);
                 v[r].x = third(v[r].x * __ldg(Eq + o + row * r) * (T)4 - p.x);
-                v[r].y = third(v[r].y * __ldg(Ep + o + row * r) * (T)4 - p.y);
+                v[r].y = third(v[r].y * __ldg(Ep + o + row * r) * (T)4 - p.y) * down;
             }
             if (store) {
 #pragma unroll
@@ -598,10 +735,14 @@ __device__ __forceinline__ void pair_combine_body(const PS &B, const PropsArgs<d
                     e1 *= e1;
                 }
                 v[r].x *= e0;
-                v[r].y *= e1;
+                v[r].y *= e1 * up;
             }
         });
     } else {
+        if (mode == 1 && x == 0 && B.rank == 0 && store && threadIdx.x == 0) *reinterpret_cast<int2 *>(ex) = nxt;
+        if (mode > 2) nxt = pair_slice_exponents(a.partials, mode - 2, a.invM);
+        if (mode > 2 && x == 0 && B.rank == 0 && store && threadIdx.x == 0) *reinterpret_cast<int2 *>(ex) = nxt;
+        up = pair_pow2(nxt.x - nxt.y);
         auto start = [&](cplx<T> *v, int o) {
 #pragma unroll
             for (int r = 0; r < PS::RA; r++) {
@@ -612,7 +753,7 @@ __device__ __forceinline__ void pair_combine_body(const PS &B, const PropsArgs<d
                     e1 *= e1;
                 }
                 v[r].x *= e0;
-                v[r].y *= e1;
+                v[r].y *= e1 * up;
             }
             if (mode == 1 && store) {
 #pragma unroll
@@ -633,7 +774,7 @@ __device__ __forceinline__ void pair_combine_body(const PS &B, const PropsArgs<d
 #pragma unroll
         for (int r = 0; r < PS::RA; r++) {
             const T e0 = __ldg(Nq + o + row * r), e1 = __ldg(Np + o + row * r);
-            v[r] = {q0[o + row * r] * (e0 * e0), q1[o + row * r] * (e1 * e1)};
+            v[r] = {q0[o + row * r] * (e0 * e0), q1[o + row * r] * (e1 * e1 * up)};
         }
     });
     B.forward_passes(specB, false, true);

@@ -27,10 +27,17 @@ __global__ void __launch_bounds__(512, 1) k_pair_combine_any(PropsArgs<T> a, int
 }
 
 template <int R2>
-__global__ void __launch_bounds__(kPencilThreads, 2) k_pair_pencil_any(PropsArgs<T> a, int ra, int rb)
+__global__ void __launch_bounds__(kPencilThreads, 2) k_pair_pencil_any(PropsArgs<T> a, int s, int nsum, int ra, int rb)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    pair_pencil_any_body<R2, kTile>(a, gridDim.x - 1 - blockIdx.x, blockIdx.y, gridDim.z - 1 - blockIdx.z, ra, rb, smem_raw);
+    const int tile = gridDim.x - 1 - blockIdx.x, slot = gridDim.z - 1 - blockIdx.z;
+    if (tile * kTile >= a.g.m1 * a.g.m2) {  // a tile past the last: the exponents of step s + 1
+        pdl_wait();
+        pdl_trigger();
+        pair_next_exponents(a, slot, s, nsum);
+        return;
+    }
+    pair_pencil_any_body<R2, kTile>(a, tile, blockIdx.y, slot, ra, rb, smem_raw);
 }
 
 }  // namespace
@@ -88,15 +95,15 @@ void pair_any_combine(const PropsArgs<T> &a, int nslots, int s, int mode, int sp
         }
 }
 
-void pair_any_pencil(const PropsArgs<T> &a, int nslots, int both, int ra, int rb, cudaStream_t st)
+void pair_any_pencil(const PropsArgs<T> &a, int nslots, int s, int both, int nsum, int ra, int rb, cudaStream_t st)
 {
     const Geo &g = a.g;
     int r1, r2;
     if (pair_x_radices(g.m0, r1, r2)) {
-        const dim3 grid((g.m1 * g.m2 + kTile - 1) / kTile, both ? 2 : 1, nslots);
+        const dim3 grid((g.m1 * g.m2 + kTile - 1) / kTile + !both, both ? 2 : 1, nslots);
         switch (r2) {
 #define X(A) \
-    case A: launch_step(k_pair_pencil_any<A>, grid, kPencilThreads, pair_any_pencil_smem(g.m0), 1, 1, st, a, ra, rb); break;
+    case A: launch_step(k_pair_pencil_any<A>, grid, kPencilThreads, pair_any_pencil_smem(g.m0), 1, 1, st, a, s, nsum, ra, rb); break;
             PAIR_RADICES(X)
 #undef X
         }

@@ -30,6 +30,16 @@ inline bool pair_slab_fixed(int m1, int m2)
     return false;
 }
 
+// CTAs that share a slab
+inline int pair_slab_ctas(int m1, int m2)
+{
+#define X(A, B) \
+    if (m1 == A && m2 == B) return kCl<A, B>;
+    PAIR_SLABS(X)
+#undef X
+    return 1;
+}
+
 inline bool pair_axis_fixed(int m0)
 {
 #define X(A) \
@@ -110,6 +120,6 @@ inline void pair_y_radices(int m1, int m2, int &ra, int &rb)
 int pair_any_setup(int m0, int m1, int m2);
 void pair_any_mid(const PropsArgs<double> &a, int nslots, int s, cudaStream_t st);
 void pair_any_combine(const PropsArgs<double> &a, int nslots, int s, int mode, int split, cudaStream_t st);
-void pair_any_pencil(const PropsArgs<double> &a, int nslots, int both, int ra, int rb, cudaStream_t st);
+void pair_any_pencil(const PropsArgs<double> &a, int nslots, int s, int both, int nsum, int ra, int rb, cudaStream_t st);
 
 }  // namespace scft

@@ -2,7 +2,8 @@
 // as one complex field, FP64.
 //
 // A pair <y, dS/dL x> needs the same pointwise products and x, y, z transforms of
-// x and of y, so x and y travel as c = x + i y through the slab and x passes of
+// x and of y, so x and y (times the power of two that makes their sizes alike, taken
+// back in the sums) travel as c = x + i y through the slab and x passes of
 // pair.cuh: half the transforms, no packing passes.  The Parseval sums come back
 // from the packed spectra: for real x, y and an even weight g,
 //   sum_k g Re(X conj Y)                = 1/2 sum_k g Im(C(k) C(-k)),
@@ -23,6 +24,13 @@ using T = double;
 struct StressSlab {
     const T *x, *y, *E4;
 };
+
+// k of pair p: the packed field is x + i 2^k y (pair.cuh)
+__device__ __forceinline__ int stress_shift(const StressArgs<T> &a, const StressPairs &P, int p)
+{
+    const int *e = a.pexp + (size_t)a.slot * (a.g.Ns + 1) * 2;
+    return pair_shift(__ldg(e + P.xe[p]), __ldg(e + P.ye[p]));
+}
 
 // real slabs of pair p at x index xi
 __device__ __forceinline__ StressSlab stress_slab(const StressArgs<T> &a, const StressPairs &P, int p, size_t off)
@@ -45,13 +53,14 @@ __device__ __forceinline__ void stress_fwd_body(const PS &B, const StressArgs<T>
     const size_t off = (size_t)xi * B.area();
     B.load_tables(a.tw, a.g.m0);
     const StressSlab s = stress_slab(a, P, p, off);
+    const T up = pair_pow2(stress_shift(a, P, p));
     B.sync();
     B.template real_space<false, true>([&](cplxd *v, int o) {
 #pragma unroll
         for (int r = 0; r < PS::RA; r++) {
             T e = __ldg(s.E4 + o + row * r);
             if (full) e *= e;
-            v[r] = {__ldg(s.x + o + row * r) * e, __ldg(s.y + o + row * r) * e};
+            v[r] = {__ldg(s.x + o + row * r) * e, __ldg(s.y + o + row * r) * e * up};
         }
     });
     B.forward_passes((full ? a.S2 : a.S4) + (size_t)p * a.g.M + off, false, false);
@@ -174,7 +183,7 @@ __global__ void __launch_bounds__(256, 2) k_pair_stress_pencil(StressArgs<T> a, 
 // The Parseval sums of pair blockIdx.y: rows 0-2 of its partials the K2 term of
 // dL_i, rows 6-8 the K1 term (the layout of k_stress_final).  r1, r2: x radices;
 // ra, rb: y radices of the position order.
-__global__ void __launch_bounds__(256) k_pair_stress_sums(StressArgs<T> a, int r1, int r2, int ra, int rb)
+__global__ void __launch_bounds__(256) k_pair_stress_sums(StressArgs<T> a, StressPairs P, int r1, int r2, int ra, int rb)
 {
     __shared__ double sh[6][8];
     const Geo &g = a.g;
@@ -220,7 +229,8 @@ __global__ void __launch_bounds__(256) k_pair_stress_sums(StressArgs<T> a, int r
         double t = 0;
         for (int j = 0; j < 8; j++) t += sh[i][j];
         const double L = a.L[i % 3];
-        a.part[((size_t)p * 9 + (i < 3 ? i : 3 + i)) * gridDim.x + blockIdx.x] = t * 8.0 * PI * PI / (L * L * L);
+        a.part[((size_t)p * 9 + (i < 3 ? i : 3 + i)) * gridDim.x + blockIdx.x] =
+            t * pair_pow2(-stress_shift(a, P, p)) * 8.0 * PI * PI / (L * L * L);
     }
 }
 
@@ -319,7 +329,7 @@ int pair_stress_chunk(const StressArgs<T> &a, const StressPairs &P, double *out,
     slab(1);
     pencil(0);
     const int nblk = std::min(g.m0, kStressSumBlocks);
-    k_pair_stress_sums<<<dim3(nblk, P.n), 256, 0, st>>>(a, r1, r2, ra, rb);
+    k_pair_stress_sums<<<dim3(nblk, P.n), 256, 0, st>>>(a, P, r1, r2, ra, rb);
     k_pair_stress_final<<<P.n, 192, 0, st>>>(a.part, nblk, P.n, 1.0 / g.M, out);
     return 6;
 }

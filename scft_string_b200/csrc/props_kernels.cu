@@ -18,6 +18,7 @@
 #include "common.cuh"
 #include "fft.cuh"
 #include "kernels.h"
+#include "pair.cuh"
 #include "pdl.cuh"
 #include "tma.cuh"
 #include "step_order.cuh"
@@ -56,8 +57,10 @@ __device__ __forceinline__ void load_tw(cplx<T> *dst, const cplx<T> *src, int n)
 // ---------------------------------------------------------------- prepare
 // E4 = exp(-wA ds/4), exp(-wB ds/4) with wA = W- + W+, wB = W+ - W-
 // (Prepare_dev_dev_expWds2_dev_expWds, GPU_kernels.h:215-225)
+// slice: also the sums of squares of that store slice of slot 0 (pair.cuh; the step
+// entry), -1: none
 template <typename T>
-__global__ void k_prepare(PropsArgs<T> a)
+__global__ void k_prepare(PropsArgs<T> a, int slice)
 {
     const Geo g = a.g;
     const int slot = blockIdx.y;
@@ -71,6 +74,9 @@ __global__ void k_prepare(PropsArgs<T> a)
         e[r + g.M] = (T)exp(-(-wm + wp) * ds / 4);
         // junction step: theta wA + (1 - theta) wB = W+ + (2 theta - 1) W-
         if (g.jon) a.jtab[(size_t)slot * g.M + r] = (T)exp(-(wp + (2.0 * g.theta - 1.0) * wm) * ds / 4);
+    }
+    if constexpr (sizeof(T) == 8) {
+        if (slice >= 0) pair_block_sums(a.hist + (size_t)slice * 2 * g.M, g.M, a.partials);
     }
 }
 
@@ -1237,11 +1243,11 @@ void launch_mid(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gs, int s, cud
 }
 
 template <typename T, int MT, int F0, int F1, int F2>
-void launch_pencil(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gp, int both, cudaStream_t st)
+void launch_pencil(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gp, int s, int both, cudaStream_t st)
 {
     if constexpr (sizeof(T) == 8) {
         if (L.pair) {
-            pair_pencil(a, gp.z, both, L.ptile_wide, st);
+            pair_pencil(a, gp.z, s, both, L.ptile_wide, st);
             return;
         }
     }
@@ -1277,7 +1283,7 @@ int launch_props_mt(const PropsArgs<T> &a, const PropsLaunch &L, int nslots, cud
 {
     const Geo &g = a.g;
     dim3 gs(g.m0, 2, nslots), gp(g.ncol_tiles, 2, nslots);
-    k_prepare<T><<<dim3(L.ew_blocks, nslots), 256, 0, st>>>(a);
+    k_prepare<T><<<dim3(L.ew_blocks, nslots), 256, 0, st>>>(a, -1);
     int n = 6;
     if constexpr (sizeof(T) == 8) {
         if (L.pair && L.persist) {
@@ -1317,9 +1323,9 @@ int launch_props_mt(const PropsArgs<T> &a, const PropsLaunch &L, int nslots, cud
     if (n == 6) {
         launch_combine<T, MT, F0, F1, F2>(a, L, gs, -1, 1, st);
         for (int s = 0; s < g.Ns; s++) {
-            launch_pencil<T, MT, F0, F1, F2>(a, L, gp, 1, st);
+            launch_pencil<T, MT, F0, F1, F2>(a, L, gp, s, 1, st);
             launch_mid<T, MT, F0, F1, F2>(a, L, gs, s, st);
-            launch_pencil<T, MT, F0, F1, F2>(a, L, gp, 0, st);
+            launch_pencil<T, MT, F0, F1, F2>(a, L, gp, s, 0, st);
             launch_combine<T, MT, F0, F1, F2>(a, L, gs, s, 0, st);
         }
         n += 4 * g.Ns;
@@ -1340,11 +1346,13 @@ int launch_single_step_mt(const PropsArgs<T> &a, const PropsLaunch &L, int s, cu
 {
     const Geo &g = a.g;
     dim3 gs(g.m0, 2, 1), gp(g.ncol_tiles, 2, 1);
-    k_prepare<T><<<dim3(L.ew_blocks, 1), 256, 0, st>>>(a);
-    launch_combine<T, MT, F0, F1, F2>(a, L, gs, s - 1, 2, st);
-    launch_pencil<T, MT, F0, F1, F2>(a, L, gp, 1, st);
+    // the packed kernels need the sizes of a slice that no step of theirs led to
+    const bool sizes = sizeof(T) == 8 && L.pair;
+    k_prepare<T><<<dim3(L.ew_blocks, 1), 256, 0, st>>>(a, sizes ? s : -1);
+    launch_combine<T, MT, F0, F1, F2>(a, L, gs, s - 1, 2 + (sizes ? L.ew_blocks : 0), st);
+    launch_pencil<T, MT, F0, F1, F2>(a, L, gp, s, 1, st);
     launch_mid<T, MT, F0, F1, F2>(a, L, gs, s, st);
-    launch_pencil<T, MT, F0, F1, F2>(a, L, gp, 0, st);
+    launch_pencil<T, MT, F0, F1, F2>(a, L, gp, s, 0, st);
     launch_combine<T, MT, F0, F1, F2>(a, L, gs, s, 0, st);
     return 6;
 }
@@ -1360,9 +1368,9 @@ int launch_chain_mt(const PropsArgs<T> &a, const PropsLaunch &L, int first_mode,
     dim3 gs(g.m0, 2, 1), gp(g.ncol_tiles, 2, 1);
     launch_combine<T, MT, F0, F1, F2>(a, L, gs, -1, first_mode, st);
     for (int s = 0; s < g.Ns; s++) {
-        launch_pencil<T, MT, F0, F1, F2>(a, L, gp, 1, st);
+        launch_pencil<T, MT, F0, F1, F2>(a, L, gp, s, 1, st);
         launch_mid<T, MT, F0, F1, F2>(a, L, gs, s, st);
-        launch_pencil<T, MT, F0, F1, F2>(a, L, gp, 0, st);
+        launch_pencil<T, MT, F0, F1, F2>(a, L, gp, s, 0, st);
         launch_combine<T, MT, F0, F1, F2>(a, L, gs, s, 0, st);
     }
     return 1 + 4 * g.Ns;
@@ -1527,7 +1535,7 @@ int launch_chain(const PropsArgs<T> &a, const PropsLaunch &L, int first_mode, cu
 template <typename T>
 int launch_prepare(const PropsArgs<T> &a, const PropsLaunch &L, cudaStream_t st)
 {
-    k_prepare<T><<<dim3(L.ew_blocks, 1), 256, 0, st>>>(a);
+    k_prepare<T><<<dim3(L.ew_blocks, 1), 256, 0, st>>>(a, -1);
     return 1;
 }
 

@@ -83,6 +83,7 @@ struct scft_ctx {
     double *partials = nullptr, *redout = nullptr;
     int npart_stride = 0, nred_rows = 0;
     int *rep_dev = nullptr, *err = nullptr;
+    int *pexp = nullptr;     // sizes of the propagators of the packed FP64 kernels (pair.cuh)
     int *sync = nullptr;     // counters of the persistent step kernel, one block per slot group
     int sync_stride = 0;
     bool persist_ok = false; // a persistent step launch exists for this context
@@ -179,6 +180,7 @@ PropsArgs<T> props_args(scft_ctx *ctx, const int *slot_rep)
     a.sync = ctx->sync;
     a.slot0 = 0;
     a.jtab = (T *)ctx->jtab;
+    a.pexp = ctx->pexp;
     return a;
 }
 
@@ -196,6 +198,7 @@ PropsArgs<T> props_args_from(scft_ctx *ctx, const int *slot_rep, int s0, int lan
     a.partials += (size_t)s0 * ctx->npart_stride;
     a.slot0 = s0;
     if (a.jtab) a.jtab += (size_t)s0 * M;
+    if (a.pexp) a.pexp += (size_t)s0 * (ctx->g.Ns + 1) * 2;
     if (a.sync && lane) a.sync += ctx->sync_stride;  // counters of the groups on the second stream
     return a;
 }
@@ -653,7 +656,7 @@ void scft_destroy(scft_ctx *ctx)
     void *ptrs[] = {ctx->W, ctx->conc, ctx->DEV, ctx->dWda, ctx->rs, ctx->partials, ctx->redout,
                     ctx->rep_dev, ctx->etab, ctx->hist, ctx->spec, ctx->pbuf, ctx->tw,
                     ctx->kfac, ctx->knots, ctx->st_S4, ctx->st_S2, ctx->st_S4p, ctx->st_part,
-                    ctx->st_out, ctx->and_X, ctx->and_D, ctx->ck_mem, ctx->jtab, ctx->jd_rbuf, ctx->sync};
+                    ctx->st_out, ctx->and_X, ctx->and_D, ctx->ck_mem, ctx->jtab, ctx->jd_rbuf, ctx->sync, ctx->pexp};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (ctx->host_mem) cudaFreeHost(ctx->host_mem);
@@ -828,6 +831,7 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
         CKC(cudaMalloc(&ctx->spec, T * 2 * 4 * (size_t)g.Mk * S));
         CKC(cudaMalloc(&ctx->pbuf, T * 2 * M * S));
         L.pair = T == 8 && pair_applicable(g.m0, g.m1, g.m2);
+        if (L.pair) CKC(cudaMalloc(&ctx->pexp, sizeof(int) * 2 * (size_t)(g.Ns + 1) * S));
         if (L.reg || L.fixed || L.pair) {  // counters of the persistent step launch
             ctx->sync_stride = reg64_sync_ints(g.Ns, (int)S);
             CKC(cudaMalloc(&ctx->sync, sizeof(int) * 2 * (size_t)ctx->sync_stride));
@@ -1550,6 +1554,7 @@ namespace {
 // `hist` (slot `slot`), E table `sel`, homopolymer (Q2) or copolymer (QC) sum
 struct StressPr {
     int xs, xf, ys, yf, sel, homo;
+    int xt, yt;  // contour steps of the slices xs and ys
 };
 
 scft_status stress_alloc(scft_ctx *ctx)
@@ -1593,6 +1598,8 @@ scft_status stress_pairs(scft_ctx *ctx, int rep, int slot, const void *hist, con
             P.ys[p] = q.ys;
             P.yf[p] = q.yf;
             P.sel[p] = q.sel;
+            P.xe[p] = 2 * q.xt + q.xf;
+            P.ye[p] = 2 * q.yt + q.yf;
         }
         int nl;
         if (ctx->prec == SCFT_FP32) {
@@ -1611,6 +1618,7 @@ scft_status stress_pairs(scft_ctx *ctx, int rep, int slot, const void *hist, con
                                  (cplx<double> *)ctx->st_S4p, ctx->st_part,
                                  {Lr[0], Lr[1], Lr[2]}, 1.0 / g.M, ctx->err};
             a.jtab = (const double *)ctx->jtab;
+            a.pexp = ctx->pexp;
             nl = ctx->L.pair ? pair_stress_chunk(a, P, ctx->st_out + 3 * c0, ctx->st)
                              : launch_stress_chunk<double>(a, P, ctx->rt_slab_threads, ctx->rt_slab_smem,
                                                            ctx->rt_pencil_threads, ctx->rt_pencil_smem,
@@ -1689,8 +1697,8 @@ scft_status scft_stress(scft_ctx *ctx, int ii, double *dlnQ_dL, double *dF_dL)
     const double Q2 = rsv(ctx, ii, kRsQ2), QC = rsv(ctx, ii, kRsQC);
     // pairs: copolymer (q(s), q^dagger(N-1-s)), homopolymer (q^dagger(j), q^dagger(Nh-1-j))
     std::vector<StressPr> pairs;
-    for (int s2 = 0; s2 < g.Ns; s2++) pairs.push_back({s2, 0, g.Ns - 1 - s2, 1, q_table(g, s2), 0});
-    for (int j = 0; j < g.Nh; j++) pairs.push_back({j, 1, g.Nh - 1 - j, 1, 1, 1});
+    for (int s2 = 0; s2 < g.Ns; s2++) pairs.push_back({s2, 0, g.Ns - 1 - s2, 1, q_table(g, s2), 0, s2, g.Ns - 1 - s2});
+    for (int j = 0; j < g.Nh; j++) pairs.push_back({j, 1, g.Nh - 1 - j, 1, 1, 1, j, g.Nh - 1 - j});
     double dQC[3] = {0, 0, 0}, dQ2[3] = {0, 0, 0};
     s = stress_pairs(ctx, ii, slot, ctx->hist, pairs, dQC, dQ2);
     if (s != SCFT_OK) return s;
@@ -1735,9 +1743,11 @@ void ckpt_chain(scft_ctx *ctx, int p0, int len, void *buf, int first_mode)
     gg.n2 = g.n2 - p0;
     gg.jq = g.jq - p0;
     gg.jqd = g.jqd - p0;
+    PropsArgs<double> ad = ckpt_args<double>(ctx, gg, buf);
+    if (ad.pexp) ad.pexp += 2 * p0;  // sizes by contour index: a piece starts with those of the chain before it
     ctx->stats.kernel_launches += ctx->prec == SCFT_FP32
                                       ? launch_chain<float>(ckpt_args<float>(ctx, gg, buf), ctx->L, first_mode, ctx->st)
-                                      : launch_chain<double>(ckpt_args<double>(ctx, gg, buf), ctx->L, first_mode, ctx->st);
+                                      : launch_chain<double>(ad, ctx->L, first_mode, ctx->st);
 }
 
 // allocation, forward pass (checkpoints, q^dagger(Nh), q(N)), then Q2, QC,
@@ -1868,17 +1878,17 @@ scft_status scft_stress_ckpt(scft_ctx *ctx, int ii, int K, double *dlnQ_dL, doub
             for (int t = a0; t < a1; t++) {
                 const int u = n - 1 - t;
                 if (homo)
-                    pairs.push_back({t - a0, 1, yb + (u - m0), 1, 1, 1});
+                    pairs.push_back({t - a0, 1, yb + (u - m0), 1, 1, 1, t, u});
                 else
-                    pairs.push_back({t - a0, 0, yb + (u - m0), 1, q_table(g, t), 0});
+                    pairs.push_back({t - a0, 0, yb + (u - m0), 1, q_table(g, t), 0, t, u});
             }
             if (!self)
                 for (int t = m0; t < m1; t++) {
                     const int u = n - 1 - t;
                     if (homo)
-                        pairs.push_back({(int)segoff + (t - m0), 1, u - a0, 1, 1, 1});
+                        pairs.push_back({(int)segoff + (t - m0), 1, u - a0, 1, 1, 1, t, u});
                     else
-                        pairs.push_back({(int)segoff + (t - m0), 0, u - a0, 1, q_table(g, t), 0});
+                        pairs.push_back({(int)segoff + (t - m0), 0, u - a0, 1, q_table(g, t), 0, t, u});
                 }
             scft_status st = stress_pairs(ctx, ii, 0, seg, pairs, dQC, dQ2);
             if (st != SCFT_OK) return st;

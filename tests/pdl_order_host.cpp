@@ -39,8 +39,7 @@ static inline void __syncwarp() {}
 static inline float __fmul_rn(float a, float b) { return a * b; }
 static inline float __fmaf_rn(float a, float b, float c) { return fmaf(a, b, c); }
 static inline unsigned __umulhi(unsigned a, unsigned b) { return (unsigned)(((unsigned long long)a * b) >> 32); }
-static inline unsigned __reduce_max_sync(unsigned, unsigned v) { return v; }
-static inline unsigned atomicMax(unsigned *p, unsigned v) { return *p > v ? *p : (*p = v); }
+static inline double __shfl_xor_sync(unsigned, double v, int) { return v; }
 static inline int __double2hiint(double v)
 {
     uint64_t b;
@@ -83,14 +82,15 @@ alignas(128) unsigned char smem_raw[1 << 18];  // the kernels' dynamic shared me
 
 using namespace scft;
 
-enum { W = 0, HIST, ETAB, JTAB, SPEC, PBUF, SCALE, CONST };
+enum { W = 0, HIST, ETAB, JTAB, SPEC, PBUF, SIZES, CONST };
 
 template <class T>
 struct Case {
     PropsArgs<T> a{};
     std::vector<T> etab, jtab, hist, pbuf, kfac;
     std::vector<cplx<T>> spec, tw;
-    std::vector<int> rep, sync;
+    std::vector<int> rep, pexp;
+    std::vector<double> partials;
     int err = 0;
 
     template <class V>
@@ -121,6 +121,8 @@ struct Case {
         own(tw, 3 * m, CONST);
         own(kfac, 3 * m, CONST);
         own(rep, 1, CONST);
+        own(pexp, 2 * (Ns + 1), SIZES);
+        own(partials, 4 * m, SIZES);
         a.etab = etab.data();
         a.jtab = jtab.data();
         a.hist = hist.data();
@@ -130,6 +132,8 @@ struct Case {
         a.kfac = kfac.data();
         a.slot_rep = rep.data();
         a.err = &err;
+        a.pexp = pexp.data();
+        a.partials = partials.data();
         a.invM = a.Mreal = (T)1;
         blockIdx = {0, 0, 0};
         gridDim = dim3(1, 2, 1);

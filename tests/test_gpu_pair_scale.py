@@ -1,0 +1,114 @@
+"""The packed FP64 step (csrc/pair.cuh) carries q + i 2^k q^dagger with k chosen so that
+both parts are of one size: each propagator keeps the precision of a transform of its
+own, whatever the mean of W- makes of the other.  Chains and single steps against the
+same scheme in 80-bit arithmetic on the host, the box stress against the FP64 oracle."""
+import numpy as np
+import pytest
+
+import oracle as O
+import scft_string_b200 as S
+
+pytestmark = pytest.mark.gpu
+
+LD = np.longdouble
+PI = LD("3.14159265358979323846264338327950288")
+EPS = np.finfo(float).eps
+
+
+def _h(m, D, N):
+    k2 = LD(0)
+    for i in range(3):
+        n = np.fft.fftfreq(m[i], 1.0 / m[i]) if i < 2 else np.arange(m[2] // 2 + 1)
+        shape = [1, 1, 1]
+        shape[i] = -1
+        k2 = k2 + ((2 * PI * n.astype(LD) / LD(D[i])) ** 2).reshape(shape)
+    return np.exp(-k2 / (12 * LD(N)))
+
+
+def _step(q, e4, h):
+    """One Richardson step in 80 bits (density.h:129-220); e4 = exp(-w ds/4)."""
+    conv = lambda v, g: np.fft.irfftn(np.fft.rfftn(v) * g, s=v.shape, axes=(0, 1, 2))  # noqa: E731
+    e2 = e4 * e4
+    return (4 * e4 * conv(e2 * conv(e4 * q, h), h) - e2 * conv(e2 * q, h * h)) / 3
+
+
+def _e4(wm, wp, m, N):
+    wm, wp = wm.astype(LD).reshape(m), wp.astype(LD).reshape(m)
+    return np.exp(-(wm + wp) / (4 * LD(N))), np.exp(-(wp - wm) / (4 * LD(N)))
+
+
+def _err(got, ref):
+    d = got.astype(LD).ravel() - ref.ravel()
+    return float(np.sqrt((d * d).sum() / (ref * ref).sum()))
+
+
+def _fields(m, mean):
+    rng = np.random.default_rng(11)
+    M = int(np.prod(m))
+    return mean + rng.normal(0, 2.0, M), rng.normal(0, 0.5, M)
+
+
+# a slab in one CTA, run-time sizes, one unmerged slab over two CTAs
+@pytest.mark.parametrize("m", [(16, 16, 16), (10, 12, 25), (4, 128, 128)])
+@pytest.mark.parametrize("mean", [0.0, 6.0, -10.0, 20.0, 40.0])
+def test_propagators_keep_their_precision(built_lib, m, mean):
+    N, f = 48, 0.375
+    D = tuple(v / 12 for v in m)
+    n1 = round(N * f)
+    wm, wp = _fields(m, mean)
+    ctx = S.Context(m, D, N, chi=20, f=f, phidb=0.8, ens=2, strn=1, dostring=0, alpha=0.2)
+    ctx.set_fields(0, wm, wp)
+    ctx.props(0)
+    eA, eB = _e4(wm, wp, m, N)
+    h = _h(m, D, N)
+    for fld, (e1, e2, n) in enumerate(((eA, eB, n1), (eB, eA, N - n1))):
+        q = np.ones(m, LD)
+        for s in range(N):
+            q = _step(q, e1 if s < n else e2, h)
+            if s + 1 in (n1, N // 2, N - n1, N):
+                # one rounding unit per step, all of one sign
+                assert _err(ctx.propagator(0, fld, s + 1), q) <= N * EPS, (fld, s + 1)
+
+
+@pytest.mark.parametrize("m", [(16, 16, 16), (35, 6, 45)])
+@pytest.mark.parametrize("size", [1e-9, 1e7, 1e-250, 1e250, "point"])
+def test_step_of_slices_of_different_size(built_lib, m, size):
+    N, s = 32, 9
+    D = tuple(v / 12 for v in m)
+    wm, wp = _fields(m, 0.0)
+    M = wm.size
+    rng = np.random.default_rng(12)
+    q = 1.0 + 0.3 * rng.normal(size=2 * M)
+    if size == "point":
+        q[:M] = 0.0
+        q[M // 3] = 1e-6
+    else:
+        q[M:] *= size
+    ctx = S.Context(m, D, N, chi=20, f=0.5, phidb=0.8, ens=2, strn=1, dostring=0)
+    ctx.set_fields(0, wm, wp)
+    out = ctx.do_step(0, q, s)
+    eA, eB = _e4(wm, wp, m, N)
+    h = _h(m, D, N)
+    # six transforms, each of a rounding unit per factor two of its length, and the
+    # pointwise products
+    tol = 6 * np.log2(M) * EPS
+    assert _err(out[:M], _step(q[:M].astype(LD).reshape(m), eA, h)) <= tol
+    assert _err(out[M:], _step(q[M:].astype(LD).reshape(m), eB, h)) <= tol
+
+
+# every kind of slab and x pass: odd axes, one column left over in the last x tile, x
+# planes beyond the blocks of the sums, merged passes, a slab over two CTAs
+@pytest.mark.parametrize("m,mean", [((8, 12, 10), 0.0), ((8, 12, 10), 10.0), ((8, 12, 10), 40.0), ((3, 5, 7), 0.0),
+                                    ((9, 15, 14), 0.0), ((7, 9, 25), 3.0), ((14, 15, 15), 0.0), ((96, 24, 24), 5.0),
+                                    ((8, 64, 96), 0.0), ((16, 48, 48), 0.0), ((4, 128, 128), 8.0)])
+@pytest.mark.parametrize("fcont", [0, 1])
+def test_stress_matches_oracle(built_lib, m, mean, fcont):
+    N, f = 20, 0.43 if fcont else 0.45
+    D = tuple(v / 12 for v in m)
+    wm, wp = _fields(m, mean)
+    ctx = S.Context(m, D, N, chi=12, f=f, phidb=0.8, ens=1, alpha=0.1, strn=1, dostring=0, fcont=fcont)
+    ctx.set_fields(0, wm, wp)
+    ref = O.Density(m, D, N).stress(np.concatenate([wm, wp]), N, 0.1, 0.8, f, 1, fcont=bool(fcont))
+    tol = 1e-10 * np.abs(ref).max()
+    assert np.abs(ctx.stress(0)[0] - ref).max() <= tol
+    assert np.abs(ctx.stress_ckpt(0, 6)[0] - ref).max() <= tol

@@ -17,7 +17,7 @@ from test_reg64_host import _cuda_include
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "..", "scft_string_b200", "csrc")
-ARRAYS = ["W", "HIST", "ETAB", "JTAB", "SPEC", "PBUF", "SCALE", "CONST"]
+ARRAYS = ["W", "HIST", "ETAB", "JTAB", "SPEC", "PBUF", "SIZES", "CONST"]
 
 PDL = """#pragma once
 #include <cstring>
