@@ -665,6 +665,11 @@ __device__ __forceinline__ void pair_mid_body(const PS &B, const PropsArgs<doubl
     }
 }
 
+// Products that the additions of the transform after them must not fuse with: whether a
+// step follows another one, starts from a stored slice or makes its spectra in two
+// CTAs, it then gives the same bits.
+__device__ __forceinline__ cplxd rounded(cplxd v, double fx, double fy) { return {__dmul_rn(v.x, fx), __dmul_rn(v.y, fy)}; }
+
 // combine, slab x of a slot: finishes step s (mode 0: Richardson combination;
 // mode 1: q(s+1) = 1; mode 2: q(s+1) from the propagator store; mode 2 + n: the same,
 // its sizes from the sums of n blocks) and starts step s + 1.  half: -1 one CTA makes both spectra; 0 / 1 this CTA makes only the
@@ -734,8 +739,7 @@ __device__ __forceinline__ void pair_combine_body(const PS &B, const PropsArgs<d
                     e0 *= e0;
                     e1 *= e1;
                 }
-                v[r].x *= e0;
-                v[r].y *= e1 * up;
+                v[r] = rounded(v[r], e0, e1 * up);
             }
         });
     } else {
@@ -752,8 +756,7 @@ __device__ __forceinline__ void pair_combine_body(const PS &B, const PropsArgs<d
                     e0 *= e0;
                     e1 *= e1;
                 }
-                v[r].x *= e0;
-                v[r].y *= e1 * up;
+                v[r] = rounded(v[r], e0, e1 * up);
             }
             if (mode == 1 && store) {
 #pragma unroll
@@ -774,7 +777,7 @@ __device__ __forceinline__ void pair_combine_body(const PS &B, const PropsArgs<d
 #pragma unroll
         for (int r = 0; r < PS::RA; r++) {
             const T e0 = __ldg(Nq + o + row * r), e1 = __ldg(Np + o + row * r);
-            v[r] = {q0[o + row * r] * (e0 * e0), q1[o + row * r] * (e1 * e1 * up)};
+            v[r] = rounded({q0[o + row * r], q1[o + row * r]}, e0 * e0, e1 * e1 * up);
         }
     });
     B.forward_passes(specB, false, true);

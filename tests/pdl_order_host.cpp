@@ -38,6 +38,7 @@ static inline void __syncthreads() {}
 static inline void __syncwarp() {}
 static inline float __fmul_rn(float a, float b) { return a * b; }
 static inline float __fmaf_rn(float a, float b, float c) { return fmaf(a, b, c); }
+static inline double __dmul_rn(double a, double b) { return a * b; }
 static inline unsigned __umulhi(unsigned a, unsigned b) { return (unsigned)(((unsigned long long)a * b) >> 32); }
 static inline double __shfl_xor_sync(unsigned, double v, int) { return v; }
 static inline int __double2hiint(double v)

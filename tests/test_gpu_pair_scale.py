@@ -96,6 +96,24 @@ def test_step_of_slices_of_different_size(built_lib, m, size):
     assert _err(out[M:], _step(q[M:].astype(LD).reshape(m), eB, h)) <= tol
 
 
+@pytest.mark.parametrize("m", [(16, 16, 16), (10, 12, 25), (48, 48, 48), (4, 128, 128)])
+@pytest.mark.parametrize("mean", [0.0, 10.0, 40.0])
+def test_checkpointed_chain_has_the_same_bits(built_lib, m, mean):
+    """A chain that starts again from a checkpoint goes on with the sizes it had and
+    rounds as the chain without a break does: the same lnQ, and the same densities up
+    to the order of the density sums."""
+    N = 48
+    wm, wp = _fields(m, mean)
+    ctx = S.Context(m, tuple(v / 12 for v in m), N, chi=20, f=0.375, phidb=0.8, ens=1, strn=1, dostring=0, alpha=0.2)
+    ctx.set_fields(0, wm, wp)
+    ctx.props(0)
+    full, lnQ, _ = ctx.get_conc(0)
+    q, _, _ = ctx.props_ckpt(0, 7)
+    ck = ctx.get_conc(0)[0]
+    assert q == lnQ
+    assert np.abs(ck - full).max() <= 4 * N * EPS * np.abs(full).max()
+
+
 # every kind of slab and x pass: odd axes, one column left over in the last x tile, x
 # planes beyond the blocks of the sums, merged passes, a slab over two CTAs
 @pytest.mark.parametrize("m,mean", [((8, 12, 10), 0.0), ((8, 12, 10), 10.0), ((8, 12, 10), 40.0), ((3, 5, 7), 0.0),
