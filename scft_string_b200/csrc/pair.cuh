@@ -518,11 +518,16 @@ __device__ __forceinline__ void pair_cta_sums(double x, double y, double *out)
         sh[1][threadIdx.x >> 5] = y;
     }
     __syncthreads();
-    if (threadIdx.x < 2) {
-        double t = 0;
-        for (int i = 0; i < (int)(blockDim.x >> 5); i++) t += sh[threadIdx.x][i];
-        out[threadIdx.x] = t;
+    if (threadIdx.x >= 32) return;
+    const bool in = threadIdx.x < blockDim.x >> 5;
+    x = in ? sh[0][threadIdx.x] : 0;
+    y = in ? sh[1][threadIdx.x] : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        x += __shfl_xor_sync(0xffffffffu, x, o);
+        y += __shfl_xor_sync(0xffffffffu, y, o);
     }
+    if (threadIdx.x == 0) *reinterpret_cast<double2 *>(out) = make_double2(x, y);
 }
 
 // Floors of the binary exponents of the root mean squares that n pairs of partial sums
@@ -630,6 +635,7 @@ __device__ __forceinline__ void pair_mid_body(const PS &B, const PropsArgs<doubl
     __syncthreads();
     pdl_wait();
     if (pdl_early(g.m0)) pdl_trigger();
+    const int eq = sp ? __ldcg(a.pexp + ((size_t)slot * (g.Ns + 1) + s) * 2) : 0;  // size of q(s)
     B.inverse_passes(spec);
     if (sp == 0) {
         B.template real_space<true, true>([&](cplx<T> *v, int o) {
@@ -651,7 +657,7 @@ __device__ __forceinline__ void pair_mid_body(const PS &B, const PropsArgs<doubl
                 v[r].x *= e0 * e0;
                 v[r].y *= e1 * e1;
             }
-            const T c = pair_pow2(-__ldcg(a.pexp + ((size_t)slot * (a.g.Ns + 1) + s) * 2));
+            const T c = pair_pow2(-eq);
 #pragma unroll
             for (int r = 0; r < PS::RA; r++) {
                 stc(P + o + row * r, v[r]);
