@@ -305,6 +305,43 @@ int groups_for(const scft_ctx *ctx, int nb)
     return ctx->ngroups > 0 ? effective_groups(ctx->ngroups, nb) : default_groups(ctx, nb);
 }
 
+// The packed FP64 kernels carry q and q^dagger as one complex field (pair.cuh), whose
+// transforms spread an infinity or a NaN of one over both.  A nonfinite q or q^dagger
+// that went into a transform leaves q(N), and so QC, nonfinite: such a replica is done
+// again on the kernels with a transform for each.
+PropsLaunch separate_launch(const scft_ctx *ctx)
+{
+    PropsLaunch L = ctx->L;
+    L.pair = L.persist = 0;
+    return L;
+}
+
+double rsv(const scft_ctx *ctx, int rep, int k) { return ctx->rs_h[(size_t)rep * kRsStride + k]; }
+
+// after a round over reps (uploaded): the replicas of nonfinite QC again; each stays in
+// its slot where it still has one
+scft_status redo_nonfinite(scft_ctx *ctx, const std::vector<int> &reps)
+{
+    int redone = 0;
+    for (size_t i = 0; i < reps.size(); i++) {
+        const int r = reps[i];
+        if (std::isfinite(rsv(ctx, r, kRsQC))) continue;
+        const int slot = std::max(ctx->slot_of[r], 0);
+        for (auto &so : ctx->slot_of)
+            if (so == slot) so = -1;
+        ctx->slot_of[r] = slot;
+        PropsArgs<double> a = props_args_from<double>(ctx, ctx->rep_dev, slot);
+        a.slot_rep = ctx->rep_dev + i;
+        ctx->stats.kernel_launches += launch_props<double>(a, separate_launch(ctx), 1, ctx->st);
+        redone++;
+    }
+    if (!redone) return SCFT_OK;
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(ctx->rs_h, ctx->rs, sizeof(double) * kRsStride * ctx->nrep_alloc, cudaMemcpyDeviceToHost,
+                       ctx->st));
+    return check_device_err(ctx);
+}
+
 // density::props for a list of replicas; scalars land in ctx->rs_h.  Without a
 // full store (nostore) each replica runs from checkpoints.
 scft_status props_list(scft_ctx *ctx, const std::vector<int> &reps)
@@ -397,10 +434,8 @@ scft_status props_list(scft_ctx *ctx, const std::vector<int> &reps)
     ctx->stats.props_calls += (long long)reps.size();
     ctx->stats.contour_steps += (long long)reps.size() * ctx->g.Ns;
     ctx->stats.kernel_launches += launches;
-    return SCFT_OK;
+    return ctx->L.pair ? redo_nonfinite(ctx, reps) : SCFT_OK;
 }
-
-double rsv(const scft_ctx *ctx, int rep, int k) { return ctx->rs_h[(size_t)rep * kRsStride + k]; }
 
 // final reduction of `rows` partial rows into ctx->red_h
 scft_status reduce_rows(scft_ctx *ctx, int rows, int nblk)
@@ -1099,6 +1134,18 @@ scft_status scft_do_step(scft_ctx *ctx, int ii, const double *in, double *out, i
     st = check_device_err(ctx);
     if (st != SCFT_OK) return st;
     copy_out_finish(ctx, dst, slice * T);
+    // A nonfinite value that went into a transform leaves q or q^dagger nonfinite at
+    // every point (separate_launch).  Slice s is still in the store.
+    if (ctx->L.pair && !(std::isfinite(out[0]) && std::isfinite(out[M]))) {
+        ctx->stats.kernel_launches += launch_single_step<double>(props_args<double>(ctx, ctx->rep_dev),
+                                                                 separate_launch(ctx), s, ctx->st);
+        CK(cudaGetLastError());
+        st = copy_out_start(ctx, dst, h0 + slice * T, slice * T);
+        if (st != SCFT_OK) return st;
+        st = check_device_err(ctx);
+        if (st != SCFT_OK) return st;
+        copy_out_finish(ctx, dst, slice * T);
+    }
     if (T == 4)
         for (size_t i = 0; i < slice; i++) out[i] = tmp[i];
     return SCFT_OK;
@@ -1935,6 +1982,16 @@ scft_status props_ckpt_impl(scft_ctx *ctx, int ii, int K, double *lnQ_out, doubl
     CkptRun R;
     scft_status s = ckpt_forward(ctx, ii, K, 6 * M * sizeof(double), R);
     if (s != SCFT_OK) return s;
+    struct KeepLaunch {
+        scft_ctx *ctx;
+        PropsLaunch L;
+        ~KeepLaunch() { ctx->L = L; }
+    } keep{ctx, ctx->L};
+    if (ctx->L.pair && !std::isfinite(rsv(ctx, ii, kRsQC))) {  // as redo_nonfinite
+        ctx->L = separate_launch(ctx);
+        s = ckpt_forward(ctx, ii, K, 6 * M * sizeof(double), R);
+        if (s != SCFT_OK) return s;
+    }
     if (bytes_out) *bytes_out = R.bytes;
     double *acc = reinterpret_cast<double *>(R.extra);
     CK(cudaMemsetAsync(acc, 0, 6 * M * sizeof(double), ctx->st));

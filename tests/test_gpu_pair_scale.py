@@ -130,3 +130,60 @@ def test_stress_matches_oracle(built_lib, m, mean, fcont):
     tol = 1e-10 * np.abs(ref).max()
     assert np.abs(ctx.stress(0)[0] - ref).max() <= tol
     assert np.abs(ctx.stress_ckpt(0, 6)[0] - ref).max() <= tol
+
+
+@pytest.mark.parametrize("m", [(16, 16, 16), (10, 12, 25)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_step_keeps_a_nonfinite_slice_to_itself(built_lib, m, bad):
+    N, s = 32, 9
+    D = tuple(v / 12 for v in m)
+    wm, wp = _fields(m, 0.0)
+    M = wm.size
+    ctx = S.Context(m, D, N, chi=20, f=0.5, phidb=0.8, ens=2, strn=1, dostring=0)
+    ctx.set_fields(0, wm, wp)
+    eA, eB = _e4(wm, wp, m, N)
+    h = _h(m, D, N)
+    q = 1.0 + 0.3 * np.random.default_rng(13).normal(size=2 * M)
+    for fld, e4 in ((0, eB), (1, eA)):
+        p = q.copy()
+        p[fld * M + M // 2] = bad
+        out = ctx.do_step(0, p, s).reshape(2, M)
+        assert not np.isfinite(out[fld]).any()
+        o = 1 - fld
+        assert _err(out[o], _step(p[o * M:(o + 1) * M].astype(LD).reshape(m), e4, h)) <= 6 * np.log2(M) * EPS
+
+
+@pytest.mark.parametrize("nostore", [0, 1])
+def test_densities_where_one_propagator_overflows(built_lib, nostore):
+    """Replica 1 of three has an A field in which q grows beyond a double at once; its
+    homopolymer, which sees the B field alone, and the other replicas do not notice."""
+    m, N, alpha = (16, 12, 10), 20, 0.2
+    D = tuple(v / 12 for v in m)
+    M = int(np.prod(m))
+    W = [_fields(m, 0.0) for _ in range(3)]
+    big = 5e3
+    W[1] = (W[1][0] - big, W[1][1] - big)  # wA = W- + W+, wB = W+ - W-
+    ctx = S.Context(m, D, N, chi=12, f=0.4, phidb=0.8, ens=1, strn=3, dostring=0, alpha=alpha, nostore=nostore, ckpt_K=6)
+    for ii in range(3):
+        ctx.set_fields(ii, *W[ii])
+    with pytest.raises(S.ScftError, match="replica 1"):
+        ctx.solve_field0_all(2, 0.0)  # one round, which then finds the residual of replica 1 to be NaN
+    for ii in (0, 2):
+        conc, lnQ, phis = ctx.get_conc(ii)
+        w = np.concatenate([*W[ii], np.zeros(4 * M)])
+        ref_lnQ, ref = O.Density(m, D, N).props(w, N, alpha, 0.8, 0.4, 1)
+        assert np.abs(conc - w[2 * M:]).max() <= 1e-12 * np.abs(w[2 * M:]).max()
+        assert abs(lnQ - ref_lnQ) <= 1e-12 * abs(ref_lnQ) and abs(phis[4] - ref[4]) <= 1e-12 * abs(ref[4])
+    # q^dagger of replica 1 in the B block, and the homopolymer's Simpson sum (density.h:404-422)
+    eB, h, Nh = _e4(*W[1], m, N)[1], _h(m, D, N), int(alpha * N)
+    q = [np.ones(m, LD)]
+    for s in range(Nh):
+        q.append(_step(q[-1], eB, h))
+    rh = 2 * q[Nh] + sum((2 if (s - 1) % 2 else 4) * q[s] * q[Nh - s] for s in range(1, Nh))
+    rh = rh * (1 - 0.8) / (q[Nh].mean() * alpha) / (3 * LD(N))
+    conc, lnQ, phis = ctx.get_conc(1)
+    assert not np.isfinite(lnQ) and not np.isfinite(conc[:2 * M]).any()
+    assert _err(conc[2 * M:3 * M], rh) <= N * EPS
+    assert abs(phis[4] - float(rh.mean())) <= N * EPS * abs(phis[4])
+    if not nostore:
+        assert _err(ctx.propagator(1, 1, Nh), q[Nh]) <= N * EPS
