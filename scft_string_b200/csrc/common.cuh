@@ -54,6 +54,24 @@ __host__ __device__ __forceinline__ int div_by(int b, unsigned mag)
 #endif
 }
 
+// Compensated sum (W. Kahan, Commun. ACM 8, 1965): the value is sum - c.
+__host__ __device__ __forceinline__ void kahan_add(double &sum, double &c, double term)
+{
+    const double y = term - c;
+    const double t = sum + y;
+    c = (t - sum) - y;
+    sum = t;
+}
+
+// (sum, c) + (sum2, c2), either of which may be the larger: the rounding of the two sums
+// by D. E. Knuth's exact addition goes into the compensation
+__host__ __device__ __forceinline__ void kahan_join(double &sum, double &c, double sum2, double c2)
+{
+    const double t = sum + sum2, b = t - sum;
+    c = (c + c2) - ((sum - (t - b)) + (sum2 - b));
+    sum = t;
+}
+
 // Mixed-radix factorisation of one FFT length (radices 2, 3, 4, 5, 7, 8).
 struct Plan1D {
     int n;

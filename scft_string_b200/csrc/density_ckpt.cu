@@ -3,19 +3,12 @@
 // (scft_props_ckpt): the terms w_s q(s) q^dagger(N-s) arrive in batches of
 // slice pairs and are Kahan-accumulated per grid point in FP64; a final
 // kernel scales them into phiA, phiB, phih, phicB and the phis averages.
+#include "common.cuh"
 #include "kernels.h"
 
 namespace scft {
 
 namespace {
-
-__device__ __forceinline__ void kahan(double &sum, double &c, double term)
-{
-    const double y = term - c;
-    const double t = sum + y;
-    c = (t - sum) - y;
-    sum = t;
-}
 
 __device__ __forceinline__ double bsum(double v, double *sh)
 {
@@ -42,9 +35,9 @@ __global__ void k_dens_acc(const T *__restrict__ base, size_t M, DensPairs P, do
         for (int k = 0; k < 6; k++) s[k] = acc[k * M + r];
         for (int p = 0; p < P.n; p++) {
             const double t = (double)base[P.x[p] + r] * (double)base[P.y[p] + r];
-            if (P.wA[p] != 0.0) kahan(s[0], s[1], P.wA[p] * t);
-            if (P.wB[p] != 0.0) kahan(s[2], s[3], P.wB[p] * t);
-            if (P.wH[p] != 0.0) kahan(s[4], s[5], P.wH[p] * t);
+            if (P.wA[p] != 0.0) kahan_add(s[0], s[1], P.wA[p] * t);
+            if (P.wB[p] != 0.0) kahan_add(s[2], s[3], P.wB[p] * t);
+            if (P.wH[p] != 0.0) kahan_add(s[4], s[5], P.wH[p] * t);
         }
 #pragma unroll
         for (int k = 0; k < 6; k++) acc[k * M + r] = s[k];

@@ -1020,17 +1020,9 @@ __global__ void k_qfinal(PropsArgs<T> a, int nblk)
     rs[kRsZC] = zC;
 }
 
-__device__ __forceinline__ void kahan_add(double &sum, double &c, double term)
-{
-    const double y = term - c;
-    const double t = sum + y;
-    c = (t - sum) - y;
-    sum = t;
-}
-
 // sum += w_s u(s) v(t - s) over part `part` of `parts` of s in [s0, s1) with Simpson interior weights
 // 4, 2, 4, ... from s0 (the reference's loops, density.h:404-422), Kahan
-// compensated, in the reference's order.  u, v are fields fu, fv of the
+// compensated; the whole range (parts = 1) in the reference's order.  u, v are fields fu, fv of the
 // propagator store at point r.  The loads of four consecutive terms are
 // issued before their additions, so each thread keeps eight loads in flight
 // instead of two.
@@ -1065,13 +1057,14 @@ __device__ __forceinline__ void simpson_run(const T *h, size_t M, int r, int s0,
 // The pass reads every slice once and is bound by memory: it needs the loads of
 // about 1000 threads per SM in flight.  One block per SM reached 1.4 TB/s at 64^3
 // (one replica); here a thread takes one point (64^3: 1024 blocks), and on grids
-// with fewer points than that PARTS threads share a point's contour.  PARTS
-// follows from the grid alone, so a replica's densities do not depend on its batch.
+// with fewer points than that PARTS threads share a point's contour, their sums joined
+// with their compensations.  PARTS follows from the grid alone, so a replica's densities
+// do not depend on its batch.
 template <typename T, int PARTS>
 __global__ void __launch_bounds__(256) k_density(PropsArgs<T> a)
 {
     constexpr int PTS = 256 / PARTS;
-    __shared__ double sh[32], part_sum[PARTS > 1 ? 3 * 256 : 1];
+    __shared__ double sh[32], part_sum[PARTS > 1 ? 6 * 256 : 1];
     const int part = threadIdx.x / PTS, lane = threadIdx.x % PTS;
     const Geo &g = a.g;
     const int slot = blockIdx.y;
@@ -1101,16 +1094,22 @@ __global__ void __launch_bounds__(256) k_density(PropsArgs<T> a)
         simpson_run(h, M, r, 1, n1, 0, 1, Ns, rCA, cA, part, PARTS);      // Q1(s) Q2(Ns - s)
         simpson_run(h, M, r, n1 + 1, Ns, 0, 1, Ns, rCB, cB, part, PARTS); // Q1(s) Q2(Ns - s)
         if constexpr (PARTS > 1) {
-            part_sum[threadIdx.x] = rhB;
-            part_sum[256 + threadIdx.x] = rCA;
-            part_sum[512 + threadIdx.x] = rCB;
+            double *p = part_sum + threadIdx.x;
+            p[0] = rhB, p[256] = chB;
+            p[512] = rCA, p[768] = cA;
+            p[1024] = rCB, p[1280] = cB;
             __syncthreads();
-            if (part == 0)
+            if (part == 0) {
                 for (int i = 1; i < PARTS; i++) {
-                    rhB += part_sum[i * PTS + lane];
-                    rCA += part_sum[256 + i * PTS + lane];
-                    rCB += part_sum[512 + i * PTS + lane];
+                    p += PTS;
+                    kahan_join(rhB, chB, p[0], p[256]);
+                    kahan_join(rCA, cA, p[512], p[768]);
+                    kahan_join(rCB, cB, p[1024], p[1280]);
                 }
+                rhB -= chB;
+                rCA -= cA;
+                rCB -= cB;
+            }
             __syncthreads();
         }
         if (part != 0 || !in) continue;
