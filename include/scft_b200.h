@@ -290,7 +290,9 @@ scft_status scft_autotune(scft_ctx *ctx, int *groups_out, int *wide_out, double 
 /* scft_autotune over more schedules: 1, 2 or 4 slot groups (four groups run
  * two after another on each of the two streams, so fewer spectra are live
  * at once; only with at least 16 replicas, and batches of fewer than 16
- * replicas then run as 2 groups), the two tile widths, and four
+ * replicas then run as 2 groups) and the count that a context takes by
+ * itself for its replicas, where that is another (*groups_out may be it, its
+ * times are not among times_ms), the two tile widths, and four
  * launches per contour step or one persistent launch per step (work items
  * claimed in order, bounded waits) where the context has one (compile-time
  * grid shapes).  times_ms[12]: times_ms[c] for c = gi + 3 wide + 6 persist

@@ -29,7 +29,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CU_SOURCES = ["scft_ctx.cu", "props_kernels.cu", "field_kernels.cu", "stress_kernels.cu", "noalloc.cu",
               "density_ckpt.cu", "reg64.cu", "pair.cu", "pair_any.cu", "pair_stress.cu", "real_slab.cu"]
 HEADERS = ["common.cuh", "fft.cuh", "kernels.h", "tma.cuh", "reg64.cuh", "step_order.cuh",
-           "dft.cuh", "pair.cuh", "pair_shapes.h", "pdl.cuh", "real_slab.cuh"]
+           "dft.cuh", "pair.cuh", "pair_shapes.h", "pdl.cuh", "real_slab.cuh", "schedule.h"]
 
 
 def _stale(target, deps):

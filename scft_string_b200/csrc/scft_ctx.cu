@@ -21,6 +21,7 @@
 
 #include "../../include/scft_b200.h"
 #include "kernels.h"
+#include "schedule.h"
 
 using namespace scft;
 
@@ -272,37 +273,9 @@ scft_status upload_list(scft_ctx *ctx, const std::vector<int> &reps)
 
 scft_status props_ckpt_impl(scft_ctx *ctx, int ii, int K, double *lnQ_out, double *phis_out, double *bytes_out);
 
-// Slot groups of a batch of nb replicas: the configured count, halved while a
-// group of more than two would get fewer than 4 replicas (a launch of 2 or 3
-// replicas leaves most SMs idle: the W+ relaxation runs many such partial
-// batches), and 1 when there are fewer than 2 replicas per group.
-int effective_groups(int ngroups, int nb)
-{
-    int ng = ngroups;
-    while (ng > 2 && nb < 4 * ng) ng /= 2;
-    return (ng > 1 && nb >= 2 * ng) ? ng : 1;
-}
-
-// The count where none is configured: two, and on the pair-packed kernels twice
-// as many as long as the replicas of the two groups that run at a time hold more
-// than L2 keeps (spectra, tables and partial result: 64 bytes a point) and a
-// group still has slabs for most SMs.  us per replica step with 2 / 4 groups: 64^3,
-// 16 replicas 14.8 / 13.9, 14 replicas 14.7 / 13.8; fewer slabs per group lose (10
-// replicas 14.7 / 15.5, 8 replicas 14.2 / 15.2 when the rule was made, 48^3 x16 5.65
-// / 6.09); 80^3 x16 33.6 / 34.1, 96^3 x8 58.3 / 58.3.
-int default_groups(const scft_ctx *ctx, int nb)
-{
-    constexpr double kLive = 135e6;
-    constexpr int kSlabs = 192;
-    int ng = 2;
-    if (ctx->L.pair)
-        while (2.0 * ((nb + ng - 1) / ng) * 64.0 * ctx->M > kLive && nb / (2 * ng) * ctx->g.m0 >= kSlabs) ng *= 2;
-    return nb >= 2 * ng ? ng : 1;
-}
-
 int groups_for(const scft_ctx *ctx, int nb)
 {
-    return ctx->ngroups > 0 ? effective_groups(ctx->ngroups, nb) : default_groups(ctx, nb);
+    return ctx->ngroups > 0 ? effective_groups(ctx->ngroups, nb) : default_groups(ctx->L.pair, ctx->M, nb);
 }
 
 // The packed FP64 kernels carry q and q^dagger as one complex field (pair.cuh), whose
@@ -2429,6 +2402,7 @@ scft_status scft_autotune_ex(scft_ctx *ctx, int *groups_out, int *wide_out, int 
     const scft_stats keep = ctx->stats;
     std::vector<int> all(ctx->strn);
     for (int i = 0; i < ctx->strn; i++) all[i] = i;
+    const int nb = std::min(ctx->strn, ctx->nslots);  // replicas of a full round
     auto drop_graphs = [&]() {
         for (auto &g : ctx->graphs)
             if (g) {
@@ -2444,12 +2418,18 @@ scft_status scft_autotune_ex(scft_ctx *ctx, int *groups_out, int *wide_out, int 
     // contour step (four, or one persistent launch); c = gi + 3 wide + 6 persist
     const int nw = (ctx->L.pair || (!ctx->L.reg && ctx->L.tmap_wide)) ? 2 : 1;
     const int np = ctx->persist_ok ? 2 : 1;
-    for (int c = 0; c < kTuneCandidates; c++) {
-        const int ng = 1 << (c % 3), wide = (c / 3) & 1, persist = c / 6;
+    // last the default count, where it is none of these
+    const int def = default_groups(ctx->L.pair, ctx->M, nb);
+    const bool def_timed = def <= 4 && effective_groups(def, nb) == def;
+    for (int c = 0; c < kTuneCandidates + (def_timed ? 0 : 2 * nw); c++) {
+        const bool extra = c >= kTuneCandidates;
+        const int ng = extra ? def : 1 << (c % 3);
+        const int wide = extra ? (c - kTuneCandidates) % nw : (c / 3) & 1;
+        const int persist = extra ? (c - kTuneCandidates) / nw : c / 6;
         if (wide >= nw || persist >= np) continue;
-        if (effective_groups(ng, (int)all.size()) != ng) continue;  // props_list would run fewer groups
+        if (!extra && effective_groups(ng, nb) != ng) continue;  // props_list would run fewer groups
         drop_graphs();
-        ctx->ngroups = ng;
+        ctx->ngroups = extra ? 0 : ng;
         ctx->L.ptile_wide = wide;
         ctx->L.persist = persist;
         scft_status s = props_list(ctx, all);
@@ -2461,7 +2441,7 @@ scft_status scft_autotune_ex(scft_ctx *ctx, int *groups_out, int *wide_out, int 
             if (s != SCFT_OK) return s;
             t = std::min(t, (ctx->stats.props_seconds - before) * 1e3);
         }
-        if (times_ms) times_ms[c] = t;
+        if (times_ms && !extra) times_ms[c] = t;
         if (first || t < best) {
             first = false;
             best = t;
@@ -2472,7 +2452,7 @@ scft_status scft_autotune_ex(scft_ctx *ctx, int *groups_out, int *wide_out, int 
     }
     drop_graphs();
     // where it is what the default takes, the default stays: it also knows partial batches
-    ctx->ngroups = best_g == default_groups(ctx, ctx->strn) ? 0 : best_g;
+    ctx->ngroups = best_g == def ? 0 : best_g;
     ctx->L.ptile_wide = best_w;
     ctx->L.persist = best_p;
     ctx->stats = keep;
