@@ -65,7 +65,7 @@ struct PropsLaunch {
     int tma_pencil;  // x pass through 2-D tensor-map tiles (fixed shapes)
     int pencil_tma_smem;
     const CUtensorMap *tmap;  // host copy of the spectrum tensor map
-    int ptile_wide;  // tensor-map x pass with tiles of twice the default width
+    int ptile_wide;  // x tiles of twice the default width: 1 yes, 0 no, -1 as the kernels choose
     int pencil_tma_smem_wide;
     const CUtensorMap *tmap_wide;  // the same spectra with the wide tile box
     int pencil_sh;   // m0 = 64: x pass as register transforms with warp-shuffle transposes (k_pencil_sh);
@@ -91,6 +91,7 @@ void reg64_step(const PropsArgs<float> &a, int nslots, int s, int grid, cudaStre
 
 // FP64 step kernels on q + i q^dagger (pair.cuh): spectra [slot][half step, full step][x][kz][y position]
 bool pair_applicable(int m0, int m1, int m2);
+bool pair_axis_wide(int m0);  // the x pass has tiles of twice the width
 int pair_setup(int m0, int m1, int m2, int *step_grid);
 void pair_mid(const PropsArgs<double> &a, int nslots, int s, cudaStream_t st);
 void pair_combine(const PropsArgs<double> &a, int nslots, int s, int mode, cudaStream_t st);
@@ -105,6 +106,7 @@ void real_mid(const PropsArgs<float> &a, int nslots, int s, cudaStream_t st);
 void real_combine(const PropsArgs<float> &a, int nslots, int s, int mode, cudaStream_t st);
 int real_pencil_setup(int m0);
 void real_pencil(const PropsArgs<float> &a, int nslots, int both, int wide, cudaStream_t st);
+int real_pencil_wide(int wide, int m0, int ncol, int both, int nslots);
 
 void pf_smem_bytes(int id, int fp32, int &mid, int &comb);
 // dynamic shared memory of k_pencil_sh for tiles of tc columns

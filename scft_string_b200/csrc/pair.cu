@@ -146,6 +146,8 @@ bool pair_applicable(int m0, int m1, int m2)
     return (pair_slab_fixed(m1, m2) || pair_any_plan(m1, m2, q)) && (pair_axis_fixed(m0) || pair_x_radices(m0, r1, r2));
 }
 
+bool pair_axis_wide(int m0) { return pair_axis_fixed(m0); }
+
 // raises the kernels' shared-memory limits; *grid = CTAs of the persistent step launch (0: none)
 int pair_setup(int m0, int m1, int m2, int *grid)
 {
@@ -225,6 +227,7 @@ void pair_combine(const PropsArgs<T> &a, int nslots, int s, int mode, cudaStream
 void pair_pencil(const PropsArgs<T> &a, int nslots, int s, int both, int wide, cudaStream_t st)
 {
     const Geo &g = a.g;
+    wide = wide > 0;  // the narrow tile where nothing is said
     const int tc = wide ? 2 * kTile : kTile;
     int ra = 1, rb = 1;
     pair_y_radices(g.m1, g.m2, ra, rb);
@@ -253,7 +256,7 @@ void pair_step(const PropsArgs<T> &a, int nslots, int s, int wide, int grid, cud
     if (g.m0 == A && g.m1 == B && g.m2 == C) {                                                                       \
         if constexpr (kCl<B, C> == 1) {                                                                             \
             constexpr int NT = PairSlab<B, C, 1>::NT;                                                                \
-            if (wide)                                                                                                \
+            if (wide > 0)                                                                                            \
                 k_pair_step<A, B, C, 2 * kTile><<<grid, NT, step_smem<A, B, C, 2 * kTile>(), st>>>(a, s, nslots);     \
             else                                                                                                     \
                 k_pair_step<A, B, C, kTile><<<grid, NT, step_smem<A, B, C, kTile>(), st>>>(a, s, nslots);             \

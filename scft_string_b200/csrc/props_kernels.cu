@@ -1265,7 +1265,7 @@ void launch_pencil(const PropsArgs<T> &a, const PropsLaunch &L, dim3 gp, int s, 
     if constexpr (F0 == 64 && sizeof(T) == 4) {
         if (L.pencil_sh) {
             constexpr int TC = kTile<T>::value, ncol = F1 * (F2 / 2 + 1);
-            if (L.ptile_wide)
+            if (L.ptile_wide > 0 && L.tmap_wide)
                 k_pencil_sh<T, MT, F0, F1, F2, 2 * TC><<<dim3((ncol + 2 * TC - 1) / (2 * TC), gp.y, gp.z), MT,
                                                          L.pencil_tma_smem_wide, st>>>(*L.tmap_wide, a, both);
             else
@@ -1309,7 +1309,7 @@ int launch_props_mt(const PropsArgs<T> &a, const PropsLaunch &L, int nslots, cud
             cudaMemsetAsync(a.sync, 0, sizeof(int) * reg64_sync_ints(g.Ns, nslots), st);
             launch_combine<T, MT, F0, F1, F2>(a, L, gs, -1, 1, st);
             for (int s = 0; s < g.Ns; s++) {
-                if (L.ptile_wide)
+                if (L.ptile_wide > 0 && L.tmap_wide)
                     k_step_pf<T, MT, F0, F1, F2, 2 * TC><<<L.step_grid_pf, MT, L.step_pf_smem, st>>>(
                         *L.tmap_wide, a, s, nslots, L.pencil_sh);
                 else

@@ -1,5 +1,6 @@
 // real_slab.cu -- launches of the FP32 slab kernels (real_slab.cuh).
 #include "real_slab.cuh"
+#include "schedule.h"
 
 namespace scft {
 
@@ -65,16 +66,16 @@ int real_pencil_setup(int m0)
     return e == cudaSuccess ? 0 : -1;
 }
 
+int real_pencil_wide(int wide, int m0, int ncol, int both, int nslots)
+{
+    return wide_tiles(wide, m0, ncol, kRealTile, both ? 4 : 2, nslots);
+}
+
 void real_pencil(const PropsArgs<float> &a, int nslots, int both, int wide, cudaStream_t st)
 {
     const Geo &g = a.g;
-    // Wide tiles where they still fill the SMs four times: 512-byte rows (16 replicas
-    // of 64^3 8.8 us per replica step against 9.2, of 48^3 79.7 us a step against
-    // 82.0).  Small batches want more blocks (one replica 24.2 us wide, 22.1
-    // narrow), and the longer axes spill at twice the butterflies per thread (eight
-    // replicas of 128^3 109 us wide, 93 narrow).
-    const int ncol = g.m1 * g.mk2, wtiles = (ncol + 2 * kRealTile - 1) / (2 * kRealTile);
-    wide = wide || (g.m0 <= 64 && wtiles * (both ? 4 : 2) * nslots >= 4 * 148);
+    const int ncol = g.m1 * g.mk2;
+    wide = real_pencil_wide(wide, g.m0, ncol, both, nslots);
     const int tc = wide ? 2 * kRealTile : kRealTile;
     const dim3 grid((ncol + tc - 1) / tc, both ? 4 : 2, nslots);
 #define X(A)                                                                                                        \

@@ -273,6 +273,22 @@ scft_status upload_list(scft_ctx *ctx, const std::vector<int> &reps)
 
 scft_status props_ckpt_impl(scft_ctx *ctx, int ii, int K, double *lnQ_out, double *phis_out, double *bytes_out);
 
+// whether the grid's x passes have tiles of twice the width: the packed FP64 ones of
+// compile-time axes, the FP32 ones of the compile-time shapes
+bool wide_available(const scft_ctx *ctx)
+{
+    const PropsLaunch &L = ctx->L;
+    if (L.pair) return pair_axis_wide(ctx->g.m0);
+    return !L.reg && L.fixed && (L.pencil_sh ? L.tmap_wide != nullptr : L.pf != 0);
+}
+
+// the FP32 kernels take wide tiles by themselves in launches of nslots replicas
+bool wide_by_rule(const scft_ctx *ctx, int nslots)
+{
+    const Geo &g = ctx->g;
+    return !ctx->L.pair && !ctx->L.pencil_sh && real_pencil_wide(-1, g.m0, g.m1 * g.mk2, 0, nslots);
+}
+
 int groups_for(const scft_ctx *ctx, int nb)
 {
     return ctx->ngroups > 0 ? effective_groups(ctx->ngroups, nb) : default_groups(ctx->L.pair, ctx->M, nb);
@@ -759,6 +775,8 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
     if (const char *ev = getenv("SCFT_REG64"))
         L.reg = (ev[0] == '1' && T == 4 && reg64_applicable(g.m0, g.m1, g.m2)) ? 1 : 0;
     L.pf = 0;
+    L.ptile_wide = -1;
+    if (const char *ev = getenv("SCFT_PENCIL_TILE_WIDE")) L.ptile_wide = ev[0] == '1';
     if (L.fixed) {
         pf_smem_bytes(L.fixed, T == 4, L.mid_pf_smem, L.combine_pf_smem);
         L.pf = (std::max(L.mid_pf_smem, L.combine_pf_smem) <= smem_optin) ? 1 : 0;
@@ -900,7 +918,6 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
                         encode(&ctx->tmap_wide, 2 * tc) == CUDA_SUCCESS) {
                         L.tmap_wide = &ctx->tmap_wide;
                         L.pencil_tma_smem_wide = smem_for(2 * tc);
-                        if (const char *ev = getenv("SCFT_PENCIL_TILE_WIDE")) L.ptile_wide = ev[0] == '1';
                     }
                 }
                 if (!L.tma_pencil) L.pencil_sh = 0;
@@ -933,8 +950,6 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
             rc = SCFT_CUDA_ERROR;
             goto done;
         }
-        if (const char *ev = getenv("SCFT_PENCIL_TILE_WIDE"))
-            if (L.pair) L.ptile_wide = ev[0] == '1';
         ctx->persist_ok = (L.pair ? L.step_grid_pair > 0 : (L.reg || L.step_grid_pf > 0)) && ctx->sync;
         if (const char *ev = getenv("SCFT_PERSIST")) L.persist = ev[0] == '1' ? 1 : 0;
         if (const char *ev = getenv("SCFT_NO_PERSIST"))
@@ -2395,7 +2410,7 @@ scft_status scft_autotune_ex(scft_ctx *ctx, int *groups_out, int *wide_out, int 
         for (int c = 0; c < kTuneCandidates; c++) times_ms[c] = -1;
     if (ctx->nostore) {  // props run one replica at a time from checkpoints: nothing to schedule
         if (groups_out) *groups_out = 1;
-        if (wide_out) *wide_out = ctx->L.ptile_wide;
+        if (wide_out) *wide_out = ctx->L.ptile_wide > 0;
         if (persist_out) *persist_out = 0;
         return SCFT_OK;
     }
@@ -2413,10 +2428,9 @@ scft_status scft_autotune_ex(scft_ctx *ctx, int *groups_out, int *wide_out, int 
     double best = 0;
     int best_g = 1, best_w = 0, best_p = 0;
     bool first = true;
-    // axes: slot groups (1, 2, 4) x x-pencil tile width (default, wide;
-    // tensor-map pencils of the shared-memory kernels only) x launches per
-    // contour step (four, or one persistent launch); c = gi + 3 wide + 6 persist
-    const int nw = (ctx->L.pair || (!ctx->L.reg && ctx->L.tmap_wide)) ? 2 : 1;
+    // axes: slot groups (1, 2, 4) x x tiles (as the kernels choose, all wide) x launches
+    // per contour step (four, or one persistent launch); c = gi + 3 wide + 6 persist
+    const int nw = wide_available(ctx) ? 2 : 1;
     const int np = ctx->persist_ok ? 2 : 1;
     // last the default count, where it is none of these
     const int def = default_groups(ctx->L.pair, ctx->M, nb);
@@ -2428,9 +2442,10 @@ scft_status scft_autotune_ex(scft_ctx *ctx, int *groups_out, int *wide_out, int 
         const int persist = extra ? (c - kTuneCandidates) / nw : c / 6;
         if (wide >= nw || persist >= np) continue;
         if (!extra && effective_groups(ng, nb) != ng) continue;  // props_list would run fewer groups
+        if (wide && !persist && wide_by_rule(ctx, nb / ng)) continue;  // the kernels chose it already
         drop_graphs();
         ctx->ngroups = extra ? 0 : ng;
-        ctx->L.ptile_wide = wide;
+        ctx->L.ptile_wide = wide ? 1 : -1;
         ctx->L.persist = persist;
         scft_status s = props_list(ctx, all);
         if (s != SCFT_OK) return s;
@@ -2453,7 +2468,7 @@ scft_status scft_autotune_ex(scft_ctx *ctx, int *groups_out, int *wide_out, int 
     drop_graphs();
     // where it is what the default takes, the default stays: it also knows partial batches
     ctx->ngroups = best_g == def ? 0 : best_g;
-    ctx->L.ptile_wide = best_w;
+    ctx->L.ptile_wide = best_w ? 1 : -1;
     ctx->L.persist = best_p;
     ctx->stats = keep;
     if (groups_out) *groups_out = best_g;

@@ -34,4 +34,16 @@ inline int default_groups(bool pair, long long M, int nb)
     return nb >= 4 ? 2 : 1;
 }
 
+// Tile width of an FP32 x pass: 1 wide (2 * tile columns), 0 default; `wide` 1 or 0 says
+// so, -1 leaves it to this rule.  Wide where the tiles still fill the SMs four times, for
+// their 512-byte rows (16 replicas of 64^3 8.8 us per replica step against 9.2, of 48^3
+// 79.7 us a step against 82.0).  Small batches want more blocks (one replica 24.2 us
+// wide, 22.1 narrow), and the longer axes spill at twice the butterflies per thread
+// (eight replicas of 128^3 109 us wide, 93 narrow).
+inline int wide_tiles(int wide, int m0, int ncol, int tile, int spectra, int nslots)
+{
+    if (wide >= 0) return wide;
+    return m0 <= 64 && (ncol + 2 * tile - 1) / (2 * tile) * spectra * nslots >= 4 * 148;
+}
+
 }  // namespace scft

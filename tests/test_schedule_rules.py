@@ -10,6 +10,7 @@ CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "scft_stri
 SRC = """#include "schedule.h"
 extern "C" int default_groups(int pair, long long M, int nb) { return scft::default_groups(pair, M, nb); }
 extern "C" int effective_groups(int ng, int nb) { return scft::effective_groups(ng, nb); }
+extern "C" int wide_tiles(int w, int m0, int ncol, int n, int nslots) { return scft::wide_tiles(w, m0, ncol, 32, n, nslots); }
 """
 
 
@@ -44,3 +45,14 @@ def test_default_groups_where_measured(rules):
                (96, 12): 2, (96, 16): 2, (128, 4): 2}
     for (m, nb), ng in fastest.items():
         assert rules.default_groups(1, m ** 3, nb) == ng, (m, nb)
+
+
+def test_tile_width_asked_for_is_taken(rules):
+    for m in (32, 48, 64, 96, 128):
+        for spectra in (2, 4):
+            for nslots in (1, 4, 16, 48):
+                ncol = m * (m // 2 + 1)
+                assert rules.wide_tiles(0, m, ncol, spectra, nslots) == 0
+                assert rules.wide_tiles(1, m, ncol, spectra, nslots) == 1
+    assert rules.wide_tiles(-1, 64, 64 * 33, 4, 16) == 1 and rules.wide_tiles(-1, 64, 64 * 33, 4, 1) == 0
+    assert rules.wide_tiles(-1, 128, 128 * 65, 4, 8) == 0
