@@ -100,7 +100,6 @@ void pair_pencil(const PropsArgs<double> &a, int nslots, int s, int both, int wi
 void pair_step(const PropsArgs<double> &a, int nslots, int s, int wide, int grid, cudaStream_t st);
 
 // FP32 slab kernels of the compile-time shapes (real_slab.cuh)
-bool real_slab_has(int m1, int m2);
 int real_slab_setup(int m1, int m2);
 void real_mid(const PropsArgs<float> &a, int nslots, int s, cudaStream_t st);
 void real_combine(const PropsArgs<float> &a, int nslots, int s, int mode, cudaStream_t st);
@@ -108,9 +107,9 @@ int real_pencil_setup(int m0);
 void real_pencil(const PropsArgs<float> &a, int nslots, int both, int wide, cudaStream_t st);
 int real_pencil_wide(int wide, int m0, int ncol, int both, int nslots);
 
-void pf_smem_bytes(int id, int fp32, int &mid, int &comb);
+void pf_smem_bytes(int id, int &mid, int &comb);
 // dynamic shared memory of k_pencil_sh for tiles of tc columns
-int pencil_sh_smem_bytes(int fp32, int tc, int m0);
+int pencil_sh_smem_bytes(int tc, int m0);
 
 int fixed_shape_id(int m0, int m1, int m2);
 int fixed_shape_threads(int id);
@@ -121,8 +120,7 @@ template <typename T>
 int launch_single_step(const PropsArgs<T> &a, const PropsLaunch &L, int s, cudaStream_t st);
 template <typename T>
 int set_props_smem(const PropsLaunch &L);
-// CTAs of the persistent step kernel of the compile-time shapes (0: none)
-template <typename T>
+// CTAs of the persistent step kernel of the FP32 compile-time shapes (0: none)
 int props_step_grid(const PropsLaunch &L);
 // chain segment of slot 0 (a.g.Ns steps; a.g.n1, n2 relative to the segment
 // start), E tables of slot 0 from its replica, Q2/QC/lnQ of slot 0 from the

@@ -425,7 +425,6 @@ __device__ __forceinline__ void mid_pf_body(const PropsArgs<T> &a, int s, int x,
         mbar_fence_init();
         mbar_expect_tx(&bars[1], L::REAL_BYTES);
         bulk_g2s(E4s, E4g, L::REAL_BYTES, &bars[1]);  // constant over the chain
-        pdl_wait();
         mbar_expect_tx(&bars[0], L::SPEC_BYTES);
         bulk_g2s(bufB, specB + slab_k, L::SPEC_BYTES, &bars[0]);
         mbar_expect_tx(&bars[2], L::SPEC_BYTES);
@@ -467,7 +466,6 @@ __device__ __forceinline__ void mid_pf_body(const PropsArgs<T> &a, int s, int x,
     }
     __syncthreads();
     slab_forward_fixed<T, m1, m2, MT>(bufA, twy, twz);
-    pdl_trigger();
     for (int i = threadIdx.x; i < m1 * mk2; i += MT) specA[slab_k + i] = bufA[i];
 }
 
@@ -505,7 +503,6 @@ __device__ __forceinline__ void combine_pf_body(const PropsArgs<T> &a, int s, in
             mbar_expect_tx(&bars[2], L::REAL_BYTES);
             bulk_g2s(E, etab_ptr(a, slot, sel_s) + slab_r, L::REAL_BYTES, &bars[2]);  // constant over the chain
         }
-        pdl_wait();
         if (mode == 0) {
             mbar_expect_tx(&bars[0], L::SPEC_BYTES);
             bulk_g2s(buf, specA + slab_k, L::SPEC_BYTES, &bars[0]);
@@ -576,7 +573,6 @@ __device__ __forceinline__ void combine_pf_body(const PropsArgs<T> &a, int s, in
     }
     __syncthreads();
     slab_forward_fixed<T, m1, m2, MT>(buf, twy, twz);
-    pdl_trigger();
     for (int i = threadIdx.x; i < m1 * mk2; i += MT) specB[slab_k + i] = buf[i];
 }
 
@@ -606,7 +602,6 @@ __device__ __forceinline__ void pencil_tma_body(const CUtensorMap &tmap, const P
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
         mbar_fence_init();
-        pdl_wait();
         mbar_expect_tx(&bars[0], BOX_BYTES);
         tma_load_2d(bufA, &tmap, x, y0, &bars[0]);
         if (both) {
@@ -641,7 +636,6 @@ __device__ __forceinline__ void pencil_tma_body(const CUtensorMap &tmap, const P
         });
         fence_proxy_async_smem();
         __syncthreads();
-        if (pass == npass - 1) pdl_trigger();
         if (threadIdx.x == 0) tma_store_2d(&tmap, x, y0 + pass * m0, buf);
     }
     if (threadIdx.x == 0) tma_store_wait_read();
@@ -677,9 +671,9 @@ struct PencilSh {
     static __device__ __forceinline__ int at(int x, int c, int m0)
     {
         const int b = c / CPB, cc = c % CPB;
-        const int chunk = sizeof(T) == 4 ? cc >> 1 : cc;
-        const int sw = chunk ^ (x & 7);
-        return b * CPB * m0 + x * CPB + (sizeof(T) == 4 ? (sw << 1) | (cc & 1) : sw);
+        static_assert(sizeof(T) == 4, "16-byte chunks of two elements");
+        const int sw = (cc >> 1) ^ (x & 7);
+        return b * CPB * m0 + x * CPB + ((sw << 1) | (cc & 1));
     }
 };
 
@@ -1417,33 +1411,22 @@ int set_smem_mt(const PropsLaunch &L)
                : -1;
 }
 
-// shared-memory bytes of the prefetching slab kernels for a fixed shape
-template <typename T>
-void pf_smem(int id, int &mid, int &comb)
+// shared-memory bytes of the prefetching slab kernels of a compile-time shape (FP32)
+void pf_smem_bytes(int id, int &mid, int &comb)
 {
     switch (id) {
-        case 32: mid = SlabSmem<T, 32, 32>::mid_bytes(); comb = SlabSmem<T, 32, 32>::combine_bytes(); return;
-        case 48: mid = SlabSmem<T, 48, 48>::mid_bytes(); comb = SlabSmem<T, 48, 48>::combine_bytes(); return;
-        case 64: mid = SlabSmem<T, 64, 64>::mid_bytes(); comb = SlabSmem<T, 64, 64>::combine_bytes(); return;
-        case 96: mid = SlabSmem<T, 96, 96>::mid_bytes(); comb = SlabSmem<T, 96, 96>::combine_bytes(); return;
-        case 128: mid = SlabSmem<T, 128, 128>::mid_bytes(); comb = SlabSmem<T, 128, 128>::combine_bytes(); return;
-        case 6496: mid = SlabSmem<T, 64, 96>::mid_bytes(); comb = SlabSmem<T, 64, 96>::combine_bytes(); return;
+#define X(ID, M1, M2)                                     \
+    case ID:                                              \
+        mid = SlabSmem<float, M1, M2>::mid_bytes();       \
+        comb = SlabSmem<float, M1, M2>::combine_bytes();  \
+        return;
+        X(32, 32, 32) X(48, 48, 48) X(64, 64, 64) X(96, 96, 96) X(128, 128, 128) X(6496, 64, 96)
+#undef X
         default: mid = comb = 0;
     }
 }
 
-void pf_smem_bytes(int id, int fp32, int &mid, int &comb)
-{
-    if (fp32)
-        pf_smem<float>(id, mid, comb);
-    else
-        pf_smem<double>(id, mid, comb);
-}
-
-int pencil_sh_smem_bytes(int fp32, int tc, int m0)
-{
-    return fp32 ? PencilSh<float>::smem(tc, m0) : PencilSh<double>::smem(tc, m0);
-}
+int pencil_sh_smem_bytes(int tc, int m0) { return PencilSh<float>::smem(tc, m0); }
 
 // op 0: props, 1: single step, 2: shared-memory attributes, 3: chain segment, 4: CTAs of the
 // persistent step kernel
@@ -1511,13 +1494,7 @@ int launch_single_step(const PropsArgs<T> &a, const PropsLaunch &L, int s, cudaS
     return dispatch<T>(1, &a, L, s, st);
 }
 
-template <typename T>
-int props_step_grid(const PropsLaunch &L)
-{
-    return dispatch<T>(4, nullptr, L, 0, nullptr);
-}
-template int props_step_grid<float>(const PropsLaunch &);
-template int props_step_grid<double>(const PropsLaunch &);
+int props_step_grid(const PropsLaunch &L) { return dispatch<float>(4, nullptr, L, 0, nullptr); }
 
 template <typename T>
 int set_props_smem(const PropsLaunch &L)

@@ -778,7 +778,7 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
     L.ptile_wide = -1;
     if (const char *ev = getenv("SCFT_PENCIL_TILE_WIDE")) L.ptile_wide = ev[0] == '1';
     if (L.fixed) {
-        pf_smem_bytes(L.fixed, T == 4, L.mid_pf_smem, L.combine_pf_smem);
+        pf_smem_bytes(L.fixed, L.mid_pf_smem, L.combine_pf_smem);
         L.pf = (std::max(L.mid_pf_smem, L.combine_pf_smem) <= smem_optin) ? 1 : 0;
         if (const char *ev = getenv("SCFT_NO_PREFETCH")) L.pf = ev[0] == '1' ? 0 : L.pf;
     }
@@ -879,7 +879,7 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
         CKC(cudaMemset(ctx->DEV, 0, sizeof(double) * 2 * M * R));
         CKC(cudaMemset(ctx->dWda, 0, sizeof(double) * M * R));
         CKC(cudaMemset(ctx->rs, 0, sizeof(double) * kRsStride * R));
-        // 2-D tensor map of all spectra: rows of 2*m1*mk2 reals, nslots*2*2*m0 rows
+        // FP32 compile-time shapes: 2-D tensor map of all spectra, rows of 2*m1*mk2 reals, nslots*2*2*m0 rows
         L.tma_pencil = 0;
         if (L.fixed && !getenv("SCFT_NO_TMA_PENCIL")) {
             typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -890,7 +890,7 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
             cudaDriverEntryPointQueryResult q;
             if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) == cudaSuccess &&
                 q == cudaDriverEntryPointSuccess && fn) {
-                const int tc = T == 4 ? 32 : 16;  // kTile<T> of the kernels
+                const int tc = 32;  // kTile<float> of the kernels
                 cuuint64_t dims[2] = {(cuuint64_t)2 * g.m1 * g.mk2, (cuuint64_t)S * 2 * 2 * g.m0};
                 cuuint64_t strides[1] = {(cuuint64_t)2 * g.m1 * g.mk2 * T};
                 cuuint32_t es[2] = {1, 1};
@@ -899,14 +899,14 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
                 const char *shv = getenv("SCFT_PENCIL_SHUFFLE");
                 L.pencil_sh = g.m0 == 64 && shv && shv[0] == '1';
                 auto encode = [&](CUtensorMap *m, int w) {
-                    cuuint32_t box[2] = {(cuuint32_t)(L.pencil_sh ? 128 / T : 2 * w), (cuuint32_t)g.m0};
-                    return ((EncodeFn)fn)(m, T == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2,
+                    cuuint32_t box[2] = {(cuuint32_t)(L.pencil_sh ? 32 : 2 * w), (cuuint32_t)g.m0};
+                    return ((EncodeFn)fn)(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
                                           ctx->spec, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                           L.pencil_sh ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
                 };
                 auto smem_for = [&](int w) {
-                    return L.pencil_sh ? pencil_sh_smem_bytes(T == 4, w, g.m0)
+                    return L.pencil_sh ? pencil_sh_smem_bytes(w, g.m0)
                                        : (int)(128 + (2 * w * g.m0 + g.m0) * 2 * T + (w + g.m0) * T);
                 };
                 if (encode(&ctx->tmap, tc) == CUDA_SUCCESS && g.m0 <= 256 && (strides[0] % 16) == 0) {
@@ -940,7 +940,7 @@ scft_status scft_create(const scft_problem *p, scft_ctx **out)
         // it, the shared-memory kernels with four launches (scft_autotune compares
         // both); SCFT_PERSIST=0|1 sets the start, SCFT_NO_PERSIST=1 rules it out
         L.persist = 0;
-        L.step_grid_pf = L.step_pf_smem > 0 ? (T == 4 ? props_step_grid<float>(L) : props_step_grid<double>(L)) : 0;
+        L.step_grid_pf = L.step_pf_smem > 0 ? props_step_grid(L) : 0;
         if (L.reg) {
             L.step_grid = reg64_step_grid();
             L.persist = 1;
