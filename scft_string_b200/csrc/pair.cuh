@@ -504,30 +504,27 @@ struct PairSlabAny {
 __device__ __forceinline__ int pair_shift(int e0, int e1) { return min(max(e0 - e1, -1000), 1000); }
 __device__ __forceinline__ double pair_pow2(int k) { return __hiloint2double((1023 + min(max(k, -1000), 1000)) << 20, 0); }
 
-// sums over the CTA's threads of x and y -> out[0], out[1]
-__device__ __forceinline__ void pair_cta_sums(double x, double y, double *out)
+// sums over the CTA's threads of x and y -> out[0], out[1]; sh: shared memory, a complex
+// per warp, that no thread reads any more (no static memory: the largest slabs leave none)
+__device__ __forceinline__ void pair_cta_sums(double x, double y, double *out, cplxd *sh)
 {
-    __shared__ double sh[2][32];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         x += __shfl_xor_sync(0xffffffffu, x, o);
         y += __shfl_xor_sync(0xffffffffu, y, o);
     }
-    if ((threadIdx.x & 31) == 0) {
-        sh[0][threadIdx.x >> 5] = x;
-        sh[1][threadIdx.x >> 5] = y;
-    }
+    if ((threadIdx.x & 31) == 0) stc(sh + (threadIdx.x >> 5), {x, y});
     __syncthreads();
     if (threadIdx.x >= 32) return;
-    const bool in = threadIdx.x < blockDim.x >> 5;
-    x = in ? sh[0][threadIdx.x] : 0;
-    y = in ? sh[1][threadIdx.x] : 0;
+    const cplxd v = threadIdx.x < blockDim.x >> 5 ? ldc(sh + threadIdx.x) : cplxd{0, 0};
+    x = v.x;
+    y = v.y;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         x += __shfl_xor_sync(0xffffffffu, x, o);
         y += __shfl_xor_sync(0xffffffffu, y, o);
     }
-    if (threadIdx.x == 0) *reinterpret_cast<double2 *>(out) = make_double2(x, y);
+    if (threadIdx.x == 0) stc(reinterpret_cast<cplxd *>(out), {x, y});
 }
 
 // Floors of the binary exponents of the root mean squares that n pairs of partial sums
@@ -666,7 +663,8 @@ __device__ __forceinline__ void pair_mid_body(const PS &B, const PropsArgs<doubl
                 sy = fma(y0, y0, sy);
             }
         });
-        pair_cta_sums(sx, sy, a.partials + (size_t)slot * a.npart_stride + 2 * (x * PS::CTAS + B.rank));
+        // the twiddle factors (m1 + m2 of them, more than warps) have done their work
+        pair_cta_sums(sx, sy, a.partials + (size_t)slot * a.npart_stride + 2 * (x * PS::CTAS + B.rank), B.twy);
         B.finish();
     }
 }

@@ -7,7 +7,7 @@
 
 namespace scft {
 
-constexpr int kSmemCta = 227 * 1024;  // dynamic shared memory a CTA may have
+constexpr int kSmemCta = 227 * 1024 - 128;  // dynamic shared memory a CTA may have, next to the kernels' few static bytes
 
 // slab shapes (m1, m2) and x lengths with kernels
 #define PAIR_SLABS(X) X(16, 16) X(24, 24) X(32, 32) X(40, 40) X(48, 48) X(64, 64) X(64, 96) X(80, 80) X(96, 96) X(128, 128)

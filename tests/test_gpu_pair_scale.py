@@ -48,8 +48,9 @@ def _fields(m, mean):
     return mean + rng.normal(0, 2.0, M), rng.normal(0, 0.5, M)
 
 
-# a slab in one CTA, run-time sizes, one unmerged slab over two CTAs
-@pytest.mark.parametrize("m", [(16, 16, 16), (10, 12, 25), (4, 128, 128)])
+# a slab in one CTA, run-time sizes, one unmerged slab over two CTAs, the largest slab
+# that a CTA's shared memory holds
+@pytest.mark.parametrize("m", [(16, 16, 16), (10, 12, 25), (4, 128, 128), (2, 144, 98)])
 @pytest.mark.parametrize("mean", [0.0, 6.0, -10.0, 20.0, 40.0])
 def test_propagators_keep_their_precision(built_lib, m, mean):
     N, f = 48, 0.375
