@@ -1117,6 +1117,10 @@ scft_status scft_do_step(scft_ctx *ctx, int ii, const double *in, double *out, i
     for (auto &so : ctx->slot_of)
         if (so == 0) so = -1;
     void *dst = T == 4 ? (void *)tmp.data() : (void *)out;
+    if (T == 8 && slice * T > kStageBytes) {  // copied straight into out, which an error leaves as it is
+        st = check_device_err(ctx);
+        if (st != SCFT_OK) return st;
+    }
     st = copy_out_start(ctx, dst, h0 + slice * T, slice * T);
     if (st != SCFT_OK) return st;
     st = check_device_err(ctx);
