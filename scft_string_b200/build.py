@@ -26,7 +26,8 @@ def _nvcc() -> str:
 
 NVCC = _nvcc()
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-CU_SOURCES = ["scft_ctx.cu", "props_kernels.cu", "field_kernels.cu", "stress_kernels.cu", "noalloc.cu",
+CU_SOURCES = ["scft_ctx.cu", "props_kernels.cu", "field_kernels.cu", "stress_kernels.cu", "stress_kernels_512.cu",
+              "stress_kernels_1024.cu", "noalloc.cu",
               "density_ckpt.cu", "reg64.cu", "pair.cu", "pair_any.cu", "pair_stress.cu", "real_slab.cu"]
 HEADERS = ["common.cuh", "fft.cuh", "kernels.h", "tma.cuh", "reg64.cuh", "step_order.cuh",
            "dft.cuh", "pair.cuh", "pair_shapes.h", "pdl.cuh", "real_slab.cuh", "schedule.h"]

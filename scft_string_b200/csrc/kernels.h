@@ -166,14 +166,25 @@ struct StressArgs {
 template <typename T>
 int launch_stress_chunk(const StressArgs<T> &a, const StressPairs &P, int slab_threads, int slab_smem,
                         int pencil_threads, int pencil_smem, double *out, cudaStream_t st);
+// threads: the larger of the slab and pencil launches
 template <typename T>
-int set_stress_smem(int slab_smem, int pencil_smem);
+int set_stress_smem(int threads, int slab_smem, int pencil_smem);
 // <y, dS_J/dtheta x> of the junction step (pair 0 of P, table 2) summed over
 // the grid: block partials into `part` (nblk), then `out` (one double)
 template <typename T>
 int launch_junction_dtheta(const StressArgs<T> &a, const StressPairs &P, int slab_threads, int slab_smem,
                            int pencil_threads, int pencil_smem, double *part, int nblk, double *out,
                            cudaStream_t st);
+
+// the builds for CTAs of up to MT threads behind these (stress_kernels.cu)
+template <typename T, int MT>
+int launch_stress_chunk_mt(const StressArgs<T> &a, const StressPairs &P, int slab_threads, int slab_smem,
+                           int pencil_threads, int pencil_smem, double *out, cudaStream_t st);
+template <typename T, int MT>
+int launch_junction_mt(const StressArgs<T> &a, const StressPairs &P, int slab_threads, int slab_smem,
+                       int pencil_threads, int pencil_smem, double *part, int nblk, double *out, cudaStream_t st);
+template <typename T, int MT>
+int set_stress_smem_mt(int slab_smem, int pencil_smem);
 
 // the same sums on pairs packed as one complex field (pair_stress.cu), FP64 grids of pair_applicable
 constexpr int kStressSumBlocks = 64;

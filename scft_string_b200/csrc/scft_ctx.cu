@@ -1611,8 +1611,9 @@ scft_status stress_alloc(scft_ctx *ctx)
         ctx->lasterr = "stress kernels: shared memory attribute";
         return SCFT_CUDA_ERROR;
     }
-    if ((T == 4 ? set_stress_smem<float>(ctx->rt_slab_smem, ctx->rt_pencil_smem)
-                : set_stress_smem<double>(ctx->rt_slab_smem, ctx->rt_pencil_smem)) != 0) {
+    const int threads = std::max(ctx->rt_slab_threads, ctx->rt_pencil_threads);
+    if ((T == 4 ? set_stress_smem<float>(threads, ctx->rt_slab_smem, ctx->rt_pencil_smem)
+                : set_stress_smem<double>(threads, ctx->rt_slab_smem, ctx->rt_pencil_smem)) != 0) {
         ctx->lasterr = "stress kernels: shared memory attribute";
         return SCFT_CUDA_ERROR;
     }

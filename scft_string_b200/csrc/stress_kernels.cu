@@ -17,6 +17,13 @@
 // Pairs are processed in chunks; per chunk four launches: slab forward (u4,
 // u2 of x and y), pencil 1 (x forward; dK1 sums; K2, x inverse of u4),
 // slab mid (E2 D2 E4), pencil 2 (x forward; dK2 sums).
+//
+// Compiled once per bound on the threads of a CTA (SCFT_STRESS_THREADS; stress_kernels.cu
+// itself is 256, stress_kernels_512.cu and _1024.cu the others): a butterfly of the
+// general transforms wants 255 registers a thread, which an SM has for 256 threads only.
+#ifndef SCFT_STRESS_THREADS
+#define SCFT_STRESS_THREADS 256
+#endif
 #include "common.cuh"
 #include "fft.cuh"
 #include "kernels.h"
@@ -24,6 +31,8 @@
 namespace scft {
 
 namespace {
+
+constexpr int kThreads = SCFT_STRESS_THREADS;
 
 template <typename T>
 __device__ __forceinline__ const T *slice(const StressArgs<T> &a, int s, int fld)
@@ -54,7 +63,7 @@ __device__ __forceinline__ double bsum(double v, double *sh)
 
 // u4 = E4 x and u2 = E2 x (and the same for y), forward slab transforms
 template <typename T>
-__global__ void k_stress_slab_fwd(StressArgs<T> a, StressPairs P)
+__global__ void __launch_bounds__(kThreads) k_stress_slab_fwd(StressArgs<T> a, StressPairs P)
 {
     const unsigned mag = div_mag(a.g.m2);
     extern __shared__ unsigned char smem_raw[];
@@ -110,7 +119,7 @@ __device__ __forceinline__ void dk_weights(const StressArgs<T> &a, int xk, int c
 
 // x forward of u4 (x, y) and u2 (x, y); dK1 sums of u2; K2/M and x inverse of u4
 template <typename T>
-__global__ void k_stress_pencil1(StressArgs<T> a)
+__global__ void __launch_bounds__(kThreads) k_stress_pencil1(StressArgs<T> a)
 {
     extern __shared__ unsigned char smem_raw[];
     __shared__ double sh[32];
@@ -179,7 +188,7 @@ __global__ void k_stress_pencil1(StressArgs<T> a)
 
 // w = E2 D2 E4 x: inverse slab, times E2, forward slab
 template <typename T>
-__global__ void k_stress_slab_mid(StressArgs<T> a, StressPairs P)
+__global__ void __launch_bounds__(kThreads) k_stress_slab_mid(StressArgs<T> a, StressPairs P)
 {
     const unsigned mag = div_mag(a.g.m2);
     extern __shared__ unsigned char smem_raw[];
@@ -218,7 +227,7 @@ __global__ void k_stress_slab_mid(StressArgs<T> a, StressPairs P)
 
 // x forward of w (x, y); dK2 sums  Re(W_x conj U4_y + U4_x conj W_y)
 template <typename T>
-__global__ void k_stress_pencil2(StressArgs<T> a)
+__global__ void __launch_bounds__(kThreads) k_stress_pencil2(StressArgs<T> a)
 {
     extern __shared__ unsigned char smem_raw[];
     __shared__ double sh[32];
@@ -323,7 +332,7 @@ __device__ void jn_pencil_tile(const StressArgs<T> &a, cplx<T> *bx, const cplx<T
 }
 
 template <typename T>
-__global__ void k_jn_pencil(StressArgs<T> a, int pass)
+__global__ void __launch_bounds__(kThreads) k_jn_pencil(StressArgs<T> a, int pass)
 {
     extern __shared__ unsigned char smem_raw[];
     const Geo &g = a.g;
@@ -358,7 +367,7 @@ __device__ void jn_slab_to_real(const StressArgs<T> &a, cplx<T> *buf, const cplx
 }
 
 template <typename T>
-__global__ void k_jn_slab(StressArgs<T> a, int pass)
+__global__ void __launch_bounds__(kThreads) k_jn_slab(StressArgs<T> a, int pass)
 {
     const unsigned mag = div_mag(a.g.m2);
     extern __shared__ unsigned char smem_raw[];
@@ -433,8 +442,8 @@ __global__ void k_jn_final(const double *part, int nblk, double *out)
 
 }  // namespace
 
-template <typename T>
-int launch_junction_dtheta(const StressArgs<T> &a, const StressPairs &P, int slab_threads, int slab_smem,
+template <typename T, int MT>
+int launch_junction_mt(const StressArgs<T> &a, const StressPairs &P, int slab_threads, int slab_smem,
                            int pencil_threads, int pencil_smem, double *part, int nblk, double *out,
                            cudaStream_t st)
 {
@@ -449,8 +458,8 @@ int launch_junction_dtheta(const StressArgs<T> &a, const StressPairs &P, int sla
     return 7;
 }
 
-template <typename T>
-int launch_stress_chunk(const StressArgs<T> &a, const StressPairs &P, int slab_threads, int slab_smem,
+template <typename T, int MT>
+int launch_stress_chunk_mt(const StressArgs<T> &a, const StressPairs &P, int slab_threads, int slab_smem,
                         int pencil_threads, int pencil_smem, double *out, cudaStream_t st)
 {
     const Geo &g = a.g;
@@ -462,8 +471,8 @@ int launch_stress_chunk(const StressArgs<T> &a, const StressPairs &P, int slab_t
     return 5;
 }
 
-template <typename T>
-int set_stress_smem(int slab_smem, int pencil_smem)
+template <typename T, int MT>
+int set_stress_smem_mt(int slab_smem, int pencil_smem)
 {
     cudaError_t e1 = raise_dyn_smem(k_stress_slab_fwd<T>, slab_smem);
     cudaError_t e2 = raise_dyn_smem(k_stress_slab_mid<T>, slab_smem);
@@ -475,13 +484,60 @@ int set_stress_smem(int slab_smem, int pencil_smem)
             e5 == cudaSuccess && e6 == cudaSuccess) ? 0 : -1;
 }
 
+#define INSTANCE(HOW, T, MT)                                                                                     \
+    HOW template int launch_stress_chunk_mt<T, MT>(const StressArgs<T> &, const StressPairs &, int, int, int, int, \
+                                                   double *, cudaStream_t);                                        \
+    HOW template int launch_junction_mt<T, MT>(const StressArgs<T> &, const StressPairs &, int, int, int, int,     \
+                                               double *, int, double *, cudaStream_t);                             \
+    HOW template int set_stress_smem_mt<T, MT>(int, int);
+INSTANCE(, float, kThreads)
+INSTANCE(, double, kThreads)
+
+#if SCFT_STRESS_THREADS == 256
+// the other builds'
+INSTANCE(extern, float, 512)
+INSTANCE(extern, double, 512)
+INSTANCE(extern, float, 1024)
+INSTANCE(extern, double, 1024)
+
+// the build whose bound the launch's threads keep
+template <typename T>
+int launch_junction_dtheta(const StressArgs<T> &a, const StressPairs &P, int slab_threads, int slab_smem,
+                           int pencil_threads, int pencil_smem, double *part, int nblk, double *out,
+                           cudaStream_t st)
+{
+    const int t = slab_threads > pencil_threads ? slab_threads : pencil_threads;
+    auto *f = t > 512 ? launch_junction_mt<T, 1024> : t > 256 ? launch_junction_mt<T, 512> : launch_junction_mt<T, 256>;
+    return f(a, P, slab_threads, slab_smem, pencil_threads, pencil_smem, part, nblk, out, st);
+}
+
+template <typename T>
+int launch_stress_chunk(const StressArgs<T> &a, const StressPairs &P, int slab_threads, int slab_smem,
+                        int pencil_threads, int pencil_smem, double *out, cudaStream_t st)
+{
+    const int t = slab_threads > pencil_threads ? slab_threads : pencil_threads;
+    auto *f = t > 512   ? launch_stress_chunk_mt<T, 1024>
+              : t > 256 ? launch_stress_chunk_mt<T, 512>
+                        : launch_stress_chunk_mt<T, 256>;
+    return f(a, P, slab_threads, slab_smem, pencil_threads, pencil_smem, out, st);
+}
+
+template <typename T>
+int set_stress_smem(int threads, int slab_smem, int pencil_smem)
+{
+    auto *f = threads > 512 ? set_stress_smem_mt<T, 1024> : threads > 256 ? set_stress_smem_mt<T, 512> : set_stress_smem_mt<T, 256>;
+    return f(slab_smem, pencil_smem);
+}
+
 template int launch_stress_chunk<float>(const StressArgs<float> &, const StressPairs &, int, int, int, int, double *, cudaStream_t);
 template int launch_stress_chunk<double>(const StressArgs<double> &, const StressPairs &, int, int, int, int, double *, cudaStream_t);
 template int launch_junction_dtheta<float>(const StressArgs<float> &, const StressPairs &, int, int, int, int,
                                            double *, int, double *, cudaStream_t);
 template int launch_junction_dtheta<double>(const StressArgs<double> &, const StressPairs &, int, int, int, int,
                                             double *, int, double *, cudaStream_t);
-template int set_stress_smem<float>(int, int);
-template int set_stress_smem<double>(int, int);
+template int set_stress_smem<float>(int, int, int);
+template int set_stress_smem<double>(int, int, int);
+#endif
+#undef INSTANCE
 
 }  // namespace scft
