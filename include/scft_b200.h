@@ -277,8 +277,9 @@ scft_status scft_load_checkpoint(scft_ctx *ctx, const char *path);
  * its content. */
 scft_status scft_checkpoint_info(const char *path, int *version, int *strn, int *m, double *D);
 /* Picks the schedule of a props round by timing rounds of all replicas at
- * their current fields: 1 or 2 concurrent slot groups, and x-pencil tiles of
- * the default or twice the width (grids with tensor-map pencils), each with
+ * their current fields: 1 or 2 concurrent slot groups, and tiles of the x
+ * pass as the kernels choose them or all of twice the width (compile-time
+ * axes, and where that is another schedule), each with
  * four launches per contour step and, where the context has it, one
  * persistent launch per step (see scft_autotune_ex).  The densities are
  * recomputed, the statistics left unchanged.  *groups_out, *wide_out = the

@@ -62,7 +62,7 @@ struct PropsLaunch {
     int fixed;       // compile-time shape id (0: runtime-shaped kernels)
     int pf;          // prefetching (bulk-copy) slab kernels for the fixed shape
     int mid_pf_smem, combine_pf_smem;
-    int tma_pencil;  // x pass through 2-D tensor-map tiles (fixed shapes)
+    int tma_pencil;  // spectra have a 2-D tensor map (FP32 compile-time shapes: persistent launch, shuffle x pass)
     int pencil_tma_smem;
     const CUtensorMap *tmap;  // host copy of the spectrum tensor map
     int ptile_wide;  // x tiles of twice the default width: 1 yes, 0 no, -1 as the kernels choose

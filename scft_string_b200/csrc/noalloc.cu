@@ -4,8 +4,9 @@
 // step: a real-time loop that must not stall on the allocator (cudaMalloc
 // can synchronise the whole device), or an embedding framework that owns
 // every device allocation through its own pool and forbids foreign ones.
-// For them, scft_do_step_noalloc runs the same runtime-shaped kernels as
-// scft_do_step (k_prepare, k_combine, k_pencil, k_mid) with all of their
+// For them, scft_do_step_noalloc runs the general step kernels (k_prepare,
+// k_combine, k_pencil, k_mid), which scft_do_step takes on grids without packed or
+// compile-time ones, with all of their
 // working buffers -- spectra, E tables, the full-step partial, the two
 // propagator slices, FFT twiddles, diffusion factors and the error word --
 // in one file-scope __device__ array of kNoAllocBytes.  The caller passes

@@ -2401,9 +2401,9 @@ scft_status scft_reset_stats(scft_ctx *ctx)
 
 // Times props rounds of every replica for each schedule -- one, two or four
 // slot groups (two concurrent streams; four groups run two after another on
-// each), x-pencil tiles of the default or twice the width (when the grid has
-// tensor-map pencils), four launches or one persistent launch per contour
-// step -- and keeps the fastest.  Each
+// each) and the default count where that is another, x tiles as the kernels
+// choose or all wide (wide_available, and where that differs), four launches or
+// one persistent launch per contour step -- and keeps the fastest.  Each
 // candidate re-captures its graphs, runs one untimed round, then the best of
 // three timed rounds counts.  The rounds recompute every replica's densities
 // at its current fields, so the state a caller sees afterwards is unchanged;
