@@ -233,9 +233,10 @@ scft_status scft_spline_redist(scft_ctx *ctx, const double *x, const double *xre
 /* One Richardson contour step for callers that cannot allocate device memory
  * when they need a step: a real-time loop that must not stall on the
  * allocator (cudaMalloc can synchronise the device), or a framework that owns
- * every device allocation through its own pool.  Same kernels and result as
- * scft_do_step, but every working buffer lives in one static __device__
- * array of 4.2 MB, so it calls no cudaMalloc/cudaFree.  All pointers are the
+ * every device allocation through its own pool.  The step of scft_do_step on
+ * the general kernels (the same result up to rounding), with every working
+ * buffer in one static __device__ array of 4.2 MB, so it calls no
+ * cudaMalloc/cudaFree.  All pointers are the
  * caller's device memory: w2M = [W-, W+], in2M = [q(s), q^dagger(s)], out2M =
  * [q(s+1), q^dagger(s+1)], each 2*M doubles; f is the A fraction (0..1) as in
  * scft_problem; stream may be NULL.  Limits: FP64, M <= 32768, each m_i <= 64
